@@ -3,6 +3,7 @@
 // flash-attn in the reference, quarot_llama.py:207-221). Not part of the parity contract of the
 // linear path: fp32 math, compared against a torch fp32 reference with a tolerance. sm_100a.
 #include "common.cuh"
+#include "attn_tile.cuh"
 #include <stdlib.h>
 #include <mutex>
 
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(128)
 decode_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ cache_k,
                         const __half* __restrict__ cache_v, const int* __restrict__ positions,
                         const int* __restrict__ seq_ids, __half* __restrict__ out,
-                        int Hq, int Hkv, int S, float sm_scale) {
+                        int Hq, int Hkv, int S, float sm_scale, int T, int min_run) {
   pdl_enter();
   constexpr int D = 128;
   extern __shared__ float scores[];                       // [S]
@@ -71,6 +72,7 @@ decode_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pos = positions[tok], seq = seq_ids[tok];
   if ((unsigned)pos >= (unsigned)S) return;               // out of the cache / rotary table: nothing valid to attend to
+  if (min_run && atile::attn_in_run(positions, seq_ids, T, tok, min_run)) return;   // attn_tile_kernel's
   const int nkeys = pos + 1;
   const int hk = h / (Hq / Hkv);
   qs[tid] = __half2float(qkv[(size_t)tok * (Hq + 2 * Hkv) * D + (size_t)h * D + tid]) * sm_scale;
@@ -575,7 +577,7 @@ template <int G>
 __global__ void __launch_bounds__(SEQ_ATTN_WARPS * 32, 4)
 seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ cache_k, const __half* __restrict__ cache_v,
                      const int* __restrict__ positions, const int* __restrict__ seq_ids, __half* __restrict__ out,
-                     int T, int Hq, int Hkv, int S, float sm_scale) {
+                     int T, int Hq, int Hkv, int S, float sm_scale, int min_run) {
   pdl_enter();
   constexpr int D = 128, R = 16 / G, NW = SEQ_ATTN_WARPS;    // R tokens x G heads <= 16 query rows per chunk; NW warps split the keys
   __shared__ int s_tok[1024];                                // tokens of this sequence in the pass (T <= 1024)
@@ -599,7 +601,28 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
     }
   }
   __syncthreads();
-  const int ntok = s_ntok;
+  int ntok = s_ntok;
+  if (min_run && ntok >= min_run) {                          // leave the tokens of prompt runs to attn_tile_kernel
+    int t_[1024 / (NW * 32)], p_[1024 / (NW * 32)];
+#pragma unroll
+    for (int q = 0; q < 1024 / (NW * 32); ++q) {
+      const int i = tid + q * NW * 32;
+      t_[q] = -1; p_[q] = 0;
+      if (i < ntok && !atile::attn_in_run(positions, seq_ids, T, s_tok[i], min_run)) { t_[q] = s_tok[i]; p_[q] = s_pos[i]; }
+    }
+    __syncthreads();
+    if (tid == 0) s_ntok = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 1024 / (NW * 32); ++q)
+      if (t_[q] >= 0) {
+        const int i = atomicAdd(&s_ntok, 1);
+        s_tok[i] = t_[q];
+        s_pos[i] = p_[q];
+      }
+    __syncthreads();
+    ntok = s_ntok;
+  }
   if (ntok == 0) return;
   const size_t row_elems = (size_t)(Hq + 2 * Hkv) * D;
   const __half* kbase = cache_k + ((size_t)seq * S * Hkv + hk) * D;
@@ -748,7 +771,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
 
 template <int G>
 static int launch_seq_attention(const void* qkv, const void* ck, const void* cv, const int* positions, const int* seq_ids,
-                                void* out, int T, int B, int Hq, int Hkv, int S, float sm_scale, cudaStream_t st) {
+                                void* out, int T, int B, int Hq, int Hkv, int S, float sm_scale, int min_run, cudaStream_t st) {
   constexpr size_t dyn = (size_t)SEQ_ATTN_WARPS * 16 * 128 * sizeof(float);
   auto kern = seq_attention_kernel<G>;
   static bool attr_set = false;                              // per instantiation
@@ -757,9 +780,26 @@ static int launch_seq_attention(const void* qkv, const void* ck, const void* cv,
     attr_set = true;
   }
   launch_pdl(kern, dim3(B, Hkv), dim3(SEQ_ATTN_WARPS * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
-             positions, seq_ids, (__half*)out, T, Hq, Hkv, S, sm_scale);
+             positions, seq_ids, (__half*)out, T, Hq, Hkv, S, sm_scale, min_run);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
+}
+
+// Prompt portions of the int4 decoder's attention. Runs of at least RUN tokens (one sequence, consecutive positions) go to
+// attn_tile_kernel, the other tokens of the pass to the kernel of the entry point; which is which is known on the device only, so both
+// are launched and each takes its own. 0 in *min_run: the tile form does not take these sizes.
+constexpr int RUN = 16;
+static int launch_runs(const void* qkv, const void* ck, const void* cv, const int* positions, const int* seq_ids, void* out, int T, int nseq, int Hq,
+                       int Hkv, int S, float sm_scale, int skip_outside, int* min_run, cudaStream_t st) {
+  atile::Args a = {};
+  a.q = qkv; a.q_ts = (long long)(Hq + 2 * Hkv) * 128; a.q_hs = 128;
+  a.k = ck; a.v = cv;
+  a.k_ss = a.v_ss = (long long)S * Hkv * 128; a.k_rs = a.v_rs = Hkv * 128; a.k_hs = a.v_hs = 128;
+  a.pos = positions; a.seq = seq_ids; a.ntok = T; a.nseq = nseq; a.rep = Hq / Hkv; a.cap = S; a.window = 1 << 30;
+  a.scale = sm_scale; a.min_run = RUN; a.skip_outside = skip_outside;
+  a.out = out; a.out_ts = (long long)Hq * 128; a.out_hs = 128; a.out_scale = 1.f;
+  *min_run = atile::supported(a, 2) ? RUN : 0;
+  return *min_run ? atile::launch<false, false>(a, Hkv, st) : QSPEC_OK;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -857,12 +897,24 @@ extern "C" int qspec_decode_attention(const void* qkv, const void* cache_k, cons
   QSPEC_REQUIRE(D == 128 && Hq % Hkv == 0, QSPEC_ERR_UNSUPPORTED, "decode_attention: need head_dim 128 and Hq %% Hkv == 0");
   QSPEC_REQUIRE(S > 0 && S <= 8192, QSPEC_ERR_UNSUPPORTED, "decode_attention: cache length %d > 8192", S);
   if (T == 0) return QSPEC_OK;
+  // passes that qspec_attn_block takes stay bit-identical to it
+  int min_run = 0;
+  if (T >= 4 * RUN && !qspec_attn_block_supported(T, Hq, Hkv, D, S)) {
+    const int rc = launch_runs(qkv, cache_k, cache_v, positions, seq_ids, out, T, 0x7fffffff, Hq, Hkv, S, sm_scale, 1, &min_run, (cudaStream_t)stream);
+    if (rc != QSPEC_OK) return rc;
+  }
   dim3 grid(T, Hq);
   launch_pdl(decode_attention_kernel, dim3(grid), dim3(128), (size_t)S * sizeof(float), (cudaStream_t)stream, 
       (const __half*)qkv, (const __half*)cache_k, (const __half*)cache_v, positions, seq_ids, (__half*)out, Hq, Hkv, S,
-      sm_scale);
+      sm_scale, T, min_run);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
+}
+
+extern "C" int qspec_attn_tile_timeouts(void) {
+  unsigned n = 0;
+  if (cudaMemcpyFromSymbol(&n, atile::attn_tile_timeouts, sizeof(n)) != cudaSuccess) return -1;
+  return (int)n;
 }
 
 extern "C" int qspec_seq_attention_supported(int T, int Hq, int Hkv, int D, int S) {
@@ -880,12 +932,17 @@ extern "C" int qspec_seq_attention(const void* qkv, const void* cache_k, const v
   QSPEC_REQUIRE(qspec_seq_attention_supported(T, Hq, Hkv, D, S), QSPEC_ERR_UNSUPPORTED,
                 "seq_attention: unsupported T=%d Hq=%d Hkv=%d D=%d S=%d (use decode_attention)", T, Hq, Hkv, D, S);
   cudaStream_t st = (cudaStream_t)stream;
+  int min_run = 0;
+  if (T >= 2 * RUN) {
+    const int rc = launch_runs(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, 0, &min_run, st);
+    if (rc != QSPEC_OK) return rc;
+  }
   switch (Hq / Hkv) {
-    case 1: return launch_seq_attention<1>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, st);
-    case 2: return launch_seq_attention<2>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, st);
-    case 4: return launch_seq_attention<4>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, st);
-    case 5: return launch_seq_attention<5>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, st);
-    default: return launch_seq_attention<8>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, st);
+    case 1: return launch_seq_attention<1>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, min_run, st);
+    case 2: return launch_seq_attention<2>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, min_run, st);
+    case 4: return launch_seq_attention<4>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, min_run, st);
+    case 5: return launch_seq_attention<5>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, min_run, st);
+    default: return launch_seq_attention<8>(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, min_run, st);
   }
 }
 

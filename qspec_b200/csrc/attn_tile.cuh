@@ -1,0 +1,673 @@
+// Softmax attention of prompt portions on the fifth-generation tensor cores, head size 128, 16-bit keys and values in a per-sequence
+// cache (rows by position, or a ring of `cap` rows), grouped-query heads, an optional window, sink and output gate. Both libraries
+// instantiate it: float16 with queries as they lie in the fused projection (attn_kernels.cu), bfloat16 with float32 queries
+// (seq_mma_kernels.cu).
+//
+// One CTA = two tiles of 128 query rows of one key/value head; a row is a (token, query head of the group) pair, so that the group's
+// heads share every key tile: 64 tokens per CTA at four heads per group. Keys are walked in blocks of 128.
+//   * S = Q K^T: both operands from shared memory, accumulator [128 x 128] float32 in tensor memory.
+//   * softmax: thread = row, so maxima and sums need no exchange. Scores are read from tensor memory (twice: maxima, then weights,
+//     64 columns at a time), weights go back over the scores they came from as a two-term 16-bit split (hi + lo: 22 / 16 mantissa
+//     bits, so that the second product is as good as one with float32 weights).
+//   * O += P V: weights from tensor memory, values from shared memory as they lie in the cache (the reduction runs over rows: the
+//     operand is "MN-major"); hi and lo terms are 8 + 8 instructions on the same value tile.
+//   * O is rescaled only when a row's maximum grew by more than 2^8 since the last rescale (weights then stay below 256, and the
+//     division by the sum at the end undoes the common factor).
+// Tensor memory: S0 | S1 | O0 | O1 = 512 columns. Warps: 2 x 4 softmax, 1 keys, 1 values (TMA), 2 that issue one tile's products
+// each. Within a tile scores, weights and value product follow one another; the two tiles run independently, so that the tensor
+// cores work on one while the other's scores pass through its softmax warps.
+//
+// Which tokens: those in RUNS, i.e. neighbours in the batch with one sequence and consecutive positions, of at least min_run
+// tokens. A CTA walks the runs of its tokens one after the other (rows of other runs are masked). Tokens outside such runs are left
+// to the caller's other kernel (attn_in_run is the common test).
+//
+// A weight of zero times a value that is not finite would be NaN: rows with a result that is not finite are computed again key by
+// key (attn_row_again), so that a row sees nothing but its own keys.
+//
+// Every wait is bounded; a CTA whose wait runs out counts itself in attn_tile_timeouts, frees its tensor memory and leaves without
+// storing.
+#pragma once
+#include "common.cuh"
+#include <cuda.h>
+#include <cuda_fp16.h>
+#include <cuda_bf16.h>
+
+namespace qspec {
+namespace atile {
+
+constexpr int TOKENS_MAX = 256;                // tokens of a CTA: 2 * (128 / heads of a group)
+constexpr int MARGIN = 16;                     // run test: links looked at on either side
+constexpr int WARP_K = 8, WARP_V = 9, WARP_MMA = 10;   // warps 0 .. 7: softmax; 10, 11: products of one tile each
+constexpr int THREADS = 12 * 32;               // three warps per scheduler: 168 registers a thread (13 warps would leave 128)
+constexpr int HALF = 128 * 128;                // 128 rows x 64 elements
+constexpr int TILE = 2 * HALF;                 // 128 rows x 128 elements
+constexpr size_t SMEM = 6 * (size_t)TILE + 1024;   // Q0 Q1 | K K | V V | slack to start on a 1024-byte boundary
+constexpr float RESCALE_LOG2 = 8.f;
+constexpr uint32_t WAIT_SPINS = 1u << 20;
+
+static __device__ unsigned attn_tile_timeouts;  // CTAs of this library that gave a wait up, since it was loaded
+
+struct Args {
+  const void* q; long long q_ts, q_hs;         // strides in elements; tokens, heads
+  const void* k; long long k_ss; int k_rs, k_hs;   // sequences, rows, heads
+  const void* v; long long v_ss; int v_rs, v_hs;
+  const int* pos; const int* seq;
+  int ntok, nseq, rep, cap, window;            // nseq: sequences the cache holds; a token of another one belongs to no run
+  float scale;
+  int min_run, ring, skip_outside;             // skip_outside: a token whose position is outside the cache is not stored
+  void* out; long long out_ts; int out_hs;
+  const float* sink; const void* gate; int gate_ld, gate_per_head; float out_scale;
+};
+
+// Is token t in a run of at least `min_run` tokens (min_run <= MARGIN)?
+__device__ __forceinline__ bool attn_link(const int* pos, const int* seq, int t) {      // t and t + 1 are of one run
+  return seq[t] == seq[t + 1] && pos[t + 1] == pos[t] + 1;
+}
+__device__ __forceinline__ bool attn_in_run(const int* pos, const int* seq, int ntok, int t, int min_run) {
+  int n = 1;
+  for (int i = t; n < min_run && i > 0 && attn_link(pos, seq, i - 1); --i) ++n;
+  for (int i = t; n < min_run && i + 1 < ntok && attn_link(pos, seq, i); ++i) ++n;
+  return n >= min_run;
+}
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count)); }
+__device__ __forceinline__ void bar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory"); }
+// false: the wait ran out, here or in another role of the CTA
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
+  for (uint32_t spins = 0; spins < WAIT_SPINS; ++spins) {
+    uint32_t done;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    if (done) return true;
+    if (*fail) return false;
+  }
+  *fail = 1;
+  return false;
+}
+__device__ __forceinline__ bool elect() {
+  uint32_t pred;
+  asm volatile(
+      "{\n"
+      ".reg .pred P;\n"
+      "elect.sync _|P, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, P;\n"
+      "}\n" : "=r"(pred));
+  return pred != 0;
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
+__device__ __forceinline__ void commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+// Shared-memory operands, 128-byte swizzle (row r at 128 r, 16-byte chunk c at c ^ (r & 7); groups of eight rows 1024 bytes apart).
+// K-major (queries, keys): 64 elements of the reduction per 128-byte row. MN-major (values): the rows ARE the reduction, the second 64
+// output columns lie one half-tile (LBO) further.
+__device__ __forceinline__ uint64_t desc_k(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ uint64_t desc_mn(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((uint32_t)HALF >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+template <bool BF> __device__ __forceinline__ constexpr uint32_t idesc(bool mn) {   // float32 += T * T, M 128, N 128
+  return (1u << 4) | (BF ? (1u << 7) | (1u << 10) : 0u) | (mn ? 1u << 16 : 0u) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+}
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(id), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a), "l"(b), "r"(id), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void tma_rows(uint32_t dst, const CUtensorMap* map, int d, int head, int row, int seq, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];\n" ::"r"(dst),
+               "l"(map), "r"(bar), "r"(d), "r"(head), "r"(row), "r"(seq) : "memory");
+}
+#define QSPEC_R8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), "=r"(r[o + 6]), "=r"(r[o + 7])
+#define QSPEC_W8(r, o) "r"(r[o]), "r"(r[o + 1]), "r"(r[o + 2]), "r"(r[o + 3]), "r"(r[o + 4]), "r"(r[o + 5]), "r"(r[o + 6]), "r"(r[o + 7])
+__device__ __forceinline__ void ld32(uint32_t addr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+               "%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+               : QSPEC_R8(r, 0), QSPEC_R8(r, 8), QSPEC_R8(r, 16), QSPEC_R8(r, 24) : "r"(addr));
+}
+__device__ __forceinline__ void st32(uint32_t addr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+               "%25,%26,%27,%28,%29,%30,%31,%32};\n"
+               ::"r"(addr), QSPEC_W8(r, 0), QSPEC_W8(r, 8), QSPEC_W8(r, 16), QSPEC_W8(r, 24) : "memory");
+}
+__device__ __forceinline__ void st16(uint32_t addr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(addr), QSPEC_W8(r, 0),
+               QSPEC_W8(r, 8) : "memory");
+}
+#undef QSPEC_R8
+#undef QSPEC_W8
+__device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x)); return y; }
+// pairs of float32 in one instruction
+__device__ __forceinline__ uint64_t pair(uint32_t a, uint32_t b) { uint64_t r; asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "r"(a), "r"(b)); return r; }
+__device__ __forceinline__ void unpair(uint64_t v, uint32_t& a, uint32_t& b) { asm("mov.b64 {%0, %1}, %2;\n" : "=r"(a), "=r"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
+// lead(): the leading bits of two weights (bits of float32, 0 <= weight < 2^15), packed, and their values; rest(): two remainders, packed.
+// Mostly on the integer units: the conversion instruction shares the special-function unit with the exponentials (with conversions for
+// both terms that unit was 95 % busy and the kernel waited for it).
+template <bool BF> struct Elem;
+template <> struct Elem<false> {
+  using T = __half;
+  static __device__ __forceinline__ uint32_t pack(float a, float b) { const __half2 h = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
+  static __device__ __forceinline__ float2 unpack(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+  // weights below 2^-14, the smallest normal number, give 2^-14: their remainder is negative
+  static __device__ __forceinline__ uint32_t lead(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
+    h0 = max(p0, 0x38800000u) & 0xffffe000u;
+    h1 = max(p1, 0x38800000u) & 0xffffe000u;
+    return (h0 >> 13) + (h1 << 3) - 0xc001c000u;           // exponent bias 127 -> 15 in both halves
+  }
+  static __device__ __forceinline__ uint32_t rest(uint32_t q0, uint32_t q1) { return pack(__uint_as_float(q0), __uint_as_float(q1)); }
+};
+template <> struct Elem<true> {
+  using T = __nv_bfloat16;
+  static __device__ __forceinline__ uint32_t pack(float a, float b) { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
+  static __device__ __forceinline__ float2 unpack(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+  static __device__ __forceinline__ uint32_t lead(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
+    h0 = p0 & 0xffff0000u;
+    h1 = p1 & 0xffff0000u;
+    return __byte_perm(p0, p1, 0x7632);
+  }
+  static __device__ __forceinline__ uint32_t rest(uint32_t q0, uint32_t q1) { return __byte_perm(q0 + 0x8000u, q1 + 0x8000u, 0x7632); }   // rounded
+};
+
+// The key blocks of a CTA: for every run the blocks of up to 128 positions from its first visible key to its last, with the tiles that
+// see something in them.
+struct Item { int kb, hi, seq, p0, ts, te; bool act[2]; };   // positions kb .. hi, at most 128
+struct Items {
+  const int *rs, *re, *pos, *seq; int nruns, tok, window, last, ring;    // ring: rows of the ring, or 0
+  int r = -1, kb = 0, hi = -1, wlo[2], whi[2];
+  __device__ __forceinline__ bool next(Item& it) {
+    for (;;) {
+      while (kb > hi) {
+        if (++r >= nruns) return false;
+        const int ts = rs[r], te = re[r], p0 = pos[ts], p1 = pos[te];
+        kb = max(0, p0 - window + 1);
+        hi = min(p1, last);
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          const int a = max(ts, w * tok), b = min(te, w * tok + tok - 1);
+          wlo[w] = a > b ? 0x7fffffff : max(0, p0 + (a - ts) - window + 1);
+          whi[w] = a > b ? -1 : min(p0 + (b - ts), last);
+        }
+      }
+      int n = 128;
+      if (ring) n = min(n, ring - kb % ring);               // a block ends where the ring does
+      it.kb = kb;
+      it.hi = min(hi, kb + n - 1);
+      kb += n;
+#pragma unroll
+      for (int w = 0; w < 2; ++w) it.act[w] = it.kb <= whi[w] && it.hi >= wlo[w];
+      if (it.act[0] || it.act[1]) break;
+    }
+    it.ts = rs[r]; it.te = re[r]; it.p0 = pos[it.ts]; it.seq = seq[it.ts];
+    return true;
+  }
+};
+
+// One row key by key on the CUDA cores (float32 weights, nothing but the row's own keys): rows whose tile result is not finite.
+template <bool BF, bool QF32>
+__device__ __noinline__ void attn_row_again(const Args& a, int tok, int head, int kvh, int seq, int lo, int hi) {
+  using T = typename Elem<BF>::T;
+  const T* kbase = (const T*)a.k + (size_t)seq * a.k_ss + (size_t)kvh * a.k_hs;
+  const T* vbase = (const T*)a.v + (size_t)seq * a.v_ss + (size_t)kvh * a.v_hs;
+  const size_t qo = (size_t)tok * a.q_ts + (size_t)head * a.q_hs;
+  auto qd = [&](int d) -> float {
+    if (QF32) return Elem<BF>::unpack(Elem<BF>::pack(((const float*)a.q)[qo + d], 0.f)).x;
+    return (float)((const T*)a.q)[qo + d];
+  };
+  auto row = [&](int j) { return a.ring && j >= a.cap ? j % a.cap : j; };
+  auto score = [&](int j) {
+    const T* kr = kbase + (size_t)row(j) * a.k_rs;
+    float s = 0.f;
+    for (int d = 0; d < 128; ++d) s = fmaf((float)kr[d], qd(d), s);
+    return s * a.scale;
+  };
+  float m = -INFINITY;
+  for (int j = lo; j <= hi; ++j) m = fmaxf(m, score(j));
+  if (a.sink) m = fmaxf(m, a.sink[head]);
+  float l = a.sink ? __expf(a.sink[head] - m) : 0.f;
+  for (int j = lo; j <= hi; ++j) l += __expf(score(j) - m);
+  for (int d0 = 0; d0 < 128; d0 += 16) {
+    float o[16];
+    for (int d = 0; d < 16; ++d) o[d] = 0.f;
+    for (int j = lo; j <= hi; ++j) {
+      const float p = __expf(score(j) - m);
+      const T* vr = vbase + (size_t)row(j) * a.v_rs + d0;
+      for (int d = 0; d < 16; ++d) o[d] = fmaf(p, (float)vr[d], o[d]);
+    }
+    for (int d = 0; d < 16; ++d) {
+      float r = o[d] / l * a.out_scale;
+      if (a.gate) r *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)tok * a.gate_ld + (a.gate_per_head ? head : head * a.out_hs + d0 + d)]));
+      ((T*)a.out)[(size_t)tok * a.out_ts + (size_t)head * a.out_hs + d0 + d] = (T)r;
+    }
+  }
+}
+
+template <bool BF, bool QF32>
+__global__ void __launch_bounds__(THREADS, 1)
+attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Args a) {
+  using T = typename Elem<BF>::T;
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  extern __shared__ __align__(16) unsigned char at_raw[];
+  __shared__ int s_pos[TOKENS_MAX + 2 * MARGIN], s_seq[TOKENS_MAX + 2 * MARGIN];
+  __shared__ int s_rs[TOKENS_MAX], s_re[TOKENS_MAX];
+  __shared__ uint32_t s_start[TOKENS_MAX / 32];
+  __shared__ __align__(8) uint64_t b_kfull[2], b_kempty[2], b_vfull[2], b_vempty[2], b_s[2], b_p[2][2], b_o[2], b_part;
+  __shared__ uint32_t s_tmem;
+  __shared__ volatile int s_fail;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rep = a.rep, tok = 128 / rep;                   // tokens per tile
+  const int c0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * tok;   // the longest key ranges first
+  const int kvh = blockIdx.y;
+  const int n2 = min(2 * tok, a.ntok - c0);
+
+  // ---- the runs among this CTA's tokens
+  for (int i = tid; i < n2 + 2 * MARGIN; i += THREADS) {
+    const int t = c0 + i - MARGIN;
+    const bool in = t >= 0 && t < a.ntok;
+    s_pos[i] = in ? a.pos[t] : 0;
+    s_seq[i] = in ? a.seq[t] : -1;
+  }
+  __syncthreads();
+  const int* pos = s_pos + MARGIN;
+  const int* seq = s_seq + MARGIN;
+  auto linked = [&](int i) { return c0 + i >= 0 && c0 + i + 1 < a.ntok && attn_link(pos, seq, i); };
+  bool start = false, end = false;
+  if (tid < TOKENS_MAX) {
+    bool in = false;
+    if (tid < n2) {
+      int n = 1;
+      for (int i = tid; n < a.min_run && linked(i - 1); --i) ++n;
+      for (int i = tid; n < a.min_run && linked(i); ++i) ++n;
+      in = n >= a.min_run && (unsigned)seq[tid] < (unsigned)a.nseq;
+      start = in && (tid == 0 || !linked(tid - 1));
+      end = in && (tid == n2 - 1 || !linked(tid));
+    }
+    const uint32_t bits = __ballot_sync(0xffffffffu, start);
+    if (lane == 0) s_start[warp] = bits;
+  }
+  if (tid == 0) s_fail = 0;
+  __syncthreads();
+  int nruns = 0, before = 0;
+  for (int w = 0; w < TOKENS_MAX / 32; ++w) {
+    if (w < warp) before += __popc(s_start[w]);
+    nruns += __popc(s_start[w]);
+  }
+  if (nruns == 0) return;                                    // nothing for this form here
+  if (tid < TOKENS_MAX) {                                    // a run's end has as many starts at or before it as its start has
+    const int rank = before + __popc(s_start[warp] & ((2u << lane) - 1u)) - 1;
+    if (start) s_rs[rank] = tid;
+    if (end) s_re[rank] = tid;
+  }
+  if (warp == WARP_MMA) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      bar_init(smem_addr(&b_kfull[i]), 1); bar_init(smem_addr(&b_kempty[i]), 2);
+      bar_init(smem_addr(&b_vfull[i]), 1); bar_init(smem_addr(&b_vempty[i]), 2);
+      bar_init(smem_addr(&b_s[i]), 1); bar_init(smem_addr(&b_o[i]), 1);
+      bar_init(smem_addr(&b_p[i][0]), 4); bar_init(smem_addr(&b_p[i][1]), 4);
+    }
+    bar_init(smem_addr(&b_part), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  const uint32_t base = (smem_addr(at_raw) + 1023u) & ~1023u;
+  unsigned char* gbase = at_raw + (base - smem_addr(at_raw));
+  // ---- queries of both tiles
+  for (int i = tid; i < 256 * 16; i += THREADS) {
+    const int row = i >> 4, c = i & 15, w = row >> 7, r = row & 127;
+    const int tl = w * tok + r / rep;
+    uint4 val = make_uint4(0u, 0u, 0u, 0u);
+    if (r < tok * rep && tl < n2) {
+      const size_t o = (size_t)(c0 + tl) * a.q_ts + (size_t)(kvh * rep + r % rep) * a.q_hs + c * 8;
+      if (QF32) {
+        const float4 x = *reinterpret_cast<const float4*>((const float*)a.q + o), y = *reinterpret_cast<const float4*>((const float*)a.q + o + 4);
+        val = make_uint4(Elem<BF>::pack(x.x, x.y), Elem<BF>::pack(x.z, x.w), Elem<BF>::pack(y.x, y.y), Elem<BF>::pack(y.z, y.w));
+      } else {
+        val = *reinterpret_cast<const uint4*>((const T*)a.q + o);
+      }
+    }
+    *reinterpret_cast<uint4*>(gbase + w * TILE + (c >> 3) * HALF + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = val;
+  }
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = s_tmem;
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // tensor memory is held: a dependent that waits for this grid cannot take it first
+
+  Items items{s_rs, s_re, pos, seq, nruns, tok, a.window, a.ring ? 0x7fffffff - 256 : a.cap - 1, a.ring ? a.cap : 0};
+  Item it;
+  if (warp >= WARP_MMA) {
+    if (elect()) {
+      const int w = warp - WARP_MMA;
+      const uint32_t id_s = idesc<BF>(false), id_o = idesc<BF>(true);
+      const uint32_t qa = base + w * TILE, p = tmem + w * 128, o = tmem + 256 + w * 128;
+      const uint32_t bs = smem_addr(&b_s[w]), bp = smem_addr(&b_p[w][0]), bo = smem_addr(&b_o[w]);
+      uint32_t done = 0;                                      // value products of this tile so far
+      for (uint32_t n = 0; items.next(it); ++n) {
+        const uint32_t stage = n & 1, phase = (n >> 1) & 1;
+        if (!bar_wait(smem_addr(&b_kfull[stage]), phase, &s_fail)) break;
+        if (it.act[w]) {
+          // the scores take the columns of the tile's previous weights: their product must be over
+          if (done && !bar_wait(bo, (done - 1) & 1, &s_fail)) break;
+          fence_after();
+          const uint64_t qd = desc_k(qa), kd = desc_k(base + (2 + stage) * TILE);
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) {
+            const uint32_t step = (uint32_t)((ks >> 2) * (HALF >> 4) + (ks & 3) * 2);
+            mma_ss(p, qd + step, kd + step, id_s, ks ? 1u : 0u);
+          }
+          commit(bs);
+        }
+        commit(smem_addr(&b_kempty[stage]));
+        if (!bar_wait(smem_addr(&b_vfull[stage]), phase, &s_fail)) break;
+        if (it.act[w]) {
+          const uint64_t vd = desc_mn(base + (4 + stage) * TILE);
+          bool ok = true;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {                       // 64 keys each: the first half's product runs during the second half's weights
+            ok = ok && bar_wait(bp + 8 * h, done & 1, &s_fail);
+            if (!ok) break;
+            fence_after();
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) {
+              const uint64_t v = vd + (h * 4 + ks) * (2048 >> 4);
+              mma_ts(o, p + h * 64 + ks * 8, v, id_o, (done | h | ks) ? 1u : 0u);
+              mma_ts(o, p + h * 64 + 32 + ks * 8, v, id_o, 1u);
+            }
+          }
+          if (!ok) break;
+          commit(bo);
+          ++done;
+        }
+        commit(smem_addr(&b_vempty[stage]));
+      }
+    }
+    __syncwarp();
+  } else if (warp == WARP_K || warp == WARP_V) {
+    // ---- key rows or value rows: two boxes of 128 rows x 64 elements per block (rows past the cache arrive as zeros)
+    const bool keys = warp == WARP_K;
+    uint64_t* full = keys ? b_kfull : b_vfull;
+    uint64_t* empty = keys ? b_kempty : b_vempty;
+    const CUtensorMap* map = keys ? &map_k : &map_v;
+    const uint32_t buf = base + (keys ? 2 : 4) * TILE;
+    bool ok = true;
+    int parts = 0;
+    for (int n = 0; items.next(it); ++n) {
+      if (n >= 2) ok = bar_wait(smem_addr(&empty[n & 1]), (uint32_t)(((n >> 1) - 1) & 1), &s_fail);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      // value rows past the block's last key are cleared before the products see them (their weights are zero, but zero times NaN is not):
+      // such a block lands on a barrier of its own first
+      const int have = it.hi - it.kb + 1;
+      const bool part = !keys && have < 128;
+      const uint32_t bar = smem_addr(part ? &b_part : &full[n & 1]), dst = buf + (n & 1) * TILE;
+      if (elect()) {
+        const int row = a.ring ? it.kb % a.cap : it.kb;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"((uint32_t)TILE) : "memory");
+        tma_rows(dst, map, 0, kvh, row, it.seq, bar);
+        tma_rows(dst + HALF, map, 64, kvh, row, it.seq, bar);
+      }
+      __syncwarp();
+      if (part) {
+        ok = bar_wait(bar, (uint32_t)(parts++ & 1), &s_fail);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        unsigned char* rows = gbase + (dst - base);
+        for (int i = have * 8 + lane; i < 128 * 8; i += 32) {
+          *reinterpret_cast<uint4*>(rows + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(rows + HALF + i * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        __syncwarp();
+        if (lane == 0) bar_arrive(smem_addr(&full[n & 1]));
+      }
+    }
+  } else {
+    // ---- softmax: thread = row of tile w
+    const int w = warp >> 2, r = (warp & 3) * 32 + lane;
+    const int tl = w * tok + r / rep, head = kvh * rep + r % rep;
+    const bool row_in = r < tok * rep && tl < n2;
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t st = tmem + lanes + w * 128, ot = tmem + lanes + 256 + w * 128;
+    const float c2 = a.scale * 1.4426950408889634f;
+    const int last = a.ring ? 0x7fffffff : a.cap - 1;
+    float m = -INFINITY, l = 0.f;                             // maximum in units of log2, sum relative to it
+    int n = 0, my_lo = 0, my_hi = -1, my_seq = 0;
+    bool ok = true, mine = false;
+    while (ok && items.next(it)) {
+      if (!it.act[w]) continue;
+      const bool in = row_in && tl >= it.ts && tl <= it.te;
+      // visible columns of the block: j0 .. j0 + span
+      int j0 = 0x7fff, span = 0;
+      if (in) {
+        const int pr = it.p0 + (tl - it.ts);
+        const int vlo = max(0, pr - a.window + 1);
+        int vhi = min(pr, last);
+        mine = true; my_lo = vlo; my_hi = vhi; my_seq = it.seq;
+        vhi = min(vhi, it.hi);
+        if (vhi >= vlo) { j0 = vlo - it.kb; span = vhi - vlo; }
+      }
+      const bool whole = !row_in || (j0 <= 0 && j0 + span >= 127);   // (rows that stand for no token are never stored)
+      const bool plain = __all_sync(0xffffffffu, whole);
+      ok = bar_wait(smem_addr(&b_s[w]), (uint32_t)(n & 1), &s_fail);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      fence_after();
+      uint32_t x[64];
+      float mx = -INFINITY;
+#pragma unroll
+      for (int h = 1; h >= 0; --h) {                          // the first half last: it stays in registers for the weights
+        ld32(st + h * 64, x);
+        ld32(st + h * 64 + 32, x + 32);
+        wait_ld();
+        if (plain) {
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int j = 0; j < 64; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(x[j]));
+          mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
+        } else {
+#pragma unroll
+          for (int j = 0; j < 64; ++j) {
+            if ((uint32_t)(h * 64 + j - j0) > (uint32_t)span) x[j] = 0xff800000u;      // hidden
+            mx = fmaxf(mx, __uint_as_float(x[j]));
+          }
+        }
+      }
+      const float mn = fmaxf(m, mx * c2);
+      if (__any_sync(0xffffffffu, mn > m + RESCALE_LOG2 || (m == -INFINITY && mn > m))) {
+        const float f = mn == -INFINITY ? 1.f : ex2(m - mn);   // 0 for a row that had seen nothing
+        m = mn;
+        l *= f;
+        if (n) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            uint32_t o[32];
+            ld32(ot + q * 32, o);
+            wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+            st32(ot + q * 32, o);
+          }
+        }
+      }
+      const float mu = m == -INFINITY ? 0.f : m;
+      const uint64_t c22 = pair(__float_as_uint(c2), __float_as_uint(c2)), mu2 = pair(__float_as_uint(-mu), __float_as_uint(-mu));
+      const uint64_t minus2 = pair(0xbf800000u, 0xbf800000u);
+      uint64_t l2[2] = {0ull, 0ull};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h == 1) {
+          ld32(st + 64, x);
+          ld32(st + 96, x + 32);
+          wait_ld();
+          if (!plain) {
+#pragma unroll
+            for (int j = 0; j < 64; ++j)
+              if ((uint32_t)(64 + j - j0) > (uint32_t)span) x[j] = 0xff800000u;
+          }
+        }
+        // weight = hi + lo: hi = the leading bits that the type keeps (cut, not rounded), lo = the rest, rounded
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          uint32_t hi[16], lo[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            uint32_t p0, p1, h0, h1, q0, q1;
+            unpair(fma2(pair(x[g * 32 + 2 * j], x[g * 32 + 2 * j + 1]), c22, mu2), p0, p1);
+            p0 = __float_as_uint(ex2(__uint_as_float(p0)));
+            p1 = __float_as_uint(ex2(__uint_as_float(p1)));
+            const uint64_t pp = pair(p0, p1);
+            l2[j & 1] = add2(l2[j & 1], pp);
+            hi[j] = Elem<BF>::lead(p0, p1, h0, h1);
+            unpair(fma2(pair(h0, h1), minus2, pp), q0, q1);
+            lo[j] = Elem<BF>::rest(q0, q1);
+          }
+          st16(st + h * 64 + g * 16, hi);
+          st16(st + h * 64 + 32 + g * 16, lo);
+        }
+        wait_st();
+        fence_before();
+        __syncwarp();
+        if (lane == 0) bar_arrive(smem_addr(&b_p[w][h]));
+      }
+      {
+        uint32_t a0, a1;
+        unpair(add2(l2[0], l2[1]), a0, a1);
+        l += __uint_as_float(a0) + __uint_as_float(a1);
+      }
+      ++n;
+    }
+    // ---- the last product is done: divide, gate, store
+    if (ok && n) ok = bar_wait(smem_addr(&b_o[w]), (uint32_t)((n - 1) & 1), &s_fail);
+    ok = __all_sync(0xffffffffu, ok);
+    fence_after();
+    // `mine` rows belong to a run; one whose position shows it no key is stored as zeros, or not at all (skip_outside)
+    if (row_in && !mine) {                                    // a run none of whose keys lie in the cache produced no block
+      for (int q = 0; q < nruns; ++q)
+        if (tl >= s_rs[q] && tl <= s_re[q]) mine = true;
+    }
+    const int pr = row_in ? pos[tl] : 0;
+    const bool store = ok && row_in && mine && !(a.skip_outside && (unsigned)pr >= (unsigned)a.cap);
+    const bool dead = l == 0.f;                               // saw no key at all
+    float f = 0.f;
+    if (!dead) {
+      float mm = m, ls = l;
+      if (a.sink && row_in) {
+        const float s2 = a.sink[head] * 1.4426950408889634f;
+        mm = fmaxf(m, s2);
+        ls = l * ex2(m - mm) + ex2(s2 - mm);
+      }
+      f = ex2(m - mm) / ls * a.out_scale;
+    }
+    if (a.gate && a.gate_per_head && store)
+      f *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)(c0 + tl) * a.gate_ld + head]));
+    T* dst = (T*)a.out + (size_t)(c0 + tl) * a.out_ts + (size_t)head * a.out_hs;
+    const T* gt = a.gate && !a.gate_per_head ? (const T*)a.gate + (size_t)(c0 + tl) * a.gate_ld + (size_t)head * a.out_hs : nullptr;
+    bool bad = false;
+    if (ok) {
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {
+        uint32_t o[32];
+        ld32(ot + q * 32, o);
+        wait_ld();
+        if (store) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              v[e] = dead ? 0.f : __uint_as_float(o[g * 8 + e]) * f;
+              bad |= !(fabsf(v[e]) < INFINITY);
+            }
+            if (gt) {
+              const uint4 gw = *reinterpret_cast<const uint4*>(gt + q * 32 + g * 8);
+              const uint32_t ww[4] = {gw.x, gw.y, gw.z, gw.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 z = Elem<BF>::unpack(ww[e]);
+                v[2 * e] *= __fdividef(1.f, 1.f + __expf(-z.x));
+                v[2 * e + 1] *= __fdividef(1.f, 1.f + __expf(-z.y));
+              }
+            }
+            *reinterpret_cast<uint4*>(dst + q * 32 + g * 8) =
+                make_uint4(Elem<BF>::pack(v[0], v[1]), Elem<BF>::pack(v[2], v[3]), Elem<BF>::pack(v[4], v[5]), Elem<BF>::pack(v[6], v[7]));
+          }
+        }
+      }
+      if (bad && store) attn_row_again<BF, QF32>(a, c0 + tl, head, kvh, my_seq, my_lo, my_hi);
+    }
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == WARP_MMA) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
+  }
+  if (tid == 0 && s_fail) atomicAdd(&attn_tile_timeouts, 1u);
+}
+
+// Heads per group that fit, positive scale (a row's maximum is the scaled maximum), rows on 16-byte boundaries.
+inline bool supported(const Args& a, int elem_q) {
+  auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
+  auto rows = [](long long ss, int rs, int hs) { return ss > 0 && rs > 0 && hs > 0 && ss % 8 == 0 && rs % 8 == 0 && hs % 8 == 0; };
+  return a.rep >= 1 && a.rep <= 64 && a.scale > 0.f && al(a.q) && al(a.k) && al(a.v) && al(a.out) && a.q_ts * elem_q % 16 == 0 &&
+         a.q_hs * elem_q % 16 == 0 && rows(a.k_ss, a.k_rs, a.k_hs) && rows(a.v_ss, a.v_rs, a.v_hs) && a.out_ts % 8 == 0 && a.out_hs % 8 == 0 &&
+         (!a.gate || a.gate_per_head || (al(a.gate) && a.gate_ld % 8 == 0));
+}
+
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// [sequence][row][head][128] with the caller's strides; a box is 128 rows x 64 elements of one head
+template <bool BF>
+inline int cache_map(CUtensorMap* map, const void* p, long long ss, int rs, int hs, int heads, int rows, int nseq) {
+  static const EncodeTiled fn = []() -> EncodeTiled {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? (EncodeTiled)f : nullptr;
+  }();
+  QSPEC_REQUIRE(fn, QSPEC_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
+  const cuuint64_t dims[4] = {128, (cuuint64_t)heads, (cuuint64_t)rows, (cuuint64_t)nseq};
+  const cuuint64_t strides[3] = {(cuuint64_t)hs * 2, (cuuint64_t)rs * 2, (cuuint64_t)ss * 2};
+  const cuuint32_t box[4] = {64, 1, 128, 1}, unit[4] = {1, 1, 1, 1};
+  const CUresult r = fn(map, BF ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(p), dims, strides, box, unit,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  QSPEC_REQUIRE(r == CUDA_SUCCESS, QSPEC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): %d rows, %d sequences", (int)r, rows, nseq);
+  return QSPEC_OK;
+}
+
+template <bool BF, bool QF32>
+inline int launch(const Args& a, int kv_heads, cudaStream_t stream) {
+  auto kern = attn_tile_kernel<BF, QF32>;
+  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
+  int dev = 0;
+  QSPEC_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
+    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
+    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
+  CUtensorMap mk, mv;
+  const int nseq = a.nseq < (1 << 20) ? a.nseq : 1 << 20;     // (a caller that does not know their number: nothing is cut off)
+  int rc = cache_map<BF>(&mk, a.k, a.k_ss, a.k_rs, a.k_hs, kv_heads, a.cap, nseq);
+  if (rc == QSPEC_OK) rc = cache_map<BF>(&mv, a.v, a.v_ss, a.v_rs, a.v_hs, kv_heads, a.cap, nseq);
+  if (rc != QSPEC_OK) return rc;
+  const int per = 2 * (128 / a.rep);
+  launch_pdl(kern, dim3((a.ntok + per - 1) / per, kv_heads), dim3(THREADS), SMEM, stream, mk, mv, a);
+  QSPEC_CHECK_LAUNCH(1);
+  return QSPEC_OK;
+}
+
+}  // namespace atile
+}  // namespace qspec

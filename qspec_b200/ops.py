@@ -642,6 +642,11 @@ def decode_attention(qkv: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Te
     return out
 
 
+def attn_tile_timeouts() -> int:
+    """CTAs of the prompt form inside seq_attention / decode_attention that gave up a bounded wait: 0 unless something is broken."""
+    return int(_lib.load().qspec_attn_tile_timeouts())
+
+
 def seq_attention_supported(T: int, num_heads: int, num_kv_heads: int, head_dim: int, cache_len: int) -> bool:
     return bool(_lib.load().qspec_seq_attention_supported(T, num_heads, num_kv_heads, head_dim, cache_len))
 

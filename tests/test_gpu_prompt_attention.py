@@ -1,0 +1,119 @@
+"""The int4 decoder's attention over prompt portions (tensor-core tiles inside seq_attention and decode_attention) against float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from qspec_b200 import ops
+    return ops
+
+
+def reference(qkv, ck, cv, pos, seq, Hq, Hkv, scale):
+    T, rep = len(pos), Hq // Hkv
+    q = qkv[:, :Hq * 128].double().view(T, Hq, 128)
+    out = torch.zeros(T, Hq, 128, dtype=torch.float64, device=qkv.device)
+    for t in range(T):
+        n = int(pos[t]) + 1
+        k = ck[int(seq[t]), :n].double().repeat_interleave(rep, 1)
+        v = cv[int(seq[t]), :n].double().repeat_interleave(rep, 1)
+        p = torch.softmax(torch.einsum("hd,jhd->hj", q[t], k) * scale, 1)
+        out[t] = torch.einsum("hj,jhd->hd", p, v)
+    return out.view(T, Hq * 128)
+
+
+def batch(segments, Hq, Hkv, S, nseq, seed=0):
+    """segments: (sequence, first position, tokens) in batch order."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    pos = torch.cat([torch.arange(p, p + n) for _, p, n in segments]).to(torch.int32)
+    seq = torch.cat([torch.full((n,), s) for s, _, n in segments]).to(torch.int32)
+    qkv = torch.randn(len(pos), (Hq + 2 * Hkv) * 128, generator=g, device="cuda").half()
+    ck = torch.randn(nseq, S, Hkv, 128, generator=g, device="cuda").half()
+    cv = torch.randn(nseq, S, Hkv, 128, generator=g, device="cuda").half()
+    return qkv, ck, cv, pos.cuda(), seq.cuda()
+
+
+def check(got, want):
+    # float16 outputs (2^-11 of a value) and a value product with 22-bit weights: two units in the last place of the largest value
+    err = (got.double() - want).abs().max().item()
+    assert err <= 2 ** -10 * want.abs().max().item(), err
+
+
+CASES = [
+    (32, 8, 300, [(0, 0, 64)]),                                   # one tile pair, exactly one block
+    (32, 8, 300, [(1, 0, 129)]),                                  # a block and one key; tokens of three CTAs
+    (32, 8, 512, [(0, 200, 150)]),                                # starts inside the cache
+    (8, 8, 400, [(0, 5, 257)]),                                   # one head per group: 128 tokens a tile
+    (40, 8, 300, [(0, 1, 77)]),                                   # five heads: rows left over in every tile
+    (64, 8, 600, [(0, 300, 45), (1, 77, 33)]),                    # eight heads; two runs in one CTA
+    (16, 8, 700, [(0, 500, 15), (1, 0, 1), (2, 30, 16), (3, 9, 40), (4, 650, 4)]),   # short runs beside long ones
+    (32, 8, 256, [(3, 100, 20), (0, 7, 1), (1, 8, 1), (2, 9, 1), (4, 255, 1), (5, 0, 256)]),
+    (32, 8, 1000, [(k, 10 * k, 4) for k in range(12)]),           # no run at all
+]
+
+
+@pytest.mark.parametrize("Hq,Hkv,S,segments", CASES)
+def test_prompt_runs_match_float64(ops, Hq, Hkv, S, segments):
+    nseq = 1 + max(s for s, _, _ in segments)
+    qkv, ck, cv, pos, seq = batch(segments, Hq, Hkv, S, nseq)
+    out = torch.full((len(pos), Hq * 128), float("nan"), dtype=torch.float16, device="cuda")
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 128 ** -0.5)
+    check(out, reference(qkv, ck, cv, pos, seq, Hq, Hkv, 128 ** -0.5))
+    assert ops.attn_tile_timeouts() == 0
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(24, 8), (48, 3), (32, 32)])
+def test_decode_attention_takes_long_runs_too(ops, Hq, Hkv):
+    """Head counts that the one-launch attention block does not take; positions that jump inside a sequence are no run."""
+    qkv, ck, cv, pos, seq = batch([(0, 3, 90), (1, 120, 1), (1, 50, 20), (1, 90, 3)], Hq, Hkv, 128, 2, seed=1)
+    out = torch.full((len(pos), Hq * 128), float("nan"), dtype=torch.float16, device="cuda")
+    ops.decode_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 0.1)
+    check(out, reference(qkv, ck, cv, pos, seq, Hq, Hkv, 0.1))
+
+
+def test_a_token_sees_nothing_but_its_own_keys(ops):
+    """Infinite values and keys at a later position of the same portion, NaN past the portion's end: earlier tokens stay finite."""
+    qkv, ck, cv, pos, seq = batch([(0, 0, 100)], 32, 8, 200, 1, seed=2)
+    cv[0, 60, :, 5] = float("inf")
+    ck[0, 60, :, 0] = float("nan")
+    ck[0, 100:] = float("nan")
+    cv[0, 100:] = float("nan")
+    out = torch.empty(100, 32 * 128, dtype=torch.float16, device="cuda")
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, 32, 8, 128, 128 ** -0.5)
+    want = reference(qkv[:60], ck, cv, pos[:60], seq[:60], 32, 8, 128 ** -0.5)
+    check(out[:60], want)
+    assert not torch.isfinite(out[60:].view(40, 32, 128)[..., 5]).any()
+
+
+def test_positions_outside_the_cache(ops):
+    """seq_attention shows such a token every row of the cache (past its end) or none (before its start: zeros), decode_attention does
+    not store it; neither reads outside."""
+    Hq, Hkv, S = 24, 8, 64
+    qkv, ck, cv, pos, seq = batch([(0, 50, 40), (1, -20, 30)], Hq, Hkv, S, 2, seed=4)
+    out = torch.full((70, Hq * 128), 7.0, dtype=torch.float16, device="cuda")
+    ops.decode_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 0.1)
+    ok = (pos >= 0) & (pos < S)
+    check(out[ok], reference(qkv[ok], ck, cv, pos[ok], seq[ok], Hq, Hkv, 0.1))
+    assert (out[~ok] == 7.0).all()
+    qkv, ck, cv, pos, seq = batch([(0, 50, 40), (1, -20, 30)], 16, 8, S, 2, seed=5)
+    out = torch.full((70, 2048), 7.0, dtype=torch.float16, device="cuda")
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, 16, 8, 128, 0.1)
+    seen = pos >= 0
+    check(out[seen], reference(qkv[seen], ck, cv, pos[seen].clamp(max=S - 1), seq[seen], 16, 8, 0.1))
+    assert (out[~seen] == 0).all()
+
+
+def test_far_apart_scores(ops):
+    """Scores that grow along the sequence (the running maximum moves in every block) and a first key that outweighs all others."""
+    qkv, ck, cv, pos, seq = batch([(0, 0, 300)], 8, 8, 300, 1, seed=3)
+    qkv[:, :1024] = 1.0
+    ramp = torch.linspace(-4, 4, 300, device="cuda").half()
+    ck[0] = ramp[:, None, None].expand(300, 8, 128)
+    ck[0, 0, 0] = 6.0
+    out = torch.empty(300, 1024, dtype=torch.float16, device="cuda")
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, 8, 8, 128, 128 ** -0.5)
+    check(out, reference(qkv, ck, cv, pos, seq, 8, 8, 128 ** -0.5))
