@@ -72,7 +72,7 @@ decode_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pos = positions[tok], seq = seq_ids[tok];
   if ((unsigned)pos >= (unsigned)S) return;               // out of the cache / rotary table: nothing valid to attend to
-  if (min_run && atile::attn_in_run(positions, seq_ids, T, tok, min_run)) return;   // attn_tile_kernel's
+  if (min_run && atile::attn_token_in_run(positions, seq_ids, T, tok, min_run)) return;   // attn_tile_kernel's
   const int nkeys = pos + 1;
   const int hk = h / (Hq / Hkv);
   qs[tid] = __half2float(qkv[(size_t)tok * (Hq + 2 * Hkv) * D + (size_t)h * D + tid]) * sm_scale;
@@ -587,7 +587,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   __shared__ __align__(16) uint4 s_qf[8][32];                // Q fragments of the chunk in mma order: [k-step][lane] = (a0, a1, a2, a3)
   extern __shared__ __align__(16) unsigned char seq_dyn[];
   float (*s_o)[16][D] = reinterpret_cast<float (*)[16][D]>(seq_dyn);   // [NW][16][D] fp32: per-warp partial outputs (64 KB)
-  const int seq = blockIdx.x, hk = blockIdx.y;
+  const int seq = blockIdx.x / Hkv, hk = blockIdx.x % Hkv;    // the heads of a sequence side by side: their rows are neighbours in the cache
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
   if (tid == 0) s_ntok = 0;
@@ -602,24 +602,19 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   }
   __syncthreads();
   int ntok = s_ntok;
-  if (min_run && ntok >= min_run) {                          // leave the tokens of prompt runs to attn_tile_kernel
-    int t_[1024 / (NW * 32)], p_[1024 / (NW * 32)];
-#pragma unroll
-    for (int q = 0; q < 1024 / (NW * 32); ++q) {
-      const int i = tid + q * NW * 32;
-      t_[q] = -1; p_[q] = 0;
-      if (i < ntok && !atile::attn_in_run(positions, seq_ids, T, s_tok[i], min_run)) { t_[q] = s_tok[i]; p_[q] = s_pos[i]; }
-    }
+  if (min_run && ntok >= min_run) {                          // gather again without the tokens of prompt runs: attn_tile_kernel's
     __syncthreads();
     if (tid == 0) s_ntok = 0;
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 1024 / (NW * 32); ++q)
-      if (t_[q] >= 0) {
+    for (int t0 = warp * 32; t0 < T; t0 += NW * 32) {
+      const int t = t0 + lane;
+      bool before, after;
+      if (!atile::attn_in_run(positions, seq_ids, T, t0, min_run, before, after) && t < T && seq_ids[t] == seq) {
         const int i = atomicAdd(&s_ntok, 1);
-        s_tok[i] = t_[q];
-        s_pos[i] = p_[q];
+        s_tok[i] = t;
+        s_pos[i] = positions[t];
       }
+    }
     __syncthreads();
     ntok = s_ntok;
   }
@@ -779,7 +774,7 @@ static int launch_seq_attention(const void* qkv, const void* ck, const void* cv,
     QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     attr_set = true;
   }
-  launch_pdl(kern, dim3(B, Hkv), dim3(SEQ_ATTN_WARPS * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
+  launch_pdl(kern, dim3(B * Hkv), dim3(SEQ_ATTN_WARPS * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
              positions, seq_ids, (__half*)out, T, Hq, Hkv, S, sm_scale, min_run);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;

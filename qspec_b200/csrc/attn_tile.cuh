@@ -3,19 +3,19 @@
 // instantiate it: float16 with queries as they lie in the fused projection (attn_kernels.cu), bfloat16 with float32 queries
 // (seq_mma_kernels.cu).
 //
-// One CTA = two tiles of 128 query rows of one key/value head; a row is a (token, query head of the group) pair, so that the group's
-// heads share every key tile: 64 tokens per CTA at four heads per group. Keys are walked in blocks of 128.
-//   * S = Q K^T: both operands from shared memory, accumulator [128 x 128] float32 in tensor memory.
-//   * softmax: thread = row, so maxima and sums need no exchange. Scores are read from tensor memory (twice: maxima, then weights,
-//     64 columns at a time), weights go back over the scores they came from as a two-term 16-bit split (hi + lo: 22 / 16 mantissa
-//     bits, so that the second product is as good as one with float32 weights).
+// One CTA = a tile of 128 query rows of one key/value head; a row is a (token, query head of the group) pair, so that the group's
+// heads share every key tile: 32 tokens per CTA at four heads per group. Keys are walked in blocks of 128.
+//   * S = Q K^T: both operands from shared memory, accumulator [128 x 128] float32 in tensor memory, two of them: the next block's
+//     scores are computed while this block's pass through the softmax.
+//   * softmax: thread = half a row (64 columns), two warps per 32 rows, which exchange the row's maximum through shared memory. Weights
+//     go back over the scores they came from as a two-term 16-bit split (hi + lo: 22 / 16 mantissa bits, so that the second product is
+//     as good as one with float32 weights).
 //   * O += P V: weights from tensor memory, values from shared memory as they lie in the cache (the reduction runs over rows: the
-//     operand is "MN-major"); hi and lo terms are 8 + 8 instructions on the same value tile.
+//     operand is "MN-major"); hi and lo terms are 8 + 8 instructions on the same value tile. It runs under the next block's softmax.
 //   * O is rescaled only when a row's maximum grew by more than 2^8 since the last rescale (weights then stay below 256, and the
 //     division by the sum at the end undoes the common factor).
-// Tensor memory: S0 | S1 | O0 | O1 = 512 columns. Warps: 2 x 4 softmax, 1 keys, 1 values (TMA), 2 that issue one tile's products
-// each. Within a tile scores, weights and value product follow one another; the two tiles run independently, so that the tensor
-// cores work on one while the other's scores pass through its softmax warps.
+// Tensor memory: S0 | S1 | O = 384 of 512 columns. Warps: 8 softmax, 1 keys, 1 values (TMA), 1 that
+// issues the products.
 //
 // Which tokens: those in RUNS, i.e. neighbours in the batch with one sequence and consecutive positions, of at least min_run
 // tokens. A CTA walks the runs of its tokens one after the other (rows of other runs are masked). Tokens outside such runs are left
@@ -35,13 +35,13 @@
 namespace qspec {
 namespace atile {
 
-constexpr int TOKENS_MAX = 256;                // tokens of a CTA: 2 * (128 / heads of a group)
-constexpr int MARGIN = 16;                     // run test: links looked at on either side
-constexpr int WARP_K = 8, WARP_V = 9, WARP_MMA = 10;   // warps 0 .. 7: softmax; 10, 11: products of one tile each
-constexpr int THREADS = 12 * 32;               // three warps per scheduler: 168 registers a thread (13 warps would leave 128)
+constexpr int TOKENS_MAX = 128;                // tokens of a CTA: 128 / heads of a group
+constexpr int WARP_K = 8, WARP_V = 9, WARP_MMA = 10;   // warps 0 .. 7: softmax
+constexpr int THREADS = 12 * 32;
 constexpr int HALF = 128 * 128;                // 128 rows x 64 elements
 constexpr int TILE = 2 * HALF;                 // 128 rows x 128 elements
-constexpr size_t SMEM = 6 * (size_t)TILE + 1024;   // Q0 Q1 | K K | V V | slack to start on a 1024-byte boundary
+constexpr int KS = 3, VS = 2;                  // key and value blocks in shared memory
+constexpr size_t SMEM = (1 + KS + VS) * (size_t)TILE + 1024;   // Q | keys | values | slack to start on a 1024-byte boundary
 constexpr float RESCALE_LOG2 = 8.f;
 constexpr uint32_t WAIT_SPINS = 1u << 20;
 
@@ -59,15 +59,25 @@ struct Args {
   const float* sink; const void* gate; int gate_ld, gate_per_head; float out_scale;
 };
 
-// Is token t in a run of at least `min_run` tokens (min_run <= MARGIN)?
-__device__ __forceinline__ bool attn_link(const int* pos, const int* seq, int t) {      // t and t + 1 are of one run
-  return seq[t] == seq[t + 1] && pos[t + 1] == pos[t] + 1;
+// Tokens t and t + 1 of the batch are of one run.
+__device__ __forceinline__ bool attn_link(const int* pos, const int* seq, int ntok, int t) {
+  return t >= 0 && t + 1 < ntok && seq[t] == seq[t + 1] && pos[t + 1] == pos[t] + 1;
 }
-__device__ __forceinline__ bool attn_in_run(const int* pos, const int* seq, int ntok, int t, int min_run) {
-  int n = 1;
-  for (int i = t; n < min_run && i > 0 && attn_link(pos, seq, i - 1); --i) ++n;
-  for (int i = t; n < min_run && i + 1 < ntok && attn_link(pos, seq, i); ++i) ++n;
-  return n >= min_run;
+// For the 32 tokens t0 .. t0 + 31 of a whole warp, token t0 + lane: is it in a run of at least min_run (<= 16) tokens? `before`, `after`: is
+// it linked to its neighbours?
+__device__ __forceinline__ bool attn_in_run(const int* pos, const int* seq, int ntok, int t0, int min_run, bool& before, bool& after) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t links = (uint64_t)__ballot_sync(0xffffffffu, attn_link(pos, seq, ntok, t0 - 16 + lane)) |
+                         (uint64_t)__ballot_sync(0xffffffffu, attn_link(pos, seq, ntok, t0 + 16 + lane)) << 32;   // bit i: token t0 - 16 + i
+  const uint64_t left = ~(links << (48 - lane)), right = ~(links >> (16 + lane));
+  before = links >> (15 + lane) & 1;
+  after = links >> (16 + lane) & 1;
+  return 1 + __clzll((long long)left) + (__ffsll((long long)right) - 1) >= min_run && t0 + lane < ntok;
+}
+// One token, asked by a whole warp.
+__device__ __forceinline__ bool attn_token_in_run(const int* pos, const int* seq, int ntok, int t, int min_run) {
+  bool x, y;
+  return __shfl_sync(0xffffffffu, attn_in_run(pos, seq, ntok, t, min_run, x, y), 0);
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -181,43 +191,30 @@ template <> struct Elem<true> {
   static __device__ __forceinline__ uint32_t rest(uint32_t q0, uint32_t q1) { return __byte_perm(q0 + 0x8000u, q1 + 0x8000u, 0x7632); }   // rounded
 };
 
-// The key blocks of a CTA: for every run the blocks of up to 128 positions from its first visible key to its last, with the tiles that
-// see something in them.
-struct Item { int kb, hi, seq, p0, ts, te; bool act[2]; };   // positions kb .. hi, at most 128
+// The key blocks of a CTA: for every run the blocks of up to 128 positions from its first visible key to its last.
+struct Item { int kb, hi, seq, p0, ts, te; };   // positions kb .. hi, at most 128; the run's tokens and its first position
 struct Items {
-  const int *rs, *re, *pos, *seq; int nruns, tok, window, last, ring;    // ring: rows of the ring, or 0
-  int r = -1, kb = 0, hi = -1, wlo[2], whi[2];
+  const int *rs, *re, *pos, *seq; int nruns, window, last, ring;    // ring: rows of the ring, or 0
+  int r = -1, kb = 0, hi = -1;
   __device__ __forceinline__ bool next(Item& it) {
-    for (;;) {
-      while (kb > hi) {
-        if (++r >= nruns) return false;
-        const int ts = rs[r], te = re[r], p0 = pos[ts], p1 = pos[te];
-        kb = max(0, p0 - window + 1);
-        hi = min(p1, last);
-#pragma unroll
-        for (int w = 0; w < 2; ++w) {
-          const int a = max(ts, w * tok), b = min(te, w * tok + tok - 1);
-          wlo[w] = a > b ? 0x7fffffff : max(0, p0 + (a - ts) - window + 1);
-          whi[w] = a > b ? -1 : min(p0 + (b - ts), last);
-        }
-      }
-      int n = 128;
-      if (ring) n = min(n, ring - kb % ring);               // a block ends where the ring does
-      it.kb = kb;
-      it.hi = min(hi, kb + n - 1);
-      kb += n;
-#pragma unroll
-      for (int w = 0; w < 2; ++w) it.act[w] = it.kb <= whi[w] && it.hi >= wlo[w];
-      if (it.act[0] || it.act[1]) break;
+    while (kb > hi) {
+      if (++r >= nruns) return false;
+      kb = max(0, pos[rs[r]] - window + 1);
+      hi = min(pos[re[r]], last);
     }
+    int n = 128;
+    if (ring) n = min(n, ring - kb % ring);                 // a block ends where the ring does
+    it.kb = kb;
+    it.hi = min(hi, kb + n - 1);
+    kb += n;
     it.ts = rs[r]; it.te = re[r]; it.p0 = pos[it.ts]; it.seq = seq[it.ts];
     return true;
   }
 };
 
-// One row key by key on the CUDA cores (float32 weights, nothing but the row's own keys): rows whose tile result is not finite.
+// 64 columns of one row key by key on the CUDA cores (float32 weights, nothing but the row's own keys): rows whose tile result is not finite.
 template <bool BF, bool QF32>
-__device__ __noinline__ void attn_row_again(const Args& a, int tok, int head, int kvh, int seq, int lo, int hi) {
+__device__ __noinline__ void attn_row_again(const Args& a, int tok, int head, int kvh, int seq, int lo, int hi, int col0) {
   using T = typename Elem<BF>::T;
   const T* kbase = (const T*)a.k + (size_t)seq * a.k_ss + (size_t)kvh * a.k_hs;
   const T* vbase = (const T*)a.v + (size_t)seq * a.v_ss + (size_t)kvh * a.v_hs;
@@ -238,7 +235,7 @@ __device__ __noinline__ void attn_row_again(const Args& a, int tok, int head, in
   if (a.sink) m = fmaxf(m, a.sink[head]);
   float l = a.sink ? __expf(a.sink[head] - m) : 0.f;
   for (int j = lo; j <= hi; ++j) l += __expf(score(j) - m);
-  for (int d0 = 0; d0 < 128; d0 += 16) {
+  for (int d0 = col0; d0 < col0 + 64; d0 += 16) {
     float o[16];
     for (int d = 0; d < 16; ++d) o[d] = 0.f;
     for (int j = lo; j <= hi; ++j) {
@@ -260,40 +257,31 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   using T = typename Elem<BF>::T;
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   extern __shared__ __align__(16) unsigned char at_raw[];
-  __shared__ int s_pos[TOKENS_MAX + 2 * MARGIN], s_seq[TOKENS_MAX + 2 * MARGIN];
+  __shared__ int pos[TOKENS_MAX], seq[TOKENS_MAX];
   __shared__ int s_rs[TOKENS_MAX], s_re[TOKENS_MAX];
   __shared__ uint32_t s_start[TOKENS_MAX / 32];
-  __shared__ __align__(8) uint64_t b_kfull[2], b_kempty[2], b_vfull[2], b_vempty[2], b_s[2], b_p[2][2], b_o[2], b_part;
+  __shared__ __align__(8) uint64_t b_kfull[KS], b_kempty[KS], b_vfull[VS], b_vempty[VS], b_s[2], b_p[2][2], b_o, b_part, b_mx[4];
+  __shared__ float s_mx[2][2][128];                         // [block & 1][half][row]
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_fail;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rep = a.rep, tok = 128 / rep;                   // tokens per tile
-  const int c0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * tok;   // the longest key ranges first
-  const int kvh = blockIdx.y;
-  const int n2 = min(2 * tok, a.ntok - c0);
+  const int rep = a.rep, tok = 128 / rep;                   // tokens per CTA
+  const int c0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * tok;   // the longest key ranges of all heads first
+  const int kvh = blockIdx.x;
+  const int n2 = min(tok, a.ntok - c0);
 
   // ---- the runs among this CTA's tokens
-  for (int i = tid; i < n2 + 2 * MARGIN; i += THREADS) {
-    const int t = c0 + i - MARGIN;
-    const bool in = t >= 0 && t < a.ntok;
-    s_pos[i] = in ? a.pos[t] : 0;
-    s_seq[i] = in ? a.seq[t] : -1;
-  }
-  __syncthreads();
-  const int* pos = s_pos + MARGIN;
-  const int* seq = s_seq + MARGIN;
-  auto linked = [&](int i) { return c0 + i >= 0 && c0 + i + 1 < a.ntok && attn_link(pos, seq, i); };
   bool start = false, end = false;
   if (tid < TOKENS_MAX) {
-    bool in = false;
-    if (tid < n2) {
-      int n = 1;
-      for (int i = tid; n < a.min_run && linked(i - 1); --i) ++n;
-      for (int i = tid; n < a.min_run && linked(i); ++i) ++n;
-      in = n >= a.min_run && (unsigned)seq[tid] < (unsigned)a.nseq;
-      start = in && (tid == 0 || !linked(tid - 1));
-      end = in && (tid == n2 - 1 || !linked(tid));
+    bool before, after;
+    bool in = attn_in_run(a.pos, a.seq, a.ntok, c0 + warp * 32, a.min_run, before, after) && tid < n2;
+    if (in) {
+      pos[tid] = a.pos[c0 + tid];
+      seq[tid] = a.seq[c0 + tid];
+      in = (unsigned)seq[tid] < (unsigned)a.nseq;
     }
+    start = in && (tid == 0 || !before);
+    end = in && (tid == n2 - 1 || !after);
     const uint32_t bits = __ballot_sync(0xffffffffu, start);
     if (lane == 0) s_start[warp] = bits;
   }
@@ -315,21 +303,22 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   if (tid == 0) {
+    for (int i = 0; i < KS; ++i) { bar_init(smem_addr(&b_kfull[i]), 1); bar_init(smem_addr(&b_kempty[i]), 1); }
+    for (int i = 0; i < VS; ++i) { bar_init(smem_addr(&b_vfull[i]), 1); bar_init(smem_addr(&b_vempty[i]), 1); }
     for (int i = 0; i < 2; ++i) {
-      bar_init(smem_addr(&b_kfull[i]), 1); bar_init(smem_addr(&b_kempty[i]), 2);
-      bar_init(smem_addr(&b_vfull[i]), 1); bar_init(smem_addr(&b_vempty[i]), 2);
-      bar_init(smem_addr(&b_s[i]), 1); bar_init(smem_addr(&b_o[i]), 1);
+      bar_init(smem_addr(&b_s[i]), 1);
       bar_init(smem_addr(&b_p[i][0]), 4); bar_init(smem_addr(&b_p[i][1]), 4);
     }
+    bar_init(smem_addr(&b_o), 1);
     bar_init(smem_addr(&b_part), 1);
+    for (int i = 0; i < 4; ++i) bar_init(smem_addr(&b_mx[i]), 2);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   const uint32_t base = (smem_addr(at_raw) + 1023u) & ~1023u;
   unsigned char* gbase = at_raw + (base - smem_addr(at_raw));
-  // ---- queries of both tiles
-  for (int i = tid; i < 256 * 16; i += THREADS) {
-    const int row = i >> 4, c = i & 15, w = row >> 7, r = row & 127;
-    const int tl = w * tok + r / rep;
+  // ---- queries
+  for (int i = tid; i < 128 * 16; i += THREADS) {
+    const int r = i >> 4, c = i & 15, tl = r / rep;
     uint4 val = make_uint4(0u, 0u, 0u, 0u);
     if (r < tok * rep && tl < n2) {
       const size_t o = (size_t)(c0 + tl) * a.q_ts + (size_t)(kvh * rep + r % rep) * a.q_hs + c * 8;
@@ -340,7 +329,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         val = *reinterpret_cast<const uint4*>((const T*)a.q + o);
       }
     }
-    *reinterpret_cast<uint4*>(gbase + w * TILE + (c >> 3) * HALF + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = val;
+    *reinterpret_cast<uint4*>(gbase + (c >> 3) * HALF + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = val;
   }
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   fence_before();
@@ -349,52 +338,52 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   const uint32_t tmem = s_tmem;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // tensor memory is held: a dependent that waits for this grid cannot take it first
 
-  Items items{s_rs, s_re, pos, seq, nruns, tok, a.window, a.ring ? 0x7fffffff - 256 : a.cap - 1, a.ring ? a.cap : 0};
+  Items items{s_rs, s_re, pos, seq, nruns, a.window, a.ring ? 0x7fffffff - 256 : a.cap - 1, a.ring ? a.cap : 0};
   Item it;
-  if (warp >= WARP_MMA) {
+  if (warp == WARP_MMA) {
     if (elect()) {
-      const int w = warp - WARP_MMA;
-      const uint32_t id_s = idesc<BF>(false), id_o = idesc<BF>(true);
-      const uint32_t qa = base + w * TILE, p = tmem + w * 128, o = tmem + 256 + w * 128;
-      const uint32_t bs = smem_addr(&b_s[w]), bp = smem_addr(&b_p[w][0]), bo = smem_addr(&b_o[w]);
-      uint32_t done = 0;                                      // value products of this tile so far
-      for (uint32_t n = 0; items.next(it); ++n) {
-        const uint32_t stage = n & 1, phase = (n >> 1) & 1;
-        if (!bar_wait(smem_addr(&b_kfull[stage]), phase, &s_fail)) break;
-        if (it.act[w]) {
-          // the scores take the columns of the tile's previous weights: their product must be over
-          if (done && !bar_wait(bo, (done - 1) & 1, &s_fail)) break;
-          fence_after();
-          const uint64_t qd = desc_k(qa), kd = desc_k(base + (2 + stage) * TILE);
+      const uint32_t id_s = idesc<BF>(false), id_o = idesc<BF>(true), o = tmem + 256, bo = smem_addr(&b_o);
+      const uint64_t qd = desc_k(base);
+      uint32_t blocks = 0;
+      while (items.next(it)) ++blocks;
+      uint32_t ks = 0, kphase = 0;                            // key stage of the next scores
+      auto scores = [&](uint32_t n) -> bool {
+        if (!bar_wait(smem_addr(&b_kfull[ks]), kphase, &s_fail)) return false;
+        // these scores take the columns of the weights of block n - 2: their product must be over
+        if (n >= 2 && !bar_wait(bo, n & 1, &s_fail)) return false;
+        fence_after();
+        const uint64_t kd = desc_k(base + (1 + ks) * TILE);
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t step = (uint32_t)((ks >> 2) * (HALF >> 4) + (ks & 3) * 2);
-            mma_ss(p, qd + step, kd + step, id_s, ks ? 1u : 0u);
-          }
-          commit(bs);
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t step = (uint32_t)((i >> 2) * (HALF >> 4) + (i & 3) * 2);
+          mma_ss(tmem + (n & 1) * 128, qd + step, kd + step, id_s, i ? 1u : 0u);
         }
-        commit(smem_addr(&b_kempty[stage]));
-        if (!bar_wait(smem_addr(&b_vfull[stage]), phase, &s_fail)) break;
-        if (it.act[w]) {
-          const uint64_t vd = desc_mn(base + (4 + stage) * TILE);
-          bool ok = true;
+        commit(smem_addr(&b_s[n & 1]));
+        commit(smem_addr(&b_kempty[ks]));
+        if (++ks == KS) { ks = 0; kphase ^= 1u; }
+        return true;
+      };
+      bool ok = blocks == 0 || scores(0);
+      for (uint32_t n = 0; ok && n < blocks; ++n) {
+        if (n + 1 < blocks && !scores(n + 1)) break;
+        if (!bar_wait(smem_addr(&b_vfull[n % VS]), (n / VS) & 1, &s_fail)) break;
+        const uint64_t vd = desc_mn(base + (1 + KS + n % VS) * TILE);
+        const uint32_t p = tmem + (n & 1) * 128;
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {                       // 64 keys each: the first half's product runs during the second half's weights
-            ok = ok && bar_wait(bp + 8 * h, done & 1, &s_fail);
-            if (!ok) break;
-            fence_after();
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              const uint64_t v = vd + (h * 4 + ks) * (2048 >> 4);
-              mma_ts(o, p + h * 64 + ks * 8, v, id_o, (done | h | ks) ? 1u : 0u);
-              mma_ts(o, p + h * 64 + 32 + ks * 8, v, id_o, 1u);
-            }
-          }
+        for (int h = 0; h < 2; ++h) {                         // 64 keys each
+          ok = ok && bar_wait(smem_addr(&b_p[n & 1][h]), (n >> 1) & 1, &s_fail);
           if (!ok) break;
-          commit(bo);
-          ++done;
+          fence_after();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint64_t v = vd + (h * 4 + i) * (2048 >> 4);
+            mma_ts(o, p + h * 64 + i * 8, v, id_o, (n | h | i) ? 1u : 0u);
+            mma_ts(o, p + h * 64 + 32 + i * 8, v, id_o, 1u);
+          }
         }
-        commit(smem_addr(&b_vempty[stage]));
+        if (!ok) break;
+        commit(bo);
+        commit(smem_addr(&b_vempty[n % VS]));
       }
     }
     __syncwarp();
@@ -404,17 +393,20 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     uint64_t* full = keys ? b_kfull : b_vfull;
     uint64_t* empty = keys ? b_kempty : b_vempty;
     const CUtensorMap* map = keys ? &map_k : &map_v;
-    const uint32_t buf = base + (keys ? 2 : 4) * TILE;
+    const uint32_t buf = base + (keys ? 1 : 1 + KS) * TILE;
+    const int stages = keys ? KS : VS;
+    int stage = 0;
+    uint32_t phase = 1;                                       // of the stage's previous release: none to wait for in the first round
     bool ok = true;
     int parts = 0;
     for (int n = 0; items.next(it); ++n) {
-      if (n >= 2) ok = bar_wait(smem_addr(&empty[n & 1]), (uint32_t)(((n >> 1) - 1) & 1), &s_fail);
+      if (n >= stages) ok = bar_wait(smem_addr(&empty[stage]), phase, &s_fail);
       if (!__all_sync(0xffffffffu, ok)) break;
       // value rows past the block's last key are cleared before the products see them (their weights are zero, but zero times NaN is not):
       // such a block lands on a barrier of its own first
       const int have = it.hi - it.kb + 1;
       const bool part = !keys && have < 128;
-      const uint32_t bar = smem_addr(part ? &b_part : &full[n & 1]), dst = buf + (n & 1) * TILE;
+      const uint32_t bar = smem_addr(part ? &b_part : &full[stage]), dst = buf + stage * TILE;
       if (elect()) {
         const int row = a.ring ? it.kb % a.cap : it.kb;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"((uint32_t)TILE) : "memory");
@@ -432,25 +424,26 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         }
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncwarp();
-        if (lane == 0) bar_arrive(smem_addr(&full[n & 1]));
+        if (lane == 0) bar_arrive(smem_addr(&full[stage]));
       }
+      if (++stage == stages) { stage = 0; phase ^= 1u; }
     }
-  } else {
-    // ---- softmax: thread = row of tile w
-    const int w = warp >> 2, r = (warp & 3) * 32 + lane;
-    const int tl = w * tok + r / rep, head = kvh * rep + r % rep;
+  } else if (warp < WARP_K) {
+    // ---- softmax: thread = 64 columns (half h) of row r
+    const int h = warp >> 2, r = (warp & 3) * 32 + lane;
+    const int tl = r / rep, head = kvh * rep + r % rep;
     const bool row_in = r < tok * rep && tl < n2;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t st = tmem + lanes + w * 128, ot = tmem + lanes + 256 + w * 128;
+    const uint32_t ot = tmem + lanes + 256 + h * 64;
+    const uint32_t bmx = smem_addr(&b_mx[warp & 3]);
     const float c2 = a.scale * 1.4426950408889634f;
     const int last = a.ring ? 0x7fffffff : a.cap - 1;
-    float m = -INFINITY, l = 0.f;                             // maximum in units of log2, sum relative to it
+    float m = -INFINITY, l = 0.f;                             // maximum in units of log2; sum of this half's weights relative to it
     int n = 0, my_lo = 0, my_hi = -1, my_seq = 0;
     bool ok = true, mine = false;
     while (ok && items.next(it)) {
-      if (!it.act[w]) continue;
       const bool in = row_in && tl >= it.ts && tl <= it.te;
-      // visible columns of the block: j0 .. j0 + span
+      // visible columns of the half block: j0 .. j0 + span
       int j0 = 0x7fff, span = 0;
       if (in) {
         const int pr = it.p0 + (tl - it.ts);
@@ -458,42 +451,47 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         int vhi = min(pr, last);
         mine = true; my_lo = vlo; my_hi = vhi; my_seq = it.seq;
         vhi = min(vhi, it.hi);
-        if (vhi >= vlo) { j0 = vlo - it.kb; span = vhi - vlo; }
+        if (vhi >= vlo) { j0 = vlo - it.kb - h * 64; span = vhi - vlo; }
       }
-      const bool whole = !row_in || (j0 <= 0 && j0 + span >= 127);   // (rows that stand for no token are never stored)
+      const bool whole = !row_in || (j0 <= 0 && j0 + span >= 63);   // (rows that stand for no token are never stored)
       const bool plain = __all_sync(0xffffffffu, whole);
-      ok = bar_wait(smem_addr(&b_s[w]), (uint32_t)(n & 1), &s_fail);
+      const uint32_t st = tmem + lanes + (n & 1) * 128 + h * 64;
+      ok = bar_wait(smem_addr(&b_s[n & 1]), (uint32_t)((n >> 1) & 1), &s_fail);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       fence_after();
       uint32_t x[64];
-      float mx = -INFINITY;
+      ld32(st, x);
+      ld32(st + 32, x + 32);
+      wait_ld();
+      if (!plain) {
 #pragma unroll
-      for (int h = 1; h >= 0; --h) {                          // the first half last: it stays in registers for the weights
-        ld32(st + h * 64, x);
-        ld32(st + h * 64 + 32, x + 32);
-        wait_ld();
-        if (plain) {
-          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-          for (int j = 0; j < 64; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(x[j]));
-          mx = fmaxf(mx, fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])));
-        } else {
-#pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            if ((uint32_t)(h * 64 + j - j0) > (uint32_t)span) x[j] = 0xff800000u;      // hidden
-            mx = fmaxf(mx, __uint_as_float(x[j]));
-          }
-        }
+        for (int j = 0; j < 64; ++j)
+          if ((uint32_t)(j - j0) > (uint32_t)span) x[j] = 0xff800000u;      // hidden
       }
-      const float mn = fmaxf(m, mx * c2);
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < 64; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(x[j]));
+      const float mine_mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      s_mx[n & 1][h][r] = mine_mx;
+      __syncwarp();
+      if (lane == 0) bar_arrive(bmx);
+      ok = bar_wait(bmx, (uint32_t)(n & 1), &s_fail);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      const float mn = fmaxf(m, fmaxf(mine_mx, s_mx[n & 1][1 - h][r]) * c2);
+      // (both warps of the rows see the same maxima and decide alike)
       if (__any_sync(0xffffffffu, mn > m + RESCALE_LOG2 || (m == -INFINITY && mn > m))) {
         const float f = mn == -INFINITY ? 1.f : ex2(m - mn);   // 0 for a row that had seen nothing
         m = mn;
         l *= f;
         if (n) {
+          ok = bar_wait(smem_addr(&b_o), (uint32_t)((n - 1) & 1), &s_fail);   // the previous block's product is in O
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          fence_after();
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
+          for (int q = 0; q < 2; ++q) {
             uint32_t o[32];
             ld32(ot + q * 32, o);
             wait_ld();
@@ -507,42 +505,29 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       const uint64_t c22 = pair(__float_as_uint(c2), __float_as_uint(c2)), mu2 = pair(__float_as_uint(-mu), __float_as_uint(-mu));
       const uint64_t minus2 = pair(0xbf800000u, 0xbf800000u);
       uint64_t l2[2] = {0ull, 0ull};
+      // weight = hi + lo: hi = the leading bits that the type keeps (cut, not rounded), lo = the rest, rounded
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h == 1) {
-          ld32(st + 64, x);
-          ld32(st + 96, x + 32);
-          wait_ld();
-          if (!plain) {
+      for (int g = 0; g < 2; ++g) {
+        uint32_t hi[16], lo[16];
 #pragma unroll
-            for (int j = 0; j < 64; ++j)
-              if ((uint32_t)(64 + j - j0) > (uint32_t)span) x[j] = 0xff800000u;
-          }
+        for (int j = 0; j < 16; ++j) {
+          uint32_t p0, p1, h0, h1, q0, q1;
+          unpair(fma2(pair(x[g * 32 + 2 * j], x[g * 32 + 2 * j + 1]), c22, mu2), p0, p1);
+          p0 = __float_as_uint(ex2(__uint_as_float(p0)));
+          p1 = __float_as_uint(ex2(__uint_as_float(p1)));
+          const uint64_t pp = pair(p0, p1);
+          l2[j & 1] = add2(l2[j & 1], pp);
+          hi[j] = Elem<BF>::lead(p0, p1, h0, h1);
+          unpair(fma2(pair(h0, h1), minus2, pp), q0, q1);
+          lo[j] = Elem<BF>::rest(q0, q1);
         }
-        // weight = hi + lo: hi = the leading bits that the type keeps (cut, not rounded), lo = the rest, rounded
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          uint32_t hi[16], lo[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            uint32_t p0, p1, h0, h1, q0, q1;
-            unpair(fma2(pair(x[g * 32 + 2 * j], x[g * 32 + 2 * j + 1]), c22, mu2), p0, p1);
-            p0 = __float_as_uint(ex2(__uint_as_float(p0)));
-            p1 = __float_as_uint(ex2(__uint_as_float(p1)));
-            const uint64_t pp = pair(p0, p1);
-            l2[j & 1] = add2(l2[j & 1], pp);
-            hi[j] = Elem<BF>::lead(p0, p1, h0, h1);
-            unpair(fma2(pair(h0, h1), minus2, pp), q0, q1);
-            lo[j] = Elem<BF>::rest(q0, q1);
-          }
-          st16(st + h * 64 + g * 16, hi);
-          st16(st + h * 64 + 32 + g * 16, lo);
-        }
-        wait_st();
-        fence_before();
-        __syncwarp();
-        if (lane == 0) bar_arrive(smem_addr(&b_p[w][h]));
+        st16(st + g * 16, hi);
+        st16(st + 32 + g * 16, lo);
       }
+      wait_st();
+      fence_before();
+      __syncwarp();
+      if (lane == 0) bar_arrive(smem_addr(&b_p[n & 1][h]));
       {
         uint32_t a0, a1;
         unpair(add2(l2[0], l2[1]), a0, a1);
@@ -550,16 +535,22 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       }
       ++n;
     }
-    // ---- the last product is done: divide, gate, store
-    if (ok && n) ok = bar_wait(smem_addr(&b_o[w]), (uint32_t)((n - 1) & 1), &s_fail);
+    // ---- the last product is done: add the halves' sums, divide, gate, store
+    if (ok && n) ok = bar_wait(smem_addr(&b_o), (uint32_t)((n - 1) & 1), &s_fail);
     ok = __all_sync(0xffffffffu, ok);
     fence_after();
+    s_mx[n & 1][h][r] = l;
+    __syncwarp();
+    if (lane == 0) bar_arrive(bmx);
+    if (ok) ok = bar_wait(bmx, (uint32_t)(n & 1), &s_fail);
+    ok = __all_sync(0xffffffffu, ok);
+    l += s_mx[n & 1][1 - h][r];
     // `mine` rows belong to a run; one whose position shows it no key is stored as zeros, or not at all (skip_outside)
     if (row_in && !mine) {                                    // a run none of whose keys lie in the cache produced no block
       for (int q = 0; q < nruns; ++q)
         if (tl >= s_rs[q] && tl <= s_re[q]) mine = true;
     }
-    const int pr = row_in ? pos[tl] : 0;
+    const int pr = row_in && mine ? pos[tl] : 0;
     const bool store = ok && row_in && mine && !(a.skip_outside && (unsigned)pr >= (unsigned)a.cap);
     const bool dead = l == 0.f;                               // saw no key at all
     float f = 0.f;
@@ -574,12 +565,12 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     }
     if (a.gate && a.gate_per_head && store)
       f *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)(c0 + tl) * a.gate_ld + head]));
-    T* dst = (T*)a.out + (size_t)(c0 + tl) * a.out_ts + (size_t)head * a.out_hs;
-    const T* gt = a.gate && !a.gate_per_head ? (const T*)a.gate + (size_t)(c0 + tl) * a.gate_ld + (size_t)head * a.out_hs : nullptr;
+    T* dst = (T*)a.out + (size_t)(c0 + tl) * a.out_ts + (size_t)head * a.out_hs + h * 64;
+    const T* gt = a.gate && !a.gate_per_head ? (const T*)a.gate + (size_t)(c0 + tl) * a.gate_ld + (size_t)head * a.out_hs + h * 64 : nullptr;
     bool bad = false;
     if (ok) {
 #pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < 2; ++q) {
         uint32_t o[32];
         ld32(ot + q * 32, o);
         wait_ld();
@@ -607,7 +598,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
           }
         }
       }
-      if (bad && store) attn_row_again<BF, QF32>(a, c0 + tl, head, kvh, my_seq, my_lo, my_hi);
+      if (bad && store) attn_row_again<BF, QF32>(a, c0 + tl, head, kvh, my_seq, my_lo, my_hi, h * 64);
     }
   }
   fence_before();
@@ -623,7 +614,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
 inline bool supported(const Args& a, int elem_q) {
   auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
   auto rows = [](long long ss, int rs, int hs) { return ss > 0 && rs > 0 && hs > 0 && ss % 8 == 0 && rs % 8 == 0 && hs % 8 == 0; };
-  return a.rep >= 1 && a.rep <= 64 && a.scale > 0.f && al(a.q) && al(a.k) && al(a.v) && al(a.out) && a.q_ts * elem_q % 16 == 0 &&
+  return a.rep >= 1 && a.rep <= 64 && a.ntok / (128 / a.rep) < 65535 && a.scale > 0.f && al(a.q) && al(a.k) && al(a.v) && al(a.out) && a.q_ts * elem_q % 16 == 0 &&
          a.q_hs * elem_q % 16 == 0 && rows(a.k_ss, a.k_rs, a.k_hs) && rows(a.v_ss, a.v_rs, a.v_hs) && a.out_ts % 8 == 0 && a.out_hs % 8 == 0 &&
          (!a.gate || a.gate_per_head || (al(a.gate) && a.gate_ld % 8 == 0));
 }
@@ -663,8 +654,8 @@ inline int launch(const Args& a, int kv_heads, cudaStream_t stream) {
   int rc = cache_map<BF>(&mk, a.k, a.k_ss, a.k_rs, a.k_hs, kv_heads, a.cap, nseq);
   if (rc == QSPEC_OK) rc = cache_map<BF>(&mv, a.v, a.v_ss, a.v_rs, a.v_hs, kv_heads, a.cap, nseq);
   if (rc != QSPEC_OK) return rc;
-  const int per = 2 * (128 / a.rep);
-  launch_pdl(kern, dim3((a.ntok + per - 1) / per, kv_heads), dim3(THREADS), SMEM, stream, mk, mv, a);
+  const int per = 128 / a.rep;
+  launch_pdl(kern, dim3(kv_heads, (a.ntok + per - 1) / per), dim3(THREADS), SMEM, stream, mk, mv, a);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
 }
