@@ -146,6 +146,7 @@ SEQ_SIGNATURES = {
                                    c_void_p, c_int, c_float, c_int, c_void_p]),
     "qspec_seq_window_attention": (c_int, [c_void_p, c_int, c_void_p]),
     "qspec_seq_window_attention_mma": (c_int, [c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_void_p]),
+    "qspec_seq_attn_tile_timeouts": (c_int, []),
     "qspec_seq_window_attention_mma_supported": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int]),
     "qspec_seq_hgrn2": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                 c_int, c_int, c_int, c_int, c_float, c_int, c_void_p]),

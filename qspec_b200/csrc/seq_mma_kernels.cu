@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 #include "seq_common.cuh"
+#include "attn_tile.cuh"
 #include "../../include/qspec_b200_seq.h"
 
 namespace qspec {
@@ -1734,6 +1735,18 @@ int window_attention_mma(const qspec_window_attn_args* p, const void* kB, long l
   a.scale = p->scale; a.token_rows = token_rows;
   a.keep = p->keep_first; a.out_ts = p->out_tok_stride ? p->out_tok_stride : (long long)p->H * DV;
   a.out_scale = p->out_scale;
+  if (token_rows && DB == 0 && DA == 128 && DV == 128 && p->keep_first == 0) {
+    atile::Args t = {};
+    t.q = p->qa; t.q_ts = p->qa_tok_stride; t.q_hs = p->qa_head_stride;
+    t.k = p->k; t.k_ss = p->k_slot_stride; t.k_rs = p->k_row_stride; t.k_hs = p->k_head_stride;
+    t.v = p->v; t.v_ss = p->v_slot_stride; t.v_rs = p->v_row_stride; t.v_hs = p->v_head_stride;
+    t.pos = p->meta + p->ntok; t.seq = p->meta;
+    t.ntok = p->ntok; t.nseq = 0x7fffffff; t.rep = p->H / p->G; t.cap = p->cap; t.window = p->window;
+    t.scale = p->scale; t.min_run = 1; t.ring = 1;
+    t.out = p->out; t.out_ts = a.out_ts; t.out_hs = DV;
+    t.sink = p->sink; t.gate = p->gate; t.gate_ld = p->gate_ld; t.gate_per_head = p->gate_per_head; t.out_scale = a.out_scale;
+    if (atile::supported(t, 4)) return atile::launch<true, true>(t, p->G, st);
+  }
   // a latent cache read in the absorbed form (keys and values are the same rows): the CTA-level kernel; QSPEC_SEQ_LATENT=sliced
   // keeps the form with one CTA per slice of 128 value columns, for comparison
   static const bool sliced = [] { const char* v = getenv("QSPEC_SEQ_LATENT"); return v && !strcmp(v, "sliced"); }();
@@ -1764,6 +1777,12 @@ extern "C" int qspec_seq_window_attention_mma(const qspec_window_attn_args* args
   QSPEC_REQUIRE(s >= 0, QSPEC_ERR_UNSUPPORTED, "seq_window_attention_mma: key parts %d + %d, value size %d, or strides / alignment not taken",
                 args->DA - DB, DB, args->DV);
   return s;
+}
+
+extern "C" int qspec_seq_attn_tile_timeouts(void) {
+  unsigned n = 0;
+  if (cudaMemcpyFromSymbol(&n, qspec::atile::attn_tile_timeouts, sizeof(n)) != cudaSuccess) return -1;
+  return (int)n;
 }
 
 extern "C" int qspec_seq_window_attention_mma_supported(int DA, int DB, int DV, int H, int G, int token_rows) {

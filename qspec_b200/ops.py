@@ -643,8 +643,9 @@ def decode_attention(qkv: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Te
 
 
 def attn_tile_timeouts() -> int:
-    """CTAs of the prompt form inside seq_attention / decode_attention that gave up a bounded wait: 0 unless something is broken."""
-    return int(_lib.load().qspec_attn_tile_timeouts())
+    """CTAs of the prompt forms inside seq_attention, decode_attention and seq_window_attention_mma that gave up a bounded wait: 0
+    unless something is broken."""
+    return int(_lib.load().qspec_attn_tile_timeouts()) + int(_lib.load_seq().qspec_seq_attn_tile_timeouts())
 
 
 def seq_attention_supported(T: int, num_heads: int, num_kv_heads: int, head_dim: int, cache_len: int) -> bool:

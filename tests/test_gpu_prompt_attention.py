@@ -117,3 +117,49 @@ def test_far_apart_scores(ops):
     out = torch.empty(300, 1024, dtype=torch.float16, device="cuda")
     ops.seq_attention(qkv, ck, cv, pos, seq, out, 8, 8, 128, 128 ** -0.5)
     check(out, reference(qkv, ck, cv, pos, seq, 8, 8, 128 ** -0.5))
+
+
+# ---- the same tiles in the sequence-mixer library: bfloat16, rings, window, sink, gates ---------------------------------------------
+@pytest.mark.parametrize("H,G,window,cap,segments,gate,sink", [
+    (16, 4, 40, 200, [(0, 150, 70)], "each", True),                    # the ring wraps inside a block, inside the portion
+    (8, 8, 1000, 600, [(1, 0, 129), (0, 300, 5)], None, True),         # window longer than anything held; two sequences in one tile
+    (12, 4, 16, 300, [(2, 1000, 33), (0, 3, 1), (1, 77, 64)], "head", False),   # three heads per group: rows left over
+    (32, 2, 129, 400, [(0, 255, 17), (1, 256, 18)], "each", False),
+])
+def test_window_tiles_match_float64(ops, H, G, window, cap, segments, gate, sink):
+    g = torch.Generator(device="cuda").manual_seed(H + window)
+    slots = 1 + max(s for s, _, _ in segments)
+    pos = torch.cat([torch.arange(p, p + n) for _, p, n in segments])
+    slot = torch.cat([torch.full((n,), s) for s, _, n in segments])
+    T = len(pos)
+    begin = torch.cat([torch.full((n,), sum(m for _, _, m in segments[:i])) for i, (_, _, n) in enumerate(segments)])
+    end = torch.cat([torch.full((n,), sum(m for _, _, m in segments[:i + 1])) for i, (_, _, n) in enumerate(segments)])
+    meta = torch.stack([slot, pos, begin, end, torch.zeros(T, dtype=torch.int64)]).to(torch.int32).cuda()
+    q = torch.randn(T, H, 128, generator=g, device="cuda")
+    ck = torch.full((slots, cap, G, 128), float("nan"), dtype=torch.bfloat16, device="cuda")      # rows that nobody wrote must not matter
+    cv = torch.full_like(ck, float("inf"))
+    for s, p, n in segments:
+        rows = torch.arange(max(0, p - window + 1), p + n) % cap
+        ck[s, rows] = torch.randn(len(rows), G, 128, generator=g, device="cuda").bfloat16()
+        cv[s, rows] = torch.randn(len(rows), G, 128, generator=g, device="cuda").bfloat16()
+    gt = torch.randn(T, H if gate == "head" else H * 128, generator=g, device="cuda").bfloat16() if gate else None
+    sk = torch.randn(H, generator=g, device="cuda") if sink else None
+    wide = torch.zeros(T, H * 128 + 64, dtype=torch.bfloat16, device="cuda")                      # rows with a stride of their own
+    out = wide[:, :H * 128].view(T, H, 128)
+    ops.seq_window_attention_mma(q, ck, None, cv, out, meta, window, 0.07, True, sink=sk, gate=gt, gate_per_head=gate == "head", out_scale=0.5)
+    want = torch.zeros(T, H, 128, dtype=torch.float64, device="cuda")
+    for t in range(T):
+        rows = torch.arange(max(0, int(pos[t]) - window + 1), int(pos[t]) + 1, device="cuda") % cap
+        k = ck[int(slot[t]), rows].double().repeat_interleave(H // G, 1)
+        v = cv[int(slot[t]), rows].double().repeat_interleave(H // G, 1)
+        s = torch.einsum("hd,jhd->hj", q[t].bfloat16().double(), k) * 0.07                        # the product takes bfloat16 queries
+        if sink:
+            s = torch.cat([s, sk.double()[:, None]], 1)
+        want[t] = torch.einsum("hj,jhd->hd", torch.softmax(s, 1)[:, :len(rows)], v) * 0.5
+    if gate:
+        z = torch.sigmoid(gt.double())
+        want *= z[:, :, None] if gate == "head" else z.view(T, H, 128)
+    err = (out.double() - want).abs().max().item()
+    assert err <= 2 ** -8 * want.abs().max().item(), err       # bfloat16 outputs: half a unit in the last place is 2^-9 of a value
+    assert float(wide[:, H * 128:].abs().max()) == 0.0
+    assert ops.attn_tile_timeouts() == 0
