@@ -250,6 +250,18 @@ int qspec_seq_lightning(const void* p, int ld, const float* decay, const float* 
                         const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, float eps, int dtype,
                         void* stream);
 
+/* The two recurrences over long segments in chunks that run side by side (the walk through a segment's tokens is a chain): same arguments
+ * and results (float32 throughout; another order of products of decays), and a workspace of qspec_seq_recurrence_chunk_bytes(..) bytes on
+ * a 16-byte boundary, which the call may leave anything in. 0 bytes: these sizes are walked token by token (segments shorter than
+ * 256 tokens on average, key or value sizes other than 64 and 128), as they are without a workspace or without seg_starts. */
+size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV);
+int qspec_seq_hgrn2_chunked(const void* p, int ld, const float* f_b, const float* lower, const float* norm_w, float* state,
+                            float* scratch, void* out, const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D,
+                            int DV, float eps, int dtype, void* workspace, size_t workspace_bytes, void* stream);
+int qspec_seq_lightning_chunked(const void* p, int ld, const float* decay, const float* norm_w, float* state, float* scratch, void* out,
+                                const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, float eps, int dtype,
+                                void* workspace, size_t workspace_bytes, void* stream);
+
 /* Router with a score function, expert groups and gate rows. z = router_w h (float32; router_w [R + n_extra, W]).
  * Scores s = softmax(z[0:R]) (score_fn 0) or sigmoid(z[0:R]) (score_fn 1); choice = s + correction (NULL: zeros). The R
  * experts form n_groups equal groups of neighbours; a group's score is the sum of its group_top largest choice scores; only

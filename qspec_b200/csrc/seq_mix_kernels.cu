@@ -306,13 +306,15 @@ window_attn_kernel(const float* __restrict__ qa, long long qa_ts, long long qa_h
 template <typename T>
 __global__ void __launch_bounds__(256)
 hgrn2_gates_kernel(const T* __restrict__ p, int ld, const float* __restrict__ f_b, const float* __restrict__ lower,
-                   float* __restrict__ gates, int HD, long long n) {
+                   float* __restrict__ gates, int HD, int ntok) {
   pdl_enter();
-  for (long long k = (long long)blockIdx.x * 256 + threadIdx.x; k < n; k += (long long)gridDim.x * 256) {
-    const long long t = k / HD;
-    const int c = (int)(k - t * HD);
+  // a thread keeps its column (an index divided by HD per element cost as much as the exponentials)
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= HD) return;
+  const float b = f_b[c], lo = lower[c];
+  for (int t = blockIdx.y; t < ntok; t += gridDim.y) {
     const T* row = p + (size_t)t * ld;
-    const float zq = to_f(row[c]), z = to_f(row[HD + c]) + f_b[c], lo = lower[c];
+    const float zq = to_f(row[c]), z = to_f(row[HD + c]) + b;
     const float om = 1.0f / (1.0f + expf(z));             // 1 - sigmoid(z)
     float* g = gates + (size_t)t * 3 * HD + c;
     g[0] = zq / (1.0f + expf(-zq));
@@ -325,11 +327,11 @@ hgrn2_gates_kernel(const T* __restrict__ p, int ld, const float* __restrict__ f_
 // ---- scalar-decay linear attention: q = silu(zq), k = silu(zk), float32, once per (token, row); gates [ntok][2][H * D] ----
 template <typename T>
 __global__ void __launch_bounds__(256)
-lightning_gates_kernel(const T* __restrict__ p, int ld, float* __restrict__ gates, int HD, long long n) {
+lightning_gates_kernel(const T* __restrict__ p, int ld, float* __restrict__ gates, int HD, int ntok) {
   pdl_enter();
-  for (long long k = (long long)blockIdx.x * 256 + threadIdx.x; k < n; k += (long long)gridDim.x * 256) {
-    const long long t = k / HD;
-    const int c = (int)(k - t * HD);
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= HD) return;
+  for (int t = blockIdx.y; t < ntok; t += gridDim.y) {
     const T* row = p + (size_t)t * ld;
     const float zq = to_f(row[c]), zk = to_f(row[HD + c]);
     float* g = gates + (size_t)t * 2 * HD + c;
@@ -557,6 +559,262 @@ hgrn2_scan_kernel(const T* __restrict__ p, int ld, const float* __restrict__ gat
   }
 }
 
+// ---- the same recurrences over long segments, in chunks that run side by side ---------------------------------------------------------
+// The walk above is a chain: 0.2 us a token whatever the GPU has left. A chunk of C tokens turns the state it starts from into
+// diag(P) S + E (P: product of its decays, E: what its own tokens add), so (1) recurrence_chunk_kernel<.., false> computes E and P of
+// every chunk, (2) recurrence_carry_kernel goes through the chunks of a segment element by element and leaves the state that each starts
+// from, and (3) recurrence_chunk_kernel<.., true> walks every chunk from its state and writes the outputs, normed per head on the way
+// out where the design norms per head. All float32, as in the walk; what changes is the order of products of decays.
+// A CTA holds the whole D x DV state of a (chunk, head) in registers, 16 rows x 4 columns a thread, as pairs of rows: 3 (outputs) or, with
+// a block's decays multiplied into its keys first, 1 (E) packed multiply-adds per pair and token. Blocks of 8 tokens arrive by cp.async,
+// two in flight; the row groups' shares of the outputs meet in shared memory once per block. What bounds it is shared
+// memory: a thread reads 56 floats for 64 elements of state, 90 wavefronts a token and warp in the output pass (73 % of the pipe), above
+// the 384 cycles a token and head that its multiply-adds need.
+// 1500 tokens, 16 heads of 128 x 128, all launches: 325 -> 146 us (gates 13, E 44, carry 9, outputs 89); 2000 tokens, 8 heads of 64 x 64:
+// 481 -> 66 us.
+constexpr int RC_BT = 8;                                     // tokens per block
+
+__device__ __forceinline__ uint64_t rc_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ uint64_t rc_mul(uint64_t a, uint64_t b) { uint64_t r; asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ uint64_t rc_pair(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float2 rc_unpair(uint64_t v) { float2 r; asm("mov.b64 {%0, %1}, %2;\n" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+
+struct RcChunk { int begin, end, first, chunks; TokMeta mt; };   // the segment's first and end row, its first chunk's number, its chunks
+// The segment that chunk b belongs to (or segment `seg` if b < 0), found by the CTA's first warp. false: there is no such chunk.
+__device__ __forceinline__ bool rc_find(const int* __restrict__ meta, const int* __restrict__ seg_starts, int nseg, int ntok, int C, int b, int seg,
+                                        RcChunk* s_chunk, bool* s_found) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int before = 0;
+    bool found = false;
+    for (int s0 = 0; s0 < nseg && !found; s0 += 32) {
+      const int s = s0 + lane;
+      int start = 0, end = 0;
+      if (s < nseg) { start = seg_starts[s]; end = meta[3 * ntok + start]; }
+      const int n = (end - start + C - 1) / C;
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+      }
+      const int first = before + incl - n;
+      const bool me = s < nseg && (b < 0 ? s == seg : b >= first && b < first + n);
+      if (me) {
+        s_chunk->begin = start; s_chunk->end = end; s_chunk->first = first; s_chunk->chunks = n;
+        s_chunk->mt = load_meta(meta, ntok, start);
+      }
+      found = __any_sync(0xffffffffu, me);
+      before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) *s_found = found;
+  }
+  __syncthreads();
+  return *s_found;
+}
+
+template <typename T, int D, int DV, bool OUT>
+__global__ void __launch_bounds__((D / 16) * (DV / 4), 32768 / (D * DV))
+recurrence_chunk_kernel(const T* __restrict__ p, int ld, const float* __restrict__ gates, float* __restrict__ E, float* __restrict__ P,
+                        float* __restrict__ state, float* __restrict__ o, T* __restrict__ out, const float* __restrict__ norm_w, float eps,
+                        const int* __restrict__ meta, const int* __restrict__ seg_starts, int nseg, int ntok, int H, int C,
+                        const float* __restrict__ decay) {
+  pdl_enter();
+  constexpr int RG = D / 16, CG = DV / 4, NT = RG * CG, BT = RC_BT, VPT = BT * DV / NT;
+  extern __shared__ __align__(16) float rc_smem[];
+  float (*sf)[BT][D] = reinterpret_cast<float (*)[BT][D]>(rc_smem);                       // [2] decays
+  float (*sg)[BT][D] = sf + 2;                                                            // [2] what multiplies v
+  float (*sv)[BT][2 * DV] = reinterpret_cast<float (*)[BT][2 * DV]>(sg + 2);              // [2] values, each twice
+  float (*sq)[BT][D] = reinterpret_cast<float (*)[BT][D]>(sv + 2);                        // [2] queries (outputs only)
+  float (*sp)[RG][DV] = reinterpret_cast<float (*)[RG][DV]>(sq + 2);                      // [BT] shares of the outputs
+  __shared__ float sF[D];
+  __shared__ RcChunk s_chunk;
+  __shared__ bool s_found;
+  const int b = blockIdx.x, h = blockIdx.y;
+  if (!rc_find(meta, seg_starts, nseg, ntok, C, b, 0, &s_chunk, &s_found)) return;
+  const int c = b - s_chunk.first;
+  if (!OUT && c == s_chunk.chunks - 1) return;               // nobody starts from where the last chunk ends
+  const int t0 = s_chunk.begin + c * C, t1 = min(t0 + C, s_chunk.end);
+  const int tid = threadIdx.x, rg = tid % RG, cg = tid / RG, HD = H * D;
+  const float dec = decay ? decay[h] : 1.f;
+  const int arrays = decay ? 2 : 3;                           // per token: q | (f) | what multiplies v
+  const float* gq = gates + (size_t)h * D;
+  const T* vp = p + 2 * (size_t)HD + (size_t)h * DV;
+  auto stage = [&](int buf, int tb) {
+#pragma unroll
+    for (int a = OUT ? 0 : 1; a < 3; ++a) {
+      if (a == 1 && decay) continue;
+      float* dst = a == 0 ? &sq[buf][0][0] : a == 1 ? &sf[buf][0][0] : &sg[buf][0][0];
+      const float* src = gq + (size_t)(a == 2 ? arrays - 1 : a) * HD;
+      for (int i = tid; i < BT * D / 4; i += NT) {
+        const int r = i / (D / 4), k = i % (D / 4) * 4;
+        cp_async_16z(dst + r * D + k, src + (size_t)min(tb + r, t1 - 1) * arrays * HD + k, true);
+      }
+    }
+    cp_async_commit();
+  };
+  float vr[VPT];
+  auto fetch_v = [&](int tb) {
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int e = tid + NT * i, t = min(tb + e / DV, t1 - 1);
+      float v = to_f(vp[(size_t)t * ld + e % DV]);
+      if (decay) v = v / (1.0f + expf(-v));                   // the scalar-decay form takes silu(v)
+      vr[i] = v;
+    }
+  };
+  // this thread's rows: 4 rg .. + 3 and the same D / 4, D / 2 and 3 D / 4 further (a load then covers neighbouring 16-byte pieces), as pairs
+  auto row_of = [&](int i) { return (i >> 1) * (D / 4) + 4 * rg + 2 * (i & 1); };
+  uint64_t S[8][4];
+  float* mine = E + ((size_t)b * H + h) * D * DV;             // OUT: the state this chunk starts from
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+    if (OUT) {
+      x = *reinterpret_cast<const float4*>(mine + (size_t)row_of(i) * DV + cg * 4);
+      y = *reinterpret_cast<const float4*>(mine + (size_t)(row_of(i) + 1) * DV + cg * 4);
+    }
+    S[i][0] = rc_pair(x.x, y.x); S[i][1] = rc_pair(x.y, y.y); S[i][2] = rc_pair(x.z, y.z); S[i][3] = rc_pair(x.w, y.w);
+  }
+  float whole = 1.f;                                          // !OUT, thread < D: product of the chunk's decays of row tid
+  stage(0, t0);
+  fetch_v(t0);
+  int buf = 0;
+  for (int tb = t0; tb < t1; tb += BT, buf ^= 1) {
+    const int nb = min(BT, t1 - tb);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int e = tid + NT * i;
+      *reinterpret_cast<float2*>(&sv[buf][e / DV][2 * (e % DV)]) = make_float2(vr[i], vr[i]);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (tb + BT < t1) { stage(buf ^ 1, tb + BT); fetch_v(tb + BT); }
+    if (!OUT) {
+      // keys times the decays that follow them in the block; the block's own decay
+      static_assert(D <= NT, "a thread per row");
+      if (tid < D) {
+        const int d = tid;
+        float f = 1.f;
+        for (int r = nb - 1; r >= 0; --r) {
+          sg[buf][r][d] *= f;
+          f *= decay ? dec : sf[buf][r][d];
+        }
+        sF[d] = f;
+      }
+      __syncthreads();
+      if (tid < D) whole *= sF[tid];
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(&sF[row_of(i)]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { S[i][j] = rc_mul(f.x, S[i][j]); S[i + 1][j] = rc_mul(f.y, S[i + 1][j]); }
+      }
+    }
+    const uint64_t dec2 = rc_pair(dec, dec);
+    for (int r = 0; r < nb; ++r) {
+      uint64_t v2[4], acc[4];
+      {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(&sv[buf][r][8 * cg]), y = *reinterpret_cast<const ulonglong2*>(&sv[buf][r][8 * cg + 4]);
+        v2[0] = x.x; v2[1] = x.y; v2[2] = y.x; v2[3] = y.y;
+      }
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(&sg[buf][r][row_of(i)]);
+        if (OUT) {
+          ulonglong2 f = make_ulonglong2(dec2, dec2);
+          if (!decay) f = *reinterpret_cast<const ulonglong2*>(&sf[buf][r][row_of(i)]);
+          const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&sq[buf][r][row_of(i)]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            S[i][j] = rc_fma(f.x, S[i][j], rc_mul(g.x, v2[j]));
+            S[i + 1][j] = rc_fma(f.y, S[i + 1][j], rc_mul(g.y, v2[j]));
+            acc[j] = i ? rc_fma(q.x, S[i][j], acc[j]) : rc_mul(q.x, S[i][j]);
+            acc[j] = rc_fma(q.y, S[i + 1][j], acc[j]);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            S[i][j] = rc_fma(g.x, v2[j], S[i][j]);
+            S[i + 1][j] = rc_fma(g.y, v2[j], S[i + 1][j]);
+          }
+        }
+      }
+      if (OUT) {
+        const float2 a = rc_unpair(acc[0]), x = rc_unpair(acc[1]), y = rc_unpair(acc[2]), z = rc_unpair(acc[3]);
+        *reinterpret_cast<float4*>(&sp[r][rg][4 * cg]) = make_float4(a.x + a.y, x.x + x.y, y.x + y.y, z.x + z.y);
+      }
+    }
+    if (OUT) {
+      __syncthreads();
+      const int lane = tid & 31;
+      for (int r = tid >> 5; r < nb; r += NT / 32) {          // a warp per token: the sums, and the per-head norm where there is one
+        const size_t at = ((size_t)(tb + r) * H + h) * DV;
+        float x[DV / 32], ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < DV / 32; ++k) {
+          x[k] = 0.f;
+#pragma unroll
+          for (int w = 0; w < RG; ++w) x[k] += sp[r][w][lane + 32 * k];
+          ss += x[k] * x[k];
+        }
+        if (out) {
+          const float rr = 1.0f / sqrtf(warp_xor_sum(ss) / (float)DV + eps);
+#pragma unroll
+          for (int k = 0; k < DV / 32; ++k) out[at + lane + 32 * k] = from_f<T>(x[k] * rr * norm_w[lane + 32 * k]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < DV / 32; ++k) o[at + lane + 32 * k] = x[k];
+        }
+      }
+    }
+  }
+  if (OUT && t1 != s_chunk.end) return;
+  // OUT: the segment's last chunk leaves the state; otherwise E, where the next chunk will look for its state
+  float* dst = OUT ? state + ((size_t)s_chunk.mt.slot * H + h) * D * DV : mine + (size_t)H * D * DV;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 a = rc_unpair(S[i][0]), x = rc_unpair(S[i][1]), y = rc_unpair(S[i][2]), z = rc_unpair(S[i][3]);
+    *reinterpret_cast<float4*>(dst + (size_t)row_of(i) * DV + cg * 4) = make_float4(a.x, x.x, y.x, z.x);
+    *reinterpret_cast<float4*>(dst + (size_t)(row_of(i) + 1) * DV + cg * 4) = make_float4(a.y, x.y, y.y, z.y);
+  }
+  if (!OUT && tid < D) P[((size_t)b * H + h) * D + tid] = whole;
+}
+
+// Through the chunks of a segment, four elements of a head's state per thread: slot c of E holds E of chunk c - 1 and becomes the state
+// that chunk c starts from (slot 0: the state before the step, zero at position 0).
+__global__ void __launch_bounds__(256)
+recurrence_carry_kernel(float* __restrict__ E, const float* __restrict__ P, const float* __restrict__ state, const int* __restrict__ meta,
+                        const int* __restrict__ seg_starts, int nseg, int ntok, int H, int D, int DV, int C) {
+  pdl_enter();
+  __shared__ RcChunk s_chunk;
+  __shared__ bool s_found;
+  if (!rc_find(meta, seg_starts, nseg, ntok, C, -1, blockIdx.x, &s_chunk, &s_found)) return;
+  const int h = blockIdx.y, e = (blockIdx.z * 256 + threadIdx.x) * 4;
+  if (e >= D * DV) return;
+  const size_t step = (size_t)H * D * DV;
+  float4* at = reinterpret_cast<float4*>(E + ((size_t)s_chunk.first * H + h) * D * DV + e);
+  const float* pr = P + ((size_t)s_chunk.first * H + h) * D + e / DV;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (s_chunk.mt.pos > 0) s = *reinterpret_cast<const float4*>(state + ((size_t)s_chunk.mt.slot * H + h) * D * DV + e);
+  at[0] = s;
+  constexpr int AHEAD = 8;
+  float4 x[AHEAD];
+  float f[AHEAD];
+  const int n = s_chunk.chunks;
+  for (int c = 1; c < n; c += AHEAD) {
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+      if (c + i < n) { x[i] = at[(c + i) * (step / 4)]; f[i] = pr[(size_t)(c + i - 1) * H * D]; }
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+      if (c + i < n) {
+        s.x = f[i] * s.x + x[i].x; s.y = f[i] * s.y + x[i].y; s.z = f[i] * s.z + x[i].z; s.w = f[i] * s.w + x[i].w;
+        at[(c + i) * (step / 4)] = s;
+      }
+  }
+}
+
 // Per-head unit-RMS norm with one weight vector shared by the heads: one warp per (token, head); src float32.
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -761,15 +1019,65 @@ extern "C" int qspec_seq_window_attention(const qspec_window_attn_args* a, int d
   return even ? launch_window_attn_n<bf16_t, 2>(a, st) : launch_window_attn_n<bf16_t, 1>(a, st);
 }
 
+// Tokens of a chunk: as many as let the chunks of all heads fill the GPU once, whole blocks, and at least 32 (below that the states on their
+// way through memory cost more than the walk).
+static int rc_chunk_tokens(int ntok, int H, int D, int DV) {
+  const long long slots = (long long)sm_count() * (32768 / (D * DV));
+  const long long c = (((long long)ntok * H + slots - 1) / slots + RC_BT - 1) / RC_BT * RC_BT;
+  return (int)(c < 32 ? 32 : c);
+}
+static bool rc_taken(int nseg, int ntok, int H, int D, int DV) {
+  if (!((D == 64 || D == 128) && (DV == 64 || DV == 128)) || nseg < 1 || sm_count() < 1) return false;
+  // The walk takes 8 us + 0.2 us a token, the chunks' four launches at least 50 us: 200 tokens of 16 heads of 128 x 128 48 against 53 us,
+  // two sequences of 300 of 16 heads of 64 x 64 82 against 52, 600 of 8 heads 86 against 39.
+  return ntok >= 256 * (long long)nseg && ntok >= 2 * (long long)nseg * rc_chunk_tokens(ntok, H, D, DV);
+}
+
+template <typename T, int D, int DV>
+static int launch_recurrence_chunks_d(const T* p, int ld, const float* gates, float* state, float* o, T* out, const float* norm_w, float eps, const int* meta,
+                                      const int* seg_starts, int nseg, int ntok, int H, const float* decay, float* ws, cudaStream_t st) {
+  const int C = rc_chunk_tokens(ntok, H, D, DV), chunks = ntok / C + nseg;
+  float* E = ws;
+  float* P = ws + (size_t)chunks * H * D * DV;
+  const dim3 grid(chunks, H), block((D / 16) * (DV / 4));
+  constexpr size_t smem_e = (size_t)RC_BT * (4 * D + 4 * DV) * sizeof(float), smem_o = smem_e + (size_t)RC_BT * (2 * D + (D / 16) * DV) * sizeof(float);
+  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
+  int dev = 0;
+  QSPEC_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
+    QSPEC_CUDA(cudaFuncSetAttribute(recurrence_chunk_kernel<T, D, DV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o));
+    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
+  launch_pdl(recurrence_chunk_kernel<T, D, DV, false>, grid, block, smem_e, st, p, ld, gates, E, P, state, o, out, norm_w, eps, meta, seg_starts, nseg, ntok, H, C, decay);
+  QSPEC_CHECK_LAUNCH(1);
+  launch_pdl(recurrence_carry_kernel, dim3(nseg, H, (D * DV + 1023) / 1024), dim3(256), 0, st, E, (const float*)P, (const float*)state, meta, seg_starts, nseg,
+             ntok, H, D, DV, C);
+  QSPEC_CHECK_LAUNCH(1);
+  launch_pdl(recurrence_chunk_kernel<T, D, DV, true>, grid, block, smem_o, st, p, ld, gates, E, P, state, o, out, norm_w, eps, meta, seg_starts, nseg, ntok, H, C, decay);
+  QSPEC_CHECK_LAUNCH(1);
+  return QSPEC_OK;
+}
+
+// o: un-normalised float32 outputs, or out (with norm_w): normed per head
+template <typename T>
+static int launch_recurrence_chunks(const void* p, int ld, const float* gates, float* state, float* o, void* out, const float* norm_w, float eps,
+                                    const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, const float* decay, void* ws,
+                                    cudaStream_t st) {
+#define RC_ARGS (const T*)p, ld, gates, state, o, (T*)out, norm_w, eps, meta, seg_starts, nseg, ntok, H, decay, (float*)ws, st
+  if (D == 128) return DV == 128 ? launch_recurrence_chunks_d<T, 128, 128>(RC_ARGS) : launch_recurrence_chunks_d<T, 128, 64>(RC_ARGS);
+  return DV == 128 ? launch_recurrence_chunks_d<T, 64, 128>(RC_ARGS) : launch_recurrence_chunks_d<T, 64, 64>(RC_ARGS);
+#undef RC_ARGS
+}
+
 template <typename T>
 static int launch_hgrn2(const void* p, int ld, const float* f_b, const float* lower, float* state, float* o, float* gates, const int* meta,
-                        const int* seg_starts, int nseg, int ntok, int H, int D, int DV, cudaStream_t st, const float* decay = nullptr) {
-  const long long n = (long long)ntok * H * D;
-  long long blocks = (n + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (decay) launch_pdl(lightning_gates_kernel<T>, dim3((unsigned)blocks), dim3(256), 0, st, (const T*)p, ld, gates, H * D, n);
-  else launch_pdl(hgrn2_gates_kernel<T>, dim3((unsigned)blocks), dim3(256), 0, st, (const T*)p, ld, f_b, lower, gates, H * D, n);
+                        const int* seg_starts, int nseg, int ntok, int H, int D, int DV, cudaStream_t st, const float* decay, void* ws, void* out,
+                        const float* norm_w, float eps) {
+  const unsigned gx = (unsigned)((H * D + 255) / 256), gy = (unsigned)max(1, min(ntok, 148 * 16 / (int)gx));
+  if (decay) launch_pdl(lightning_gates_kernel<T>, dim3(gx, gy), dim3(256), 0, st, (const T*)p, ld, gates, H * D, ntok);
+  else launch_pdl(hgrn2_gates_kernel<T>, dim3(gx, gy), dim3(256), 0, st, (const T*)p, ld, f_b, lower, gates, H * D, ntok);
   QSPEC_CHECK_LAUNCH(1);
+  if (ws) return launch_recurrence_chunks<T>(p, ld, gates, state, o, out, norm_w, eps, meta, seg_starts, nseg, ntok, H, D, DV, decay, ws, st);
   const dim3 grid(seg_starts ? nseg : ntok, H, (DV + 15) / 16);
 #define HG_ARGS dim3(256), 0, st, (const T*)p, ld, (const float*)gates, state, o, meta, seg_starts, ntok, H, D, DV, decay
   // blocks of 16 tokens for prompt portions (fewer barriers and copies per token); 8 for decoding steps, where the state's
@@ -783,9 +1091,20 @@ static int launch_hgrn2(const void* p, int ld, const float* f_b, const float* lo
   return QSPEC_OK;
 }
 
-extern "C" int qspec_seq_hgrn2(const void* p, int ld, const float* f_b, const float* lower, const float* norm_w, float* state,
-                               float* scratch, void* out, const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D,
-                               int DV, float eps, int dtype, void* stream) {
+extern "C" size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV) {
+  if (ntok < 1 || H < 1 || D < 1 || DV < 1 || !rc_taken(nseg, ntok, H, D, DV)) return 0;
+  return (size_t)(ntok / rc_chunk_tokens(ntok, H, D, DV) + nseg) * H * ((size_t)D * DV + D) * sizeof(float);
+}
+
+// The chunk form's buffer, if these sizes take it and the caller brought one that fits (rows are read 16 bytes at a time).
+static void* chunk_workspace(void* ws, size_t bytes, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, const void* scratch, const void* state) {
+  const size_t need = seg_starts && ws ? qspec_seq_recurrence_chunk_bytes(nseg, ntok, H, D, DV) : 0;
+  return need && bytes >= need && (((uintptr_t)ws | (uintptr_t)scratch | (uintptr_t)state) & 15) == 0 ? ws : nullptr;
+}
+
+extern "C" int qspec_seq_hgrn2_chunked(const void* p, int ld, const float* f_b, const float* lower, const float* norm_w, float* state,
+                                       float* scratch, void* out, const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D,
+                                       int DV, float eps, int dtype, void* workspace, size_t workspace_bytes, void* stream) {
   QSPEC_REQUIRE(!seg_starts || (nseg >= 1 && nseg <= ntok) || ntok == 0, QSPEC_ERR_INVALID_ARG, "seq_hgrn2: %d segments for %d tokens", nseg, ntok);
   QSPEC_REQUIRE(p && f_b && lower && norm_w && state && scratch && out && meta, QSPEC_ERR_INVALID_ARG, "seq_hgrn2: null pointer");
   QSPEC_REQUIRE(ntok >= 0 && H > 0 && H <= 65535 && D > 0 && D <= 256 && DV > 0 && DV <= 65535 * 16 && ld >= 2 * H * D + H * DV,
@@ -793,10 +1112,12 @@ extern "C" int qspec_seq_hgrn2(const void* p, int ld, const float* f_b, const fl
   MIX_DTYPE_OK(dtype);
   if (ntok == 0) return QSPEC_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  void* ws = chunk_workspace(workspace, workspace_bytes, seg_starts, nseg, ntok, H, D, DV, scratch, state);
   float* gates = scratch + (size_t)ntok * H * DV;          // scratch: un-normalised outputs, then the gates
-  int s = dtype == QSPEC_DTYPE_F32 ? launch_hgrn2<float>(p, ld, f_b, lower, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st)
-                                   : launch_hgrn2<bf16_t>(p, ld, f_b, lower, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st);
-  if (s) return s;
+  int s = dtype == QSPEC_DTYPE_F32
+              ? launch_hgrn2<float>(p, ld, f_b, lower, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, nullptr, ws, out, norm_w, eps)
+              : launch_hgrn2<bf16_t>(p, ld, f_b, lower, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, nullptr, ws, out, norm_w, eps);
+  if (s || ws) return s;                                    // (chunks leave normed)
   const long long rows = (long long)ntok * H;
   const unsigned blocks = (unsigned)((rows + 3) / 4);
   if (dtype == QSPEC_DTYPE_F32)
@@ -805,6 +1126,12 @@ extern "C" int qspec_seq_hgrn2(const void* p, int ld, const float* f_b, const fl
     launch_pdl(head_norm_kernel<bf16_t>, dim3(blocks), dim3(128), 0, st, (const float*)scratch, norm_w, (bf16_t*)out, rows, DV, eps);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
+}
+
+extern "C" int qspec_seq_hgrn2(const void* p, int ld, const float* f_b, const float* lower, const float* norm_w, float* state,
+                               float* scratch, void* out, const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D,
+                               int DV, float eps, int dtype, void* stream) {
+  return qspec_seq_hgrn2_chunked(p, ld, f_b, lower, norm_w, state, scratch, out, meta, seg_starts, nseg, ntok, H, D, DV, eps, dtype, nullptr, 0, stream);
 }
 
 extern "C" int qspec_seq_side_gate(void* g, const void* table, const int* ids, int col0, int sd, int table_ld, int V, int ntok, int dtype,
@@ -932,9 +1259,9 @@ extern "C" int qspec_seq_silu_mul(const void* gu, int ld, void* out, int ntok, i
   return qspec_seq_glu(gu, ld, out, ntok, F, QSPEC_GLU_SILU, dtype, stream);
 }
 
-extern "C" int qspec_seq_lightning(const void* p, int ld, const float* decay, const float* norm_w, float* state, float* scratch, void* out,
-                                   const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, float eps, int dtype,
-                                   void* stream) {
+extern "C" int qspec_seq_lightning_chunked(const void* p, int ld, const float* decay, const float* norm_w, float* state, float* scratch, void* out,
+                                           const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, float eps, int dtype,
+                                           void* workspace, size_t workspace_bytes, void* stream) {
   QSPEC_REQUIRE(!seg_starts || (nseg >= 1 && nseg <= ntok) || ntok == 0, QSPEC_ERR_INVALID_ARG, "seq_lightning: %d segments for %d tokens", nseg, ntok);
   QSPEC_REQUIRE(p && decay && norm_w && state && scratch && out && meta, QSPEC_ERR_INVALID_ARG, "seq_lightning: null pointer");
   QSPEC_REQUIRE(ntok >= 0 && H > 0 && H <= 65535 && D > 0 && D <= 256 && DV > 0 && DV <= 65535 * 16 && ld >= 2 * H * D + 2 * H * DV,
@@ -943,9 +1270,10 @@ extern "C" int qspec_seq_lightning(const void* p, int ld, const float* decay, co
   if (ntok == 0) return QSPEC_OK;
   cudaStream_t st = (cudaStream_t)stream;
   float* gates = scratch + (size_t)ntok * H * DV;          // scratch: un-normalised outputs, then silu(q) and silu(k)
+  void* ws = chunk_workspace(workspace, workspace_bytes, seg_starts, nseg, ntok, H, D, DV, scratch, state);
   int s = dtype == QSPEC_DTYPE_F32
-              ? launch_hgrn2<float>(p, ld, nullptr, nullptr, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, decay)
-              : launch_hgrn2<bf16_t>(p, ld, nullptr, nullptr, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, decay);
+              ? launch_hgrn2<float>(p, ld, nullptr, nullptr, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, decay, ws, nullptr, nullptr, eps)
+              : launch_hgrn2<bf16_t>(p, ld, nullptr, nullptr, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, decay, ws, nullptr, nullptr, eps);
   if (s) return s;
   const int N = H * DV, goff = 2 * H * D + H * DV;         // the output gate's logits follow q, k and v in the row
   if (dtype == QSPEC_DTYPE_F32)
@@ -956,4 +1284,10 @@ extern "C" int qspec_seq_lightning(const void* p, int ld, const float* decay, co
                (bf16_t*)out, N, eps);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
+}
+
+extern "C" int qspec_seq_lightning(const void* p, int ld, const float* decay, const float* norm_w, float* state, float* scratch, void* out,
+                                   const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, float eps, int dtype,
+                                   void* stream) {
+  return qspec_seq_lightning_chunked(p, ld, decay, norm_w, state, scratch, out, meta, seg_starts, nseg, ntok, H, D, DV, eps, dtype, nullptr, 0, stream);
 }

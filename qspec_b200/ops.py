@@ -1103,6 +1103,13 @@ def seq_window_attention_mma(q: torch.Tensor, cache_k: torch.Tensor, k_shared: O
          "seq_window_attention_mma")
 
 
+def _chunk_workspace(lib, nseg: int, ntok: int, H: int, D: int, DV: int, device) -> Optional[torch.Tensor]:
+    """Room for the states between the chunks of a recurrence over long segments: of the call's own (the caching allocator ties it to
+    the current stream), so that calls on several streams do not meet in it."""
+    nbytes = lib.qspec_seq_recurrence_chunk_bytes(nseg, ntok, H, D, DV) if nseg else 0
+    return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
+
+
 def seq_hgrn2(p: torch.Tensor, f_b: torch.Tensor, lower: torch.Tensor, norm_w: torch.Tensor, state: torch.Tensor, scratch: torch.Tensor,
               out: torch.Tensor, meta: torch.Tensor, H: int, D: int, DV: int, eps: float, seg_starts: Optional[torch.Tensor] = None) -> None:
     """HGRN2 recurrence over rows [zq | zf | v] with the per-slot state float32 [slots, H, D, DV]; out [ntok, H * DV] after the
@@ -1116,9 +1123,11 @@ def seq_hgrn2(p: torch.Tensor, f_b: torch.Tensor, lower: torch.Tensor, norm_w: t
     if out.shape != (ntok, H * DV) or state.shape[1:] != (H, D, DV) or scratch.numel() < ntok * H * (DV + 3 * D) or norm_w.numel() != DV \
             or f_b.numel() != H * D or lower.numel() != H * D:
         raise ValueError("seq_hgrn2: shapes do not match")
-    _seq(_lib.load_seq().qspec_seq_hgrn2(_ptr(p), p.shape[1], _ptr(f_b), _ptr(lower), _ptr(norm_w), _ptr(state), _ptr(scratch), _ptr(out),
-                                         _ptr(meta), _ptr(seg_starts), 0 if seg_starts is None else seg_starts.numel(), ntok, H, D, DV,
-                                         float(eps), _sdt(p), _stream()), "seq_hgrn2")
+    lib, nseg = _lib.load_seq(), 0 if seg_starts is None else seg_starts.numel()
+    ws = _chunk_workspace(lib, nseg, ntok, H, D, DV, p.device)
+    _seq(lib.qspec_seq_hgrn2_chunked(_ptr(p), p.shape[1], _ptr(f_b), _ptr(lower), _ptr(norm_w), _ptr(state), _ptr(scratch), _ptr(out),
+                                     _ptr(meta), _ptr(seg_starts), nseg, ntok, H, D, DV, float(eps), _sdt(p), _ptr(ws),
+                                     0 if ws is None else ws.numel(), _stream()), "seq_hgrn2")
 
 
 def seq_side_gate(g: torch.Tensor, table: torch.Tensor, ids: torch.Tensor, col0: int) -> None:
@@ -1209,9 +1218,11 @@ def seq_lightning(p: torch.Tensor, decay: torch.Tensor, norm_w: torch.Tensor, st
     if out.shape != (ntok, H * DV) or state.shape[1:] != (H, D, DV) or scratch.numel() < ntok * H * (DV + 2 * D) or \
             norm_w.numel() != H * DV or decay.numel() != H or p.shape[1] < 2 * H * (D + DV) or meta.shape != (5, ntok):
         raise ValueError("seq_lightning: shapes do not match")
-    _seq(_lib.load_seq().qspec_seq_lightning(_ptr(p), p.shape[1], _ptr(decay), _ptr(norm_w), _ptr(state), _ptr(scratch), _ptr(out),
-                                             _ptr(meta), _ptr(seg_starts), 0 if seg_starts is None else seg_starts.numel(), ntok, H, D,
-                                             DV, float(eps), _sdt(p), _stream()), "seq_lightning")
+    lib, nseg = _lib.load_seq(), 0 if seg_starts is None else seg_starts.numel()
+    ws = _chunk_workspace(lib, nseg, ntok, H, D, DV, p.device)
+    _seq(lib.qspec_seq_lightning_chunked(_ptr(p), p.shape[1], _ptr(decay), _ptr(norm_w), _ptr(state), _ptr(scratch), _ptr(out), _ptr(meta),
+                                         _ptr(seg_starts), nseg, ntok, H, D, DV, float(eps), _sdt(p), _ptr(ws),
+                                         0 if ws is None else ws.numel(), _stream()), "seq_lightning")
 
 
 def moe_route_grouped(h: torch.Tensor, router_w: torch.Tensor, correction: Optional[torch.Tensor], idx: torch.Tensor,
