@@ -12,6 +12,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("QSPEC_LIB") or os.path.join(_HERE, "_C", "libqspec_b200.so")
 
 QSPEC_OK = 0
+QSPEC_ERR_WORKSPACE = 4
 DTYPE_F16 = 0
 DTYPE_BF16 = 1
 

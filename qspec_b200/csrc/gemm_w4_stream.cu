@@ -1242,11 +1242,10 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   return pl;
 }
 
-static size_t workspace_bytes(int mode, int M, int N, int K) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const Plan pl = make_plan(mode, M, N, K);
+static size_t workspace_bytes(const Plan& pl) {
   return COUNTER_BYTES + 2 * (size_t)pl.G * (pl.pair ? 2 : 1) * pl.slot_bytes;
 }
+static size_t workspace_bytes(int mode, int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? 0 : workspace_bytes(make_plan(mode, M, N, K)); }
 
 template <int MODE, bool PAIR>
 static int launch(const CUtensorMap& mw, const CUtensorMap& ma, const Params& p, const Plan& pl, cudaStream_t st) {
@@ -1294,9 +1293,9 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   QSPEC_REQUIRE(((uintptr_t)act & 15) == 0 && ((uintptr_t)w & 15) == 0, QSPEC_ERR_UNSUPPORTED,
                 "%s: operand pointers must be 16-byte aligned", who);
   if (M == 0) return QSPEC_OK;
-  const size_t need = workspace_bytes(mode, M, N, K);
-  QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
   const Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
+  const size_t need = split_out ? workspace_bytes(mode, M, N, K) : workspace_bytes(pl);
+  QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
   if (split_out) {
     QSPEC_REQUIRE(pl.split >= 1 && pl.tiles_m == 1, QSPEC_ERR_UNSUPPORTED, "%s: no even k-split for M=%d N=%d K=%d", who, M, N, K);
     QSPEC_REQUIRE(split_bytes >= (size_t)pl.split * M * N * 4, QSPEC_ERR_WORKSPACE, "%s: partial buffer too small (%zu < %zu)", who,

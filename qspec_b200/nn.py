@@ -83,6 +83,12 @@ def get_hadK(n: int):
 # Linear4bit  (quarot_nn/linear.py:28-152)
 # ----------------------------------------------------------------------------------------------
 
+def _row_scales(x: "PackedQuantizedTensor") -> torch.Tensor:
+    """The scales of the tensor's rows: the buffer they lie in may be longer or of another shape."""
+    rows, scales = x.quantized_x.shape[0], x.scales_x
+    return scales if scales.dim() == 1 and scales.shape[0] == rows else scales.view(-1)[:rows]
+
+
 class Linear4bit(torch.nn.Module):
     """Symmetric 4-bit linear layer: ONE packed weight serves W4A4 (draft) and W4A16 (verify)."""
 
@@ -113,50 +119,51 @@ class Linear4bit(torch.nn.Module):
         else:
             return self.forward_w4a16(x, C)
 
-    def _lazy_views(self):
-        if self.weight_scales.dim() == 2:                      # linear.py:75-78
-            self.weight_scales = self.weight_scales.view(-1)
-        if self.weight.dtype != torch.int8:
-            self.weight = self.weight.view(torch.int8)
+    def _packed(self):
+        """(weight, weight_scales) as the kernels take them: int8 and flat (linear.py:75-78). Straight from the buffer table where they
+        are buffers: Module.__getattr__ costs half a microsecond a name."""
+        weight, scales = self._buffers.get("weight"), self._buffers.get("weight_scales")
+        if weight is None or scales is None:
+            weight, scales = self.weight, self.weight_scales
+        if scales.dim() == 2:
+            self.weight_scales = scales = scales.view(-1)
+        if weight.dtype != torch.int8:
+            self.weight = weight = weight.view(torch.int8)
+        return weight, scales
 
     def forward_w4a4(self, x, C=None):
         assert type(x) == PackedQuantizedTensor                # linear.py:72
-        xq, scales_x = x.quantized_x, x.scales_x
-        self._lazy_views()
+        xq = x.quantized_x
+        weight, scales = self._packed()
         if C is None:
-            C = torch.empty(xq.shape[0], self.weight.shape[0], dtype=self.weight_scales.dtype, device=xq.device)
-        ops.rowwise_scaled_linear_cutlass_s4s4_unified(xq, scales_x.view(-1)[: xq.shape[0]], self.weight,
-                                                       self.weight_scales, self.bias, C)
+            C = torch.empty(xq.shape[0], weight.shape[0], dtype=scales.dtype, device=xq.device)
+        ops.rowwise_scaled_linear_cutlass_s4s4_unified(xq, _row_scales(x), weight, scales, self.bias, C)
         return C
 
     def forward_w4a8(self, x, C=None):
         """linear.py:86-99: int8 activations (PackedQuantizedTensor carrying [T, K] int8) x the same packed int4 weight."""
         assert type(x) == PackedQuantizedTensor
-        xq, scales_x = x.quantized_x, x.scales_x
-        self._lazy_views()
-        return ops.rowwise_scaled_linear_cutlass_s8s4(xq, scales_x.view(-1)[: xq.shape[0]], self.weight, self.weight_scales,
-                                                      self.bias, C)
+        weight, scales = self._packed()
+        return ops.rowwise_scaled_linear_cutlass_s8s4(x.quantized_x, _row_scales(x), weight, scales, self.bias, C)
 
     def forward_w4a16(self, x, C=None):
-        self._lazy_views()
+        weight, scales = self._packed()
         if C is None:
-            C = torch.empty(x.shape[0], self.weight.shape[0], dtype=x.dtype, device=x.device)
-        ops.gemm_w4a16(x, self.weight, self.weight_scales, self.bias, C)
+            C = torch.empty(x.shape[0], weight.shape[0], dtype=x.dtype, device=x.device)
+        ops.gemm_w4a16(x, weight, scales, self.bias, C)
         return C
 
     def forward_split(self, x, partials, w4a4=False):
         """Deferred reduction (qspec_b200 extension, no reference counterpart): the GEMM leaves its per-k-slice partial
         accumulators in `partials`; ops.split_add_rms_norm_* finishes the epilogue inside the next norm."""
-        self._lazy_views()
+        weight, scales = self._packed()
         if w4a4:
             assert type(x) == PackedQuantizedTensor
             xq = x.quantized_x
-            if xq.shape[-1] == 2 * self.weight.shape[1]:       # int8 container: one int4 value per byte
-                return ops.gemm_w4a4_c8_split(xq, x.scales_x.view(-1)[: xq.shape[0]], self.weight, self.weight_scales,
-                                              self.bias, partials)
-            return ops.gemm_w4a4_split(xq, x.scales_x.view(-1)[: xq.shape[0]], self.weight, self.weight_scales, self.bias,
-                                       partials)
-        return ops.gemm_w4a16_split(x, self.weight, self.weight_scales, self.bias, partials)
+            if xq.shape[-1] == 2 * weight.shape[1]:            # int8 container: one int4 value per byte
+                return ops.gemm_w4a4_c8_split(xq, _row_scales(x), weight, scales, self.bias, partials)
+            return ops.gemm_w4a4_split(xq, _row_scales(x), weight, scales, self.bias, partials)
+        return ops.gemm_w4a16_split(x, weight, scales, self.bias, partials)
 
     @staticmethod
     def from_float(module: torch.nn.Linear, weight_scales=None, **kwargs):

@@ -37,10 +37,12 @@ def _dt(t: torch.Tensor) -> int:
 
 def _stream() -> int:
     # the raw handle of the current stream of the current device, without building a torch.cuda.Stream object per launch
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _chk(t: Optional[torch.Tensor], name: str, dtypes=None, allow_none=False):
+    if t is not None and t.is_cuda and (dtypes is None or t.dtype in dtypes) and t.is_contiguous():
+        return
     if t is None:
         if allow_none:
             return
@@ -79,6 +81,19 @@ def _workspace(kind: str, nbytes: int, device: torch.device) -> torch.Tensor:
         ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
         _workspaces[key] = ws
     return ws
+
+
+def _with_workspace(kind: str, need, shape, device: torch.device, call) -> int:
+    """call(pointer, bytes) with the workspace as it is; where it is too small, once more with one of need(*shape) bytes. (Asking for the
+    size before every call plans every product twice.)"""
+    index = device.index
+    ws = _workspaces.get((kind, index if index is not None else torch.cuda.current_device()))
+    if ws is not None:
+        status = call(ws.data_ptr(), ws.numel())
+        if status != _lib.QSPEC_ERR_WORKSPACE:
+            return status
+    ws = _workspace(kind, need(*shape), device)
+    return call(ws.data_ptr(), ws.numel())
 
 
 def reserve_workspaces(max_tokens: int, shapes, device) -> None:
@@ -346,11 +361,9 @@ def rowwise_scaled_linear_cutlass_s4s4_unified(input: torch.Tensor, input_scale:
         return result
     lib = _lib.load()
     K = 2 * K2
-    need = lib.qspec_gemm_w4a4_workspace_bytes(M, N, K)
-    ws = _workspace("w4a4", need, input.device)
-    _lib.check(lib.qspec_gemm_w4a4(_ptr(input), _ptr(input_scale), _ptr(weight), _ptr(weight_scale), _ptr(bias),
-                                   _ptr(result), M, N, K, _dt(result), _ptr(ws), ws.numel(), _stream()),
-               "rowwise_scaled_linear_cutlass_s4s4_unified")
+    _lib.check(_with_workspace("w4a4", lib.qspec_gemm_w4a4_workspace_bytes, (M, N, K), input.device, lambda ws, n: lib.qspec_gemm_w4a4(
+        input.data_ptr(), input_scale.data_ptr(), weight.data_ptr(), weight_scale.data_ptr(), _ptr(bias), result.data_ptr(), M, N, K,
+        _dt(result), ws, n, _stream())), "rowwise_scaled_linear_cutlass_s4s4_unified")
     return result
 
 
@@ -386,10 +399,9 @@ def gemm_w4a16(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor
     if M == 0:
         return out
     lib = _lib.load()
-    need = lib.qspec_gemm_w4a16_workspace_bytes(M, N, K)
-    ws = _workspace("w4a16", need, x.device)
-    _lib.check(lib.qspec_gemm_w4a16(_ptr(x), _ptr(weight), _ptr(weight_scale), _ptr(bias), _ptr(out), M, N, K,
-                                    _dt(x), _ptr(ws), ws.numel(), _stream()), "gemm_w4a16")
+    _lib.check(_with_workspace("w4a16", lib.qspec_gemm_w4a16_workspace_bytes, (M, N, K), x.device, lambda ws, n: lib.qspec_gemm_w4a16(
+        x.data_ptr(), weight.data_ptr(), weight_scale.data_ptr(), _ptr(bias), out.data_ptr(), M, N, K, _dt(x), ws, n, _stream())),
+        "gemm_w4a16")
     return out
 
 
@@ -455,11 +467,9 @@ def rowwise_scaled_linear_cutlass_s8s4(input: torch.Tensor, input_scale: torch.T
     if M == 0:
         return result
     lib = _lib.load()
-    need = lib.qspec_gemm_w4a8_workspace_bytes(M, N, K)
-    ws = _workspace("w4a4", need, input.device)
-    _lib.check(lib.qspec_gemm_w4a8(_ptr(input), _ptr(input_scale), _ptr(weight), _ptr(weight_scale), _ptr(bias),
-                                   _ptr(result), M, N, K, _dt(result), _ptr(ws), ws.numel(), _stream()),
-               "rowwise_scaled_linear_cutlass_s8s4")
+    _lib.check(_with_workspace("w4a4", lib.qspec_gemm_w4a8_workspace_bytes, (M, N, K), input.device, lambda ws, n: lib.qspec_gemm_w4a8(
+        input.data_ptr(), input_scale.data_ptr(), weight.data_ptr(), weight_scale.data_ptr(), _ptr(bias), result.data_ptr(), M, N, K,
+        _dt(result), ws, n, _stream())), "rowwise_scaled_linear_cutlass_s8s4")
     return result
 
 
