@@ -260,7 +260,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   __shared__ int pos[TOKENS_MAX], seq[TOKENS_MAX];
   __shared__ int s_rs[TOKENS_MAX], s_re[TOKENS_MAX];
   __shared__ uint32_t s_start[TOKENS_MAX / 32];
-  __shared__ __align__(8) uint64_t b_kfull[KS], b_kempty[KS], b_vfull[VS], b_vempty[VS], b_s[2], b_p[2][2], b_o, b_part, b_mx[4];
+  __shared__ __align__(8) uint64_t b_kfull[KS], b_kempty[KS], b_vfull[VS], b_vempty[VS], b_s[2], b_p[2][2], b_o, b_done, b_part, b_mx[4];
   __shared__ float s_mx[2][2][128];                         // [block & 1][half][row]
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_fail;
@@ -310,6 +310,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       bar_init(smem_addr(&b_p[i][0]), 4); bar_init(smem_addr(&b_p[i][1]), 4);
     }
     bar_init(smem_addr(&b_o), 1);
+    bar_init(smem_addr(&b_done), 1);
     bar_init(smem_addr(&b_part), 1);
     for (int i = 0; i < 4; ++i) bar_init(smem_addr(&b_mx[i]), 2);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -383,6 +384,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         }
         if (!ok) break;
         commit(bo);
+        if (n + 1 == blocks) commit(smem_addr(&b_done));
         commit(smem_addr(&b_vempty[n % VS]));
       }
     }
@@ -536,7 +538,8 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       ++n;
     }
     // ---- the last product is done: add the halves' sums, divide, gate, store
-    if (ok && n) ok = bar_wait(smem_addr(&b_o), (uint32_t)((n - 1) & 1), &s_fail);
+    // (A barrier of its own: a warp may get here two products ahead, where the parity of b_o's phase n - 3 reads like that of n - 1.)
+    if (ok && n) ok = bar_wait(smem_addr(&b_done), 0, &s_fail);
     ok = __all_sync(0xffffffffu, ok);
     fence_after();
     s_mx[n & 1][h][r] = l;

@@ -89,6 +89,21 @@ def test_a_token_sees_nothing_but_its_own_keys(ops):
     assert not torch.isfinite(out[60:].view(40, 32, 128)[..., 5]).any()
 
 
+def test_values_that_arrive_late(ops):
+    """Caches that no kernel has read yet and an L2 full of something else: the last blocks' values come from DRAM, after the weights they
+    are multiplied with. The outputs wait for both of the products that can then still be under way."""
+    Hq, Hkv, S, n = 32, 8, 1200, 160
+    junk = torch.empty(300 << 20, dtype=torch.uint8, device="cuda")
+    for i in range(48):
+        qkv, ck, cv, pos, seq = batch([(0, 1000, n)], Hq, Hkv, S, 1, seed=i)
+        junk.fill_(i)
+        out = torch.empty(n, Hq * 128, dtype=torch.float16, device="cuda")
+        ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 128 ** -0.5)
+        first = out.clone()
+        ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 128 ** -0.5)
+        assert torch.equal(first, out), i
+
+
 def test_positions_outside_the_cache(ops):
     """seq_attention shows such a token every row of the cache (past its end) or none (before its start: zeros), decode_attention does
     not store it; neither reads outside."""
