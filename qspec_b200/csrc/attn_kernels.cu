@@ -538,18 +538,24 @@ static int launch_attn_block(const void* qkv, const void* cos_sin, const int* po
 }
 
 // ------------------------------------------------------------------------------------------
-// Attention for passes with MANY sequences (BASELINE configs[2]/[3]: 64 / 32 concurrent sequences; verify passes of
+// Attention for passes with MANY sequences (32 and 64 concurrent sequences are typical; verify passes of
 // (k + 1) tokens per sequence): one 128-thread CTA per (sequence, kv head) reads that head's key and value rows ONCE
 // for all tokens of the sequence in the pass and all G query heads of the GQA group (decode_attention_kernel reads them
 // once per (token, query head): 16x the cache traffic at G = 4, k + 1 = 4), and does the arithmetic on the tensor
 // cores (mma.sync m16n8k16, f16 operands, fp32 accumulate) -- on CUDA cores the same loop is issue-bound at ~45-70 us
-// for 64 sequences (profiles/r02g_notes.md).
+// for 64 sequences.
 //   * 16 query rows per chunk = R tokens x G heads (R = 16 / G). The 4 warps split the keys; every warp runs a
 //     flash-decoding loop over 16-key blocks with an online softmax, then the warps' (max, sum, O) are merged in shared memory.
-//   * No shared-memory staging of K / V: the fragments are loaded straight from the cache with 128-bit loads by permuting
-//     the reduction index (QK^T: lane (gid, tig) takes dims [32 tig, 32 tig + 32) of key row gid -- both operands use the
-//     same permutation, so the dot products are unchanged) and the output index (P.V: n-tile t of lane gid is dim
-//     16 gid + t, so a lane needs 32 contiguous bytes of 4 value rows and ends up holding 32 contiguous output dims).
+//   * Keys and values come by bulk copies, one per 256-byte row, into a ring of ST 16-key blocks per warp: a block's successor in its place
+//     is asked for as soon as its keys (values) are multiplied. Loaded straight into the fragments, 16-byte pieces of 32 different sectors
+//     per instruction kept the L1 at 71 % and a warp waited for every block; prefetching into the L2 made that slower. ST = 1 leaves room for
+//     four CTAs per SM, so that 64 sequences x 8 heads fit the GPU at once; ST = 2 (two CTAs) is for fewer, whose loads have to hide behind
+//     their own work, with eight warps per CTA instead of four once an SM each is left for them (us; before = loads into the fragments;
+//     32 query heads): 64 x 4 tokens after 900 51 (ST 2: 61; before: 54), 20 x 4 after 2000 69 (ST 1: 73; before: 88), 33 x 1 after 1000
+//     39 (41; 50), 8 x 5 after 1900 72 (ST 1: 125, ST 2 with four warps: 118; before: 104).
+//     The rows are padded so that the fragment reads are free of bank conflicts, and the fragments are met without a transposition by
+//     permuting the reduction index (QK^T: lane (gid, tig) takes dims [32 i + 8 tig, + 8), i < 4, of key row gid -- both operands use the same
+//     permutation) and the output index (P.V: n-tiles t and 8 + t of lane gid are dims 8 gid + t and 64 + 8 gid + t).
 //   * Accuracy is fp32-like although the operands are f16: q and k ARE f16 (products exact, fp32 accumulate; the softmax
 //     scale is applied to the fp32 scores), and the probabilities enter P.V as a two-term f16 split P = P_hi + P_lo.
 // qkv holds the ROTATED queries (rope_kvcache ran before), the cache already contains this pass's keys / values.
@@ -571,26 +577,35 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t& hi, uint32_
   lo = pack_h2(x - hf.x, y - hf.y);
 }
 
-constexpr int SEQ_ATTN_WARPS = 4;                          // warps of a CTA that split the keys of one (sequence, kv head)
+constexpr int SEQ_KS = 256 + 64, SEQ_VS = 256 + 16;         // bytes between the rows of a block in shared memory
+constexpr int SEQ_BLOCK = 16 * (SEQ_KS + SEQ_VS);           // 16 keys and values
 
-template <int G>
-__global__ void __launch_bounds__(SEQ_ATTN_WARPS * 32, 4)
+template <int G, int ST, int NW>                              // NW warps split the keys of one (sequence, kv head)
+__global__ void __launch_bounds__(NW * 32, ST == 1 ? 4 : NW == 4 ? 2 : 1)
 seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ cache_k, const __half* __restrict__ cache_v,
                      const int* __restrict__ positions, const int* __restrict__ seq_ids, __half* __restrict__ out,
                      int T, int Hq, int Hkv, int S, float sm_scale, int min_run) {
   pdl_enter();
-  constexpr int D = 128, R = 16 / G, NW = SEQ_ATTN_WARPS;    // R tokens x G heads <= 16 query rows per chunk; NW warps split the keys
+  constexpr int D = 128, R = 16 / G;                         // R tokens x G heads <= 16 query rows per chunk
   __shared__ int s_tok[1024];                                // tokens of this sequence in the pass (T <= 1024)
   __shared__ int s_pos[1024];                                // ... and their positions (loaded in the same round trip as the scan)
   __shared__ int s_ntok;
   __shared__ float s_m[NW][16], s_l[NW][16];
   __shared__ __align__(16) uint4 s_qf[8][32];                // Q fragments of the chunk in mma order: [k-step][lane] = (a0, a1, a2, a3)
-  extern __shared__ __align__(16) unsigned char seq_dyn[];
-  float (*s_o)[16][D] = reinterpret_cast<float (*)[16][D]>(seq_dyn);   // [NW][16][D] fp32: per-warp partial outputs (64 KB)
+  __shared__ __align__(8) uint64_t s_full[NW][2][ST];         // keys, values of a warp's blocks
+  __shared__ volatile int s_fail;                            // a bounded wait ran out: nothing is stored
+  extern __shared__ __align__(16) unsigned char seq_dyn[];   // [NW][ST] blocks; after the keys:
+  constexpr int OS = D + 4;                                  // (row stride of the partial outputs: the rows of a store fall on different banks)
+  float (*s_o)[16][OS] = reinterpret_cast<float (*)[16][OS]>(seq_dyn);   // [NW][16][OS] fp32: per-warp partial outputs
   const int seq = blockIdx.x / Hkv, hk = blockIdx.x % Hkv;    // the heads of a sequence side by side: their rows are neighbours in the cache
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
-  if (tid == 0) s_ntok = 0;
+  if (tid == 0) {
+    s_ntok = 0;
+    s_fail = 0;
+    for (int i = 0; i < NW * 2 * ST; ++i) atile::bar_init(atile::smem_addr(&s_full[0][0][0] + i), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
   __syncthreads();
   for (int t = tid; t < T; t += NW * 32) {
     const int sq = __ldg(seq_ids + t), ps = __ldg(positions + t);
@@ -623,6 +638,18 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   const __half* kbase = cache_k + ((size_t)seq * S * Hkv + hk) * D;
   const __half* vbase = cache_v + ((size_t)seq * S * Hkv + hk) * D;
   const size_t kv_stride = (size_t)Hkv * D;                  // elements between consecutive positions
+  unsigned char* ring = seq_dyn + (size_t)warp * ST * SEQ_BLOCK;   // this warp's blocks: 16 key rows, 16 value rows each
+  uint32_t blocks = 0;                                       // blocks this warp has consumed: place and phase in the ring
+  // rows kb .. of the keys or of the values into place `at` of the ring, one row per lane
+  auto fetch = [&](bool values, uint32_t at, int kb, int nkeys) {
+    const uint32_t bar = atile::smem_addr(&s_full[warp][values][at]);
+    const int n = min(16, nkeys - kb);
+    if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"((uint32_t)n * 256u) : "memory");
+    __syncwarp();
+    if (lane < n)
+      bulk_row_256(atile::smem_addr(ring) + at * SEQ_BLOCK + (values ? 16 * SEQ_KS + lane * SEQ_VS : lane * SEQ_KS),
+                   (values ? vbase : kbase) + (size_t)(kb + lane) * kv_stride, bar);
+  };
   for (int c0 = 0; c0 < ntok; c0 += R) {
     const int nr = min(R, ntok - c0);
     // rows gid and gid + 8 of this lane: (token slot, head) and the position limit of the row (-1 = padding row)
@@ -634,56 +661,55 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) pmax = max(pmax, __shfl_xor_sync(0xffffffffu, pmax, off));
     const int nkeys = min(pmax + 1, S);
-    // ---- Q fragments: dims [32 tig, 32 tig + 32) of rows gid / gid + 8 (zero for padding rows). Identical for every warp:
+    // ---- Q fragments: dims [32 i + 8 tig, + 8) of rows gid / gid + 8 (zero for padding rows). Identical for every warp:
     // warp 0 loads them and leaves them in shared memory in mma order (registers are needed for the accumulators).
-    __syncthreads();                                         // the previous chunk is done with s_qf
+    __syncthreads();                                         // the previous chunk is done with s_qf and with its partial outputs
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+#pragma unroll
+    for (uint32_t i = 0; i < ST; ++i) {
+      const int kb = (warp + (int)i * NW) * 16;
+      if (kb < nkeys) {
+        fetch(false, (blocks + i) % ST, kb, nkeys);
+        fetch(true, (blocks + i) % ST, kb, nkeys);
+      }
+    }
     if (warp == 0) {
       const uint4 z = make_uint4(0, 0, 0, 0);
-      const uint4* pa = tokA >= 0 ? reinterpret_cast<const uint4*>(qkv + (size_t)tokA * row_elems + (size_t)(hk * G + gA) * D + tig * 32) : nullptr;
-      const uint4* pb = tokB >= 0 ? reinterpret_cast<const uint4*>(qkv + (size_t)tokB * row_elems + (size_t)(hk * G + gB) * D + tig * 32) : nullptr;
+      const uint4* pa = tokA >= 0 ? reinterpret_cast<const uint4*>(qkv + (size_t)tokA * row_elems + (size_t)(hk * G + gA) * D) + tig : nullptr;
+      const uint4* pb = tokB >= 0 ? reinterpret_cast<const uint4*>(qkv + (size_t)tokB * row_elems + (size_t)(hk * G + gB) * D) + tig : nullptr;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {                          // 16-byte piece i holds the words of k-steps 2 i and 2 i + 1
-        const uint4 va = pa ? __ldg(pa + i) : z, vb = pb ? __ldg(pb + i) : z;
+        const uint4 va = pa ? __ldg(pa + 4 * i) : z, vb = pb ? __ldg(pb + 4 * i) : z;
         s_qf[2 * i][lane] = make_uint4(va.x, vb.x, va.y, vb.y);
         s_qf[2 * i + 1][lane] = make_uint4(va.z, vb.z, va.w, vb.w);
       }
     }
     __syncthreads();
-    float o[16][4];                                          // n-tile t: (row gid: dims 32 tig + t, 32 tig + 16 + t), (row gid + 8: same)
+    float o[16][4];                                          // n-tile t < 8: (row gid: dims 16 tig + t, 16 tig + 8 + t), (row gid + 8: same); 8 + t: 64 dims further
 #pragma unroll
     for (int t = 0; t < 16; ++t) { o[t][0] = 0.f; o[t][1] = 0.f; o[t][2] = 0.f; o[t][3] = 0.f; }
     float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;
     // this warp's keys: blocks of 16, interleaved over the warps
     for (int kb = warp * 16; kb < nkeys; kb += NW * 16) {
-      // ---- loads of the block: K rows kb + gid, kb + 8 + gid (64 B each), V rows kb + 2 tig (+1), kb + 8 + 2 tig (+1) (32 B each)
-      // (requesting a warp's first block before the Q fragments are staged was tried: the 16 vectors do not fit the 128 registers
-      // beside the 64 accumulators across the staging -- ~200 bytes of spills)
-      uint4 k0[4], k1[4], v[4][2];
-      {
-        const int j0 = min(kb + gid, nkeys - 1), j1 = min(kb + 8 + gid, nkeys - 1);
-        const uint4* p0 = reinterpret_cast<const uint4*>(kbase + (size_t)j0 * kv_stride + tig * 32);
-        const uint4* p1 = reinterpret_cast<const uint4*>(kbase + (size_t)j1 * kv_stride + tig * 32);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { k0[i] = __ldg(p0 + i); k1[i] = __ldg(p1 + i); }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int jv = min(kb + (i >> 1) * 8 + 2 * tig + (i & 1), nkeys - 1);
-          const uint4* pv = reinterpret_cast<const uint4*>(vbase + (size_t)jv * kv_stride + gid * 16);
-          v[i][0] = __ldg(pv); v[i][1] = __ldg(pv + 1);
-        }
-      }
+      const int next = kb + ST * NW * 16;                    // the block that takes this one's place
+      const uint32_t at = blocks % ST, phase = (blocks / ST) & 1;
+      const unsigned char* blk = ring + at * SEQ_BLOCK;
+      unsigned char* blv = ring + at * SEQ_BLOCK + 16 * SEQ_KS;
+      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][0][at]), phase, &s_fail))) break;
       // ---- S = Q K^T for the two 8-key tiles
       float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-      {
-        const uint32_t* w0 = reinterpret_cast<const uint32_t*>(k0);
-        const uint32_t* w1 = reinterpret_cast<const uint32_t*>(k1);
 #pragma unroll
-        for (int st = 0; st < 8; ++st) {
-          const uint4 a = s_qf[st][lane];
-          mma16816(s0, a.x, a.y, a.z, a.w, w0[2 * st], w0[2 * st + 1]);
-          mma16816(s1, a.x, a.y, a.z, a.w, w1[2 * st], w1[2 * st + 1]);
-        }
+      for (int i = 0; i < 4; ++i) {
+        const uint4 k0 = *reinterpret_cast<const uint4*>(blk + gid * SEQ_KS + i * 64 + tig * 16);
+        const uint4 k1 = *reinterpret_cast<const uint4*>(blk + (gid + 8) * SEQ_KS + i * 64 + tig * 16);
+        const uint4 a = s_qf[2 * i][lane], c = s_qf[2 * i + 1][lane];
+        mma16816(s0, a.x, a.y, a.z, a.w, k0.x, k0.y);
+        mma16816(s1, a.x, a.y, a.z, a.w, k1.x, k1.y);
+        mma16816(s0, c.x, c.y, c.z, c.w, k0.z, k0.w);
+        mma16816(s1, c.x, c.y, c.z, c.w, k1.z, k1.w);
       }
+      __syncwarp();
+      if (next < nkeys) fetch(false, at, next, nkeys);
       // ---- scale, mask (key j <= position of the row), online softmax
       const int j00 = kb + 2 * tig, j10 = kb + 8 + 2 * tig;
       float pA[4], pB[4];                                    // row gid: keys j00, j00 + 1, j10, j10 + 1; row gid + 8 likewise
@@ -711,29 +737,47 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
       uint32_t ah[4], al[4];
       split_h2(pA[0], pA[1], ah[0], al[0]); split_h2(pB[0], pB[1], ah[1], al[1]);
       split_h2(pA[2], pA[3], ah[2], al[2]); split_h2(pB[2], pB[3], ah[3], al[3]);
-#pragma unroll
-      for (int t = 0; t < 16; ++t) {
-        const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
-        const uint32_t* x0 = reinterpret_cast<const uint32_t*>(&v[0][0]);   // 8 words: dims 16 gid + 2 w, + 1 of value row kb + 2 tig
-        const uint32_t* x1 = reinterpret_cast<const uint32_t*>(&v[1][0]);
-        const uint32_t* x2 = reinterpret_cast<const uint32_t*>(&v[2][0]);
-        const uint32_t* x3 = reinterpret_cast<const uint32_t*>(&v[3][0]);
-        const uint32_t b0 = __byte_perm(x0[t >> 1], x1[t >> 1], sel), b1 = __byte_perm(x2[t >> 1], x3[t >> 1], sel);
-        mma16816(o[t], ah[0], ah[1], ah[2], ah[3], b0, b1);
-        mma16816(o[t], al[0], al[1], al[2], al[3], b0, b1);
+      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][1][at]), phase, &s_fail))) break;
+      if (kb + 16 > nkeys) {                                 // rows past the last key: their weights are zero, their values must be finite
+        for (int i = (nkeys - kb) * 16 + lane; i < 256; i += 32) *reinterpret_cast<uint4*>(blv + (i >> 4) * SEQ_VS + (i & 15) * 16) = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();                                        // (a warp's last block: the barrier before the next chunk's copies follows)
       }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {                          // value rows 2 tig, + 1, + 8, + 9: dims 8 gid .. + 7, and 64 further
+        uint4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          v[i] = *reinterpret_cast<const uint4*>(blv + ((i >> 1) * 8 + 2 * tig + (i & 1)) * SEQ_VS + h * 128 + gid * 16);
+        const uint32_t x0[4] = {v[0].x, v[0].y, v[0].z, v[0].w}, x1[4] = {v[1].x, v[1].y, v[1].z, v[1].w};
+        const uint32_t x2[4] = {v[2].x, v[2].y, v[2].z, v[2].w}, x3[4] = {v[3].x, v[3].y, v[3].z, v[3].w};
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
+          const uint32_t b0 = __byte_perm(x0[t >> 1], x1[t >> 1], sel), b1 = __byte_perm(x2[t >> 1], x3[t >> 1], sel);
+          mma16816(o[h * 8 + t], ah[0], ah[1], ah[2], ah[3], b0, b1);
+          mma16816(o[h * 8 + t], al[0], al[1], al[2], al[3], b0, b1);
+        }
+      }
+      ++blocks;
+      __syncwarp();
+      if (next < nkeys) fetch(true, at, next, nkeys);
     }
     // ---- quad-reduce the row sums, publish this warp's (m, l, O)
     lA += __shfl_xor_sync(0xffffffffu, lA, 1); lA += __shfl_xor_sync(0xffffffffu, lA, 2);
     lB += __shfl_xor_sync(0xffffffffu, lB, 1); lB += __shfl_xor_sync(0xffffffffu, lB, 2);
-    __syncthreads();                                         // the previous chunk's merge is done with shared memory
+    __syncthreads();                                         // every warp is done with its blocks, where the partial outputs go
     if (tig == 0) { s_m[warp][gid] = mA; s_l[warp][gid] = lA; s_m[warp][gid + 8] = mB; s_l[warp][gid + 8] = lB; }
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
-      s_o[warp][gid][32 * tig + t] = o[t][0];      s_o[warp][gid][32 * tig + 16 + t] = o[t][1];
-      s_o[warp][gid + 8][32 * tig + t] = o[t][2];  s_o[warp][gid + 8][32 * tig + 16 + t] = o[t][3];
+      const int d = (t & 8) * 8 + 16 * tig + (t & 7);
+      s_o[warp][gid][d] = o[t][0];      s_o[warp][gid][d + 8] = o[t][1];
+      s_o[warp][gid + 8][d] = o[t][2];  s_o[warp][gid + 8][d + 8] = o[t][3];
     }
     __syncthreads();
+    if (s_fail) {                                            // (written before the barrier: uniform)
+      if (tid == 0) atomicAdd(&atile::attn_tile_timeouts, 1u);
+      return;
+    }
     // ---- merge the warps: thread = (row r, 16 dims); out = sum_w e^{m_w - m} O_w / sum_w e^{m_w - m} l_w
     for (int item = tid; item < 16 * 8; item += NW * 32) {
       const int r = item >> 3, dq = item & 7;
@@ -764,20 +808,33 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   }
 }
 
-template <int G>
-static int launch_seq_attention(const void* qkv, const void* ck, const void* cv, const int* positions, const int* seq_ids,
+template <int G, int ST, int NW>
+static int launch_seq_attention_st(const void* qkv, const void* ck, const void* cv, const int* positions, const int* seq_ids,
                                 void* out, int T, int B, int Hq, int Hkv, int S, float sm_scale, int min_run, cudaStream_t st) {
-  constexpr size_t dyn = (size_t)SEQ_ATTN_WARPS * 16 * 128 * sizeof(float);
-  auto kern = seq_attention_kernel<G>;
+  constexpr size_t dyn = (size_t)NW * ST * SEQ_BLOCK;
+  static_assert(SEQ_BLOCK >= 16 * (128 + 4) * (int)sizeof(float), "the partial outputs lie in the blocks");
+  auto kern = seq_attention_kernel<G, ST, NW>;
   static bool attr_set = false;                              // per instantiation
   if (!attr_set) {
     QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     attr_set = true;
   }
-  launch_pdl(kern, dim3(B * Hkv), dim3(SEQ_ATTN_WARPS * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
+  launch_pdl(kern, dim3(B * Hkv), dim3(NW * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
              positions, seq_ids, (__half*)out, T, Hq, Hkv, S, sm_scale, min_run);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
+}
+
+template <int G>
+static int launch_seq_attention(const void* qkv, const void* ck, const void* cv, const int* positions, const int* seq_ids, void* out, int T, int B, int Hq,
+                                int Hkv, int S, float sm_scale, int min_run, cudaStream_t st) {
+  // CTAs with work: at most one per (sequence with a token, kv head)
+  const long long ctas = (long long)min(B, T) * Hkv;
+#define SEQ_ARGS qkv, ck, cv, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, min_run, st
+  if (ctas <= sm_count()) return launch_seq_attention_st<G, 2, 8>(SEQ_ARGS);
+  if (2 * ctas <= 5ll * sm_count()) return launch_seq_attention_st<G, 2, 4>(SEQ_ARGS);
+  return launch_seq_attention_st<G, 1, 4>(SEQ_ARGS);
+#undef SEQ_ARGS
 }
 
 // Prompt portions of the int4 decoder's attention. Runs of at least RUN tokens (one sequence, consecutive positions) go to
