@@ -307,7 +307,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     for (int i = 0; i < VS; ++i) { bar_init(smem_addr(&b_vfull[i]), 1); bar_init(smem_addr(&b_vempty[i]), 1); }
     for (int i = 0; i < 2; ++i) {
       bar_init(smem_addr(&b_s[i]), 1);
-      bar_init(smem_addr(&b_p[i][0]), 4); bar_init(smem_addr(&b_p[i][1]), 4);
+      bar_init(smem_addr(&b_p[i][0]), 8); bar_init(smem_addr(&b_p[i][1]), 4);
     }
     bar_init(smem_addr(&b_o), 1);
     bar_init(smem_addr(&b_done), 1);
@@ -501,7 +501,15 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
             st32(ot + q * 32, o);
           }
+          wait_st();
         }
+      }
+      // The product of the first 64 keys adds to all columns of O, those of the second half's warps among them: b_p[.][0] counts their
+      // rescale, done or not needed, beside the first half's weights.
+      if (h) {
+        fence_before();
+        __syncwarp();
+        if (lane == 0) bar_arrive(smem_addr(&b_p[n & 1][0]));
       }
       const float mu = m == -INFINITY ? 0.f : m;
       const uint64_t c22 = pair(__float_as_uint(c2), __float_as_uint(c2)), mu2 = pair(__float_as_uint(-mu), __float_as_uint(-mu));

@@ -43,6 +43,14 @@ def check(got, want):
     assert err <= 2 ** -10 * want.abs().max().item(), err
 
 
+def check_rows(got, want, Hq, most):
+    """Every (token, head) by itself: half a unit in the last place of float16 of its largest value, and 2^-16 of the largest value in the
+    cache, `most`: scores of up to 2^7 (units of log2) carry an error of a few 2^-17 out of float32 sums, and so do their weights."""
+    err = (got.double() - want).abs().view(-1, Hq, 128).amax(2)
+    bound = 2 ** -11 * want.abs().view(-1, Hq, 128).amax(2) + 2 ** -16 * most
+    assert (err <= bound).all(), (err / bound).max().item()
+
+
 CASES = [
     (32, 8, 300, [(0, 0, 64)]),                                   # one tile pair, exactly one block
     (32, 8, 300, [(1, 0, 129)]),                                  # a block and one key; tokens of three CTAs
@@ -102,6 +110,32 @@ def test_values_that_arrive_late(ops):
         first = out.clone()
         ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 128 ** -0.5)
         assert torch.equal(first, out), i
+
+
+@pytest.mark.parametrize("Hq,Hkv,segments", [
+    (32, 8, [(0, 1900, 96)]),                                     # 16 blocks, the maximum moves in each
+    (32, 8, [(0, 1000, 16), (1, 1500, 16), (2, 700, 40)]),        # two runs in a tile: the second's rows start when the first's are done
+    (8, 8, [(1, 1400, 129), (0, 900, 127)]),
+])
+def test_the_maximum_moves_in_every_block(ops, Hq, Hkv, segments):
+    """Scores that rise by more than the rescale threshold (8 in units of log2) from block to block: the outputs so far are scaled before
+    each product. A product that did not wait for every warp's part of that shows in the rows against float64, or between repetitions."""
+    S, nseq, scale = 2048, 1 + max(s for s, _, _ in segments), 128 ** -0.5
+    qkv, ck, cv, pos, seq = batch(segments, Hq, Hkv, S, nseq, seed=7)
+    direction = torch.randn(128, generator=torch.Generator(device="cuda").manual_seed(8), device="cuda")
+    direction /= direction.norm()
+    score = (torch.arange(S, device="cuda") - S / 2) * (8.3 / 128)                     # 8.3 (12 in units of log2) a block
+    qkv[:, :Hq * 128] = (qkv[:, :Hq * 128].view(-1, Hq, 128) * 0.3 + 40 * direction).half().view(-1, Hq * 128)
+    ck.copy_((ck * 0.3 + (score / (40 * scale))[None, :, None, None] * direction).half())
+    first = None
+    for _ in range(300):
+        out = torch.full((len(pos), Hq * 128), float("nan"), dtype=torch.float16, device="cuda")
+        ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, scale)
+        if first is None:
+            first = out
+        assert torch.equal(first, out)
+    check_rows(first, reference(qkv, ck, cv, pos, seq, Hq, Hkv, scale), Hq, cv.abs().max().item())
+    assert ops.attn_tile_timeouts() == 0
 
 
 def test_positions_outside_the_cache(ops):
