@@ -21,8 +21,9 @@
 // tokens. A CTA walks the runs of its tokens one after the other (rows of other runs are masked). Tokens outside such runs are left
 // to the caller's other kernel (attn_in_run is the common test).
 //
-// A weight of zero times a value that is not finite would be NaN: rows with a result that is not finite are computed again key by
-// key (attn_row_again), so that a row sees nothing but its own keys.
+// A row sees nothing but its own keys, bit for bit: hidden keys enter the products with weights of exactly zero, and a row is rescaled by
+// its own maximum alone. A weight of zero times a value that is not finite would be NaN: rows with a result that is not finite are computed
+// again key by key (attn_row_again).
 //
 // Every wait is bounded; a CTA whose wait runs out counts itself in attn_tile_timeouts, frees its tensor memory and leaves without
 // storing.
@@ -163,19 +164,28 @@ __device__ __forceinline__ void unpair(uint64_t v, uint32_t& a, uint32_t& b) { a
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b)); return r; }
 
-// lead(): the leading bits of two weights (bits of float32, 0 <= weight < 2^15), packed, and their values; rest(): two remainders, packed.
-// Mostly on the integer units: the conversion instruction shares the special-function unit with the exponentials (with conversions for
-// both terms that unit was 95 % busy and the kernel waited for it).
+// lead(): the leading bits of two weights (bits of float32, 0 <= weight < 2^15), rounded and packed, and their values; rest(): two
+// remainders, packed. Mostly on the integer units: the conversion instruction shares the special-function unit with the exponentials (with
+// conversions for both terms that unit was 95 % busy and the kernel waited for it). ZEROS: whether lead() and rest() give zero for a weight
+// of zero; lead_zero() does in any case.
 template <bool BF> struct Elem;
 template <> struct Elem<false> {
   using T = __half;
   static __device__ __forceinline__ uint32_t pack(float a, float b) { const __half2 h = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
   static __device__ __forceinline__ float2 unpack(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+  static constexpr bool ZEROS = false;
   // weights below 2^-14, the smallest normal number, give 2^-14: their remainder is negative
   static __device__ __forceinline__ uint32_t lead(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
-    h0 = max(p0, 0x38800000u) & 0xffffe000u;
-    h1 = max(p1, 0x38800000u) & 0xffffe000u;
+    h0 = __viaddmax_u32(p0, 0x1000u, 0x38800000u) & 0xffffe000u;
+    h1 = __viaddmax_u32(p1, 0x1000u, 0x38800000u) & 0xffffe000u;
     return (h0 >> 13) + (h1 << 3) - 0xc001c000u;           // exponent bias 127 -> 15 in both halves
+  }
+  static __device__ __forceinline__ uint32_t lead_zero(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
+    const uint32_t w = pack(__uint_as_float(p0), __uint_as_float(p1));
+    const float2 f = unpack(w);
+    h0 = __float_as_uint(f.x);
+    h1 = __float_as_uint(f.y);
+    return w;
   }
   static __device__ __forceinline__ uint32_t rest(uint32_t q0, uint32_t q1) { return pack(__uint_as_float(q0), __uint_as_float(q1)); }
 };
@@ -183,11 +193,15 @@ template <> struct Elem<true> {
   using T = __nv_bfloat16;
   static __device__ __forceinline__ uint32_t pack(float a, float b) { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
   static __device__ __forceinline__ float2 unpack(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+  static constexpr bool ZEROS = true;
   static __device__ __forceinline__ uint32_t lead(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
+    p0 += 0x8000u;
+    p1 += 0x8000u;
     h0 = p0 & 0xffff0000u;
     h1 = p1 & 0xffff0000u;
     return __byte_perm(p0, p1, 0x7632);
   }
+  static __device__ __forceinline__ uint32_t lead_zero(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) { return lead(p0, p1, h0, h1); }
   static __device__ __forceinline__ uint32_t rest(uint32_t q0, uint32_t q1) { return __byte_perm(q0 + 0x8000u, q1 + 0x8000u, 0x7632); }   // rounded
 };
 
@@ -483,9 +497,10 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       if (!ok) break;
       const float mn = fmaxf(m, fmaxf(mine_mx, s_mx[n & 1][1 - h][r]) * c2);
       // (both warps of the rows see the same maxima and decide alike)
-      if (__any_sync(0xffffffffu, mn > m + RESCALE_LOG2 || (m == -INFINITY && mn > m))) {
-        const float f = mn == -INFINITY ? 1.f : ex2(m - mn);   // 0 for a row that had seen nothing
-        m = mn;
+      const bool grown = mn > m + RESCALE_LOG2 || (m == -INFINITY && mn > m);
+      if (__any_sync(0xffffffffu, grown)) {
+        const float f = grown ? ex2(m - mn) : 1.f;             // 0 for a row that had seen nothing; other rows of the warp keep theirs
+        if (grown) m = mn;
         l *= f;
         if (n) {
           ok = bar_wait(smem_addr(&b_o), (uint32_t)((n - 1) & 1), &s_fail);   // the previous block's product is in O
@@ -515,25 +530,29 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       const uint64_t c22 = pair(__float_as_uint(c2), __float_as_uint(c2)), mu2 = pair(__float_as_uint(-mu), __float_as_uint(-mu));
       const uint64_t minus2 = pair(0xbf800000u, 0xbf800000u);
       uint64_t l2[2] = {0ull, 0ull};
-      // weight = hi + lo: hi = the leading bits that the type keeps (cut, not rounded), lo = the rest, rounded
+      // weight = hi + lo: hi = the leading bits that the type keeps, rounded, lo = the rest, rounded
+      auto weights = [&](auto lead) {
 #pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        uint32_t hi[16], lo[16];
+        for (int g = 0; g < 2; ++g) {
+          uint32_t hi[16], lo[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          uint32_t p0, p1, h0, h1, q0, q1;
-          unpair(fma2(pair(x[g * 32 + 2 * j], x[g * 32 + 2 * j + 1]), c22, mu2), p0, p1);
-          p0 = __float_as_uint(ex2(__uint_as_float(p0)));
-          p1 = __float_as_uint(ex2(__uint_as_float(p1)));
-          const uint64_t pp = pair(p0, p1);
-          l2[j & 1] = add2(l2[j & 1], pp);
-          hi[j] = Elem<BF>::lead(p0, p1, h0, h1);
-          unpair(fma2(pair(h0, h1), minus2, pp), q0, q1);
-          lo[j] = Elem<BF>::rest(q0, q1);
+          for (int j = 0; j < 16; ++j) {
+            uint32_t p0, p1, h0, h1, q0, q1;
+            unpair(fma2(pair(x[g * 32 + 2 * j], x[g * 32 + 2 * j + 1]), c22, mu2), p0, p1);
+            p0 = __float_as_uint(ex2(__uint_as_float(p0)));
+            p1 = __float_as_uint(ex2(__uint_as_float(p1)));
+            const uint64_t pp = pair(p0, p1);
+            l2[j & 1] = add2(l2[j & 1], pp);
+            hi[j] = lead(p0, p1, h0, h1);
+            unpair(fma2(pair(h0, h1), minus2, pp), q0, q1);
+            lo[j] = Elem<BF>::rest(q0, q1);
+          }
+          st16(st + g * 16, hi);
+          st16(st + 32 + g * 16, lo);
         }
-        st16(st + g * 16, hi);
-        st16(st + 32 + g * 16, lo);
-      }
+      };
+      if (Elem<BF>::ZEROS || plain) weights([](uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) { return Elem<BF>::lead(p0, p1, h0, h1); });
+      else weights([](uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) { return Elem<BF>::lead_zero(p0, p1, h0, h1); });   // some are hidden
       wait_st();
       fence_before();
       __syncwarp();

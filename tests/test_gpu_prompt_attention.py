@@ -97,6 +97,79 @@ def test_a_token_sees_nothing_but_its_own_keys(ops):
     assert not torch.isfinite(out[60:].view(40, 32, 128)[..., 5]).any()
 
 
+def test_hidden_keys_leave_no_trace(ops):
+    """The same tokens with other keys and values at later positions and in the sequence that shares their tile: bit for bit the same rows.
+    Their own values are small, so that even a remainder of a hidden value of 6e4 times the smallest normal weight would show."""
+    segments = [(0, 0, 100), (1, 0, 28)]
+    qkv, ck, cv, pos, seq = batch(segments, 32, 8, 200, 2, seed=11)
+    cv[0, :60] *= 1e-3
+    outs = []
+    for k, size in enumerate((1.0, 6e4)):
+        g = torch.Generator(device="cuda").manual_seed(20 + k)
+        for part in (ck[0, 60:100], ck[1], qkv[60:100], qkv[100:]):
+            part.copy_(3 * torch.randn(part.shape, generator=g, device="cuda"))
+        for part in (cv[0, 60:100], cv[1]):
+            part.copy_(size * (2 * torch.rand(part.shape, generator=g, device="cuda") - 1))
+        out = torch.empty(128, 32 * 128, dtype=torch.float16, device="cuda")
+        ops.seq_attention(qkv, ck, cv, pos, seq, out, 32, 8, 128, 128 ** -0.5)
+        outs.append(out[:60])
+    check_rows(outs[0], reference(qkv[:60], ck, cv, pos[:60], seq[:60], 32, 8, 128 ** -0.5), 32, 1e-3 * 5)
+    assert torch.equal(*outs)
+
+
+def signs_that_cancel(p):
+    """p [heads, keys] weights of one row -> values +-1 [heads, keys, 128] whose weighted sums nearly vanish: what is left of the output is
+    the error of the weights."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    v = torch.where(torch.rand(*p.shape, 128, generator=g, device="cuda") < 0.5, -1.0, 1.0).double()
+    for _ in range(40):                                           # turn the key whose part is closest to half of what is left
+        left = torch.einsum("hj,hjd->hd", p, v)
+        j = (left[:, None, :] - 2 * p[:, :, None] * v).abs().argmin(1, keepdim=True)
+        turned = v.scatter(1, j, -v.gather(1, j))
+        better = torch.einsum("hj,hjd->hd", p, turned).abs() < left.abs()
+        v = torch.where(better[:, None, :], turned, v)
+    return v
+
+
+def split_error(w, dtype):
+    """w minus its two-term split with both terms rounded."""
+    hi = w.to(dtype).double()
+    return w - hi - (w - hi).to(dtype).double()
+
+
+def test_weights_keep_both_terms(ops):
+    """float16: 1000 keys of comparable weights whose values cancel. Without the second term of the weights (2^-12 of each) the outputs would
+    be off by 2^-12 / sqrt(3000), 4e-6; with it by float32 sums and the smallest float16 numbers."""
+    H, n = 8, 1000
+    qkv, ck, cv, pos, seq = batch([(0, n - 40, 40)], H, H, n, 1, seed=12)
+    q = qkv[-1, :H * 128].double().view(H, 128)
+    p = torch.softmax(torch.einsum("hd,jhd->hj", q, ck[0].double()) * 128 ** -0.5, 1)
+    cv[0] = signs_that_cancel(p).permute(1, 0, 2).half()
+    out = torch.empty(40, H * 128, dtype=torch.float16, device="cuda")
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, H, H, 128, 128 ** -0.5)
+    want = torch.einsum("hj,jhd->hd", p, cv[0].double())
+    assert (out[-1].double().view(H, 128) - want).abs().max() <= 2 ** -21
+
+
+def test_window_weights_are_rounded_twice(ops):
+    """bfloat16: as above; the error is that of a split with both terms rounded and of float32 sums and exponentials (half as much again). A
+    leading term that is cut instead leaves a remainder, and an error, of twice the size."""
+    H, n = 32, 1000
+    g = torch.Generator(device="cuda").manual_seed(13)
+    q = torch.randn(40, H, 128, generator=g, device="cuda").bfloat16().float()
+    ck = torch.randn(1, n, H, 128, generator=g, device="cuda").bfloat16()
+    s = torch.einsum("hd,jhd->hj", q[-1].double(), ck[0].double()) * 128 ** -0.5
+    p = torch.softmax(s, 1)
+    cv = signs_that_cancel(p).permute(1, 0, 2)[None].bfloat16().contiguous()
+    meta = torch.stack([torch.zeros(40), torch.arange(n - 40, n), torch.zeros(40), torch.full((40,), 40), torch.zeros(40)]).to(torch.int32).cuda()
+    out = torch.empty(40, H, 128, dtype=torch.bfloat16, device="cuda")
+    ops.seq_window_attention_mma(q, ck, None, cv, out, meta, 4096, 128 ** -0.5, True)
+    err = out[-1].double() - torch.einsum("hj,jhd->hd", p, cv[0].double())
+    w = torch.exp(s - s.amax(1, keepdim=True))
+    expected = (split_error(w, torch.bfloat16).pow(2).sum(1).sqrt() / w.sum(1)).pow(2).mean().sqrt()
+    assert err.pow(2).mean().sqrt() <= 1.5 * expected, (err.pow(2).mean().sqrt() / expected).item()
+
+
 def test_values_that_arrive_late(ops):
     """Caches that no kernel has read yet and an L2 full of something else: the last blocks' values come from DRAM, after the weights they
     are multiplied with. The outputs wait for both of the products that can then still be under way."""
