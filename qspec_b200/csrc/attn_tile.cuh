@@ -582,7 +582,10 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     }
     const int pr = row_in && mine ? pos[tl] : 0;
     const bool store = ok && row_in && mine && !(a.skip_outside && (unsigned)pr >= (unsigned)a.cap);
-    const bool dead = l == 0.f;                               // saw no key at all
+    // No key had a weight: none was visible, or every score was -inf. As in the kernels beside this one: 0 / 0 in the window form without
+    // a sink and in decode_attention, zeros otherwise.
+    const bool dead = l == 0.f;
+    const float none = (a.ring && !a.sink) || a.skip_outside ? __int_as_float(0x7fffffff) : 0.f;
     float f = 0.f;
     if (!dead) {
       float mm = m, ls = l;
@@ -610,7 +613,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             float v[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              v[e] = dead ? 0.f : __uint_as_float(o[g * 8 + e]) * f;
+              v[e] = dead ? none : __uint_as_float(o[g * 8 + e]) * f;
               bad |= !(fabsf(v[e]) < INFINITY);
             }
             if (gt) {
@@ -628,7 +631,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
           }
         }
       }
-      if (bad && store) attn_row_again<BF, QF32>(a, c0 + tl, head, kvh, my_seq, my_lo, my_hi, h * 64);
+      if (bad && store && !dead) attn_row_again<BF, QF32>(a, c0 + tl, head, kvh, my_seq, my_lo, my_hi, h * 64);
     }
   }
   fence_before();

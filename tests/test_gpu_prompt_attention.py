@@ -241,6 +241,28 @@ def test_far_apart_scores(ops):
     check(out, reference(qkv, ck, cv, pos, seq, 8, 8, 128 ** -0.5))
 
 
+@pytest.mark.parametrize("form", ["seq", "decode", "window", "sink"])
+def test_rows_without_a_weight(ops, form):
+    """Every score of the first 20 tokens is -inf: what softmax makes of it, 0 / 0, where the forms for few tokens say so (decode_attention,
+    window attention without a sink), zeros where they say that."""
+    T, S, dtype = 64, 100, torch.float16 if form in ("seq", "decode") else torch.bfloat16
+    Hq, Hkv = (24, 8) if form == "decode" else (16, 8)
+    qkv, ck, cv, pos, seq = batch([(0, 0, T)], Hq, Hkv, S, 1, seed=14)
+    qkv[:, :Hq * 128:128] = 1.0
+    ck, cv = ck.to(dtype), cv.to(dtype)
+    ck[0, :20, :, 0] = float("-inf")
+    if form in ("seq", "decode"):
+        out = torch.full((T, Hq * 128), 7.0, dtype=dtype, device="cuda")
+        (ops.seq_attention if form == "seq" else ops.decode_attention)(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 0.1)
+    else:
+        out = torch.full((T, Hq, 128), 7.0, dtype=dtype, device="cuda")
+        meta = torch.stack([seq, pos, 0 * pos, 0 * pos + T, 0 * pos]).contiguous()
+        sink = torch.zeros(Hq, device="cuda") if form == "sink" else None
+        ops.seq_window_attention_mma(qkv[:, :Hq * 128].float().reshape(T, Hq, 128), ck, None, cv, out, meta, 1000, 0.1, True, sink=sink)
+    assert torch.isfinite(out[20:]).all()
+    assert out[:20].isnan().all() if form in ("decode", "window") else (out[:20] == 0).all()
+
+
 # ---- the same tiles in the sequence-mixer library: bfloat16, rings, window, sink, gates ---------------------------------------------
 @pytest.mark.parametrize("H,G,window,cap,segments,gate,sink", [
     (16, 4, 40, 200, [(0, 150, 70)], "each", True),                    # the ring wraps inside a block, inside the portion
