@@ -287,13 +287,15 @@ int qspec_decode_attention(const void* qkv, const void* cache_k, const void* cac
  * queries, the cache already contains this pass's keys); B = number of sequences the cache holds (seq_ids < B).
  * fp32 math; agrees with qspec_decode_attention to fp32 rounding, not bit for bit. qspec_seq_attention_supported():
  * D == 128, Hq/Hkv in {1,2,4,5,8}, T <= 1024, S small enough for shared memory (~1500 positions at Hq/Hkv = 4). */
-/* CTAs of the tensor-core prompt form (inside qspec_seq_attention and qspec_decode_attention) that gave up a bounded wait since the
- * library was loaded on the current device: 0 unless something is broken; -1 if it cannot be read. Synchronises. No counterpart. */
-int qspec_attn_tile_timeouts(void);
 int qspec_seq_attention_supported(int T, int Hq, int Hkv, int D, int S);
 int qspec_seq_attention(const void* qkv, const void* cache_k, const void* cache_v, const int* positions,
                         const int* seq_ids, void* out, int T, int B, int Hq, int Hkv, int D, int S, float sm_scale,
                         void* stream);
+
+/* CTAs of qspec_seq_attention, and of the tensor-core prompt form inside it and qspec_decode_attention, that gave up a bounded wait since
+ * the library was loaded on the current device (the rows that such a CTA would have written are NaN): 0 unless something is broken; -1 if
+ * it cannot be read. Synchronises. No counterpart. */
+int qspec_attn_tile_timeouts(void);
 
 /* The attention block between qkv_proj and o_proj as one launch for decode-sized passes: rotary embedding and
  * cache append (qspec_rope_kvcache), attention over the cache (qspec_decode_attention), the o_proj rotation over

@@ -190,10 +190,11 @@ int qspec_seq_window_attention(const qspec_window_attn_args* args, int dtype, vo
  * tokens, head) -- prompts. */
 int qspec_seq_window_attention_mma(const qspec_window_attn_args* args, const void* k_shared, long long k_shared_slot_stride,
                                    int k_shared_row_stride, int DB, int token_rows, void* stream);
-/* CTAs of the tensor-core prompt form (inside qspec_seq_window_attention_mma with token_rows) that gave up a bounded wait since the
- * library was loaded on the current device: 0 unless something is broken; -1 if it cannot be read. Synchronises. */
-int qspec_seq_attn_tile_timeouts(void);
 int qspec_seq_window_attention_mma_supported(int DA, int DB, int DV, int H, int G, int token_rows);
+/* CTAs of the tensor-core prompt form (inside qspec_seq_window_attention_mma with token_rows) that gave up a bounded wait since the
+ * library was loaded on the current device (the rows that such a CTA would have written are NaN): 0 unless something is broken; -1 if it
+ * cannot be read. Synchronises. */
+int qspec_seq_attn_tile_timeouts(void);
 
 /* HGRN2 recurrence. Row t of p = [zq (H x D) | zf (H x D) | v (H x DV)]. q = silu(zq), f = lower + (1 - lower) *
  * sigmoid(zf + f_b); per head S <- diag(f) S + (1 - f) v^T, o = S^T q; out[t, h] = unit_rms(o over DV) * norm_w.

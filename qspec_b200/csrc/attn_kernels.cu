@@ -593,7 +593,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   __shared__ float s_m[NW][16], s_l[NW][16];
   __shared__ __align__(16) uint4 s_qf[8][32];                // Q fragments of the chunk in mma order: [k-step][lane] = (a0, a1, a2, a3)
   __shared__ __align__(8) uint64_t s_full[NW][2][ST];         // keys, values of a warp's blocks
-  __shared__ volatile int s_fail;                            // a bounded wait ran out: nothing is stored
+  __shared__ volatile int s_fail;                            // a bounded wait ran out: NaN is stored
   extern __shared__ __align__(16) unsigned char seq_dyn[];   // [NW][ST] blocks; after the keys:
   constexpr int OS = D + 4;                                  // (row stride of the partial outputs: the rows of a store fall on different banks)
   float (*s_o)[16][OS] = reinterpret_cast<float (*)[16][OS]>(seq_dyn);   // [NW][16][OS] fp32: per-warp partial outputs
@@ -650,6 +650,13 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
       bulk_row_256(atile::smem_addr(ring) + at * SEQ_BLOCK + (values ? 16 * SEQ_KS + lane * SEQ_VS : lane * SEQ_KS),
                    (values ? vbase : kbase) + (size_t)(kb + lane) * kv_stride, bar);
   };
+  // before giving up at block kb: the keys of the blocks from `keys` places on (0: itself), the values from itself on, if they were asked for
+  auto drain = [&](uint32_t keys, int kb, int nkeys) {
+    for (uint32_t i = keys; i < ST + keys; ++i)
+      if (kb + (int)i * NW * 16 < nkeys) atile::bar_drain(atile::smem_addr(&s_full[warp][0][(blocks + i) % ST]), ((blocks + i) / ST) & 1);
+    for (uint32_t i = 0; i < ST; ++i)
+      if (kb + (int)i * NW * 16 < nkeys) atile::bar_drain(atile::smem_addr(&s_full[warp][1][(blocks + i) % ST]), ((blocks + i) / ST) & 1);
+  };
   for (int c0 = 0; c0 < ntok; c0 += R) {
     const int nr = min(R, ntok - c0);
     // rows gid and gid + 8 of this lane: (token slot, head) and the position limit of the row (-1 = padding row)
@@ -695,7 +702,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
       const uint32_t at = blocks % ST, phase = (blocks / ST) & 1;
       const unsigned char* blk = ring + at * SEQ_BLOCK;
       unsigned char* blv = ring + at * SEQ_BLOCK + 16 * SEQ_KS;
-      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][0][at]), phase, &s_fail))) break;
+      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][0][at]), phase, &s_fail))) { drain(0, kb, nkeys); break; }
       // ---- S = Q K^T for the two 8-key tiles
       float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -737,7 +744,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
       uint32_t ah[4], al[4];
       split_h2(pA[0], pA[1], ah[0], al[0]); split_h2(pB[0], pB[1], ah[1], al[1]);
       split_h2(pA[2], pA[3], ah[2], al[2]); split_h2(pB[2], pB[3], ah[3], al[3]);
-      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][1][at]), phase, &s_fail))) break;
+      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][1][at]), phase, &s_fail))) { drain(1, kb, nkeys); break; }
       if (kb + 16 > nkeys) {                                 // rows past the last key: their weights are zero, their values must be finite
         for (int i = (nkeys - kb) * 16 + lane; i < 256; i += 32) *reinterpret_cast<uint4*>(blv + (i >> 4) * SEQ_VS + (i & 15) * 16) = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();                                        // (a warp's last block: the barrier before the next chunk's copies follows)
@@ -776,6 +783,9 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
     __syncthreads();
     if (s_fail) {                                            // (written before the barrier: uniform)
       if (tid == 0) atomicAdd(&atile::attn_tile_timeouts, 1u);
+      for (int i = tid; i < (ntok - c0) * G * 16; i += NW * 32)   // nobody takes what the buffer held for a result
+        *reinterpret_cast<uint4*>(out + ((size_t)s_tok[c0 + i / (G * 16)] * Hq + hk * G + i / 16 % G) * D + (i & 15) * 8) =
+            make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
       return;
     }
     // ---- merge the warps: thread = (row r, 16 dims); out = sum_w e^{m_w - m} O_w / sum_w e^{m_w - m} l_w

@@ -25,8 +25,8 @@
 // its own maximum alone. A weight of zero times a value that is not finite would be NaN: rows with a result that is not finite are computed
 // again key by key (attn_row_again).
 //
-// Every wait is bounded; a CTA whose wait runs out counts itself in attn_tile_timeouts, frees its tensor memory and leaves without
-// storing.
+// Every wait is bounded; a CTA whose wait runs out waits (again with a limit) for its copies and products under way, fills its rows with
+// NaN, so that nobody takes what the buffer held for a result, counts itself in attn_tile_timeouts and frees its tensor memory.
 #pragma once
 #include "common.cuh"
 #include <cuda.h>
@@ -46,7 +46,7 @@ constexpr size_t SMEM = (1 + KS + VS) * (size_t)TILE + 1024;   // Q | keys | val
 constexpr float RESCALE_LOG2 = 8.f;
 constexpr uint32_t WAIT_SPINS = 1u << 20;
 
-static __device__ unsigned attn_tile_timeouts;  // CTAs of this library that gave a wait up, since it was loaded
+static __device__ unsigned attn_tile_timeouts;  // CTAs of this library's attention kernels that gave a wait up, since it was loaded
 
 struct Args {
   const void* q; long long q_ts, q_hs;         // strides in elements; tokens, heads
@@ -99,6 +99,11 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile
   }
   *fail = 1;
   return false;
+}
+// For what is under way at the end: waits, as long as any wait, whether or not the CTA has given up.
+__device__ __noinline__ void bar_drain(uint32_t bar, uint32_t parity) {
+  int none = 0;
+  bar_wait(bar, parity, &none);
 }
 __device__ __forceinline__ bool elect() {
   uint32_t pred;
@@ -378,7 +383,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         if (++ks == KS) { ks = 0; kphase ^= 1u; }
         return true;
       };
-      bool ok = blocks == 0 || scores(0);
+      bool ok = blocks == 0 || scores(0), over = blocks == 0;
       for (uint32_t n = 0; ok && n < blocks; ++n) {
         if (n + 1 < blocks && !scores(n + 1)) break;
         if (!bar_wait(smem_addr(&b_vfull[n % VS]), (n / VS) & 1, &s_fail)) break;
@@ -398,9 +403,11 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         }
         if (!ok) break;
         commit(bo);
-        if (n + 1 == blocks) commit(smem_addr(&b_done));
+        if (n + 1 == blocks) { commit(smem_addr(&b_done)); over = true; }
         commit(smem_addr(&b_vempty[n % VS]));
       }
+      if (!over) commit(smem_addr(&b_done));                   // given up: the products issued so far
+      if (blocks) bar_drain(smem_addr(&b_done), 0);
     }
     __syncwarp();
   } else if (warp == WARP_K || warp == WARP_V) {
@@ -414,8 +421,8 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     int stage = 0;
     uint32_t phase = 1;                                       // of the stage's previous release: none to wait for in the first round
     bool ok = true;
-    int parts = 0;
-    for (int n = 0; items.next(it); ++n) {
+    int parts = 0, n = 0;
+    for (; items.next(it); ++n) {
       if (n >= stages) ok = bar_wait(smem_addr(&empty[stage]), phase, &s_fail);
       if (!__all_sync(0xffffffffu, ok)) break;
       // value rows past the block's last key are cleared before the products see them (their weights are zero, but zero times NaN is not):
@@ -431,8 +438,12 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       }
       __syncwarp();
       if (part) {
-        ok = bar_wait(bar, (uint32_t)(parts++ & 1), &s_fail);
-        if (!__all_sync(0xffffffffu, ok)) break;
+        ok = bar_wait(bar, (uint32_t)(parts & 1), &s_fail);
+        if (!__all_sync(0xffffffffu, ok)) {
+          bar_drain(bar, (uint32_t)(parts & 1));
+          break;
+        }
+        ++parts;
         unsigned char* rows = gbase + (dst - base);
         for (int i = have * 8 + lane; i < 128 * 8; i += 32) {
           *reinterpret_cast<uint4*>(rows + i * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -444,6 +455,8 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       }
       if (++stage == stages) { stage = 0; phase ^= 1u; }
     }
+    // blocks 0 .. n - 1 were asked for: the CTA does not leave before the last of each stage has landed
+    for (int j = max(0, n - stages); j < n; ++j) bar_drain(smem_addr(&full[j % stages]), (uint32_t)(j / stages) & 1u);
   } else if (warp < WARP_K) {
     // ---- softmax: thread = 64 columns (half h) of row r
     const int h = warp >> 2, r = (warp & 3) * 32 + lane;
@@ -640,7 +653,16 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
   }
-  if (tid == 0 && s_fail) atomicAdd(&attn_tile_timeouts, 1u);
+  if (s_fail) {                                               // (written before the barrier: uniform)
+    if (tid == 0) atomicAdd(&attn_tile_timeouts, 1u);
+    for (int q = 0; q < nruns; ++q)
+      for (int i = s_rs[q] * rep * 16 + tid; i < (s_re[q] + 1) * rep * 16; i += THREADS) {
+        const int tl = i / (rep * 16), head = kvh * rep + i / 16 % rep;
+        if (a.skip_outside && (unsigned)pos[tl] >= (unsigned)a.cap) continue;
+        *reinterpret_cast<uint4*>((T*)a.out + (size_t)(c0 + tl) * a.out_ts + (size_t)head * a.out_hs + (i & 15) * 8) =
+            make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+      }
+  }
 }
 
 // Heads per group that fit, positive scale (a row's maximum is the scaled maximum), rows on 16-byte boundaries.

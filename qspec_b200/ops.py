@@ -653,9 +653,16 @@ def decode_attention(qkv: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Te
 
 
 def attn_tile_timeouts() -> int:
-    """CTAs of the prompt forms inside seq_attention, decode_attention and seq_window_attention_mma that gave up a bounded wait: 0
-    unless something is broken."""
-    return int(_lib.load().qspec_attn_tile_timeouts()) + int(_lib.load_seq().qspec_seq_attn_tile_timeouts())
+    """CTAs of seq_attention and of the prompt forms inside it, decode_attention and seq_window_attention_mma that gave up a bounded wait
+    (their rows are NaN): 0 unless something is broken. Counts those of the current device, synchronises."""
+    counts = []
+    if _lib._lib is not None:
+        counts.append(_lib._lib.qspec_attn_tile_timeouts())
+    if _lib._seq_lib is not None:
+        counts.append(_lib._seq_lib.qspec_seq_attn_tile_timeouts())
+    if any(n < 0 for n in counts):
+        raise RuntimeError("attn_tile_timeouts: the count of waits that were given up cannot be read")
+    return sum(counts)
 
 
 def seq_attention_supported(T: int, num_heads: int, num_kv_heads: int, head_dim: int, cache_len: int) -> bool:

@@ -205,3 +205,37 @@ def test_plugin_binds_to_the_importable_vllm_registry():
     assert tuple(layer.weight.shape) == (256, 128) and layer.weight.dtype == torch.int8
     assert tuple(layer.weight_scales.shape) == (256, 1) and layer.weight.input_dim == 1 and layer.weight.packed_dim == 1
     assert callable(layer.weight.weight_loader)
+
+
+# ---- waits that attention gave up ----------------------------------------------------------------------------------------------------
+def _counters(monkeypatch, main, seq):
+    import types
+    from qspec_b200 import _lib
+    monkeypatch.setattr(_lib, "_lib", None if main is None else types.SimpleNamespace(qspec_attn_tile_timeouts=lambda: main))
+    monkeypatch.setattr(_lib, "_seq_lib", None if seq is None else types.SimpleNamespace(qspec_seq_attn_tile_timeouts=lambda: seq))
+
+
+@pytest.mark.parametrize("main,seq,total", [(0, 0, 0), (2, 3, 5), (None, 3, 3), (2, None, 2), (None, None, 0)])
+def test_given_up_waits_are_counted_over_the_loaded_libraries(monkeypatch, main, seq, total):
+    from qspec_b200 import ops
+    _counters(monkeypatch, main, seq)
+    assert ops.attn_tile_timeouts() == total
+
+
+@pytest.mark.parametrize("main,seq", [(-1, 1), (1, -1), (-1, None)])
+def test_a_counter_that_cannot_be_read_is_an_error(monkeypatch, main, seq):
+    from qspec_b200 import ops
+    _counters(monkeypatch, main, seq)
+    with pytest.raises(RuntimeError):
+        ops.attn_tile_timeouts()
+
+
+def test_engine_metrics_report_given_up_waits(monkeypatch):
+    import types
+    from qspec_b200.engine import QSpecEngine
+    engine = types.SimpleNamespace(model=types.SimpleNamespace(peers=None), counters=torch.tensor([3, 6, 5]), B=2, k=3)
+    _counters(monkeypatch, 0, None)
+    assert QSpecEngine.metrics(engine)["accepted_tokens"] == 3
+    _counters(monkeypatch, 1, None)
+    with pytest.raises(RuntimeError, match="gave up"):
+        QSpecEngine.metrics(engine)
