@@ -824,10 +824,12 @@ static int launch_seq_attention_st(const void* qkv, const void* ck, const void* 
   constexpr size_t dyn = (size_t)NW * ST * SEQ_BLOCK;
   static_assert(SEQ_BLOCK >= 16 * (128 + 4) * (int)sizeof(float), "the partial outputs lie in the blocks");
   auto kern = seq_attention_kernel<G, ST, NW>;
-  static bool attr_set = false;                              // per instantiation
-  if (!attr_set) {
+  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
+  int dev = 0;
+  QSPEC_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
     QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    attr_set = true;
+    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
   }
   launch_pdl(kern, dim3(B * Hkv), dim3(NW * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
              positions, seq_ids, (__half*)out, T, Hq, Hkv, S, sm_scale, min_run);
