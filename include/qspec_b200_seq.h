@@ -186,8 +186,10 @@ int qspec_seq_window_attention(const qspec_window_attn_args* args, int dtype, vo
  * 128), value size 64 or 128; rows and strides on 16-byte boundaries). args->qa is the whole query [DA] (args->DB = 0); the
  * last DB entries of a key come from k_shared (one row per slot and ring row, shared by all heads: the rotary part of a
  * latent cache), the first DA - DB from args->k. token_rows = 0: one CTA per (token, key/value head), the rows of the
- * products are the query heads of the group (H / G <= 16) -- decode-shaped batches; 1: one CTA per (16 consecutive batch
- * tokens, head) -- prompts. */
+ * products are the query heads of the group (H / G <= 16) -- decode-shaped batches. 1: prompts, alone or beside decoding sequences:
+ * head size 128 without a shared part and without kept tokens in tiles of 128 (token, head of a group) rows, where tokens of segments
+ * shorter than 16 take the rows of token_rows = 0; other sizes one CTA per (16 consecutive batch tokens, head). 2: as 1 where the caller
+ * knows that every segment has at least 16 tokens. */
 int qspec_seq_window_attention_mma(const qspec_window_attn_args* args, const void* k_shared, long long k_shared_slot_stride,
                                    int k_shared_row_stride, int DB, int token_rows, void* stream);
 int qspec_seq_window_attention_mma_supported(int DA, int DB, int DV, int H, int G, int token_rows);

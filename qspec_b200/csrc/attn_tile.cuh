@@ -19,7 +19,8 @@
 //
 // Which tokens: those in RUNS, i.e. neighbours in the batch with one sequence and consecutive positions, of at least min_run
 // tokens. A CTA walks the runs of its tokens one after the other (rows of other runs are masked). Tokens outside such runs are left
-// to the caller's other kernel (attn_in_run is the common test).
+// to the caller's other kernel (attn_in_run is the common test). Where the caller has a table of segments, the test is the length of the
+// token's segment instead, and runs end where segments do.
 //
 // A row sees nothing but its own keys, bit for bit: hidden keys enter the products with weights of exactly zero, and a row is rescaled by
 // its own maximum alone. A weight of zero times a value that is not finite would be NaN: rows with a result that is not finite are computed
@@ -55,6 +56,7 @@ struct Args {
   const int* pos; const int* seq;
   int ntok, nseq, rep, cap, window;            // nseq: sequences the cache holds; a token of another one belongs to no run
   float scale;
+  const int* seg;                              // or NULL: [2][ntok] first batch row and end of each token's segment
   int min_run, ring, skip_outside;             // skip_outside: a token whose position is outside the cache is not stored
   void* out; long long out_ts; int out_hs;
   const float* sink; const void* gate; int gate_ld, gate_per_head; float out_scale;
@@ -294,6 +296,12 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   if (tid < TOKENS_MAX) {
     bool before, after;
     bool in = attn_in_run(a.pos, a.seq, a.ntok, c0 + warp * 32, a.min_run, before, after) && tid < n2;
+    if (a.seg && tid < n2) {
+      const int t = c0 + tid, s0 = a.seg[t], s1 = a.seg[a.ntok + t];
+      in = s1 - s0 >= a.min_run;
+      before = before && t > s0;
+      after = after && t + 1 < s1;
+    }
     if (in) {
       pos[tid] = a.pos[c0 + tid];
       seq[tid] = a.seq[c0 + tid];

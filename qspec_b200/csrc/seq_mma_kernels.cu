@@ -986,9 +986,10 @@ struct WinMma {
 
 // STREAM: key rows are loaded inside the product loop instead of a whole step ahead (long keys: the fragments of a step
 // would not fit the register file); blockIdx.z selects a slice of DV value columns (values longer than DV).
+// bx: the block of 16 tokens (token_rows) or the token whose heads are the rows; with `toks` the rows are the heads of a group of `toks`
+// tokens of one sequence from bx on (toks * H / G <= 16).
 template <int DA, int DB, int DV, bool STREAM>
-__global__ void __launch_bounds__(128, 2) window_attn_mma_kernel(const WinMma a) {
-  pdl_enter();
+__device__ __forceinline__ void window_attn_mma_rows(const WinMma& a, int bx, int toks = 0) {
   constexpr int DK = DA + DB, QS = DK / 2 + 4;
   extern __shared__ __align__(16) unsigned char wm_raw[];
   uint32_t* sQ = reinterpret_cast<uint32_t*>(wm_raw);       // [16][QS]
@@ -1000,8 +1001,9 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_kernel(const WinMma a)
   const int kvh = a.token_rows ? (int)blockIdx.y / rep : (int)blockIdx.y;
   if (tid < 16) {
     int tok = -1, head = 0;
-    if (a.token_rows) { tok = blockIdx.x * 16 + tid; head = blockIdx.y; if (tok >= a.ntok) tok = -1; }
-    else if (tid < rep) { tok = blockIdx.x; head = kvh * rep + tid; }
+    if (a.token_rows) { tok = bx * 16 + tid; head = blockIdx.y; if (tok >= a.ntok) tok = -1; }
+    else if (toks) { if (tid < toks * rep) { tok = bx + tid / rep; head = kvh * rep + tid % rep; } }
+    else if (tid < rep) { tok = bx; head = kvh * rep + tid; }
     s_tok[tid] = tok; s_head[tid] = head;
     s_pos[tid] = tok >= 0 ? a.meta[a.ntok + tok] : -1;
     s_seg[tid] = tok >= 0 ? a.meta[2 * a.ntok + tok] : -1;
@@ -1033,7 +1035,7 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_kernel(const WinMma a)
     int r1 = r0 + 1;
     while (r1 < 16 && s_tok[r1] >= 0 && s_seg[r1] == s_seg[r0]) ++r1;
     const int seg = s_seg[r0], slot = s_slot[r0];
-    const int pmax = a.token_rows ? s_pos[r1 - 1] : s_pos[r0];
+    const int pmax = a.token_rows || toks ? s_pos[r1 - 1] : s_pos[r0];
     // keys in order: nk kept positions that the first row's window has left behind, then positions from jlo on
     const int jlo = max(0, s_pos[r0] - a.window + 1), nk = min(a.keep, jlo);
     const int nkeys = nk + pmax - jlo + 1;
@@ -1066,8 +1068,8 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_kernel(const WinMma a)
         for (int sp = 0; sp < DV / 64; ++sp) r.v[q][sp] = ok ? __ldg(reinterpret_cast<const uint4*>(vp + 64 * sp + 8 * gid)) : zero4;
       }
     };
-    const bool inA = a.token_rows ? (segA == seg && s_tok[rA] >= 0) : rA < rep;
-    const bool inB = a.token_rows ? (segB == seg && s_tok[rB] >= 0) : rB < rep;
+    const bool inA = a.token_rows || toks ? (segA == seg && s_tok[rA] >= 0) : rA < rep;
+    const bool inB = a.token_rows || toks ? (segB == seg && s_tok[rB] >= 0) : rB < rep;
     Rows cur, nxt;
     int hb = warp;
     if (!STREAM && hb * 16 < nkeys) fetch(hb, cur);
@@ -1205,6 +1207,44 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_kernel(const WinMma a)
     float r = acc / L * a.out_scale;
     if (a.gate) r *= __fdividef(1.0f, 1.0f + __expf(-__bfloat162float(a.gate[(size_t)tok * a.gate_ld + (a.gate_per_head ? (size_t)head : (size_t)head * a.out_hs + (size_t)blockIdx.z * DV + d)])));
     a.out[(size_t)tok * a.out_ts + (size_t)head * a.out_hs + (size_t)blockIdx.z * DV + d] = __float2bfloat16_rn(r);
+  }
+}
+
+template <int DA, int DB, int DV, bool STREAM>
+__global__ void __launch_bounds__(128, 2) window_attn_mma_kernel(const WinMma a) {
+  pdl_enter();
+  window_attn_mma_rows<DA, DB, DV, STREAM>(a, blockIdx.x);
+}
+
+// The same for the tokens of a batch whose segment is shorter than WIN_RUN (decoding sequences, rests of prompts), beside
+// attn_tile_kernel, which takes the others: the rows are the heads of a group of up to 16 / heads tokens of a segment. CTA x takes the pieces
+// that begin at tokens x, x + gridDim.x, ...: neighbours go to different CTAs, and a warp looks at 32 of its CTA's tokens at once, so that a
+// batch without short segments costs a launch and little more.
+constexpr int WIN_RUN = 16;
+template <int DA, int DV>
+__global__ void __launch_bounds__(128, 2) window_attn_mma_short_kernel(const WinMma a) {
+  pdl_enter();
+  __shared__ uint32_t s_short;
+  const int most = 16 / (a.H / a.G);                          // tokens of a piece
+  for (int t0 = blockIdx.x; t0 < a.ntok; t0 += 32 * (int)gridDim.x) {
+    if (threadIdx.x < 32) {
+      const int t = t0 + (int)threadIdx.x * (int)gridDim.x;
+      bool begins = false;
+      if (t < a.ntok) {
+        const int s0 = a.meta[2 * a.ntok + t], s1 = a.meta[3 * a.ntok + t];
+        begins = s1 - s0 < WIN_RUN && (t - s0) % most == 0;
+      }
+      const uint32_t bits = __ballot_sync(0xffffffffu, begins);
+      if (threadIdx.x == 0) s_short = bits;
+    }
+    __syncthreads();
+    uint32_t left = s_short;
+    for (; left; left &= left - 1u) {
+      const int t = t0 + (__ffs(left) - 1) * (int)gridDim.x;
+      window_attn_mma_rows<DA, 0, DV, false>(a, t, min(most, a.meta[3 * a.ntok + t] - t));
+      __syncthreads();
+    }
+    __syncthreads();
   }
 }
 
@@ -1705,6 +1745,17 @@ static int launch_window_mma(const WinMma& a, int slices, cudaStream_t st) {
   return QSPEC_OK;
 }
 
+// Tokens of segments shorter than WIN_RUN, beside attn_tile_kernel.
+static int launch_window_short(WinMma a, cudaStream_t st) {
+  constexpr size_t smem = (size_t)16 * (128 / 2 + 4) * 4 + (size_t)4 * 16 * 128 * sizeof(float);   // below the limit that needs no asking for
+  static_assert(smem <= 48 * 1024, "dynamic shared memory");
+  a.token_rows = 0;
+  const int per = (2 * sm_count() / a.G) | 1;                 // two CTAs per SM; odd, so that pieces of 2, 4, .. tokens go to all of them
+  launch_pdl(window_attn_mma_short_kernel<128, 128>, dim3(min(a.ntok, per), a.G), dim3(128), smem, st, a);
+  QSPEC_CHECK_LAUNCH(1);
+  return QSPEC_OK;
+}
+
 // Shapes: per-head key part 64 or 128 with values of 64 or 128; 128 + a shared part of 64 with values of 128 (a latent
 // layer's expanded form); 256 or 512 + a shared part of 64 with values of 128, 256, 384 or 512 in slices of 128 columns (a
 // latent cache read in the absorbed form: key and value are the same rows).
@@ -1742,10 +1793,21 @@ int window_attention_mma(const qspec_window_attn_args* p, const void* kB, long l
     t.v = p->v; t.v_ss = p->v_slot_stride; t.v_rs = p->v_row_stride; t.v_hs = p->v_head_stride;
     t.pos = p->meta + p->ntok; t.seq = p->meta;
     t.ntok = p->ntok; t.nseq = 0x7fffffff; t.rep = p->H / p->G; t.cap = p->cap; t.window = p->window;
-    t.scale = p->scale; t.min_run = 1; t.ring = 1;
+    t.scale = p->scale; t.ring = 1;
+    // A tile walks its runs one after the other: 32 decoding tokens in it would be 32 walks for four rows each (64 of them beside 2000
+    // tokens, 16 / 4 heads, window 1024: 560 us; before the tiles 762, now see window_attn_mma_short_kernel). Tokens of short segments go
+    // there unless the caller says that there are none (or the heads of a group are too many).
+    const bool mixed = token_rows == 1 && t.rep <= 16;
+    t.seg = p->meta + 2 * p->ntok; t.min_run = mixed ? WIN_RUN : 1;
     t.out = p->out; t.out_ts = a.out_ts; t.out_hs = DV;
     t.sink = p->sink; t.gate = p->gate; t.gate_ld = p->gate_ld; t.gate_per_head = p->gate_per_head; t.out_scale = a.out_scale;
-    if (atile::supported(t, 4)) return atile::launch<true, true>(t, p->G, st);
+    if (atile::supported(t, 4)) {
+      if (!mixed || p->ntok >= WIN_RUN) {
+        const int rc = atile::launch<true, true>(t, p->G, st);
+        if (rc != QSPEC_OK) return rc;
+      }
+      return mixed ? launch_window_short(a, st) : QSPEC_OK;
+    }
   }
   // a latent cache read in the absorbed form (keys and values are the same rows): the CTA-level kernel; QSPEC_SEQ_LATENT=sliced
   // keeps the form with one CTA per slice of 128 value columns, for comparison

@@ -1085,15 +1085,19 @@ def seq_window_attention_mma_supported(out_dtype, DA: int, DB: int, DV: int, H: 
     return bool(out_dtype == _BF16 and _lib.load_seq().qspec_seq_window_attention_mma_supported(DA, DB, DV, H, G, int(token_rows)))
 
 
+WINDOW_ROWS_SEGMENT = 16
+
+
 def seq_window_attention_mma(q: torch.Tensor, cache_k: torch.Tensor, k_shared: Optional[torch.Tensor], cache_v: torch.Tensor,
-                             out: torch.Tensor, meta: torch.Tensor, window: int, scale: float, token_rows: bool,
+                             out: torch.Tensor, meta: torch.Tensor, window: int, scale: float, token_rows: int,
                              sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None,
                              gate_per_head: bool = False, keep_first: int = 0, out_scale: float = 1.0) -> None:
     """`seq_window_attention` on the tensor cores (bfloat16). q [ntok, H, DK] float32; cache_k [slots, cap, G, DA] holds the
     per-head part of the keys and k_shared [slots, cap, DB] (or None) the part all heads share, DK = DA + DB; cache_v
-    [slots, cap, G, DV] (views: a slot stride of 0 serves one buffer to every slot). token_rows: False = the rows of the
-    products are the query heads of a group, one CTA per (token, key/value head): decoding; True = 16 consecutive batch
-    tokens per CTA and head: prompts."""
+    [slots, cap, G, DV] (views: a slot stride of 0 serves one buffer to every slot). token_rows: 0 / False = the rows of the
+    products are the query heads of a group, one CTA per (token, key/value head): decoding; 1 / True = consecutive batch
+    tokens share a CTA: prompts, alone or beside decoding sequences; 2 = the same where every segment is known to have at least
+    WINDOW_ROWS_SEGMENT tokens, which saves the launch that looks for shorter ones."""
     import ctypes
     if q.dtype != _F32 or cache_k.dtype != _BF16 or cache_v.dtype != _BF16 or out.dtype != _BF16:
         raise ValueError("seq_window_attention_mma: float32 queries, bfloat16 caches and output")

@@ -35,6 +35,7 @@ from typing import Dict, List, Optional
 import torch
 
 from . import ops
+from .seq_layers import token_rows
 from .state import BatchMeta
 
 
@@ -438,7 +439,7 @@ class PitudraModel(torch.nn.Module):
         torch.bmm(olat.transpose(0, 1), p.uv_t, out=att.transpose(0, 1))
         return att.view(T, H * m.vdim)
 
-    def _attention(self, i, m, p, h, tab, T, prompt_shaped):
+    def _attention(self, i, m, p, h, tab, T, rows):
         HD, GD, GDV, HDV = m.heads * m.dim, m.kv_heads * m.dim, m.kv_heads * m.vdim, m.heads * m.vdim
         ld = HD + GD + GDV + HDV
         proj = self.buf_proj[:T * ld].view(T, ld)
@@ -450,8 +451,8 @@ class PitudraModel(torch.nn.Module):
         cap = ck.shape[1]
         k4, v4 = ck.view(self.n_slots, cap, m.kv_heads, m.dim), cv.view(self.n_slots, cap, m.kv_heads, m.vdim)
         gate = proj[:, HD + GD + GDV:]
-        if self.use_tiles and ld % 8 == 0 and ops.seq_window_attention_mma_supported(self.dtype, m.dim, 0, m.vdim, m.heads, m.kv_heads, prompt_shaped):
-            ops.seq_window_attention_mma(qf.view(T, m.heads, m.dim), k4, None, v4, att, tab, m.window, m.scale, prompt_shaped, sink=p.sink,
+        if self.use_tiles and ld % 8 == 0 and ops.seq_window_attention_mma_supported(self.dtype, m.dim, 0, m.vdim, m.heads, m.kv_heads, rows):
+            ops.seq_window_attention_mma(qf.view(T, m.heads, m.dim), k4, None, v4, att, tab, m.window, m.scale, rows, sink=p.sink,
                                          gate=gate)
         else:
             ops.seq_window_attention(qf.view(T, m.heads, m.dim), None, k4, v4, att, tab, m.window, m.scale, sink=p.sink, gate=gate)
@@ -486,7 +487,7 @@ class PitudraModel(torch.nn.Module):
             if m.kind == "latent_attention":
                 att = self._latent_attention(i, m, p, h, meta, T, prompt_shaped)
             elif m.kind == "attention":
-                att = self._attention(i, m, p, h, tab, T, prompt_shaped)
+                att = self._attention(i, m, p, h, tab, T, token_rows(meta, prompt_shaped))
             else:
                 att = self._hgrn2(i, m, p, h, meta, T)
             torch.matmul(att, p.o.t(), out=y)

@@ -10,6 +10,11 @@ TILES_MIN_TOKENS = 64           # a step with fewer tokens, or fewer than 16 per
 PROMPT_TILES_MIN_CTAS = 64      # (64-token blocks x heads) from which a prompt portion takes the tile form of its attention
 
 
+def token_rows(meta: BatchMeta, prompt_shaped: bool) -> int:
+    """What `ops.seq_window_attention_mma` is told about the step's segments."""
+    return 0 if not prompt_shaped else 2 if all(n >= ops.WINDOW_ROWS_SEGMENT for _, _, _, n in meta.segments) else 1
+
+
 def attend_window(qf: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor, out: torch.Tensor, meta: BatchMeta, window: int,
                   scale: float, *, tiles: bool, min_tokens: int = TILES_MIN_TOKENS, min_ctas: int = PROMPT_TILES_MIN_CTAS, **kw) -> None:
     """Softmax attention of the step's queries qf [T, H, D] over a layer's cache rows (window, kept tokens, sink, gates: see
@@ -25,7 +30,7 @@ def attend_window(qf: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tensor
             ops.seq_prompt_attention_mma(qf, cache_k, None, cache_v, out, meta.segments[0][1], meta.segments[0][2], window, scale, **kw)
             return
         if ops.seq_window_attention_mma_supported(out.dtype, D, 0, DV, H, G, prompt_shaped):
-            ops.seq_window_attention_mma(qf, cache_k, None, cache_v, out, meta.table, window, scale, prompt_shaped, **kw)
+            ops.seq_window_attention_mma(qf, cache_k, None, cache_v, out, meta.table, window, scale, token_rows(meta, prompt_shaped), **kw)
             return
     ops.seq_window_attention(qf, None, cache_k, cache_v, out, meta.table, window, scale, **kw)
 

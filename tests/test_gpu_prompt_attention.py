@@ -307,3 +307,38 @@ def test_window_tiles_match_float64(ops, H, G, window, cap, segments, gate, sink
     assert err <= 2 ** -8 * want.abs().max().item(), err       # bfloat16 outputs: half a unit in the last place is 2^-9 of a value
     assert float(wide[:, H * 128:].abs().max()) == 0.0
     assert ops.attn_tile_timeouts() == 0
+
+
+@pytest.mark.parametrize("segments", [
+    [(k, 700 + 5 * k, 1) for k in range(37)] + [(40, 300, 170)],               # decoding sequences in front of a prompt
+    [(0, 0, 15), (1, 900, 16), (2, 40, 17), (3, 1500, 3), (4, 7, 1)],           # both sides of the line
+    [(0, 500, 4), (1, 0, 2)],                                                   # fewer tokens than a run
+    [(k, 620 + 11 * k, 2 + k % 14) for k in range(30)],                         # pieces of every size, more than there are CTAs in a row
+    [(0, 10, 20), (0, 30, 5), (1, 0, 16)],                                      # a segment that continues its neighbour
+])
+@pytest.mark.parametrize("H,G", [(16, 4), (12, 4), (16, 1), (32, 1)])            # 32 heads per group: no form with heads as rows
+def test_window_of_mixed_steps(ops, H, G, segments):
+    """Prompt portions beside decoding sequences: every token once, whichever form takes it."""
+    g = torch.Generator(device="cuda").manual_seed(31)
+    window, cap = 600, 900
+    slots = 1 + max(s for s, _, _ in segments)
+    meta, at = [], 0
+    for s, p0, n in segments:
+        meta += [(s, p0 + i, at, at + n, 0) for i in range(n)]
+        at += n
+    meta = torch.tensor(meta, dtype=torch.int32).T.contiguous().cuda()
+    q = torch.randn(at, H, 128, generator=g, device="cuda")
+    ck = torch.randn(slots, cap, G, 128, generator=g, device="cuda").bfloat16()
+    cv = torch.randn(slots, cap, G, 128, generator=g, device="cuda").bfloat16()
+    sink = torch.randn(H, generator=g, device="cuda")
+    for rows in (1, 2) if min(n for _, _, n in segments) >= 16 else (1,):
+        out = torch.full((at, H, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.seq_window_attention_mma(q, ck, None, cv, out, meta, window, 0.09, rows, sink=sink)
+        for t in range(at):
+            slot, pos = int(meta[0, t]), int(meta[1, t])
+            j = torch.arange(max(0, pos - window + 1), pos + 1, device="cuda") % cap
+            s = torch.einsum("hd,jhd->hj", q[t].bfloat16().double(), ck[slot, j].double().repeat_interleave(H // G, 1)) * 0.09
+            w = torch.softmax(torch.cat([s, sink.double()[:, None]], 1), 1)[:, :-1]
+            want = torch.einsum("hj,jhd->hd", w, cv[slot, j].double().repeat_interleave(H // G, 1))
+            assert (out[t].double() - want).abs().max() <= 2 ** -8 * want.abs().max(), t
+    assert ops.attn_tile_timeouts() == 0
