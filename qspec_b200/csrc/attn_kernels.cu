@@ -539,12 +539,13 @@ static int launch_attn_block(const void* qkv, const void* cos_sin, const int* po
 
 // ------------------------------------------------------------------------------------------
 // Attention for passes with MANY sequences (32 and 64 concurrent sequences are typical; verify passes of
-// (k + 1) tokens per sequence): one 128-thread CTA per (sequence, kv head) reads that head's key and value rows ONCE
+// (k + 1) tokens per sequence): one CTA per (sequence, kv head) reads that head's key and value rows ONCE
 // for all tokens of the sequence in the pass and all G query heads of the GQA group (decode_attention_kernel reads them
 // once per (token, query head): 16x the cache traffic at G = 4, k + 1 = 4), and does the arithmetic on the tensor
 // cores (mma.sync m16n8k16, f16 operands, fp32 accumulate) -- on CUDA cores the same loop is issue-bound at ~45-70 us
 // for 64 sequences.
-//   * 16 query rows per chunk = R tokens x G heads (R = 16 / G). The 4 warps split the keys; every warp runs a
+//   * 16 query rows per chunk = R tokens x G heads (R = 16 / G). In passes of up to SEQ_CHUNKS tokens a CTA takes one chunk, so that a
+//     prompt portion spreads over the GPU as well as many sequences do, in one launch. The 4 or 8 warps split the keys; every warp runs a
 //     flash-decoding loop over 16-key blocks with an online softmax, then the warps' (max, sum, O) are merged in shared memory.
 //   * Keys and values come by bulk copies, one per 256-byte row, into a ring of ST 16-key blocks per warp: a block's successor in its place
 //     is asked for as soon as its keys (values) are multiplied. Loaded straight into the fragments, 16-byte pieces of 32 different sectors
@@ -577,6 +578,7 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t& hi, uint32_
   lo = pack_h2(x - hf.x, y - hf.y);
 }
 
+constexpr int SEQ_CHUNKS = 64;                               // passes of up to so many tokens: a CTA per chunk of 16 query rows
 constexpr int SEQ_KS = 256 + 64, SEQ_VS = 256 + 16;         // bytes between the rows of a block in shared memory
 constexpr int SEQ_BLOCK = 16 * (SEQ_KS + SEQ_VS);           // 16 keys and values
 
@@ -584,12 +586,12 @@ template <int G, int ST, int NW>                              // NW warps split 
 __global__ void __launch_bounds__(NW * 32, ST == 1 ? 4 : NW == 4 ? 2 : 1)
 seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ cache_k, const __half* __restrict__ cache_v,
                      const int* __restrict__ positions, const int* __restrict__ seq_ids, __half* __restrict__ out,
-                     int T, int Hq, int Hkv, int S, float sm_scale, int min_run) {
+                     int T, int B, int Hq, int Hkv, int S, float sm_scale, int min_run) {
   pdl_enter();
   constexpr int D = 128, R = 16 / G;                         // R tokens x G heads <= 16 query rows per chunk
   __shared__ int s_tok[1024];                                // tokens of this sequence in the pass (T <= 1024)
   __shared__ int s_pos[1024];                                // ... and their positions (loaded in the same round trip as the scan)
-  __shared__ int s_ntok;
+  __shared__ int s_ntok, s_seq;
   __shared__ float s_m[NW][16], s_l[NW][16];
   __shared__ __align__(16) uint4 s_qf[8][32];                // Q fragments of the chunk in mma order: [k-step][lane] = (a0, a1, a2, a3)
   __shared__ __align__(8) uint64_t s_full[NW][2][ST];         // keys, values of a warp's blocks
@@ -597,25 +599,69 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   extern __shared__ __align__(16) unsigned char seq_dyn[];   // [NW][ST] blocks; after the keys:
   constexpr int OS = D + 4;                                  // (row stride of the partial outputs: the rows of a store fall on different banks)
   float (*s_o)[16][OS] = reinterpret_cast<float (*)[16][OS]>(seq_dyn);   // [NW][16][OS] fp32: per-warp partial outputs
-  const int seq = blockIdx.x / Hkv, hk = blockIdx.x % Hkv;    // the heads of a sequence side by side: their rows are neighbours in the cache
+  int seq = blockIdx.x / Hkv;                                 // (T <= SEQ_CHUNKS: the number of a chunk, see below)
+  const int hk = blockIdx.x % Hkv;                            // the heads of a sequence side by side: their rows are neighbours in the cache
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
   if (tid == 0) {
     s_ntok = 0;
     s_fail = 0;
-    for (int i = 0; i < NW * 2 * ST; ++i) atile::bar_init(atile::smem_addr(&s_full[0][0][0] + i), 1);
+  }
+  if (tid < NW * 2 * ST) {
+    atile::bar_init(atile::smem_addr(&s_full[0][0][0] + tid), 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  __syncthreads();
-  for (int t = tid; t < T; t += NW * 32) {
-    const int sq = __ldg(seq_ids + t), ps = __ldg(positions + t);
-    if (sq == seq) {
-      const int i = atomicAdd(&s_ntok, 1);
-      s_tok[i] = t;
-      s_pos[i] = ps;
+  if (T <= SEQ_CHUNKS) {
+    // chunk c of the pass: R tokens of one sequence, in batch order; the chunks are numbered by their first tokens
+    const int chunk = seq;
+    if (tid < T) { s_tok[SEQ_CHUNKS + tid] = __ldg(seq_ids + tid); s_pos[SEQ_CHUNKS + tid] = __ldg(positions + tid); }
+    __syncthreads();
+    if (warp == 0) {
+      int sq[2], rank[2] = {0, 0};                            // tokens lane and lane + 32: sequence (-1: none), how many of it come before
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = lane + 32 * i;
+        sq[i] = t < T ? s_tok[SEQ_CHUNKS + t] : -1;
+        if ((unsigned)sq[i] >= (unsigned)B) sq[i] = -1;
+      }
+      const uint32_t before = (1u << lane) - 1u;
+      rank[0] = __popc(__match_any_sync(0xffffffffu, sq[0]) & before);
+      if (T > 32) {
+        rank[1] = __popc(__match_any_sync(0xffffffffu, sq[1]) & before);
+        for (int u = 0; u < 32; ++u) rank[1] += s_tok[SEQ_CHUNKS + u] == sq[1];
+      }
+      const uint32_t first0 = __ballot_sync(0xffffffffu, sq[0] >= 0 && rank[0] % R == 0), first1 = __ballot_sync(0xffffffffu, sq[1] >= 0 && rank[1] % R == 0);
+      const int n0 = __popc(first0);
+      int n = 0;
+      if (chunk < n0 + __popc(first1)) {
+        const bool low = chunk < n0;                          // the chunk's first token: among the first 32 or the others
+        const uint32_t first = low ? first0 : first1;
+        const int src = __ffs(__ballot_sync(0xffffffffu, (first >> lane & 1u) && __popc(first & before) == (low ? chunk : chunk - n0))) - 1;
+        const int my_seq = __shfl_sync(0xffffffffu, low ? sq[0] : sq[1], src), from = __shfl_sync(0xffffffffu, low ? rank[0] : rank[1], src);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const bool mine = sq[i] == my_seq && rank[i] >= from && rank[i] < from + R;
+          if (mine) { s_tok[rank[i] - from] = lane + 32 * i; s_pos[rank[i] - from] = s_pos[SEQ_CHUNKS + lane + 32 * i]; }
+          n += __popc(__ballot_sync(0xffffffffu, mine));
+        }
+        if (lane == 0) s_seq = my_seq;
+      }
+      if (lane == 0) s_ntok = n;
     }
+    __syncthreads();
+    seq = s_seq;
+  } else {
+    __syncthreads();
+    for (int t = tid; t < T; t += NW * 32) {
+      const int sq = __ldg(seq_ids + t), ps = __ldg(positions + t);
+      if (sq == seq) {
+        const int i = atomicAdd(&s_ntok, 1);
+        s_tok[i] = t;
+        s_pos[i] = ps;
+      }
+    }
+    __syncthreads();
   }
-  __syncthreads();
   int ntok = s_ntok;
   if (min_run && ntok >= min_run) {                          // gather again without the tokens of prompt runs: attn_tile_kernel's
     __syncthreads();
@@ -831,8 +877,10 @@ static int launch_seq_attention_st(const void* qkv, const void* ck, const void* 
     QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
   }
-  launch_pdl(kern, dim3(B * Hkv), dim3(NW * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
-             positions, seq_ids, (__half*)out, T, Hq, Hkv, S, sm_scale, min_run);
+  // T <= SEQ_CHUNKS: sequences with a token and whole chunks bound the number of chunks
+  const int units = T <= SEQ_CHUNKS ? min(T, min(B, T) + T / (16 / G)) : B;
+  launch_pdl(kern, dim3(units * Hkv), dim3(NW * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,
+             positions, seq_ids, (__half*)out, T, B, Hq, Hkv, S, sm_scale, min_run);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
 }
@@ -997,7 +1045,9 @@ extern "C" int qspec_seq_attention(const void* qkv, const void* cache_k, const v
                 "seq_attention: unsupported T=%d Hq=%d Hkv=%d D=%d S=%d (use decode_attention)", T, Hq, Hkv, D, S);
   cudaStream_t st = (cudaStream_t)stream;
   int min_run = 0;
-  if (T >= 2 * RUN) {
+  // Up to 64 tokens the chunks of a prompt portion spread over the GPU as they are, and the launch that looks for runs costs more than it
+  // gives: it made 8 x 4 tokens after 20 .. 400 9.0 .. 13.7 us that were 5.8 .. 11.9 without it (32 / 8 heads).
+  if (T > SEQ_CHUNKS) {
     const int rc = launch_runs(qkv, cache_k, cache_v, positions, seq_ids, out, T, B, Hq, Hkv, S, sm_scale, 0, &min_run, st);
     if (rc != QSPEC_OK) return rc;
   }

@@ -74,6 +74,25 @@ def test_prompt_runs_match_float64(ops, Hq, Hkv, S, segments):
     assert ops.attn_tile_timeouts() == 0
 
 
+@pytest.mark.parametrize("Hq,Hkv", [(8, 8), (16, 8), (32, 8), (40, 8), (64, 8)])
+@pytest.mark.parametrize("segments", [
+    [(0, 100, 64)],                                               # one sequence: every chunk its own CTA
+    [(5, 7, 63)],
+    [(3, 40, 1)],
+    [(1, 250, 33), (0, 0, 31)],                                   # the numbering passes from the first 32 tokens to the others
+    [(k % 9, 20 * (k % 9) + k // 9, 1) for k in range(64)],       # a sequence's tokens all over the batch
+    [(k, 299 - 3 * k, 1 + k % 3) for k in range(30)],
+])
+def test_passes_of_up_to_64_tokens_are_one_launch(ops, Hq, Hkv, segments):
+    from qspec_b200 import _lib
+    qkv, ck, cv, pos, seq = batch(segments, Hq, Hkv, 310, 1 + max(s for s, _, _ in segments) + 40, seed=9)
+    out = torch.full((len(pos), Hq * 128), float("nan"), dtype=torch.float16, device="cuda")
+    before = _lib.load().qspec_launch_count()
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 128 ** -0.5)
+    assert _lib.load().qspec_launch_count() - before == 1
+    check_rows(out, reference(qkv, ck, cv, pos, seq, Hq, Hkv, 128 ** -0.5), Hq, 5.0)
+
+
 @pytest.mark.parametrize("Hq,Hkv", [(24, 8), (48, 3), (32, 32)])
 def test_decode_attention_takes_long_runs_too(ops, Hq, Hkv):
     """Head counts that the one-launch attention block does not take; positions that jump inside a sequence are no run."""
