@@ -68,15 +68,25 @@ decode_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict
   __shared__ float qs[D];
   __shared__ float red[4];
   __shared__ float accs[4][D];
+  __shared__ bool run;
   const int tok = blockIdx.x, h = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pos = positions[tok], seq = seq_ids[tok];
+  // (the neighbours in the same round trip: a token with neither next to it in its sequence is in no run, and the others are asked by one
+  // warp; 256 x 1 tokens over 20 keys, 24 / 8 heads: 18.9 us against 19.4 with all four warps asking for every token)
+  const int tl = max(tok - 1, 0), tr = min(tok + 1, T - 1);
+  const int pl = positions[tl], sl = seq_ids[tl], pr = positions[tr], sr = seq_ids[tr];
+  const bool ask = min_run && ((sl == seq && pl + 1 == pos) || (sr == seq && pr == pos + 1));
   if ((unsigned)pos >= (unsigned)S) return;               // out of the cache / rotary table: nothing valid to attend to
-  if (min_run && atile::attn_token_in_run(positions, seq_ids, T, tok, min_run)) return;   // attn_tile_kernel's
   const int nkeys = pos + 1;
   const int hk = h / (Hq / Hkv);
   qs[tid] = __half2float(qkv[(size_t)tok * (Hq + 2 * Hkv) * D + (size_t)h * D + tid]) * sm_scale;
+  if (ask && warp == 0) {
+    const bool r = atile::attn_token_in_run(positions, seq_ids, T, tok, min_run);
+    if (lane == 0) run = r;
+  }
   __syncthreads();
+  if (ask && run) return;                                 // attn_tile_kernel's
   const __half* kbase = cache_k + ((size_t)seq * S * Hkv + hk) * D;
   const __half* vbase = cache_v + ((size_t)seq * S * Hkv + hk) * D;
   float lmax = -INFINITY;
