@@ -254,10 +254,12 @@ int qspec_seq_lightning(const void* p, int ld, const float* decay, const float* 
                         void* stream);
 
 /* The two recurrences over long segments in chunks that run side by side (the walk through a segment's tokens is a chain): same arguments
- * and results (float32 throughout; another order of products of decays), and a workspace of qspec_seq_recurrence_chunk_bytes(..) bytes on
- * a 16-byte boundary, which the call may leave anything in. 0 bytes: these sizes are walked token by token (segments shorter than
- * 256 tokens on average, key or value sizes other than 64 and 128), as they are without a workspace or without seg_starts. */
+ * and results (float32 throughout; another order of products of decays), and a workspace of qspec_seq_recurrence_chunk_bytes(..) bytes
+ * (qspec_seq_lightning_chunk_bytes for the scalar decay) on a 16-byte boundary, which the call may leave anything in. 0 bytes: these sizes
+ * are walked token by token (segments shorter than 256 to 336 tokens on average, key or value sizes other than 64 and 128, a scalar decay
+ * with more segments and heads than the walk leaves room for), as they are without a workspace or without seg_starts. */
 size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV);
+size_t qspec_seq_lightning_chunk_bytes(int nseg, int ntok, int H, int D, int DV);
 int qspec_seq_hgrn2_chunked(const void* p, int ld, const float* f_b, const float* lower, const float* norm_w, float* state,
                             float* scratch, void* out, const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D,
                             int DV, float eps, int dtype, void* workspace, size_t workspace_bytes, void* stream);

@@ -324,19 +324,27 @@ hgrn2_gates_kernel(const T* __restrict__ p, int ld, const float* __restrict__ f_
 }
 
 
-// ---- scalar-decay linear attention: q = silu(zq), k = silu(zk), float32, once per (token, row); gates [ntok][2][H * D] ----
+// ---- scalar-decay linear attention: q = silu(zq), k = silu(zk), float32, once per (token, row); gates [ntok][2][H * D]. vs (or NULL)
+// [ntok][H * DV]: silu(zv), for the chunk form, whose passes would compute it once each (64 heads of 64 x 64, 9 x 600
+// tokens: 1101 -> 748 us) ----
 template <typename T>
 __global__ void __launch_bounds__(256)
-lightning_gates_kernel(const T* __restrict__ p, int ld, float* __restrict__ gates, int HD, int ntok) {
+lightning_gates_kernel(const T* __restrict__ p, int ld, float* __restrict__ gates, int HD, int ntok, float* __restrict__ vs, int HDV) {
   pdl_enter();
   const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c >= HD) return;
+  const bool qk = c < HD, v = vs && c < HDV;
   for (int t = blockIdx.y; t < ntok; t += gridDim.y) {
     const T* row = p + (size_t)t * ld;
-    const float zq = to_f(row[c]), zk = to_f(row[HD + c]);
-    float* g = gates + (size_t)t * 2 * HD + c;
-    g[0] = zq / (1.0f + expf(-zq));
-    g[HD] = zk / (1.0f + expf(-zk));
+    if (qk) {
+      const float zq = to_f(row[c]), zk = to_f(row[HD + c]);
+      float* g = gates + (size_t)t * 2 * HD + c;
+      g[0] = zq / (1.0f + expf(-zq));
+      g[HD] = zk / (1.0f + expf(-zk));
+    }
+    if (v) {
+      const float zv = to_f(row[2 * HD + c]);
+      vs[(size_t)t * HDV + c] = zv / (1.0f + expf(-zv));
+    }
   }
 }
 
@@ -570,8 +578,8 @@ hgrn2_scan_kernel(const T* __restrict__ p, int ld, const float* __restrict__ gat
 // two in flight; the row groups' shares of the outputs meet in shared memory once per block. What bounds it is shared
 // memory: a thread reads 56 floats for 64 elements of state, 90 wavefronts a token and warp in the output pass (73 % of the pipe), above
 // the 384 cycles a token and head that its multiply-adds need.
-// 1500 tokens, 16 heads of 128 x 128, all launches: 325 -> 146 us (gates 13, E 44, carry 9, outputs 89); 2000 tokens, 8 heads of 64 x 64:
-// 481 -> 66 us.
+// 1500 tokens, 16 heads of 128 x 128, all launches: 325 -> 144 us (each by itself, overlaps not taken off: gates 13, E 44, carry 9, outputs
+// 89); 2000 tokens, 8 heads of 64 x 64: 473 -> 61 us.
 constexpr int RC_BT = 8;                                     // tokens per block
 
 __device__ __forceinline__ uint64_t rc_fma(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
@@ -658,9 +666,8 @@ recurrence_chunk_kernel(const T* __restrict__ p, int ld, const float* __restrict
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int e = tid + NT * i, t = min(tb + e / DV, t1 - 1);
-      float v = to_f(vp[(size_t)t * ld + e % DV]);
-      if (decay) v = v / (1.0f + expf(-v));                   // the scalar-decay form takes silu(v)
-      vr[i] = v;
+      // the scalar-decay form takes silu(v), which waits where the row's outputs will go: every row is read a block before it is written
+      vr[i] = decay ? o[((size_t)t * H + h) * DV + e % DV] : to_f(vp[(size_t)t * ld + e % DV]);
     }
   };
   // this thread's rows: 4 rg .. + 3 and the same D / 4, D / 2 and 3 D / 4 further (a load then covers neighbouring 16-byte pieces), as pairs
@@ -1026,11 +1033,18 @@ static int rc_chunk_tokens(int ntok, int H, int D, int DV) {
   const long long c = (((long long)ntok * H + slots - 1) / slots + RC_BT - 1) / RC_BT * RC_BT;
   return (int)(c < 32 ? 32 : c);
 }
-static bool rc_taken(int nseg, int ntok, int H, int D, int DV) {
+static bool rc_taken(int nseg, int ntok, int H, int D, int DV, bool scalar_decay) {
   if (!((D == 64 || D == 128) && (DV == 64 || DV == 128)) || nseg < 1 || sm_count() < 1) return false;
-  // The walk takes 8 us + 0.2 us a token, the chunks' four launches at least 50 us: 200 tokens of 16 heads of 128 x 128 48 against 53 us,
-  // two sequences of 300 of 16 heads of 64 x 64 82 against 52, 600 of 8 heads 86 against 39.
-  return ntok >= 256 * (long long)nseg && ntok >= 2 * (long long)nseg * rc_chunk_tokens(ntok, H, D, DV);
+  // The walk takes 0.2 us a token while its CTAs (a segment, a head, 16 columns each) fit the GPU side by side; the chunks take four launches,
+  // 35 to 60 us, and from there what their multiply-adds need. Where the two meet (us, walk : chunks; 300 tokens and less to a segment):
+  // 128 x 128, 256 tokens: 8 heads 58 : 62, 32 heads 63 : 68; 300 tokens: 16 heads 69 : 61, 32 heads 72 : 75; 600 tokens: 32 heads 138 : 120.
+  // 64 x 64, 256 tokens: 8 heads 57 : 35, 64 heads 75 : 57.
+  // The walk of a scalar decay is the cheaper one once its CTAs come in several rounds: 64 x 64, 8 segments of 300, 32 heads 167 : 178, 9 of
+  // 600, 64 heads 706 : 748, against 2 of 600, 64 heads 192 : 173, 4 of 1500, 64 heads 791 : 771.
+  const long long walkers = (long long)nseg * H * (DV / 16);
+  int least = D * DV < 128 * 128 || walkers <= 32 ? 256 : walkers <= 128 ? 288 : 336;
+  if (scalar_decay && D * DV < 128 * 128 && walkers > 512) least = walkers > 1024 ? 0x7fffffff : 1000;
+  return ntok >= least * (long long)nseg && ntok >= 2 * (long long)nseg * rc_chunk_tokens(ntok, H, D, DV);
 }
 
 template <typename T, int D, int DV>
@@ -1073,8 +1087,8 @@ template <typename T>
 static int launch_hgrn2(const void* p, int ld, const float* f_b, const float* lower, float* state, float* o, float* gates, const int* meta,
                         const int* seg_starts, int nseg, int ntok, int H, int D, int DV, cudaStream_t st, const float* decay, void* ws, void* out,
                         const float* norm_w, float eps) {
-  const unsigned gx = (unsigned)((H * D + 255) / 256), gy = (unsigned)max(1, min(ntok, 148 * 16 / (int)gx));
-  if (decay) launch_pdl(lightning_gates_kernel<T>, dim3(gx, gy), dim3(256), 0, st, (const T*)p, ld, gates, H * D, ntok);
+  const unsigned gx = (unsigned)((H * (decay && ws ? max(D, DV) : D) + 255) / 256), gy = (unsigned)max(1, min(ntok, 148 * 16 / (int)gx));
+  if (decay) launch_pdl(lightning_gates_kernel<T>, dim3(gx, gy), dim3(256), 0, st, (const T*)p, ld, gates, H * D, ntok, ws ? o : nullptr, H * DV);
   else launch_pdl(hgrn2_gates_kernel<T>, dim3(gx, gy), dim3(256), 0, st, (const T*)p, ld, f_b, lower, gates, H * D, ntok);
   QSPEC_CHECK_LAUNCH(1);
   if (ws) return launch_recurrence_chunks<T>(p, ld, gates, state, o, out, norm_w, eps, meta, seg_starts, nseg, ntok, H, D, DV, decay, ws, st);
@@ -1091,14 +1105,18 @@ static int launch_hgrn2(const void* p, int ld, const float* f_b, const float* lo
   return QSPEC_OK;
 }
 
-extern "C" size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV) {
-  if (ntok < 1 || H < 1 || D < 1 || DV < 1 || !rc_taken(nseg, ntok, H, D, DV)) return 0;
+static size_t rc_bytes(int nseg, int ntok, int H, int D, int DV, bool scalar_decay) {
+  if (ntok < 1 || H < 1 || D < 1 || DV < 1 || !rc_taken(nseg, ntok, H, D, DV, scalar_decay)) return 0;
   return (size_t)(ntok / rc_chunk_tokens(ntok, H, D, DV) + nseg) * H * ((size_t)D * DV + D) * sizeof(float);
 }
 
+extern "C" size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV) { return rc_bytes(nseg, ntok, H, D, DV, false); }
+extern "C" size_t qspec_seq_lightning_chunk_bytes(int nseg, int ntok, int H, int D, int DV) { return rc_bytes(nseg, ntok, H, D, DV, true); }
+
 // The chunk form's buffer, if these sizes take it and the caller brought one that fits (rows are read 16 bytes at a time).
-static void* chunk_workspace(void* ws, size_t bytes, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, const void* scratch, const void* state) {
-  const size_t need = seg_starts && ws ? qspec_seq_recurrence_chunk_bytes(nseg, ntok, H, D, DV) : 0;
+static void* chunk_workspace(void* ws, size_t bytes, const int* seg_starts, int nseg, int ntok, int H, int D, int DV, const void* scratch, const void* state,
+                             bool scalar_decay) {
+  const size_t need = seg_starts && ws ? rc_bytes(nseg, ntok, H, D, DV, scalar_decay) : 0;
   return need && bytes >= need && (((uintptr_t)ws | (uintptr_t)scratch | (uintptr_t)state) & 15) == 0 ? ws : nullptr;
 }
 
@@ -1112,7 +1130,7 @@ extern "C" int qspec_seq_hgrn2_chunked(const void* p, int ld, const float* f_b, 
   MIX_DTYPE_OK(dtype);
   if (ntok == 0) return QSPEC_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  void* ws = chunk_workspace(workspace, workspace_bytes, seg_starts, nseg, ntok, H, D, DV, scratch, state);
+  void* ws = chunk_workspace(workspace, workspace_bytes, seg_starts, nseg, ntok, H, D, DV, scratch, state, false);
   float* gates = scratch + (size_t)ntok * H * DV;          // scratch: un-normalised outputs, then the gates
   int s = dtype == QSPEC_DTYPE_F32
               ? launch_hgrn2<float>(p, ld, f_b, lower, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, nullptr, ws, out, norm_w, eps)
@@ -1270,7 +1288,7 @@ extern "C" int qspec_seq_lightning_chunked(const void* p, int ld, const float* d
   if (ntok == 0) return QSPEC_OK;
   cudaStream_t st = (cudaStream_t)stream;
   float* gates = scratch + (size_t)ntok * H * DV;          // scratch: un-normalised outputs, then silu(q) and silu(k)
-  void* ws = chunk_workspace(workspace, workspace_bytes, seg_starts, nseg, ntok, H, D, DV, scratch, state);
+  void* ws = chunk_workspace(workspace, workspace_bytes, seg_starts, nseg, ntok, H, D, DV, scratch, state, true);
   int s = dtype == QSPEC_DTYPE_F32
               ? launch_hgrn2<float>(p, ld, nullptr, nullptr, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, decay, ws, nullptr, nullptr, eps)
               : launch_hgrn2<bf16_t>(p, ld, nullptr, nullptr, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, decay, ws, nullptr, nullptr, eps);

@@ -102,3 +102,30 @@ def test_scalar_decay_recurrence(ops, H, D, DV, segments, dtype):
     assert (out.double() - want).abs().max() <= tol * want.abs().max()
     for slot, _, _ in segments:
         assert (state[slot].double() - want_state[slot]).abs().max() <= 2e-5 * want_state[slot].abs().max()
+
+
+@pytest.mark.parametrize("H,D,DV,segments,gated,scalar", [
+    (64, 64, 64, [(0, 0, 300), (1, 5, 300), (2, 0, 300), (3, 9, 300)], True, False),   # the scalar decay's walk is the faster one here
+    (32, 128, 128, [(0, 0, 300)], False, False),                                       # and both are here
+    (16, 128, 64, [(0, 3, 700)], True, True),
+])
+def test_both_sides_of_the_rule(ops, H, D, DV, segments, gated, scalar):
+    """Which form is taken, and that the scalar decay gives the same on either side."""
+    from qspec_b200 import _lib
+    meta, starts = table(segments)
+    T, lib = meta.shape[1], _lib.load_seq()
+    assert (lib.qspec_seq_recurrence_chunk_bytes(len(segments), T, H, D, DV) > 0) == gated
+    assert (lib.qspec_seq_lightning_chunk_bytes(len(segments), T, H, D, DV) > 0) == scalar
+    g = torch.Generator(device="cuda").manual_seed(H)
+    p = torch.randn(T, 2 * H * (D + DV), generator=g, device="cuda")
+    decay, norm = torch.rand(H, generator=g, device="cuda") * 0.5 + 0.5, torch.randn(H * DV, generator=g, device="cuda")
+    state = torch.randn(len(segments), H, D, DV, generator=g, device="cuda")
+    want_state, z = state.double(), p.double()
+    s = z * torch.sigmoid(z)
+    q, k, v = s[:, :H * D].view(T, H, D), s[:, H * D:2 * H * D].view(T, H, D), s[:, 2 * H * D:2 * H * D + H * DV].view(T, H, DV)
+    o = walk(q, decay.double()[None, :, None].expand(T, H, D), k, v, segments, want_state).reshape(T, H * DV)
+    want = o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-5) * norm.double() * torch.sigmoid(z[:, 2 * H * D + H * DV:])
+    out = torch.empty(T, H * DV, device="cuda")
+    ops.seq_lightning(p, decay, norm, state, torch.empty(T * H * (DV + 2 * D), device="cuda"), out, meta, H, D, DV, 1e-5, seg_starts=starts)
+    assert (out.double() - want).abs().max() <= 2e-5 * want.abs().max()
+    assert (state.double() - want_state).abs().max() <= 2e-5 * want_state.abs().max()
