@@ -24,7 +24,7 @@
 //
 // A row sees nothing but its own keys, bit for bit: hidden keys enter the products with weights of exactly zero, and a row is rescaled by
 // its own maximum alone. A weight of zero times a value that is not finite would be NaN: rows with a result that is not finite are computed
-// again key by key (attn_row_again).
+// again key by key (attn_rows_again).
 //
 // Every wait is bounded; a CTA whose wait runs out waits (again with a limit) for its copies and products under way, fills its rows with
 // NaN, so that nobody takes what the buffer held for a result, counts itself in attn_tile_timeouts and frees its tensor memory.
@@ -233,41 +233,84 @@ struct Items {
   }
 };
 
-// 64 columns of one row key by key on the CUDA cores (float32 weights, nothing but the row's own keys): rows whose tile result is not finite.
+// Rows whose tile result is not finite, once more on the CUDA cores: float32 weights, nothing but the row's own keys. A whole warp per row,
+// every lane with keys of its own (a thread per row took 100 times as long, and one infinite value in a cache is enough for every later row).
+// rows: the lanes that ask; 64 columns from col0 on of the row that each describes.
 template <bool BF, bool QF32>
-__device__ __noinline__ void attn_row_again(const Args& a, int tok, int head, int kvh, int seq, int lo, int hi, int col0) {
+__device__ __noinline__ void attn_rows_again(const Args& a, uint32_t rows, int tok_, int head_, int kvh, int seq_, int lo_, int hi_, int col0) {
   using T = typename Elem<BF>::T;
-  const T* kbase = (const T*)a.k + (size_t)seq * a.k_ss + (size_t)kvh * a.k_hs;
-  const T* vbase = (const T*)a.v + (size_t)seq * a.v_ss + (size_t)kvh * a.v_hs;
-  const size_t qo = (size_t)tok * a.q_ts + (size_t)head * a.q_hs;
-  auto qd = [&](int d) -> float {
-    if (QF32) return Elem<BF>::unpack(Elem<BF>::pack(((const float*)a.q)[qo + d], 0.f)).x;
-    return (float)((const T*)a.q)[qo + d];
-  };
-  auto row = [&](int j) { return a.ring && j >= a.cap ? j % a.cap : j; };
-  auto score = [&](int j) {
-    const T* kr = kbase + (size_t)row(j) * a.k_rs;
-    float s = 0.f;
-    for (int d = 0; d < 128; ++d) s = fmaf((float)kr[d], qd(d), s);
-    return s * a.scale;
-  };
-  float m = -INFINITY;
-  for (int j = lo; j <= hi; ++j) m = fmaxf(m, score(j));
-  if (a.sink) m = fmaxf(m, a.sink[head]);
-  float l = a.sink ? __expf(a.sink[head] - m) : 0.f;
-  for (int j = lo; j <= hi; ++j) l += __expf(score(j) - m);
-  for (int d0 = col0; d0 < col0 + 64; d0 += 16) {
-    float o[16];
-    for (int d = 0; d < 16; ++d) o[d] = 0.f;
-    for (int j = lo; j <= hi; ++j) {
+  const int lane = threadIdx.x & 31;
+  for (; rows; rows &= rows - 1u) {
+    const int src = __ffs(rows) - 1;
+    const int tok = __shfl_sync(0xffffffffu, tok_, src), head = __shfl_sync(0xffffffffu, head_, src), seq = __shfl_sync(0xffffffffu, seq_, src);
+    const int lo = __shfl_sync(0xffffffffu, lo_, src), hi = __shfl_sync(0xffffffffu, hi_, src);
+    const T* kbase = (const T*)a.k + (size_t)seq * a.k_ss + (size_t)kvh * a.k_hs;
+    const T* vbase = (const T*)a.v + (size_t)seq * a.v_ss + (size_t)kvh * a.v_hs + col0;
+    const size_t qo = (size_t)tok * a.q_ts + (size_t)head * a.q_hs;
+    auto row = [&](int j) { return a.ring && j >= a.cap ? j % a.cap : j; };
+    auto score = [&](int j) {
+      const uint4* kr = reinterpret_cast<const uint4*>(kbase + (size_t)row(j) * a.k_rs);
+      float s = 0.f;
+#pragma unroll 2
+      for (int c = 0; c < 16; ++c) {
+        const uint4 kw = kr[c];
+        const uint32_t kk[4] = {kw.x, kw.y, kw.z, kw.w};
+        uint32_t qq[4];
+        if (QF32) {
+          const float4 x = *reinterpret_cast<const float4*>((const float*)a.q + qo + c * 8), y = *reinterpret_cast<const float4*>((const float*)a.q + qo + c * 8 + 4);
+          qq[0] = Elem<BF>::pack(x.x, x.y); qq[1] = Elem<BF>::pack(x.z, x.w); qq[2] = Elem<BF>::pack(y.x, y.y); qq[3] = Elem<BF>::pack(y.z, y.w);
+        } else {
+          const uint4 w = *reinterpret_cast<const uint4*>((const T*)a.q + qo + c * 8);
+          qq[0] = w.x; qq[1] = w.y; qq[2] = w.z; qq[3] = w.w;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = Elem<BF>::unpack(kk[e]), y = Elem<BF>::unpack(qq[e]);
+          s = fmaf(x.y, y.y, fmaf(x.x, y.x, s));
+        }
+      }
+      return s * a.scale;
+    };
+    float m = -INFINITY;
+    for (int j = lo + lane; j <= hi; j += 32) m = fmaxf(m, score(j));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (a.sink) m = fmaxf(m, a.sink[head]);
+    float l = a.sink && lane == 0 ? __expf(a.sink[head] - m) : 0.f;
+    float acc[64];
+#pragma unroll
+    for (int d = 0; d < 64; ++d) acc[d] = 0.f;
+    for (int j = lo + lane; j <= hi; j += 32) {
       const float p = __expf(score(j) - m);
-      const T* vr = vbase + (size_t)row(j) * a.v_rs + d0;
-      for (int d = 0; d < 16; ++d) o[d] = fmaf(p, (float)vr[d], o[d]);
+      l += p;
+      const uint4* vr = reinterpret_cast<const uint4*>(vbase + (size_t)row(j) * a.v_rs);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint4 vw = vr[c];
+        const uint32_t vv[4] = {vw.x, vw.y, vw.z, vw.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = Elem<BF>::unpack(vv[e]);
+          acc[c * 8 + 2 * e] = fmaf(p, x.x, acc[c * 8 + 2 * e]);
+          acc[c * 8 + 2 * e + 1] = fmaf(p, x.y, acc[c * 8 + 2 * e + 1]);
+        }
+      }
     }
-    for (int d = 0; d < 16; ++d) {
-      float r = o[d] / l * a.out_scale;
-      if (a.gate) r *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)tok * a.gate_ld + (a.gate_per_head ? head : head * a.out_hs + d0 + d)]));
-      ((T*)a.out)[(size_t)tok * a.out_ts + (size_t)head * a.out_hs + d0 + d] = (T)r;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    float mine[2] = {0.f, 0.f};                               // columns 2 lane, + 1
+#pragma unroll
+    for (int d = 0; d < 64; ++d) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
+      if (lane == d >> 1) mine[d & 1] = acc[d];
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int d = col0 + 2 * lane + e;
+      float r = mine[e] / l * a.out_scale;
+      if (a.gate) r *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)tok * a.gate_ld + (a.gate_per_head ? head : head * a.out_hs + d)]));
+      ((T*)a.out)[(size_t)tok * a.out_ts + (size_t)head * a.out_hs + d] = (T)r;
     }
   }
 }
@@ -652,7 +695,9 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
           }
         }
       }
-      if (bad && store && !dead) attn_row_again<BF, QF32>(a, c0 + tl, head, kvh, my_seq, my_lo, my_hi, h * 64);
+      // (a sum of weights that is not a number makes every column so: nothing to do again)
+      const uint32_t again = __ballot_sync(0xffffffffu, bad && store && !dead && l == l);
+      if (again) attn_rows_again<BF, QF32>(a, again, c0 + tl, head, kvh, my_seq, my_lo, my_hi, h * 64);
     }
   }
   fence_before();

@@ -116,6 +116,24 @@ def test_a_token_sees_nothing_but_its_own_keys(ops):
     assert not torch.isfinite(out[60:].view(40, 32, 128)[..., 5]).any()
 
 
+@pytest.mark.parametrize("Hq,Hkv", [(32, 8), (40, 8)])
+def test_infinite_values_and_scores_without_a_number(ops, Hq, Hkv):
+    """One infinite value that every later row sees, one NaN in a query, one in a key: what float64 makes of them, column by column."""
+    qkv, ck, cv, pos, seq = batch([(0, 150, 200)], Hq, Hkv, 400, 1, seed=15)
+    cv[0, 40, 0, 7] = float("inf")
+    cv[0, 200, 0, 7] = float("-inf")
+    cv[0, 170, 1, 64] = float("nan")
+    qkv[30, 2 * 128 + 3] = float("nan")                           # head 2 of token 30
+    ck[0, 300, 2, 9] = float("nan")                               # key/value head 2 from position 300 on
+    out = torch.empty(200, Hq * 128, dtype=torch.float16, device="cuda")
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 128 ** -0.5)
+    want = reference(qkv, ck, cv, pos, seq, Hq, Hkv, 128 ** -0.5)
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.isinf(), want.isinf()) and torch.equal(out[out.isinf()].sign().double(), want[want.isinf()].sign())
+    fine = want.isfinite()
+    check(torch.where(fine, out, 0), torch.where(fine, want, 0))
+
+
 def test_hidden_keys_leave_no_trace(ops):
     """The same tokens with other keys and values at later positions and in the sequence that shares their tile: bit for bit the same rows.
     Their own values are small, so that even a remainder of a hidden value of 6e4 times the smallest normal weight would show."""
