@@ -11,10 +11,12 @@
 //     go back over the scores they came from as a two-term 16-bit split (hi + lo: 22 / 16 mantissa bits, so that the second product is
 //     as good as one with float32 weights).
 //   * O += P V: weights from tensor memory, values from shared memory as they lie in the cache (the reduction runs over rows: the
-//     operand is "MN-major"); hi and lo terms are 8 + 8 instructions on the same value tile. It runs under the next block's softmax.
+//     operand is "MN-major"); hi and lo terms are 8 + 8 instructions on the same value tile. It runs under the next block's softmax. The lo
+//     terms have an accumulator of their own: every accumulation cuts at the accumulator's last bit, and half as many of them go to O
+//     (sums over 3000 keys whose values cancel: off by 8.0e-9 of the values, 5.6e-8 with one accumulator).
 //   * O is rescaled only when a row's maximum grew by more than 2^8 since the last rescale (weights then stay below 256, and the
 //     division by the sum at the end undoes the common factor).
-// Tensor memory: S0 | S1 | O = 384 of 512 columns. Warps: 8 softmax, 1 keys, 1 values (TMA), 1 that
+// Tensor memory: S0 | S1 | O | O of the lo terms = 512 columns. Warps: 8 softmax, 1 keys, 1 values (TMA), 1 that
 // issues the products.
 //
 // Which tokens: those in RUNS, i.e. neighbours in the batch with one sequence and consecutive positions, of at least min_run
@@ -449,7 +451,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
           for (int i = 0; i < 4; ++i) {
             const uint64_t v = vd + (h * 4 + i) * (2048 >> 4);
             mma_ts(o, p + h * 64 + i * 8, v, id_o, (n | h | i) ? 1u : 0u);
-            mma_ts(o, p + h * 64 + 32 + i * 8, v, id_o, 1u);
+            mma_ts(o + 128, p + h * 64 + 32 + i * 8, v, id_o, (n | h | i) ? 1u : 0u);
           }
         }
         if (!ok) break;
@@ -572,13 +574,14 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
           if (!ok) break;
           fence_after();
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t at = ot + (q >> 1) * 128 + (q & 1) * 32;
             uint32_t o[32];
-            ld32(ot + q * 32, o);
+            ld32(at, o);
             wait_ld();
 #pragma unroll
             for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-            st32(ot + q * 32, o);
+            st32(at, o);
           }
           wait_st();
         }
@@ -668,8 +671,9 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     if (ok) {
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {
-        uint32_t o[32];
+        uint32_t o[32], low[32];
         ld32(ot + q * 32, o);
+        ld32(ot + 128 + q * 32, low);
         wait_ld();
         if (store) {
 #pragma unroll
@@ -677,7 +681,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
             float v[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-              v[e] = dead ? none : __uint_as_float(o[g * 8 + e]) * f;
+              v[e] = dead ? none : (__uint_as_float(o[g * 8 + e]) + __uint_as_float(low[g * 8 + e])) * f;
               bad |= !(fabsf(v[e]) < INFINITY);
             }
             if (gt) {

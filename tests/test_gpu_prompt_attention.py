@@ -188,6 +188,20 @@ def test_weights_keep_both_terms(ops):
     assert (out[-1].double().view(H, 128) - want).abs().max() <= 2 ** -21
 
 
+def test_long_sums_do_not_drift(ops):
+    """3000 keys whose values cancel: every accumulation of a product cuts at the accumulator's last bit, always towards zero. The sums stay
+    within 2^-25 of the values, which four partial sums in registers also do (2^-25.8); 375 accumulations in a row do not (2^-24.1)."""
+    H, n = 8, 3000
+    qkv, ck, cv, pos, seq = batch([(0, n - 100, 100)], H, H, n, 1, seed=16)
+    q = qkv[-1, :H * 128].double().view(H, 128)
+    p = torch.softmax(torch.einsum("hd,jhd->hj", q, ck[0].double()) * 128 ** -0.5, 1)
+    cv[0] = (signs_that_cancel(p) * 1024).permute(1, 0, 2).half()
+    out = torch.empty(100, H * 128, dtype=torch.float16, device="cuda")
+    ops.seq_attention(qkv, ck, cv, pos, seq, out, H, H, 128, 128 ** -0.5)
+    err = out[-1].double().view(H, 128) - torch.einsum("hj,jhd->hd", p, cv[0].double())
+    assert err.pow(2).mean().sqrt() <= 2 ** -25 * 1024, (err.pow(2).mean().sqrt() / 1024).item()
+
+
 def test_window_weights_are_rounded_twice(ops):
     """bfloat16: as above; the error is that of a split with both terms rounded and of float32 sums and exponentials (half as much again). A
     leading term that is cut instead leaves a remainder, and an error, of twice the size."""
