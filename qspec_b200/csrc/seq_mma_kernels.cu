@@ -1798,7 +1798,7 @@ int window_attention_mma(const qspec_window_attn_args* p, const void* kB, long l
     // tokens, 16 / 4 heads, window 1024: 560 us; before the tiles 762, now see window_attn_mma_short_kernel). Tokens of short segments go
     // there unless the caller says that there are none (or the heads of a group are too many).
     const bool mixed = token_rows == 1 && t.rep <= 16;
-    t.seg = p->meta + 2 * p->ntok; t.min_run = mixed ? WIN_RUN : 1;
+    t.seg = mixed ? p->meta + 2 * p->ntok : nullptr; t.min_run = mixed ? WIN_RUN : 1;
     t.out = p->out; t.out_ts = a.out_ts; t.out_hs = DV;
     t.sink = p->sink; t.gate = p->gate; t.gate_ld = p->gate_ld; t.gate_per_head = p->gate_per_head; t.out_scale = a.out_scale;
     if (atile::supported(t, 4)) {
