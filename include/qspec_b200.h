@@ -276,17 +276,19 @@ int qspec_rope_kvcache(void* qkv, const void* cos_sin_cache, const int* position
                        void* cache_k, void* cache_v, int T, int Hq, int Hkv, int D, int S, void* stream);
 /* Causal decode attention over the cache (stands in for the reference's flash-attn call,
  * quarot_llama.py:221): token t attends keys 0..positions[t] of sequence seq_ids[t].
- * out [T, Hq, D] f16. D == 128. */
+ * out [T, Hq, D] f16. D == 128. float32 math; runs of 16 or more neighbouring tokens with consecutive positions, in passes of 64 or more
+ * tokens that qspec_attn_block does not take, go to the tensor-core tiles of qspec_seq_attention (weights of two float16 terms). */
 int qspec_decode_attention(const void* qkv, const void* cache_k, const void* cache_v,
                            const int* positions, const int* seq_ids, void* out, int T, int Hq,
                            int Hkv, int D, int S, float sm_scale, void* stream);
 
-/* qspec_decode_attention for passes with many sequences / several tokens per sequence (verify passes of large batches,
- * BASELINE configs[2]/[3]): one CTA per (sequence, kv head) reads that head's keys and values once for ALL tokens of the
- * sequence in the pass and all Hq/Hkv query heads. Same inputs and output as qspec_decode_attention (qkv holds the rotated
- * queries, the cache already contains this pass's keys); B = number of sequences the cache holds (seq_ids < B).
- * fp32 math; agrees with qspec_decode_attention to fp32 rounding, not bit for bit. qspec_seq_attention_supported():
- * D == 128, Hq/Hkv in {1,2,4,5,8}, T <= 1024, S small enough for shared memory (~1500 positions at Hq/Hkv = 4). */
+/* qspec_decode_attention for passes with many sequences / several tokens per sequence (verify passes of large batches): one CTA per
+ * (sequence, kv head), or per chunk of 16 query rows in passes of up to 64 tokens, reads that head's keys and values once for ALL its
+ * tokens and all Hq/Hkv query heads. Runs of 16 or more neighbouring tokens with consecutive positions in longer passes go to tensor-core
+ * tiles. Same inputs and output as qspec_decode_attention (qkv holds the rotated queries, the cache already contains this pass's keys);
+ * B = number of sequences the cache holds (seq_ids < B; a token of another one is not stored). float32 scores and sums, the softmax weights
+ * enter the value product as two float16 terms (22 bits): agrees with float32 math to the rounding of the outputs, not bit for bit.
+ * qspec_seq_attention_supported(): D == 128, Hq/Hkv in {1,2,4,5,8}, T <= 1024, any S. */
 int qspec_seq_attention_supported(int T, int Hq, int Hkv, int D, int S);
 int qspec_seq_attention(const void* qkv, const void* cache_k, const void* cache_v, const int* positions,
                         const int* seq_ids, void* out, int T, int B, int Hq, int Hkv, int D, int S, float sm_scale,
