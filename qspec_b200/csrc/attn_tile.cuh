@@ -235,17 +235,27 @@ struct Items {
   }
 };
 
-// Rows whose tile result is not finite, once more on the CUDA cores: float32 weights, nothing but the row's own keys. A whole warp per row,
-// every lane with keys of its own (a thread per row took 100 times as long, and one infinite value in a cache is enough for every later row).
-// rows: the lanes that ask; 64 columns from col0 on of the row that each describes.
+// Columns of rows whose tile result is not finite, once more on the CUDA cores: float32 weights, nothing but the row's own keys. (hi and lo
+// terms of opposite signs turn an infinite value into NaN, and so does a hidden key's weight of zero.) A whole warp per row, every lane with
+// keys of its own. First the row's own values that are not finite: where a column has one, they decide. A column without one was spoilt by a
+// key that the row does not see and is summed again.
+// rows: the lanes that ask; 64 columns from col0 on of the row that each describes, of which `bad`; f and m: factor and reference of the row's
+// weights, as in the kernel.
+// 1000 tokens after 1000, 32 / 8 heads, one infinite value that all see in one head / in two columns of every head: whole sums by a thread per
+// row 104 / 300 ms, by a warp 10.2 / 19.3, now 1.5 / 3.3; before the tiles 7.7, as any other prompt.
 template <bool BF, bool QF32>
-__device__ __noinline__ void attn_rows_again(const Args& a, uint32_t rows, int tok_, int head_, int kvh, int seq_, int lo_, int hi_, int col0) {
+__device__ __noinline__ void attn_rows_again(const Args& a, uint32_t rows, int tok_, int head_, int kvh, int seq_, int lo_, int hi_, int col0, uint64_t bad_,
+                                             float m_, float f_) {
   using T = typename Elem<BF>::T;
+  constexpr uint32_t EXPONENTS = BF ? 0x7f807f80u : 0x7c007c00u;
   const int lane = threadIdx.x & 31;
+  __syncwarp();                                               // the rows' lanes have stored them
   for (; rows; rows &= rows - 1u) {
     const int src = __ffs(rows) - 1;
     const int tok = __shfl_sync(0xffffffffu, tok_, src), head = __shfl_sync(0xffffffffu, head_, src), seq = __shfl_sync(0xffffffffu, seq_, src);
     const int lo = __shfl_sync(0xffffffffu, lo_, src), hi = __shfl_sync(0xffffffffu, hi_, src);
+    const uint64_t bad = __shfl_sync(0xffffffffu, bad_, src);
+    const float mt = __shfl_sync(0xffffffffu, m_, src), ft = __shfl_sync(0xffffffffu, f_, src);
     const T* kbase = (const T*)a.k + (size_t)seq * a.k_ss + (size_t)kvh * a.k_hs;
     const T* vbase = (const T*)a.v + (size_t)seq * a.v_ss + (size_t)kvh * a.v_hs + col0;
     const size_t qo = (size_t)tok * a.q_ts + (size_t)head * a.q_hs;
@@ -273,13 +283,61 @@ __device__ __noinline__ void attn_rows_again(const Args& a, uint32_t rows, int t
       }
       return s * a.scale;
     };
+    auto store = [&](int d, float r) {                        // (a gate per head is in ft)
+      if (a.gate && !a.gate_per_head) r *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)tok * a.gate_ld + head * a.out_hs + col0 + d]));
+      ((T*)a.out)[(size_t)tok * a.out_ts + (size_t)head * a.out_hs + col0 + d] = (T)r;
+    };
+    float acc[64];
+#pragma unroll
+    for (int d = 0; d < 64; ++d) acc[d] = 0.f;
+    bool found = false;
+    for (int j = lo + lane; j <= hi; j += 32) {
+      const uint4* vr = reinterpret_cast<const uint4*>(vbase + (size_t)row(j) * a.v_rs);
+      uint4 vw[8];
+      uint32_t odd = 0u;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        vw[c] = vr[c];
+        odd |= __vcmpeq2(vw[c].x & EXPONENTS, EXPONENTS) | __vcmpeq2(vw[c].y & EXPONENTS, EXPONENTS) | __vcmpeq2(vw[c].z & EXPONENTS, EXPONENTS) |
+               __vcmpeq2(vw[c].w & EXPONENTS, EXPONENTS);
+      }
+      if (!odd) continue;
+      found = true;
+      const float p = ex2(score(j) * 1.4426950408889634f - mt);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const uint32_t vv[4] = {vw[c].x, vw[c].y, vw[c].z, vw[c].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 x = Elem<BF>::unpack(vv[e]);
+          if (!(fabsf(x.x) < INFINITY)) acc[c * 8 + 2 * e] = fmaf(p, x.x, acc[c * 8 + 2 * e]);
+          if (!(fabsf(x.y) < INFINITY)) acc[c * 8 + 2 * e + 1] = fmaf(p, x.y, acc[c * 8 + 2 * e + 1]);
+        }
+      }
+    }
+    float mine[2] = {0.f, 0.f};                               // columns 2 lane, + 1
+    if (__any_sync(0xffffffffu, found)) {
+#pragma unroll
+      for (int d = 0; d < 64; ++d) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
+        if (lane == d >> 1) mine[d & 1] = acc[d];
+      }
+    }
+    bool again[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const bool ask = bad >> (2 * lane + e) & 1;
+      again[e] = ask && mine[e] == 0.f;
+      if (ask && !again[e]) store(2 * lane + e, mine[e] * ft);
+    }
+    if (!__any_sync(0xffffffffu, again[0] || again[1])) continue;
     float m = -INFINITY;
     for (int j = lo + lane; j <= hi; j += 32) m = fmaxf(m, score(j));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (a.sink) m = fmaxf(m, a.sink[head]);
     float l = a.sink && lane == 0 ? __expf(a.sink[head] - m) : 0.f;
-    float acc[64];
 #pragma unroll
     for (int d = 0; d < 64; ++d) acc[d] = 0.f;
     for (int j = lo + lane; j <= hi; j += 32) {
@@ -300,20 +358,17 @@ __device__ __noinline__ void attn_rows_again(const Args& a, uint32_t rows, int t
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    float mine[2] = {0.f, 0.f};                               // columns 2 lane, + 1
 #pragma unroll
     for (int d = 0; d < 64; ++d) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
       if (lane == d >> 1) mine[d & 1] = acc[d];
     }
+    float gh = a.out_scale / l;
+    if (a.gate && a.gate_per_head) gh *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)tok * a.gate_ld + head]));
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int d = col0 + 2 * lane + e;
-      float r = mine[e] / l * a.out_scale;
-      if (a.gate) r *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)tok * a.gate_ld + (a.gate_per_head ? head : head * a.out_hs + d)]));
-      ((T*)a.out)[(size_t)tok * a.out_ts + (size_t)head * a.out_hs + d] = (T)r;
-    }
+    for (int e = 0; e < 2; ++e)
+      if (again[e]) store(2 * lane + e, mine[e] * gh);
   }
 }
 
@@ -667,7 +722,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       f *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)(c0 + tl) * a.gate_ld + head]));
     T* dst = (T*)a.out + (size_t)(c0 + tl) * a.out_ts + (size_t)head * a.out_hs + h * 64;
     const T* gt = a.gate && !a.gate_per_head ? (const T*)a.gate + (size_t)(c0 + tl) * a.gate_ld + (size_t)head * a.out_hs + h * 64 : nullptr;
-    bool bad = false;
+    uint64_t bad = 0;                                         // columns that are not finite
     if (ok) {
 #pragma unroll 1
       for (int q = 0; q < 2; ++q) {
@@ -682,7 +737,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               v[e] = dead ? none : (__uint_as_float(o[g * 8 + e]) + __uint_as_float(low[g * 8 + e])) * f;
-              bad |= !(fabsf(v[e]) < INFINITY);
+              if (!(fabsf(v[e]) < INFINITY)) bad |= 1ull << (q * 32 + g * 8 + e);
             }
             if (gt) {
               const uint4 gw = *reinterpret_cast<const uint4*>(gt + q * 32 + g * 8);
@@ -700,8 +755,8 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         }
       }
       // (a sum of weights that is not a number makes every column so: nothing to do again)
-      const uint32_t again = __ballot_sync(0xffffffffu, bad && store && !dead && l == l);
-      if (again) attn_rows_again<BF, QF32>(a, again, c0 + tl, head, kvh, my_seq, my_lo, my_hi, h * 64);
+      const uint32_t again = __ballot_sync(0xffffffffu, bad != 0 && store && !dead && l == l);
+      if (again) attn_rows_again<BF, QF32>(a, again, c0 + tl, head, kvh, my_seq, my_lo, my_hi, h * 64, bad, m, f);
     }
   }
   fence_before();
