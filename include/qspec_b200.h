@@ -84,7 +84,7 @@ int qspec_add_norm_f16(void* x, const void* delta, void* out, int rows, int K, f
  *   delta = T(epilogue(sum over slices)), x += delta, norm (+ quantiser)
  * with exactly the arithmetic and summation order of the in-GEMM reduction: for W4A4 (exact int32 sums) x and the norm
  * outputs are bit-identical to qspec_gemm_* followed by qspec_add_norm_*; for W4A16 they are when both calls split k the
- * same way, and equal up to fp32 summation order otherwise. What it saves: the GEMM's cross-CTA reduction
+ * same way, and equal up to fp32 summation order otherwise. (Few tokens: split = 1, whole sums.) What it saves: the GEMM's cross-CTA reduction
  * (partial store, counter atomic, reload: three serialized L2 round trips at the end of every launch).
  * Reference semantics: quarot_nn/linear.py:34-56 (Linear4bit.forward) + quarot_llama.py:380,389 (residual add)
  * + layernorm_kernels.cu:569-720. */
@@ -294,9 +294,9 @@ int qspec_seq_attention(const void* qkv, const void* cache_k, const void* cache_
                         const int* seq_ids, void* out, int T, int B, int Hq, int Hkv, int D, int S, float sm_scale,
                         void* stream);
 
-/* CTAs of qspec_seq_attention, and of the tensor-core prompt form inside it and qspec_decode_attention, that gave up a bounded wait since
- * the library was loaded on the current device (the rows that such a CTA would have written are NaN): 0 unless something is broken; -1 if
- * it cannot be read. Synchronises. No counterpart. */
+/* CTAs of qspec_seq_attention, of the tensor-core prompt form inside it and qspec_decode_attention, and of the few-token form of the
+ * qspec_gemm_* calls that gave up a bounded wait since the library was loaded on the current device (what such a CTA would have written is
+ * NaN, raw integer sums the lowest integer): 0 unless something is broken; -1 if it cannot be read. Synchronises. No counterpart. */
 int qspec_attn_tile_timeouts(void);
 
 /* The attention block between qkv_proj and o_proj as one launch for decode-sized passes: rotary embedding and

@@ -31,7 +31,7 @@ def _nvcc() -> str:
 
 
 def _newest_source_mtime(sources=None) -> float:
-    names = os.listdir(CSRC) if sources is None else list(sources) + ["common.cuh", "seq_common.cuh", "attn_tile.cuh"]
+    names = os.listdir(CSRC) if sources is None else list(sources) + ["common.cuh", "seq_common.cuh", "attn_tile.cuh", "gemm_w4_rows.cuh"]
     paths = [os.path.join(CSRC, f) for f in names]
     paths.append(os.path.join(HERE, "..", "include", "qspec_b200.h"))
     paths.append(os.path.join(HERE, "..", "include", "qspec_b200_seq.h"))

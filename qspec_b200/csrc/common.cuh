@@ -16,6 +16,7 @@ namespace qspec {
 void set_error(const char* fmt, ...);            // stores thread-local text for qspec_last_error()
 void count_launch(int n = 1);                    // bumps qspec_launch_count()
 int  sm_count();
+int  gemm_rows_timeouts();                         // CTAs of the few-token GEMM that gave a wait up; -1: not readable
 
 #define QSPEC_REQUIRE(cond, code, ...)                                                       \
   do {                                                                                       \

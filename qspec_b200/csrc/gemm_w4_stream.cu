@@ -7,6 +7,8 @@
 // rowwise_scaled_linear_cutlass/rowwise_scaled_linear_cutlass_unified.cuh:240-488, an SM80 mma.sync.s4
 // kernel) and the BitBLAS Matmul + per-call `weight ^ 0x88` pass (quarot_nn/linear.py:102-124,156-211).
 //
+// Products of few tokens take another kernel (gemm_w4_rows.cuh; rule: rows_wanted below).
+//
 // Design (nothing here follows the reference's kernels):
 //  * swap-AB: the 128 output channels of a tile are the UMMA M dimension, tokens are UMMA N (16..128).
 //  * The weight operand never exists in shared memory in MMA form. A dedicated TMA warp streams packed
@@ -37,7 +39,7 @@ namespace qspec {
 namespace w4s {
 
 constexpr int MODE_I8 = 0, MODE_F16 = 1, MODE_BF16 = 2, MODE_A8 = 3;   // A8: int8 activations x int4 weights (W4A8)
-constexpr bool mode_is_int(int m) { return m == MODE_I8 || m == MODE_A8; }
+__host__ __device__ constexpr bool mode_is_int(int m) { return m == MODE_I8 || m == MODE_A8; }
 
 constexpr int TM = 128;              // channels per tile (UMMA M)
 constexpr int UK = 256;              // k per unit
@@ -1028,6 +1030,8 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
 }
 
+#include "gemm_w4_rows.cuh"
+
 // ---- host side -----------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1045,27 +1049,29 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// 2-D row-major tensor [rows][row_bytes], tiles of box_rows x 128 bytes, SWIZZLE_128B. Encoded maps are
+// Row-major tensor [rows][row_bytes], tiles of box_rows x 128 bytes, SWIZZLE_128B; with pieces > 1, tiles of `pieces` neighbouring 128-byte
+// columns, one after the other (the tensor then has three dimensions: byte of a piece, row, piece). Encoded maps are
 // cached by (pointer, geometry): weights and arena activations keep their addresses across calls.
 struct MapKey {
-  const void* ptr; uint64_t rows, row_bytes; uint32_t box_rows, elem;
+  const void* ptr; uint64_t rows, row_bytes; uint32_t box_rows, elem, pieces;
   bool operator==(const MapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && row_bytes == o.row_bytes && box_rows == o.box_rows && elem == o.elem;
+    return ptr == o.ptr && rows == o.rows && row_bytes == o.row_bytes && box_rows == o.box_rows && elem == o.elem && pieces == o.pieces;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = (size_t)k.ptr;
     h = h * 1000003u ^ k.rows; h = h * 1000003u ^ k.row_bytes; h = h * 1000003u ^ k.box_rows; h = h * 1000003u ^ k.elem;
+    h = h * 1000003u ^ k.pieces;
     return h;
   }
 };
 
 static int get_map(const void* ptr, uint64_t rows, uint64_t row_bytes, uint32_t box_rows, uint32_t elem_bytes,
-                   CUtensorMap* out) {
+                   CUtensorMap* out, uint32_t pieces = 1) {
   static std::mutex mu;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  const MapKey key{ptr, rows, row_bytes, box_rows, elem_bytes};
+  const MapKey key{ptr, rows, row_bytes, box_rows, elem_bytes, pieces};
   {
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(key);
@@ -1073,11 +1079,11 @@ static int get_map(const void* ptr, uint64_t rows, uint64_t row_bytes, uint32_t 
   }
   EncodeTiledFn fn = encode_fn();
   QSPEC_REQUIRE(fn, QSPEC_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
-  const cuuint64_t dims[2] = {row_bytes / elem_bytes, rows};
-  const cuuint64_t strides[1] = {row_bytes};
-  const cuuint32_t box[2] = {128u / elem_bytes, box_rows};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = fn(out, elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2,
+  const cuuint64_t dims[3] = {pieces > 1 ? 128u / elem_bytes : row_bytes / elem_bytes, rows, row_bytes / 128};
+  const cuuint64_t strides[2] = {row_bytes, 128};
+  const cuuint32_t box[3] = {128u / elem_bytes, box_rows, pieces};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(out, elem_bytes == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, pieces > 1 ? 3 : 2,
                         const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   QSPEC_REQUIRE(r == CUDA_SUCCESS, QSPEC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) ptr=%p rows=%llu row_bytes=%llu box_rows=%u",
@@ -1281,6 +1287,82 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& ma, const Params& p,
   return QSPEC_OK;
 }
 
+// Which calls the few-token kernel takes (gemm_w4_rows.cuh). Its time grows with the tokens (mma.sync, and for W4A16 the widening, which every
+// CTA does for its tokens at half the tensor rate), that of the tcgen05 form hardly: the line lies where they meet, later for products whose
+// time is mostly latency (up to 2^26 weights). us, few-token | tcgen05 form, on both sides of the lines:
+//   W4A4              28672 x 4096: 32 tokens 19.6 | 19.9, 48: 24.4 | 21.2   8192 x 8192: 64 tokens 18.5 | 19.1   10240 x 8192: 64: 31.0 | 21.7
+//   W4A4 bytes, W4A8  28672 x 4096: 24 tokens 16.6 | 17.6, 32: 27.1 | 17.8   8192 x 8192: 32 tokens 15.3 | 15.3   10240 x 8192: 32: 25.0 | 16.7
+//   W4A16             28672 x 4096: 16 tokens 20.0 | 26.1, 24: 31.1 | 27.0   8192 x 8192: 32 tokens 19.1 | 19.3   10240 x 8192: 24: 29.6 | 22.5
+// QSPEC_GEMM_ROWS, read at every call, for measurements and tests: 0 = none, 2 = all that it can run.
+static bool rows_wanted(int mode, int M, int N, int K) {
+  const int want = env_int("QSPEC_GEMM_ROWS", 1);
+  const int most = mode == MODE_I8 ? ROWS_MAX_M : ROWS_MAX_M / 2;         // what is instantiated
+  if (want == 0 || M > most) return false;
+  return want == 2 || (long long)N * K <= (1ll << 26) || M <= (mode == MODE_I8 ? 32 : mode == MODE_A8 ? 24 : 16);
+}
+
+template <int MODE, int NT, int NW, int CTAS>
+static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, RowsArgs p, int sms, cudaStream_t st) {
+  using Sh = RowsShape<MODE, NT>;
+  // a CTA's share of the SM's 228 KB (1 KB a CTA is the system's), less the static part
+  constexpr size_t BUDGET = (CTAS == 1 ? 227 : 113) * 1024 - 1024, SUMS = (size_t)NW * Sh::T * Sh::LD * 4, FIXED = 1024 + SUMS;
+  constexpr int FIT = (int)((BUDGET - FIXED) / (Sh::SLOT * NW)), DEPTH = FIT < ROWS_SLOTS / NW ? FIT : ROWS_SLOTS / NW;
+  static_assert(DEPTH >= 1, "a slot per warp");
+  auto kern = w4_rows_kernel<MODE, NT, NW, CTAS>;
+  const int grid = p.tiles < sms * CTAS ? p.tiles : sms * CTAS;
+  const int most = (p.tiles + grid - 1) / grid * ((p.items + NW - 1) / NW);      // items of a warp
+  p.depth = most < DEPTH ? most : DEPTH;
+  static std::atomic<uint64_t> raised{0};                   // devices on which the kernel's shared-memory limit has been raised
+  int dev = 0;
+  QSPEC_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !(raised.load(std::memory_order_relaxed) >> dev & 1)) {
+    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BUDGET));
+    if (dev < 64) raised.fetch_or(1ull << dev);
+  }
+  QSPEC_CUDA(launch_pdl(kern, dim3(grid), dim3(NW * 32), FIXED + (size_t)p.depth * NW * Sh::SLOT, st, mw, ma, p));
+  count_launch(1);
+  return QSPEC_OK;
+}
+
+// One CTA of eight warps where every tile gets an SM of its own; otherwise two CTAs per SM, of four warps, or of eight where the slots are
+// small (W4A4, up to 8 tokens): the second CTA loads while the first one adds its sums up. 28672 x 4096, one | two CTAs per SM: W4A4, 4 tokens
+// 12.4 | 10.3 us, W4A16, 16 tokens 23.4 | 20.4.
+template <int MODE, int NT>
+static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, const RowsArgs& p, cudaStream_t st) {
+  const int sms = sm_count() > 0 ? sm_count() : 148;
+  if (p.tiles <= sms) return rows_launch<MODE, NT, 8, 1>(mw, ma, p, sms, st);
+  return rows_launch<MODE, NT, (MODE == MODE_I8 && NT == 1) ? 8 : 4, 2>(mw, ma, p, sms, st);
+}
+template <int MODE>
+static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, const RowsArgs& p, cudaStream_t st) {
+  switch ((p.M + 7) / 8) {
+    case 1: return rows_launch<MODE, 1>(mw, ma, p, st);
+    case 2: return rows_launch<MODE, 2>(mw, ma, p, st);
+    case 3: return rows_launch<MODE, 3>(mw, ma, p, st);
+    case 4: return rows_launch<MODE, 4>(mw, ma, p, st);
+    default: break;
+  }
+  if constexpr (MODE == MODE_I8) return p.M <= 48 ? rows_launch<MODE, 6>(mw, ma, p, st) : rows_launch<MODE, 8>(mw, ma, p, st);
+  return QSPEC_ERR_UNSUPPORTED;
+}
+static int rows_run(int mode, const void* act, const int8_t* w, const RowsArgs& a, int K, cudaStream_t st) {
+  CUtensorMap mw, ma;
+  int rc = get_map(w, (uint64_t)a.N, (uint64_t)K / 2, ROWS_R, 1, &mw);
+  if (rc != QSPEC_OK) return rc;
+  const int groups = (a.M + 7) / 8;
+  const uint32_t box = 8u * (groups <= 4 ? groups : groups <= 6 ? 6 : 8);
+  rc = mode == MODE_I8 ? get_map(act, (uint64_t)a.M, (uint64_t)K / 2, box, 1, &ma)
+     : mode == MODE_A8 ? get_map(act, (uint64_t)a.M, (uint64_t)K, box, 1, &ma, RowsShape<MODE_A8, 1>::ABOX)
+                       : get_map(act, (uint64_t)a.M, (uint64_t)K * 2, box, 2, &ma, RowsShape<MODE_F16, 1>::ABOX);
+  if (rc != QSPEC_OK) return rc;
+  switch (mode) {
+    case MODE_I8: return rows_launch<MODE_I8>(mw, ma, a, st);
+    case MODE_A8: return rows_launch<MODE_A8>(mw, ma, a, st);
+    case MODE_F16: return rows_launch<MODE_F16>(mw, ma, a, st);
+    default: return rows_launch<MODE_BF16>(mw, ma, a, st);
+  }
+}
+
 static int run(int mode, const void* act, const void* sA, const int8_t* w, const void* sW, const void* bias, void* out,
                int32_t* acc_out, int M, int N, int K, int out_bf16, void* workspace, size_t ws_bytes, cudaStream_t st,
                const char* who, uint32_t* split_out = nullptr, size_t split_bytes = 0) {
@@ -1293,14 +1375,18 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   QSPEC_REQUIRE(((uintptr_t)act & 15) == 0 && ((uintptr_t)w & 15) == 0, QSPEC_ERR_UNSUPPORTED,
                 "%s: operand pointers must be 16-byte aligned", who);
   if (M == 0) return QSPEC_OK;
-  const Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
+  const bool rows = rows_wanted(mode, M, N, K);
+  Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
+  if (rows) pl.split = 1;                                   // whole sums: one slice
   const size_t need = split_out ? workspace_bytes(mode, M, N, K) : workspace_bytes(pl);
   QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
   if (split_out) {
-    QSPEC_REQUIRE(pl.split >= 1 && pl.tiles_m == 1, QSPEC_ERR_UNSUPPORTED, "%s: no even k-split for M=%d N=%d K=%d", who, M, N, K);
+    QSPEC_REQUIRE(pl.split >= 1 && (rows || pl.tiles_m == 1), QSPEC_ERR_UNSUPPORTED, "%s: no even k-split for M=%d N=%d K=%d", who, M, N, K);
     QSPEC_REQUIRE(split_bytes >= (size_t)pl.split * M * N * 4, QSPEC_ERR_WORKSPACE, "%s: partial buffer too small (%zu < %zu)", who,
                   split_bytes, (size_t)pl.split * M * N * 4);
   }
+  if (rows)
+    return rows_run(mode, act, w, RowsArgs{sA, sW, bias, out, acc_out, split_out, M, N, (K + ROWS_UK - 1) / ROWS_UK, (N + ROWS_R - 1) / ROWS_R, 0, out_bf16}, K, st);
   CUtensorMap mw, ma;
   int rc = get_map(w, (uint64_t)N, (uint64_t)K / 2, TM, 1, &mw);
   if (rc != QSPEC_OK) return rc;
@@ -1336,6 +1422,11 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
 }
 
 }  // namespace w4s
+
+int gemm_rows_timeouts() {
+  unsigned n = 0;
+  return cudaMemcpyFromSymbol(&n, w4s::rows_timeouts, sizeof(n)) == cudaSuccess ? (int)(n & 0x3fffffffu) : -1;
+}
 }  // namespace qspec
 
 using namespace qspec;
@@ -1394,7 +1485,9 @@ extern "C" int qspec_debug_gemm_plan(int mode, int M, int N, int K, int deferred
 
 extern "C" int qspec_gemm_split_factor(int w4a16, int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0 || K % 128 || N % 8) return 0;
-  const w4s::Plan pl = w4s::make_plan(w4a16 == 2 ? w4s::MODE_A8 : w4a16 ? w4s::MODE_F16 : w4s::MODE_I8, M, N, K, true);   // 2: int8-container W4A4
+  const int mode = w4a16 == 2 ? w4s::MODE_A8 : w4a16 ? w4s::MODE_F16 : w4s::MODE_I8;   // 2: int8-container W4A4
+  if (w4s::rows_wanted(mode, M, N, K)) return 1;
+  const w4s::Plan pl = w4s::make_plan(mode, M, N, K, true);
   return pl.tiles_m == 1 ? pl.split : 0;
 }
 

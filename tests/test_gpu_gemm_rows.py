@@ -1,0 +1,119 @@
+"""The few-token form of the int4 products (csrc/gemm_w4_rows.cuh) against exact sums: token counts around its groups of 8, channel counts
+around its tiles of 32 and around one tile per SM, k around its items of 256, and both sides of the rule that chooses it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from qspec_b200 import ops
+    return ops
+
+
+def _int4(w):
+    low = (w << 4) >> 4
+    return torch.stack((low, w >> 4), -1).reshape(w.shape[0], -1).double()
+
+
+def _operands(M, N, K, dt, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    w = torch.randint(-128, 128, (N, K // 2), generator=g, dtype=torch.int8, device="cuda")
+    sW = ((0.5 + torch.rand(N, generator=g, device="cuda")) * 2.0 ** -7).to(dt)
+    bias = (torch.randn(N, generator=g, device="cuda") * 0.1).to(dt)
+    sA = (0.01 + 0.1 * torch.rand(M, generator=g, device="cuda")).to(dt)
+    q = torch.randint(-8, 8, (M, K), generator=g, dtype=torch.int8, device="cuda")
+    x = torch.randn(M, K, generator=g, device="cuda").to(dt)
+    return w, sW, bias, sA, q, x
+
+
+SHAPES = [(1, 8, 128), (8, 32, 256), (9, 40, 384), (16, 136, 128), (4, 4096, 4096), (16, 4736, 640), (17, 4768, 384), (24, 9504, 256), (25, 776, 2176),
+          (32, 14336, 512), (33, 1000, 1152), (48, 4800, 256), (49, 512, 3840), (64, 6144, 896), (16, 28672, 4096)]
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_rows_products_are_the_exact_sums(ops, monkeypatch, M, N, K, dt, with_bias):
+    w, sW, bias, sA, q, x = _operands(M, N, K, dt, M * 131 + N + K)
+    b = bias if with_bias else None
+    packed = ((q[:, 0::2] & 15) | (q[:, 1::2] << 4)).contiguous()
+    monkeypatch.setenv("QSPEC_GEMM_ROWS", "2")
+    sums = q.double() @ _int4(w).T                                       # whole numbers: exact
+    want = (sums.float() * sA.float()[:, None]) * sW.float()[None, :]
+    want = (want + bias.float() if with_bias else want).to(dt)
+    out = torch.full((M, N), float("nan"), dtype=dt, device="cuda")
+    ops.rowwise_scaled_linear_cutlass_s4s4_unified(packed, sA, w, sW, b, out)
+    assert torch.equal(out, want)
+    assert torch.equal(ops.gemm_w4a4_acc_i32(packed, w), sums.int())
+    if M <= 32:
+        out.fill_(float("nan"))
+        ops.rowwise_scaled_linear_cutlass_s8s4(q, sA, w, sW, b, out)
+        assert torch.equal(out, want)
+        out.fill_(float("nan"))
+        ops.gemm_w4a16(x, w, sW, b, out)
+        exact = x.double() @ _int4(w).T * sW.double()
+        exact = exact + bias.double() if with_bias else exact
+        # float32: the tensor cores cut the sum of 256 products (16 steps, 2^-23 each at most, of a partial sum's magnitude), the K / 256 sums and the
+        # two epilogue operations round; partial sums stay below 6 standard deviations. Then one rounding to 8 or 11 bits.
+        mag = (x.double().abs().square().sum(1, keepdim=True) * 21.5).sqrt() * 6 * sW.double()
+        bound = mag * (16 + K / 256 + 2) * 2.0 ** -23 + exact.abs() * (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11) + 2.0 ** -24
+        assert ((out.double() - exact).abs() <= bound).all()
+    assert ops.attn_tile_timeouts() == 0
+
+
+@pytest.mark.parametrize("mode,M,N,K", [("w4a4", 32, 28672, 4096), ("w4a4", 33, 28672, 4096), ("w4a4", 64, 8192, 8192), ("w4a4", 65, 8192, 8192),
+                                        ("w4a8", 24, 10240, 8192), ("w4a8", 25, 10240, 8192), ("w4a8", 32, 8192, 8192), ("w4a8", 33, 8192, 8192),
+                                        ("w4a16", 16, 10240, 8192), ("w4a16", 17, 10240, 8192), ("w4a16", 32, 8192, 8192), ("w4a16", 33, 8192, 8192)])
+def test_both_sides_of_the_rule(ops, monkeypatch, mode, M, N, K):
+    """Which form runs shows in the deferred split (the few-token form leaves one slice); both agree, run twice in a row on two inputs."""
+    w, sW, _, sA, q, x = _operands(M, N, K, torch.float16, M + N)
+    kind = {"w4a4": 0, "w4a16": 1, "w4a8": 2}[mode]
+    rows = M <= {0: 64, 1: 32, 2: 32}[kind] if N * K <= 2 ** 26 else M <= {0: 32, 1: 16, 2: 24}[kind]
+    packed = ((q[:, 0::2] & 15) | (q[:, 1::2] << 4)).contiguous()
+
+    def call(form, flip):
+        monkeypatch.setenv("QSPEC_GEMM_ROWS", form)
+        out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+        if mode == "w4a4":
+            ops.rowwise_scaled_linear_cutlass_s4s4_unified(packed.flip(0).contiguous() if flip else packed, sA, w, sW, None, out)
+        elif mode == "w4a8":
+            ops.rowwise_scaled_linear_cutlass_s8s4(q.flip(0).contiguous() if flip else q, sA, w, sW, None, out)
+        else:
+            ops.gemm_w4a16(x.flip(0).contiguous() if flip else x, w, sW, None, out)
+        return out
+
+    if rows:
+        assert ops.gemm_split_factor(kind, M, N, K) == 1
+    for flip in (False, True, False):
+        a, b = call("1", flip), call("0", flip)
+        if mode == "w4a16":                                               # another order of float32 sums, then a rounding to 11 bits
+            assert (a.float() - b.float()).norm() <= 1e-4 * b.float().norm()
+        else:
+            assert torch.equal(a, b)
+
+
+def test_capture_and_two_streams(ops):
+    """Captured calls replay; calls on two streams with weights of their own do not meet."""
+    M, N, K = 4, 4096, 4096
+    sets = [_operands(M, N, K, torch.float16, s) for s in (1, 2)]
+    want = [ops.gemm_w4a16(s[5], s[0], s[1], None, torch.empty(M, N, dtype=torch.float16, device="cuda")) for s in sets]
+    outs = [torch.zeros(M, N, dtype=torch.float16, device="cuda") for _ in sets]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for s, o in zip(sets, outs):
+            ops.gemm_w4a16(s[5], s[0], s[1], None, o)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, w) for o, w in zip(outs, want))
+    streams = [torch.cuda.Stream() for _ in sets]
+    for o in outs:
+        o.zero_()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for st, s, o in zip(streams, sets, outs):
+            with torch.cuda.stream(st):
+                ops.gemm_w4a16(s[5], s[0], s[1], None, o)
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, w) for o, w in zip(outs, want))
