@@ -443,38 +443,89 @@ struct GroupPlan {
   int* offsets;      // [E + 1] first sorted row of every expert
   int* status;       // [1] status word at the start of the workspace: set to 1 by a CTA whose bounded wait ran out, never cleared
   int* ntiles;       // [1]
-  int* tile_expert;  // [max tiles]
-  int* tile_row0;    // [max tiles]
+  int4* tile;        // [max tiles] expert, first sorted row, end of its rows, rows it is made for (multiple of 16)
   int* perm;         // [npairs] sorted row -> pair index
 };
 
-__global__ void __launch_bounds__(1024) moe_group_kernel(const int* __restrict__ idx, int npairs, int E, GroupPlan p) {
+// One CTA: counts, prefix sums over the experts, then every pair takes the next row of its expert. The pairs' experts are read once, and the
+// sorted rows leave as whole lines, where they fit (MOE_KEEP * 1024 pairs). 8192 pairs of 16 experts: 7.8 us. Counting inside each
+// warp first (ballots, counts of each warp's own) took 10: the block spends its time on issuing instructions.
+// tile_rows: rows of a tile; 0: an expert's rows are divided evenly into tiles of at most 256, multiples of 16 (tc_rows).
+__host__ __device__ __forceinline__ int tc_rows(int c) {
+  const int n = (c + 255) / 256;
+  return n ? ((c + n - 1) / n + 15) & ~15 : 16;
+}
+__device__ __forceinline__ int block_scan_1024(int v, int* sums, int& total) {      // exclusive prefix sum over 1024 threads
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();                        // sums may still be read from an earlier call
+  if (lane == 31) sums[warp] = x;
+  __syncthreads();
+  int w = sums[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, w, o);
+    if (lane >= o) w += y;
+  }
+  total = __shfl_sync(0xffffffffu, w, 31);
+  return x - v + (warp ? __shfl_sync(0xffffffffu, w, warp - 1) : 0);
+}
+constexpr int MOE_KEEP = 16;                                  // pairs of a thread that stay in registers
+static bool moe_group_kept(int npairs) { return npairs <= MOE_KEEP * 1024; }
+static size_t moe_group_smem(int npairs, int E) { return 4 * ((size_t)E + 1 + (moe_group_kept(npairs) ? npairs : 0)); }
+__global__ void __launch_bounds__(1024) moe_group_kernel(const int* __restrict__ idx, int npairs, int E, int tile_rows, int kept, GroupPlan p) {
   pdl_enter();
-  extern __shared__ int s_cnt[];          // [E + 1]
+  extern __shared__ int s_cnt[];          // [E + 1] pairs of an expert, then its next sorted row; where the pairs are kept, the sorted rows behind
+  __shared__ int s_sums[32];
   const int tid = threadIdx.x;
+  int* s_perm = s_cnt + E + 1;
   for (int e = tid; e <= E; e += 1024) s_cnt[e] = 0;
-  __syncthreads();
-  for (int k = tid; k < npairs; k += 1024) {
-    const int e = idx[k];
-    if (e >= 0 && e < E) atomicAdd(&s_cnt[e], 1);
+  int ex[MOE_KEEP];
+#pragma unroll
+  for (int j = 0; j < MOE_KEEP; ++j) {
+    const int k = tid + j * 1024;
+    ex[j] = kept && k < npairs ? idx[k] : -1;
   }
   __syncthreads();
-  if (tid == 0) {
-    int at = 0, nt = 0;
-    for (int e = 0; e < E; ++e) {
-      const int c = s_cnt[e];
-      p.offsets[e] = at;
-      for (int r = 0; r < c; r += GG_BM) { p.tile_expert[nt] = e; p.tile_row0[nt] = at + r; ++nt; }
-      s_cnt[e] = at;                      // becomes the cursor
-      at += c;
+  auto in = [&](int e) { return e >= 0 && e < E; };
+#pragma unroll
+  for (int j = 0; j < MOE_KEEP; ++j)
+    if (in(ex[j])) atomicAdd(&s_cnt[ex[j]], 1);
+  if (!kept)
+    for (int k = tid; k < npairs; k += 1024)
+      if (in(idx[k])) atomicAdd(&s_cnt[idx[k]], 1);
+  __syncthreads();
+  int rows = 0, tiles = 0;
+  for (int e0 = 0; e0 < E; e0 += 1024) {
+    const int e = e0 + tid, c = e < E ? s_cnt[e] : 0;
+    int total, ttotal;
+    const int first = rows + block_scan_1024(c, s_sums, total);
+    const int size = tile_rows ? tile_rows : tc_rows(c);
+    int nt = tiles + block_scan_1024((c + size - 1) / size, s_sums, ttotal);
+    if (e < E) {
+      p.offsets[e] = first;
+      s_cnt[e] = first;
+      for (int r = 0; r < c; r += size, ++nt) p.tile[nt] = make_int4(e, first + r, first + min(c, r + size), size);
     }
-    p.offsets[E] = at;
-    *p.ntiles = nt;
+    rows += total;
+    tiles += ttotal;
   }
+  if (tid == 0) { p.offsets[E] = rows; *p.ntiles = tiles; }
   __syncthreads();
-  for (int k = tid; k < npairs; k += 1024) {
-    const int e = idx[k];
-    if (e >= 0 && e < E) p.perm[atomicAdd(&s_cnt[e], 1)] = k;
+  if (kept) {
+#pragma unroll
+    for (int j = 0; j < MOE_KEEP; ++j)
+      if (in(ex[j])) s_perm[atomicAdd(&s_cnt[ex[j]], 1)] = tid + j * 1024;
+    __syncthreads();
+    for (int m = tid; m < rows; m += 1024) p.perm[m] = s_perm[m];
+  } else {
+    for (int k = tid; k < npairs; k += 1024)
+      if (in(idx[k])) p.perm[atomicAdd(&s_cnt[idx[k]], 1)] = k;
   }
 }
 
@@ -517,7 +568,7 @@ grouped_gemm_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16
   if (tile >= *p.ntiles) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gid = lane >> 2, tig = lane & 3;
   const int wm = warp >> 2, wn = warp & 3;
-  const int e = p.tile_expert[tile], m0 = p.tile_row0[tile];
+  const int e = p.tile[tile].x, m0 = p.tile[tile].y;
   const int mend = p.offsets[e + 1];
   constexpr int BN = DUAL ? 64 : 128;                    // output columns per CTA
   const int n0 = blockIdx.y * BN;
@@ -626,25 +677,38 @@ grouped_gemm_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// The same product on the fifth-generation tensor cores. One CTA = 128 rows of one expert x 128 B-rows, accumulator
-// [128 lanes x 128 columns] float32 in tensor memory. A and B k-steps of 64 (128 bytes per row) land in shared memory
-// through the same gathering cp.async ring, laid out as the K-major 128-byte-swizzle operand layout (row r at r * 128
-// bytes, 16-byte chunk c at position c ^ (r & 7); 8-row groups 1024 bytes apart), so that one elected thread multiplies a
-// stage with four tcgen05.mma (M 128, N 128, K 16) whose completion (tcgen05.commit on an mbarrier) frees the slot.
-// Every wait is bounded: a barrier that does not complete raises the plan's error word, and the CTA drains its copies,
-// frees its tensor memory and leaves without storing.
+// The same product on the fifth-generation tensor cores: pairs of CTAs that stay, one CTA per SM, walk tiles of 256 channels x up to 256 rows
+// of one expert. The channels are the M of tcgen05.mma (cta_group::2, 128 in each CTA's tensor memory; for the gated product 64 gate and the
+// 64 up channels of the same columns), the rows its N: an expert's rows are divided evenly into tiles of a multiple of 16, so that hardly any
+// product is spent on padding. Operands are k-steps of 128 (two atoms of 64, 128 bytes per row) in a ring of three stages, laid out K-major with the 128-byte
+// swizzle (row r at r * 128 bytes, 16-byte chunk c at c ^ (r & 7); 8-row groups 1024 bytes apart): a CTA holds its own 128 channels and half
+// of the rows. Warps: 0 .. 7 epilogue, 8 .. 15 gather token rows (cp.async; scattered over the batch, which rules out a plain tile copy),
+// (in the down product, whose rows lie sorted, the first of them copies tiles), 16 the weights (TMA), 17 in the first CTA the products. A stage has one barrier, in the first CTA:
+// under this load a wait costs its warp 250 cycles even where nothing is left to wait for, so there are few: three a k-step of 64 made it 1000
+// cycles, one a k-step of 64 600 where rows are gathered (products: 410 for 205 rows). Two accumulators of 256 columns in tensor memory: a tile's activation and stores run under the next tile's products.
+// What bounds it: operands from L2, of which an SM gets about 60 bytes a cycle (64 KB k-steps of 128: 1000 to 1140 cycles, products 820; 2000 cycles
+// from request to arrival). 128 x 128 tiles, with a barrier of the whole CTA each k-step and an epilogue on its own, took 131 / 80 us (gated / down product; 8192
+// rows of 16 experts, 2048 x 1024), 128 x 256 tiles of one CTA 85 / 39; this form 80 / 38
+// with cold caches, the whole call 227 -> 130 in a row of calls (the pass over pairs without an expert, 10.5, is gone).
+// Every wait is bounded: a role whose barrier does not complete raises the plan's status word, the others follow; copies and products under
+// way are waited for (with the same limit), the tile is not stored, and the tensor memory is freed.
 // ---------------------------------------------------------------------------------------------------------------------
-constexpr int TC_STAGES = 3;                                               // 97 KB: two CTAs per SM
-constexpr int TC_TILE_BYTES = 128 * 128;                                   // 128 rows x 64 bf16
-constexpr size_t TC_SMEM = (size_t)TC_STAGES * 2 * TC_TILE_BYTES + 1024;   // + slack to start on a 1024-byte boundary
-constexpr uint32_t TC_COLS = 128;                                          // tensor-memory columns of the accumulator
+constexpr int TC_STAGES = 3, TC_BK = 128, TC_ATOMS = TC_BK / 64;           // k of a stage, in atoms of 64
+constexpr int TC_ROWS = 256;                                               // rows of a tile, at most
+constexpr int TC_W_ATOM = 128 * 128, TC_X_ATOM = TC_ROWS / 2 * 128;        // bytes
+constexpr int TC_W_BYTES = TC_ATOMS * TC_W_ATOM, TC_STAGE = TC_W_BYTES + TC_ATOMS * TC_X_ATOM;
+constexpr int TC_SWAP = 32 * 128 * 2;                                      // bytes: 32 rows x 128 channels of bf16 on their way out, per group of epilogue warps
+constexpr size_t TC_SMEM = (size_t)TC_STAGES * TC_STAGE + 2 * TC_SWAP + 1024;   // + slack to start on a 1024-byte boundary
+constexpr int TC_EPI = 8, TC_GATHER = 8, TC_WARP_TMA = TC_EPI + TC_GATHER, TC_WARP_MMA = TC_WARP_TMA + 1, TC_THREADS = (TC_WARP_MMA + 1) * 32;
+constexpr int TC_LAG = 2;                                                  // k-steps that a gathering warp has under way
+constexpr uint32_t TC_SPINS = 1u << 20;
 
 __device__ __forceinline__ uint32_t tc_smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void tc_mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
 }
-__device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t spins = 0; spins < (1u << 20); ++spins) {
+__device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity, volatile int* fail) {   // false: given up, here or by another role
+  for (uint32_t spins = 0; spins < TC_SPINS; ++spins) {
     uint32_t done;
     asm volatile(
         "{\n"
@@ -653,8 +717,22 @@ __device__ __forceinline__ bool tc_mbar_wait(uint32_t bar, uint32_t parity) {
         "selp.u32 %0, 1, 0, p;\n"
         "}\n" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
+    if (*fail) return false;
   }
+  *fail = 1;
   return false;
+}
+__device__ __noinline__ void tc_drain(uint32_t bar, uint32_t parity) {      // what is under way when the CTA gives up
+  int none = 0;
+  tc_mbar_wait(bar, parity, &none);
+}
+__device__ __forceinline__ void tc_arrive_first(uint32_t bar) {             // the barrier at this place in the pair's first CTA
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(mapa_shared(bar, 0)) : "memory");
+}
+__device__ __forceinline__ void tc_load(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  // cta_group::2: the barrier may be the other CTA's
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::"r"(dst), "l"(map),
+               "r"(bar), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ bool tc_elect_one() {
   uint32_t pred;
@@ -672,13 +750,13 @@ __device__ __forceinline__ uint64_t tc_desc_sw128(uint32_t smem_addr) {
   return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 // float32 accumulator [4,6) = 1, bfloat16 A [7,10) = 1 and B [10,13) = 1, both K-major, N >> 3 at [17,23), M >> 4 at [24,29)
-constexpr uint32_t TC_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-__device__ __forceinline__ void tc_mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-               ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(TC_IDESC), "r"(accumulate) : "memory");
+__device__ __forceinline__ uint32_t tc_idesc(int n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)n >> 3 << 17) | ((256u >> 4) << 24); }
+__device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+__device__ __forceinline__ void tc_commit_both(uint32_t bar) {              // the barrier at this place in both CTAs
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
@@ -689,160 +767,349 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
-// MODE 0: down product (rows in sorted order, output scattered to [token, choice]); 1: [gate ; up] product with the clamped
-// gated activation; 2: up product alone with the squared-ReLU activation (rows gathered, output in sorted order).
+// MODE 0: down product (rows in sorted order, output scattered to [token, choice]); 1 and 3: [gate ; up] product with the SiLU / the clamped
+// gated activation; 2: up product alone with the squared-ReLU activation (rows gathered, output in sorted order). Modes 1, 2 and 3 also
+// copy the rows of pairs without an expert from A to `whole` [npairs][K].
 template <int MODE>
-__global__ void __launch_bounds__(256)
-grouped_gemm_tc_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16* __restrict__ C, GroupPlan p, int K, int N, int top,
-                       float limit, int act) {
-  pdl_enter();
+__global__ void __launch_bounds__(TC_THREADS, 1)
+grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const bf16* __restrict__ A, bf16* __restrict__ C,
+                       const GroupPlan p, int K, int N, int top, int npairs, int E, float limit, const int* __restrict__ idx,
+                       bf16* __restrict__ whole) {
+  constexpr bool DUAL = MODE == 1 || MODE == 3, GATHER = MODE != 0;
+  constexpr int BN = DUAL ? 128 : 256;                   // output channels of a tile, half of them in this CTA
   extern __shared__ __align__(16) unsigned char tc_smem_raw[];
-  __shared__ int s_row[GG_BM];
-  __shared__ __align__(8) uint64_t s_bar[TC_STAGES];
+  __shared__ __align__(8) uint64_t s_full[TC_STAGES], s_free[TC_STAGES], s_done[2], s_taken[2], s_last;
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_fail;
-  const int tile = blockIdx.x;
-  if (tile >= *p.ntiles) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t base = (tc_smem_u32(tc_smem_raw) + 1023u) & ~1023u;      // stage s: A at base + s * 32 KB, B 16 KB after it
-  const int e = p.tile_expert[tile], m0 = p.tile_row0[tile];
-  const int mend = p.offsets[e + 1];
-  constexpr bool DUAL = MODE == 1, GATHER = MODE != 0;
-  constexpr int BN = DUAL ? 64 : 128;                    // output columns per CTA
-  const int n0 = blockIdx.y * BN;
-  if (tid < GG_BM) {
-    const int m = m0 + tid;
-    s_row[tid] = m < mend ? p.perm[m] : -1;
-  }
+  const uint32_t base = (tc_smem_u32(tc_smem_raw) + 1023u) & ~1023u;      // stage s: weights at base + s * TC_STAGE, rows after them
+  const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   if (tid == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) tc_mbar_init(tc_smem_u32(&s_bar[s]), 1);
+    for (int s = 0; s < TC_STAGES; ++s) {
+      tc_mbar_init(tc_smem_u32(&s_full[s]), 1 + (GATHER ? 2 * TC_GATHER : 0));     // first CTA's: the copies and gathering warps of both
+      tc_mbar_init(tc_smem_u32(&s_free[s]), 1);
+    }
+    for (int d = 0; d < 2; ++d) {
+      tc_mbar_init(tc_smem_u32(&s_done[d]), 1);
+      tc_mbar_init(tc_smem_u32(&s_taken[d]), 2 * TC_EPI);
+    }
+    tc_mbar_init(tc_smem_u32(&s_last), 1);
     s_fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem_u32(&s_tmem)), "r"(TC_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  if (warp == TC_WARP_MMA) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(tc_smem_u32(&s_tmem)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
+  cluster_sync_all();                                    // both CTAs' barriers and allocations are there
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  pdl_enter();                                           // the plan
   const uint32_t tmem = s_tmem;
-  const bf16* Be = B + (size_t)e * (DUAL ? 2 : 1) * N * K;
-  constexpr int NV = GG_BM * (GG_BK / 8) / 256, VPR = GG_BK / 8;        // 4 vectors of A and 4 of B per thread and stage
-  const bf16* a_src[NV];
-  const bf16* b_src[NV];
-  bool a_ok[NV], b_ok[NV];
-  uint32_t dst[NV];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) {
-    const int v = tid + q * 256, r = v / VPR, c8 = v % VPR;
-    const int pr = s_row[r];
-    a_ok[q] = pr >= 0;
-    a_src[q] = a_ok[q] ? (GATHER ? A + (size_t)(pr / top) * K : A + (size_t)(m0 + r) * K) + c8 * 8 : A;
-    int brow;
-    if (DUAL) brow = (r < 64 ? 0 : N) + n0 + (r & 63);
-    else brow = n0 + r;
-    b_ok[q] = (DUAL ? n0 + (r & 63) : n0 + r) < N;
-    b_src[q] = b_ok[q] ? Be + (size_t)brow * K + c8 * 8 : Be;
-    dst[q] = (uint32_t)(r * 128 + ((c8 ^ (r & 7)) << 4));
-  }
-  auto issue = [&](int stage, int k0) {
-    const uint32_t sa = base + (uint32_t)stage * (2 * TC_TILE_BYTES), sb = sa + TC_TILE_BYTES;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      const bool in_k = k0 + (((tid + q * 256) % VPR) * 8) < K;
-      const int na = (a_ok[q] && in_k) ? 16 : 0, nb = (b_ok[q] && in_k) ? 16 : 0;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa + dst[q]), "l"(a_src[q] + (na ? k0 : 0)), "r"(na) : "memory");
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sb + dst[q]), "l"(b_src[q] + (nb ? k0 : 0)), "r"(nb) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  const int nb = (N + BN - 1) / BN, nk = (K + TC_BK - 1) / TC_BK, count = *p.ntiles * nb;
+  struct Tile { int e, m0, mend, n0, rows; };            // expert, first sorted row, end of the expert's rows, first channel, N of the products
+  auto tile_at = [&](int it) {                           // (the roles ask for a tile while they are at the one before: the table lies in L2)
+    if (it >= count) return Tile{0, 0, 0, 0, 16};
+    const int tile = it / nb;
+    const int4 v = p.tile[tile];
+    return Tile{v.x, v.y, v.z, (it - tile * nb) * BN, v.w};
   };
-  const int nk = (K + GG_BK - 1) / GG_BK;
-  // ring: k-step kt lives in slot kt % TC_STAGES; TC_STAGES - 1 steps are in flight while one is multiplied. Past the end
-  // of K the copies are zero-size, so that every iteration commits exactly one group and the wait count stays fixed.
-#pragma unroll
-  for (int s = 0; s < TC_STAGES - 1; ++s) issue(s, s * GG_BK);
-  for (int kt = 0; kt < nk; ++kt) {
-    const int st = kt % TC_STAGES;
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(TC_STAGES - 2) : "memory");
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // this thread's rows, for the tensor cores' reads
-    __syncthreads();                                                    // k-step kt has landed for everyone
-    if (s_fail) break;                                                  // written before the barrier: uniform
-    if (warp == 0) {
+
+  if (warp < TC_EPI) {
+    if (GATHER) {                                        // pairs without an expert: this CTA's share, a warp per pair
+      const int share = (npairs + (int)gridDim.x - 1) / (int)gridDim.x, first = blockIdx.x * share, end = min(npairs, first + share);
+      for (int k0 = first + warp * 32; k0 < end; k0 += TC_EPI * 32) {
+        const int e = k0 + lane < end ? idx[k0 + lane] : 0;
+        unsigned m = __ballot_sync(0xffffffffu, k0 + lane < end && (e < 0 || e >= E));
+        for (; m; m &= m - 1) {
+          const int k = k0 + __ffs(m) - 1;
+          const uint4* src = reinterpret_cast<const uint4*>(A + (size_t)(k / top) * K);
+          uint4* dst = reinterpret_cast<uint4*>(whole + (size_t)k * K);
+          for (int c = lane; c < K / 8; c += 32) dst[c] = src[c];
+        }
+      }
+    }
+    // Warp w reads lanes 32 * (w & 3) .. + 31 (channels); the two groups of four warps take chunks of 32 rows in turn. A chunk goes through shared
+    // memory ([row][CH channels] bf16, CH = 128, or 64 of the gated product) to leave in 16-byte pieces (32 stores of two bytes a thread took
+    // 10 000 cycles a tile). Gated product: the gate channels' warps (0, 1) and the up channels' (2, 3) finish 16 rows of a chunk each, the other
+    // half's values cross through the same place. The loops are short: unrolled whole they ran at the speed of the instruction fetch.
+    constexpr int CH = BN / 2;
+    const int q = warp & 3, group = warp >> 2, gtid = tid & 127;
+    const int c_in = DUAL ? (q & 1) * 32 + lane : q * 32 + lane;
+    __nv_bfloat16* swap = reinterpret_cast<__nv_bfloat16*>(tc_smem_raw + (base - tc_smem_u32(tc_smem_raw)) + (size_t)TC_STAGES * TC_STAGE + (size_t)group * TC_SWAP);
+    auto meet = [&]() { asm volatile("bar.sync %0, 128;\n" ::"r"(1 + group) : "memory"); };
+    int i = 0;
+    Tile next = tile_at(pair);
+    for (int it = pair; it < count; it += pairs, ++i) {
+      const Tile t = next;
+      next = tile_at(it + pairs);
+      const int d = i & 1, rows = t.mend - t.m0, ch0 = t.n0 + rank * CH;
+      // the four warps go on or leave together: they meet below
+      const uint32_t given_up = tc_mbar_wait(tc_smem_u32(&s_done[d]), (uint32_t)(i >> 1) & 1, &s_fail) ? 0 : 1;
+      uint32_t leave;
+      asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, %2, 128, q;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leave) : "r"(given_up),
+                   "r"(1 + group) : "memory");
+      if (leave) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      if (tc_elect_one()) {
-        const uint64_t ad = tc_desc_sw128(base + (uint32_t)st * (2 * TC_TILE_BYTES));
-        const uint64_t bd = tc_desc_sw128(base + (uint32_t)st * (2 * TC_TILE_BYTES) + TC_TILE_BYTES);
+      const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + d * TC_ROWS;
+      for (int c0 = group * 32; c0 < rows; c0 += 64) {
+        uint32_t a[16], b[16];
+        __syncwarp();
+        tc_ld16(trow + (uint32_t)c0, a);
+        tc_ld16(trow + (uint32_t)c0 + 16, b);
+        tc_wait_ld();
+        if (DUAL) {
+          // projections leave the matrix unit in bfloat16, like the dense layers' products
+          const bool gate = q < 2;
+          __nv_bfloat16 *mine = swap + (gate ? 0 : 16) * CH + c_in, *theirs = swap + (gate ? 16 : 0) * CH + c_in;
 #pragma unroll
-        for (int ks = 0; ks < GG_BK / 16; ++ks) tc_mma_ss(tmem, ad + 2 * ks, bd + 2 * ks, (kt | ks) ? 1u : 0u);
-        tc_commit(tc_smem_u32(&s_bar[st]));
+          for (int x = 0; x < 16; ++x) theirs[x * CH] = __float2bfloat16_rn(__uint_as_float(gate ? b[x] : a[x]));
+          if (!gate) {
+#pragma unroll
+            for (int x = 0; x < 16; ++x) a[x] = b[x];
+          }
+          meet();
+#pragma unroll
+          for (int x0 = 0; x0 < 16; x0 += 4) {
+#pragma unroll
+            for (int x = x0; x < x0 + 4; ++x) {
+              const float own = __bfloat162float(__float2bfloat16_rn(__uint_as_float(a[x]))), other = __bfloat162float(mine[x * CH]);
+              float gv = gate ? own : other, uv = gate ? other : own, v;
+              if (MODE == 1) {
+                v = gv / (1.0f + expf(-gv)) * uv;
+              } else {
+                gv = fminf(gv, limit);
+                uv = fminf(fmaxf(uv, -limit), limit);
+                v = gv * (1.0f / (1.0f + expf(-1.702f * gv))) * (uv + 1.0f);
+              }
+              mine[x * CH] = __float2bfloat16_rn(v);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int x = 0; x < 32; ++x) {
+            float v = __uint_as_float(x < 16 ? a[x & 15] : b[x & 15]);
+            if (MODE == 2) {
+              v = fmaxf(__bfloat162float(__float2bfloat16_rn(v)), 0.f);
+              v = v * v;
+            }
+            swap[x * CH + c_in] = __float2bfloat16_rn(v);
+          }
+        }
+        meet();
+#pragma unroll
+        for (int j = 0; j < CH / 32; ++j) {              // 16-byte pieces: CH / 8 of them a row
+          const int piece = gtid + j * 128, x = piece / (CH / 8), c = piece % (CH / 8) * 8, m = t.m0 + c0 + x;
+          if (c0 + x < rows && ch0 + c < N)
+            *reinterpret_cast<uint4*>(C + (size_t)(MODE == 0 ? p.perm[m] : m) * N + ch0 + c) = *reinterpret_cast<const uint4*>(swap + x * CH + c);
+        }
+        meet();                                          // read before the next chunk is written
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc_arrive_first(tc_smem_u32(&s_taken[d]));            // the accumulator is read: it may be written again
+    }
+  } else if (warp < TC_WARP_TMA) {
+    if (GATHER) {
+      // A warp gathers 16 rows of a stage: eight lanes a row (16 bytes each), four rows at a time.
+      const int w = warp - TC_EPI, c8 = lane & 7;
+      int s = 0, hs = 0, under_way = 0;                  // next stage to fill, next to hand over
+      uint32_t parity = 1;                               // the first round of the ring finds its stages free
+      bool ok = true;
+      auto hand_over = [&](int left) {                   // all but the newest `left` k-steps have landed
+        if (left) asm volatile("cp.async.wait_group %0;\n" ::"n"(TC_LAG - 1) : "memory");
+        else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");    // this thread's rows, for the tensor cores' reads
+        __syncwarp();
+        for (; under_way > left; --under_way) {
+          if (lane == 0) tc_arrive_first(tc_smem_u32(&s_full[hs]));
+          hs = hs + 1 == TC_STAGES ? 0 : hs + 1;
+        }
+      };
+      auto rows_of = [&](const Tile& t, int (&pr)[4]) {                     // the pairs of this thread's rows; -1: padding
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int r = w * 16 + j * 4 + (lane >> 3), m = t.m0 + rank * (t.rows / 2) + r;
+          pr[j] = r < t.rows / 2 && m < t.mend ? p.perm[m] : -1;
+        }
+      };
+      const uint32_t place = (uint32_t)((w * 16 + (lane >> 3)) * 128);
+      const uint32_t even = (uint32_t)((c8 ^ (lane >> 3)) << 4), odd = even ^ 64u;        // rows 4 further: chunk ^ 4
+      Tile next = tile_at(pair);
+      int next_pr[4];
+      rows_of(next, next_pr);
+      for (int it = pair; it < count && ok; it += pairs) {
+        const Tile t = next;
+        const bf16* src[4];
+        unsigned read = 0, real = 0;                     // rows that the products read, and those of them that are not padding
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (w * 16 + j * 4 + (lane >> 3) < t.rows / 2) read |= 1u << j;
+          if (next_pr[j] >= 0) real |= 1u << j;
+          src[j] = A + (next_pr[j] >= 0 ? (size_t)(next_pr[j] / top) * K + c8 * 8 : 0);
+        }
+        next = tile_at(it + pairs);
+        for (int k = 0; k < nk; ++k) {
+          if (k == 1 || nk == 1) rows_of(next, next_pr);                    // used when the tile is done
+          if (under_way == TC_LAG) hand_over(TC_LAG - 1);                   // before the wait: the products must not wait for themselves
+          if (!__all_sync(0xffffffffu, tc_mbar_wait(tc_smem_u32(&s_free[s]), parity, &s_fail))) { ok = false; break; }
+          const uint32_t dst = base + s * TC_STAGE + TC_W_BYTES + place;
+#pragma unroll
+          for (int u = 0; u < TC_ATOMS; ++u) {
+            const unsigned full = k * TC_BK + u * 64 + c8 * 8 < K ? real : 0u;            // past the end of K: zeros
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (read >> j & 1)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + u * TC_X_ATOM + j * 512 + (j & 1 ? odd : even)),
+                             "l"(full >> j & 1 ? src[j] + u * 64 : A), "r"(full >> j & 1 ? 16 : 0) : "memory");
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) src[j] += TC_BK;
+          asm volatile("cp.async.commit_group;\n" ::: "memory");
+          ++under_way;
+          if (++s == TC_STAGES) { s = 0; parity ^= 1u; }
+        }
+      }
+      hand_over(0);
+    } else if (warp == TC_EPI) {                         // the sorted rows of the down product
+      if (tc_elect_one()) {
+        int s = 0;
+        uint32_t parity = 1;
+        bool ok = true;
+        Tile next = tile_at(pair);
+        for (int it = pair; it < count && ok; it += pairs) {
+          const Tile t = next;
+          next = tile_at(it + pairs);
+          const int boxes = (t.rows / 2 + 63) / 64, x0 = t.m0 + rank * (t.rows / 2);
+          for (int k = 0; k < nk; ++k) {
+            if (!tc_mbar_wait(tc_smem_u32(&s_free[s]), parity, &s_fail)) { ok = false; break; }
+            const uint32_t at = base + s * TC_STAGE + TC_W_BYTES, bar = mapa_shared(tc_smem_u32(&s_full[s]), 0);
+            for (int u = 0; u < TC_ATOMS; ++u)
+              for (int j = 0; j < boxes; ++j) tc_load(at + u * TC_X_ATOM + j * 64 * 128, &map_x, k * TC_BK + u * 64, x0 + j * 64, bar);
+            if (++s == TC_STAGES) { s = 0; parity ^= 1u; }
+          }
+        }
       }
       __syncwarp();
     }
-    // slot (kt - 1) % TC_STAGES is refilled next: the products of k-step kt - 1 must have read it
-    if (kt >= 1 && !tc_mbar_wait(tc_smem_u32(&s_bar[(kt - 1) % TC_STAGES]), (uint32_t)(((kt - 1) / TC_STAGES) & 1))) s_fail = 1;
-    issue((kt + TC_STAGES - 1) % TC_STAGES, (kt + TC_STAGES - 1) * GG_BK);
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  if (!s_fail && !tc_mbar_wait(tc_smem_u32(&s_bar[(nk - 1) % TC_STAGES]), (uint32_t)(((nk - 1) / TC_STAGES) & 1))) s_fail = 1;
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  if (s_fail) {
-    if (tid == 0) atomicExch(p.status, 1);
-  } else {
-    // warp w reads lanes 32 * (w & 3) .. + 31 (rows of the tile); the two warps of a lane quarter split the columns
-    const int r = (warp & 3) * 32 + lane, half = warp >> 2;
-    const int pr = s_row[r];
-    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-    bf16* crow = GATHER ? C + (size_t)(m0 + r) * N : C + (size_t)(pr < 0 ? 0 : pr) * N;
-    constexpr int GROUPS = DUAL ? 2 : 4;                 // groups of 16 output columns per warp
+  } else if (warp == TC_WARP_TMA) {
+    if (tc_elect_one()) {
+      int s = 0, issued = 0;
+      uint32_t parity = 1;
+      bool ok = true;
+      Tile next = tile_at(pair);
+      for (int it = pair; it < count && ok; it += pairs) {
+        const Tile t = next;
+        next = tile_at(it + pairs);
+        const int row0 = t.e * (DUAL ? 2 : 1) * N + t.n0 + rank * (BN / 2), row1 = row0 + N;                 // rows of a tensor: they fit an int
+        const int bytes = 2 * (TC_W_BYTES + (GATHER ? 0 : TC_ATOMS * ((t.rows / 2 + 63) / 64) * 64 * 128));               // of both CTAs
+        for (int k = 0; k < nk; ++k) {
+          if (!tc_mbar_wait(tc_smem_u32(&s_free[s]), parity, &s_fail)) { ok = false; break; }
+          const uint32_t at = base + s * TC_STAGE, bar = mapa_shared(tc_smem_u32(&s_full[s]), 0);
+          if (rank == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(tc_smem_u32(&s_full[s])), "r"(bytes) : "memory");
 #pragma unroll
-    for (int gq = 0; gq < GROUPS; ++gq) {
-      const int col = half * (GROUPS * 16) + gq * 16;    // output column inside the CTA's BN
-      uint32_t a[16], b[16];
-      tc_ld16(trow + (uint32_t)col, a);
-      if (DUAL) tc_ld16(trow + (uint32_t)(64 + col), b);
-      tc_wait_ld();
-      float v[16];
-#pragma unroll
-      for (int x = 0; x < 16; ++x) {
-        if (DUAL) {
-          // projections leave the matrix unit in bfloat16, like the dense layers' products
-          if (act == QSPEC_EXPERT_ACT_SILU) {
-            const float gv = __bfloat162float(__float2bfloat16_rn(__uint_as_float(a[x])));
-            const float uv = __bfloat162float(__float2bfloat16_rn(__uint_as_float(b[x])));
-            v[x] = gv / (1.0f + expf(-gv)) * uv;
-          } else {
-            const float gv = fminf(__bfloat162float(__float2bfloat16_rn(__uint_as_float(a[x]))), limit);
-            const float uv = fminf(fmaxf(__bfloat162float(__float2bfloat16_rn(__uint_as_float(b[x]))), -limit), limit);
-            v[x] = gv * (1.0f / (1.0f + expf(-1.702f * gv))) * (uv + 1.0f);
+          for (int u = 0; u < TC_ATOMS; ++u) {
+            tc_load(at + u * TC_W_ATOM, &map_w, k * TC_BK + u * 64, row0, bar);
+            if (DUAL) tc_load(at + u * TC_W_ATOM + TC_W_ATOM / 2, &map_w, k * TC_BK + u * 64, row1, bar);
           }
-        } else if (MODE == 2) {
-          const float u = fmaxf(__bfloat162float(__float2bfloat16_rn(__uint_as_float(a[x]))), 0.f);
-          v[x] = u * u;
-        } else {
-          v[x] = __uint_as_float(a[x]);
+          ++issued;
+          if (++s == TC_STAGES) { s = 0; parity ^= 1u; }
         }
       }
-      const int n = n0 + col;
-      if (pr >= 0) {
-        if (n + 16 <= N) {
-          uint4 w0, w1;
-          w0.x = pack_bf2(v[0], v[1]); w0.y = pack_bf2(v[2], v[3]); w0.z = pack_bf2(v[4], v[5]); w0.w = pack_bf2(v[6], v[7]);
-          w1.x = pack_bf2(v[8], v[9]); w1.y = pack_bf2(v[10], v[11]); w1.z = pack_bf2(v[12], v[13]); w1.w = pack_bf2(v[14], v[15]);
-          *reinterpret_cast<uint4*>(crow + n) = w0;
-          *reinterpret_cast<uint4*>(crow + n + 8) = w1;
-        } else {
-#pragma unroll
-          for (int x = 0; x < 16; ++x)
-            if (n + x < N) crow[n + x] = __float2bfloat16_rn(v[x]);
-        }
+      if (!ok && rank == 0) {                            // the newest copies of the ring, of both CTAs (which leave together)
+        for (int j = max(0, issued - TC_STAGES); j < issued; ++j) tc_drain(tc_smem_u32(&s_full[j % TC_STAGES]), (uint32_t)(j / TC_STAGES) & 1);
       }
     }
+    __syncwarp();
+  } else {
+    if (rank == 0 && tc_elect_one()) {
+      int s = 0, i = 0;
+      uint32_t parity = 0;
+      Tile next = tile_at(pair);
+      bool ok = true;
+      for (int it = pair; it < count && ok; it += pairs, ++i) {
+        const int d = i & 1;
+        const uint32_t idesc = tc_idesc(next.rows);
+        next = tile_at(it + pairs);
+        if (!tc_mbar_wait(tc_smem_u32(&s_taken[d]), ((uint32_t)(i >> 1) & 1) ^ 1, &s_fail)) { ok = false; break; }
+        for (int k = 0; k < nk; ++k) {
+          if (!tc_mbar_wait(tc_smem_u32(&s_full[s]), parity, &s_fail)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+          for (int u = 0; u < TC_ATOMS; ++u) {
+            const uint64_t wd = tc_desc_sw128(base + s * TC_STAGE + u * TC_W_ATOM), xd = tc_desc_sw128(base + s * TC_STAGE + TC_W_BYTES + u * TC_X_ATOM);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) tc_mma_pair(tmem + d * TC_ROWS, wd + 2 * ks, xd + 2 * ks, idesc, (k | u | ks) ? 1u : 0u);
+          }
+          tc_commit_both(tc_smem_u32(&s_free[s]));
+          if (k == nk - 1) tc_commit_both(tc_smem_u32(&s_done[d]));
+          if (++s == TC_STAGES) { s = 0; parity ^= 1u; }
+        }
+      }
+      if (!ok) {
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(tc_smem_u32(&s_last)) : "memory");
+        tc_drain(tc_smem_u32(&s_last), 0);
+      }
+    }
+    __syncwarp();
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TC_COLS) : "memory");
+  cluster_sync_all();                                    // neither CTA leaves while products read its operands or arrivals are on their way to it
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (tid == 0 && s_fail) atomicExch(p.status, 1);
+  if (warp == TC_WARP_MMA) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
+}
+
+// [rows][width] bf16 as it lies, boxes of box_rows x 64 elements, 128-byte swizzle
+static int tc_map(CUtensorMap* map, const void* ptr, size_t rows, int width, int box_rows) {
+  static const atile::EncodeTiled fn = []() -> atile::EncodeTiled {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess ? (atile::EncodeTiled)f
+                                                                                                                                        : nullptr;
+  }();
+  QSPEC_REQUIRE(fn, QSPEC_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
+  const cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)width * 2};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows}, unit[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, unit, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  QSPEC_REQUIRE(r == CUDA_SUCCESS, QSPEC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): %zu rows of %d", (int)r, rows, width);
+  return QSPEC_OK;
+}
+
+template <int MODE>
+static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mb, const bf16* A, bf16* C, const GroupPlan& p, int tiles, int K, int N, int top, int npairs,
+                          int E, float limit, const int* idx, bf16* whole, cudaStream_t st) {
+  auto kern = grouped_gemm_tc_kernel<MODE>;
+  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
+  int dev = 0;
+  QSPEC_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
+    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
+    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
+  constexpr int BN = MODE & 1 ? 128 : 256;
+  const long long most = (long long)tiles * ((N + BN - 1) / BN);
+  const int pairs = (sm_count() > 0 ? sm_count() : 148) / 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (unsigned)(most < pairs ? most : pairs));
+  cfg.blockDim = dim3(TC_THREADS);
+  cfg.dynamicSmemBytes = TC_SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  QSPEC_CUDA(cudaLaunchKernelEx(&cfg, kern, ma, mb, A, C, p, K, N, top, npairs, E, limit, idx, whole));
+  count_launch(1);
+  return QSPEC_OK;
 }
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -880,8 +1147,7 @@ static size_t grouped_layout(int ntok, int top, int E, int F, size_t* off) {
   off[1] = at; at = align_up(at + 4, 16);                        // status word (first, wherever the rest lies)
   off[0] = at; at = align_up(at + (size_t)(E + 1) * 4, 16);      // offsets
   off[2] = at; at = align_up(at + 4, 16);                        // ntiles
-  off[3] = at; at = align_up(at + max_tiles * 4, 16);            // tile_expert
-  off[4] = at; at = align_up(at + max_tiles * 4, 16);            // tile_row0
+  off[3] = off[4] = at; at = align_up(at + max_tiles * 16, 16);  // tile
   off[5] = at; at = align_up(at + npairs * 4, 16);               // perm
   off[6] = at; at = align_up(at + npairs * (size_t)F * 2, 16);   // Y
   return at;
@@ -910,40 +1176,45 @@ extern "C" int qspec_moe_expert_grouped_act(const void* h, const void* gate_up, 
   unsigned char* ws = (unsigned char*)workspace;
   GroupPlan p;
   p.offsets = (int*)(ws + off[0]); p.status = (int*)(ws + off[1]); p.ntiles = (int*)(ws + off[2]);
-  p.tile_expert = (int*)(ws + off[3]); p.tile_row0 = (int*)(ws + off[4]); p.perm = (int*)(ws + off[5]);
+  p.tile = (int4*)(ws + off[3]); p.perm = (int*)(ws + off[5]);
   bf16* Y = (bf16*)(ws + off[6]);
   const int npairs = ntok * top;
   const int max_tiles = npairs / 128 + E + 1;
-  launch_pdl(moe_identity_kernel, dim3(npairs), dim3(128), 0, st, (const bf16*)h, idx, (bf16*)out, W, E, top);
-  QSPEC_CHECK_LAUNCH(1);
+  // QSPEC_SEQ_GROUPED=mma selects the warp-level (mma.sync) tiles, kept as the comparison form for timing and tests
+  static const bool warp_level = [] { const char* v = getenv("QSPEC_SEQ_GROUPED"); return v && !strcmp(v, "mma"); }();
+  if (E == 0 || warp_level) {                                 // pairs without an expert; the tcgen05 form copies them itself
+    launch_pdl(moe_identity_kernel, dim3(npairs), dim3(128), 0, st, (const bf16*)h, idx, (bf16*)out, W, E, top);
+    QSPEC_CHECK_LAUNCH(1);
+  }
   if (E == 0) return QSPEC_OK;
-  launch_pdl(moe_group_kernel, dim3(1), dim3(1024), (size_t)(E + 1) * sizeof(int), st, idx, npairs, E, p);
+  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
+  int dev = 0;
+  QSPEC_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
+    QSPEC_CUDA(cudaFuncSetAttribute(moe_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_group_smem(MOE_KEEP * 1024, 8192)));
+    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
+  launch_pdl(moe_group_kernel, dim3(1), dim3(1024), moe_group_smem(npairs, E), st, idx, npairs, E, warp_level ? GG_BM : 0, moe_group_kept(npairs) ? 1 : 0, p);
   QSPEC_CHECK_LAUNCH(1);
+  QSPEC_REQUIRE(!warp_level || act == QSPEC_EXPERT_ACT_GATED, QSPEC_ERR_UNSUPPORTED,
+                "moe_expert_grouped: the warp-level comparison form has the gated activation only");
+  if (!warp_level) {
+    CUtensorMap mg, my, md;
+    const bool dual = act != QSPEC_EXPERT_ACT_RELU2;
+    int rc = tc_map(&mg, gate_up, (size_t)E * F * (dual ? 2 : 1), W, dual ? 64 : 128);
+    if (rc == QSPEC_OK) rc = tc_map(&my, Y, npairs, F, 64);
+    if (rc == QSPEC_OK) rc = tc_map(&md, down, (size_t)E * W, F, 128);
+    if (rc != QSPEC_OK) return rc;
+    auto first = act == QSPEC_EXPERT_ACT_SILU ? launch_grouped<1> : dual ? launch_grouped<3> : launch_grouped<2>;
+    rc = first(mg, mg, (const bf16*)h, Y, p, max_tiles, W, F, top, npairs, E, limit, idx, (bf16*)out, st);
+    if (rc != QSPEC_OK) return rc;
+    return launch_grouped<0>(my, md, nullptr, (bf16*)out, p, max_tiles, F, W, top, npairs, E, limit, idx, nullptr, st);
+  }
   static bool configured = false;
   if (!configured) {
     QSPEC_CUDA(cudaFuncSetAttribute(grouped_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM));
     QSPEC_CUDA(cudaFuncSetAttribute(grouped_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM));
-    QSPEC_CUDA(cudaFuncSetAttribute(grouped_gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-    QSPEC_CUDA(cudaFuncSetAttribute(grouped_gemm_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-    QSPEC_CUDA(cudaFuncSetAttribute(grouped_gemm_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
     configured = true;
-  }
-  // QSPEC_SEQ_GROUPED=mma selects the warp-level (mma.sync) tiles, kept as the comparison form for timing and tests
-  static const bool warp_level = [] { const char* v = getenv("QSPEC_SEQ_GROUPED"); return v && !strcmp(v, "mma"); }();
-  QSPEC_REQUIRE(!warp_level || act == QSPEC_EXPERT_ACT_GATED, QSPEC_ERR_UNSUPPORTED,
-                "moe_expert_grouped: the warp-level comparison form has the gated activation only");
-  if (!warp_level) {
-    if (act == QSPEC_EXPERT_ACT_RELU2)
-      launch_pdl(grouped_gemm_tc_kernel<2>, dim3(max_tiles, (F + 127) / 128), dim3(256), TC_SMEM, st, (const bf16*)h, (const bf16*)gate_up, Y,
-                 p, W, F, top, limit, act);
-    else
-      launch_pdl(grouped_gemm_tc_kernel<1>, dim3(max_tiles, (F + 63) / 64), dim3(256), TC_SMEM, st, (const bf16*)h, (const bf16*)gate_up, Y,
-                 p, W, F, top, limit, act);
-    QSPEC_CHECK_LAUNCH(1);
-    launch_pdl(grouped_gemm_tc_kernel<0>, dim3(max_tiles, (W + 127) / 128), dim3(256), TC_SMEM, st, (const bf16*)Y, (const bf16*)down,
-               (bf16*)out, p, F, W, top, limit, act);
-    QSPEC_CHECK_LAUNCH(1);
-    return QSPEC_OK;
   }
   launch_pdl(grouped_gemm_kernel<true>, dim3(max_tiles, (F + 63) / 64), dim3(256), GG_SMEM, st, (const bf16*)h, (const bf16*)gate_up, Y, p, W,
              F, top, limit);
