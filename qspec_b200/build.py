@@ -31,7 +31,7 @@ def _nvcc() -> str:
 
 
 def _newest_source_mtime(sources=None) -> float:
-    names = os.listdir(CSRC) if sources is None else list(sources) + ["common.cuh", "seq_common.cuh", "attn_tile.cuh", "gemm_w4_rows.cuh"]
+    names = [f for f in os.listdir(CSRC) if f != "fast_call.cpp"] if sources is None else list(sources) + ["common.cuh", "seq_common.cuh", "attn_tile.cuh", "gemm_w4_rows.cuh"]
     paths = [os.path.join(CSRC, f) for f in names]
     paths.append(os.path.join(HERE, "..", "include", "qspec_b200.h"))
     paths.append(os.path.join(HERE, "..", "include", "qspec_b200_seq.h"))
@@ -70,6 +70,25 @@ def build_seq_library(force: bool = False, verbose: bool = False) -> str:
     return SEQ_LIB_PATH
 
 
+def build_fast(force: bool = False) -> str:
+    """_C/_fast.so: the linear layers' call path (csrc/fast_call.cpp), against the headers of the torch that is installed."""
+    src, path = os.path.join(CSRC, "fast_call.cpp"), os.path.join(OUT_DIR, "_fast.so")
+    os.makedirs(OUT_DIR, exist_ok=True)
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= os.path.getmtime(src):
+        return path
+    import sysconfig
+    import torch
+    root, cuda = os.path.dirname(torch.__file__), os.path.dirname(os.path.dirname(_nvcc())) or "/usr/local/cuda"
+    tmp = f"{path}.{os.getpid()}"
+    r = subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+                        f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda}/include", src, "-o", tmp,
+                        f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for fast_call.cpp:\n{r.stderr}")
+    os.replace(tmp, path)
+    return path
+
+
 def build_variant(suffix: str, defines, verbose: bool = False) -> str:
     """Experiment builds: libqspec_b200<suffix>.so compiled with extra -D flags (select with QSPEC_LIB=<path>)."""
     os.makedirs(OUT_DIR, exist_ok=True)
@@ -97,7 +116,7 @@ def build_library(force: bool = False, verbose: bool = False, prof: bool = False
     """prof=True builds libqspec_b200_prof.so with the GEMM cycle counters compiled in (scripts/gpu_gemm_trace.py;
     select it with QSPEC_LIB=<path>); watchdog=True builds libqspec_b200_wd.so whose pipeline waits trap instead of
     hanging (for protocol changes). The product library carries neither."""
-    os.makedirs(OUT_DIR, exist_ok=True)
+    build_fast(force=force)
     lib_path = LIB_PATH.replace(".so", "_prof.so") if prof else LIB_PATH.replace(".so", "_wd.so") if watchdog else LIB_PATH
     if not force and os.path.exists(lib_path) and os.path.getmtime(lib_path) >= _newest_source_mtime(SOURCES):
         build_seq_library(force=False, verbose=verbose)

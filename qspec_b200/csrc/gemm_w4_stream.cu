@@ -1345,6 +1345,14 @@ static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, const RowsA
   if constexpr (MODE == MODE_I8) return p.M <= 48 ? rows_launch<MODE, 6>(mw, ma, p, st) : rows_launch<MODE, 8>(mw, ma, p, st);
   return QSPEC_ERR_UNSUPPORTED;
 }
+// workspace_bytes(mode, M, N, K), remembered for the sizes asked for last: the plan behind it takes a microsecond of a call of three
+static size_t rows_workspace_bytes(int mode, int M, int N, int K) {
+  struct Known { int mode, M, N, K; size_t bytes; };
+  static thread_local Known known[16];                        // (bytes 0: nothing known)
+  Known& k = known[((unsigned)N * 31u + (unsigned)K * 7u + (unsigned)M * 3u + (unsigned)mode) >> 3 & 15u];
+  if (!k.bytes || k.mode != mode || k.M != M || k.N != N || k.K != K) k = Known{mode, M, N, K, workspace_bytes(mode, M, N, K)};
+  return k.bytes;
+}
 static int rows_run(int mode, const void* act, const int8_t* w, const RowsArgs& a, int K, cudaStream_t st) {
   CUtensorMap mw, ma;
   int rc = get_map(w, (uint64_t)a.N, (uint64_t)K / 2, ROWS_R, 1, &mw);
@@ -1375,18 +1383,22 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   QSPEC_REQUIRE(((uintptr_t)act & 15) == 0 && ((uintptr_t)w & 15) == 0, QSPEC_ERR_UNSUPPORTED,
                 "%s: operand pointers must be 16-byte aligned", who);
   if (M == 0) return QSPEC_OK;
-  const bool rows = rows_wanted(mode, M, N, K);
-  Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
-  if (rows) pl.split = 1;                                   // whole sums: one slice
+  if (rows_wanted(mode, M, N, K)) {
+    // (it needs no workspace, but asks for the one of the stream form all the same: which form runs is not the caller's business)
+    const size_t need = rows_workspace_bytes(mode, M, N, K);
+    QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
+    QSPEC_REQUIRE(!split_out || split_bytes >= (size_t)M * N * 4, QSPEC_ERR_WORKSPACE, "%s: partial buffer too small (%zu < %zu)", who, split_bytes,
+                  (size_t)M * N * 4);
+    return rows_run(mode, act, w, RowsArgs{sA, sW, bias, out, acc_out, split_out, M, N, (K + ROWS_UK - 1) / ROWS_UK, (N + ROWS_R - 1) / ROWS_R, 0, out_bf16}, K, st);
+  }
+  const Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
   const size_t need = split_out ? workspace_bytes(mode, M, N, K) : workspace_bytes(pl);
   QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
   if (split_out) {
-    QSPEC_REQUIRE(pl.split >= 1 && (rows || pl.tiles_m == 1), QSPEC_ERR_UNSUPPORTED, "%s: no even k-split for M=%d N=%d K=%d", who, M, N, K);
+    QSPEC_REQUIRE(pl.split >= 1 && pl.tiles_m == 1, QSPEC_ERR_UNSUPPORTED, "%s: no even k-split for M=%d N=%d K=%d", who, M, N, K);
     QSPEC_REQUIRE(split_bytes >= (size_t)pl.split * M * N * 4, QSPEC_ERR_WORKSPACE, "%s: partial buffer too small (%zu < %zu)", who,
                   split_bytes, (size_t)pl.split * M * N * 4);
   }
-  if (rows)
-    return rows_run(mode, act, w, RowsArgs{sA, sW, bias, out, acc_out, split_out, M, N, (K + ROWS_UK - 1) / ROWS_UK, (N + ROWS_R - 1) / ROWS_R, 0, out_bf16}, K, st);
   CUtensorMap mw, ma;
   int rc = get_map(w, (uint64_t)N, (uint64_t)K / 2, TM, 1, &mw);
   if (rc != QSPEC_OK) return rc;

@@ -17,6 +17,7 @@ from __future__ import annotations
 
 from typing import Optional
 
+import ctypes
 import os
 
 import torch
@@ -60,6 +61,35 @@ def _ptr(t: Optional[torch.Tensor]):
 
 
 _I4 = (torch.int8, torch.uint8)
+
+# csrc/fast_call.cpp: the linear layers' calls without the Python below them. It takes what the functions here take without an error and
+# returns None for everything else, which then goes the ordinary way (and so does everything where it has not been built).
+try:
+    from ._C import _fast
+except ImportError:
+    _fast = None
+_addresses: dict = {}
+
+
+def _address(name: str) -> int:
+    found = _addresses.get(name)
+    if found is None:
+        lib = _lib.load()
+        found = ctypes.cast(getattr(lib, name), ctypes.c_void_p).value if isinstance(lib, ctypes.CDLL) else 0
+        _addresses[name] = found
+    return found
+
+
+def _fast_linear(name: str, kind: int, x, x_scale, weight, weight_scale, bias, out, what: str) -> bool:
+    """True: the call has been made."""
+    if _fast is None or out is None:
+        return False
+    status = _fast.linear(_address(name), kind, x, x_scale, weight, weight_scale, bias, out, _workspaces, "w4a16" if kind == 1 else "w4a4")
+    if status is None:
+        return False
+    if status:
+        _lib.check(status, what)
+    return True
 
 # ---------------------------------------------------------------------------------------------
 # workspaces: one zero-initialised, self-cleaning buffer per (device, kind); grown on demand.
@@ -343,6 +373,8 @@ def rowwise_scaled_linear_cutlass_s4s4_unified(input: torch.Tensor, input_scale:
                                                weight: torch.Tensor, weight_scale: torch.Tensor,
                                                bias: Optional[torch.Tensor], result: torch.Tensor) -> torch.Tensor:
     """W4A4: result = T(((acc * input_scale[m]) * weight_scale[n]) + bias[n]); exact int32 acc."""
+    if _fast_linear("qspec_gemm_w4a4", 0, input, input_scale, weight, weight_scale, bias, result, "rowwise_scaled_linear_cutlass_s4s4_unified"):
+        return result
     _chk(input, "input", _I4); _chk(weight, "weight", _I4)
     _chk(result, "result", (_F16, _BF16))
     _chk(input_scale, "input_scale", (result.dtype,)); _chk(weight_scale, "weight_scale", (result.dtype,))
@@ -387,6 +419,8 @@ def gemm_w4a16(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor
                bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
     """W4A16: out = x @ (int4(weight) * weight_scale[:, None]).T (+ bias); weight is the SAME
     two's-complement packed tensor the W4A4 path reads (no `^ 0x88` copy)."""
+    if _fast_linear("qspec_gemm_w4a16", 1, x, None, weight, weight_scale, bias, out, "gemm_w4a16"):
+        return out
     _chk(x, "x", (_F16, _BF16)); _chk(weight, "weight", _I4); _chk(out, "out", (x.dtype,))
     _chk(weight_scale, "weight_scale", (x.dtype,)); _chk(bias, "bias", (x.dtype,), True)
     N, K2 = weight.shape
@@ -447,6 +481,8 @@ def rowwise_scaled_linear_cutlass_s8s4(input: torch.Tensor, input_scale: torch.T
                                        weight_scale: torch.Tensor, bias: Optional[torch.Tensor] = None,
                                        result: Optional[torch.Tensor] = None) -> torch.Tensor:
     """W4A8: result = T(((acc * input_scale[m]) * weight_scale[n]) + bias[n]); input int8 [M, K], weight packed int4 [N, K/2]."""
+    if _fast_linear("qspec_gemm_w4a8", 2, input, input_scale, weight, weight_scale, bias, result, "rowwise_scaled_linear_cutlass_s8s4"):
+        return result
     _chk(input, "input", (torch.int8,)); _chk(weight, "weight", _I4)
     _chk(input_scale, "input_scale", (_F16, _BF16)); _chk(weight_scale, "weight_scale", (input_scale.dtype,))
     _chk(bias, "bias", (input_scale.dtype,), True)

@@ -117,3 +117,46 @@ def test_capture_and_two_streams(ops):
                 ops.gemm_w4a16(s[5], s[0], s[1], None, o)
     torch.cuda.synchronize()
     assert all(torch.equal(o, w) for o, w in zip(outs, want))
+
+
+def _outcome(call):
+    try:
+        return call().clone()
+    except Exception as e:
+        return type(e), str(e)
+
+
+@pytest.mark.parametrize("kind", ["w4a4", "w4a8", "w4a16"])
+def test_native_call_path_takes_and_refuses_what_the_python_path_does(ops, monkeypatch, kind):
+    """Every form of call, with and without csrc/fast_call.cpp: the same values, the same errors."""
+    if ops._fast is None:
+        pytest.skip("csrc/fast_call.cpp is not built")
+    M, N, K = 5, 96, 256
+    w, sW, bias, sA, q, x = _operands(M, N, K, torch.float16, 3)
+    packed = ((q[:, 0::2] & 15) | (q[:, 1::2] << 4)).contiguous()
+    act = {"w4a4": packed, "w4a8": q, "w4a16": x}[kind]
+    new = lambda *s, dtype=torch.float16: torch.zeros(*(s or (M, N)), dtype=dtype, device="cuda")  # noqa: E731
+
+    def run(act=act, sA=sA, w=w, sW=sW, bias=bias, out=None):
+        out = new() if out is None else out
+        if kind == "w4a16":
+            return ops.gemm_w4a16(act, w, sW, bias, out)
+        return {"w4a4": ops.rowwise_scaled_linear_cutlass_s4s4_unified, "w4a8": ops.rowwise_scaled_linear_cutlass_s8s4}[kind](act, sA, w, sW, bias, out)
+
+    wide = torch.cat([w, w], 1)
+    forms = [
+        {}, {"bias": None}, {"w": w.view(torch.uint8)}, {"sW": sW.view(-1, 1)}, {"act": act.view(1, M, -1)}, {"out": new(1, M, N)}, {"w": torch.nn.Parameter(w, requires_grad=False)},
+        {"act": act.cpu()}, {"w": w.cpu()}, {"act": act.t().contiguous().t()}, {"w": wide[:, :K // 2]}, {"out": new(M, 2 * N)[:, :N]}, {"out": new(M + 1, N)},
+        {"out": new(dtype=torch.float32)}, {"out": new(dtype=torch.bfloat16)}, {"sW": sW.float()}, {"sW": sW[:-1].contiguous()}, {"bias": bias[:-1].contiguous()},
+        {"bias": bias.bfloat16()}, {"w": w.view(-1)}, {"w": wide}, {"act": act[:, :-128].contiguous()}, {"act": act[:0]}, {"act": act.float()}, {"w": w.int()},
+        {"w": w[:N - 4].contiguous(), "sW": sW[:N - 4].contiguous(), "bias": None, "out": new(M, N - 4)}, {"act": None}, {"out": "no tensor"},
+    ]
+    if kind != "w4a16":
+        forms += [{"sA": sA.view(-1, 1)}, {"sA": sA[:-1].contiguous()}, {"sA": sA.bfloat16()}, {"sA": None}, {"act": act.view(torch.uint8)}]
+    fast = ops._fast
+    for form in forms:
+        got = _outcome(lambda: run(**form))
+        monkeypatch.setattr(ops, "_fast", None)
+        want = _outcome(lambda: run(**form))
+        monkeypatch.setattr(ops, "_fast", fast)
+        assert (torch.equal(got, want) if isinstance(want, torch.Tensor) and isinstance(got, torch.Tensor) else got == want), (form.keys(), got, want)
