@@ -51,7 +51,8 @@ constexpr int WARP_MMA = NCONV + NEPI;
 constexpr int WARP_TMA = WARP_MMA + 1;
 constexpr int THREADS = (WARP_TMA + 1) * 32;   // 448
 constexpr int MAX_STAGES = 12;
-constexpr int MAX_TA = 14;           // TMEM operand slots of 32 columns (I8: 128 k, F16: 64 k)
+constexpr int TA_COLS = 64;          // columns of a TMEM operand slot (I8: 256 k, F16: 128 k): what one hand-over from converters to products covers
+constexpr int MAX_TA = 7;
 
 // ---- PTX wrappers ----------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -372,10 +373,12 @@ __device__ __forceinline__ void finalize16(const Params& p, const uint32_t (&r)[
 
 // ---- the kernel --------------------------------------------------------------------------------
 // Shared-memory map (dynamic, 1024-aligned): [stages][16 KB packed W] | [stages][act stage] |
-// (I8 only) [ta][np * 128 B] int8 token tiles. act stage = np*128 B (I8: packed int4) or np*512 B
+// (I8 only) [ta][2][np * 128 B] int8 token tiles. act stage = np*128 B (I8: packed int4) or np*512 B
 // (F16: 4 K-major SW128 atoms of 64 k).
-// Tensor-memory map: D0 at column 0, D1 at dcols, then `ta` operand slots of 32 columns; one slot is what
-// 4 UMMAs consume (I8: 128 k, F16: 64 k). Decode tiles (np <= 64) take 256 columns and ~100 KB of shared
+// Tensor-memory map: D0 at column 0, D1 at dcols, then `ta` operand slots of 64 columns; one slot is what
+// 8 UMMAs consume (I8: 256 k, F16: 128 k). With slots of 32 columns the issuing thread met a barrier every 4 UMMAs, and a wait costs it about 220
+// cycles under this load even where nothing is left to wait for, as much as the products themselves: W4A16 10240 x 8192, 256 tokens 50.1 -> 47.6 us,
+// 1999 tokens 279 -> 264; W4A4 4096 x 14336, 256 tokens 31.8 -> 30.7. Decode tiles (np <= 64) take 256 columns and ~100 KB of shared
 // memory so that two CTAs -- the tail of one GEMM and the head of the next -- share an SM.
 struct Ring {                         // (index, phase) of an mbarrier ring, advanced without divisions
   int idx, n; uint32_t phase;
@@ -416,7 +419,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   constexpr bool I8 = MODE == MODE_I8 || MODE == MODE_A8; // integer accumulate, per-token activation scale in the epilogue
   constexpr bool A8 = MODE == MODE_A8;                    // int8 activations, used as TMA delivers them (like F16)
   constexpr bool ACONV = MODE == MODE_I8;                 // packed int4 activations, widened by the converters into sm_b
-  constexpr int SPU = I8 ? 2 : 4;                         // TMEM operand slots per 256-k unit
+  constexpr int SPU = I8 ? 1 : 2;                         // TMEM operand slots per 256-k unit
   constexpr int ATOMS = A8 ? 2 : 4, ATOM_ELEMS = A8 ? 128 : 64;   // 128-byte K-major atoms of the TMA'd activation stage
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t w_full[MAX_STAGES], w_empty[MAX_STAGES];
@@ -446,7 +449,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   unsigned char* sm_w = base;
   unsigned char* sm_act = sm_w + (size_t)S * W_STAGE;
   unsigned char* sm_b = sm_act + (size_t)S * act_stage;   // I8 only
-  unsigned char* sm_recv = sm_b + (ACONV ? (size_t)TA * npl * 128 : 0);   // cluster reduction: [cs-1][np][128] partial sums pushed by the peers
+  unsigned char* sm_recv = sm_b + (ACONV ? (size_t)TA * npl * 256 : 0);   // cluster reduction: [cs-1][np][128] partial sums pushed by the peers
 
   const uint32_t stage_tx = (uint32_t)(W_STAGE + act_stage);
   int pt = u0 / KB, kb = u0 - pt * KB;                // (producer warp) tile / k-unit of the next unit to load
@@ -565,17 +568,21 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             mbar_wait(smem_u32(&a_full[sl.idx]), sl.phase);
             PROF(1);
             tc_fence_after();
-            const uint32_t a_tmem = tmem + tmem_a_col + sl.idx * 32;
-            // I8: slot = half unit, tokens from the converted int8 ring; F16: slot = one 64-k atom of x
+            const uint32_t a_tmem = tmem + tmem_a_col + sl.idx * TA_COLS;
+            // I8: slot = unit, tokens from the converted int8 ring; F16: slot = half a unit, two 64-k atoms of x
             // (PAIR: each CTA holds npl = np / 2 token rows at this offset; the instruction reads both halves)
-            const uint32_t b0 = ACONV ? smem_u32(sm_b + (size_t)sl.idx * (npl * 128))
-                                   : smem_u32(sm_act + (size_t)st.idx * act_stage + sub * (npl * 128));
-            const uint64_t bdesc = make_desc_sw128(b0);
+            const uint32_t b0 = ACONV ? smem_u32(sm_b + (size_t)sl.idx * (npl * 256))
+                                   : smem_u32(sm_act + (size_t)st.idx * act_stage + sub * (npl * 256));
             const uint32_t first = (k > ka || sub > 0) ? 1u : 0u;
-            umma_ts<MODE, PAIR>(d_tmem, a_tmem, bdesc, idesc, first);
-            umma_ts<MODE, PAIR>(d_tmem, a_tmem + 8, bdesc + 2, idesc, 1u);     // +32 B along K = +2 in the (>>4) start field
-            umma_ts<MODE, PAIR>(d_tmem, a_tmem + 16, bdesc + 4, idesc, 1u);
-            umma_ts<MODE, PAIR>(d_tmem, a_tmem + 24, bdesc + 6, idesc, 1u);
+#pragma unroll
+            for (int atom = 0; atom < 2; ++atom) {
+              const uint64_t bdesc = make_desc_sw128(b0 + atom * (npl * 128));
+              const uint32_t a0 = a_tmem + atom * 32;
+              umma_ts<MODE, PAIR>(d_tmem, a0, bdesc, idesc, atom ? 1u : first);
+              umma_ts<MODE, PAIR>(d_tmem, a0 + 8, bdesc + 2, idesc, 1u);       // +32 B along K = +2 in the (>>4) start field
+              umma_ts<MODE, PAIR>(d_tmem, a0 + 16, bdesc + 4, idesc, 1u);
+              umma_ts<MODE, PAIR>(d_tmem, a0 + 24, bdesc + 6, idesc, 1u);
+            }
             PROF(4);
             umma_commit<PAIR>(smem_u32(&a_empty[sl.idx]));
             if (!ACONV && sub == SPU - 1) umma_commit<PAIR>(smem_u32(&w_empty[st.idx]));
@@ -621,24 +628,20 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 #pragma unroll
       for (int c = 0; c < 8; ++c) pk[c] = *reinterpret_cast<const uint4*>(wrow + ((c ^ swz) << 4));
       if (A8) {
-        // W4A8: weights widened in natural k order into the two half-unit slots; the int8 activations stay where TMA put them
-        Ring s1 = sl;
-        s1.next();
+        // W4A8: weights widened in natural k order into the unit's slot; the int8 activations stay where TMA put them
         mbar_wait(smem_u32(&a_empty[sl.idx]), sl.phase ^ 1u);
-        mbar_wait(smem_u32(&a_empty[s1.idx]), s1.phase ^ 1u);
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint32_t r[8];
           widen_i8_nat(pk[c], r);
-          tmem_st8(lane_base + (c < 4 ? sl.idx : s1.idx) * 32 + (c & 3) * 8, r);
+          tmem_st8(lane_base + sl.idx * TA_COLS + c * 8, r);
         }
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           arrive_a_full(sl.idx);
-          arrive_a_full(s1.idx);
           mbar_arrive(smem_u32(&w_empty[st.idx]));     // the weight half of the stage; the MMA commit releases the activation half
         }
       } else if (ACONV) {
@@ -662,22 +665,19 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             if (tok < npl) akb[j] = *reinterpret_cast<const uint4*>(act + tok * 128 + ((ac ^ (tok & 7)) << 4));
           }
         }
-        Ring s1 = sl;                                    // second half-unit slot
-        s1.next();
         mbar_wait(smem_u32(&a_empty[sl.idx]), sl.phase ^ 1u);
-        mbar_wait(smem_u32(&a_empty[s1.idx]), s1.phase ^ 1u);
         tc_fence_after();
         PROF(1);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint32_t r[8];
           widen_i8(pk[c], r);
-          tmem_st8(lane_base + (c < 4 ? sl.idx : s1.idx) * 32 + (c & 3) * 8, r);
+          tmem_st8(lane_base + sl.idx * TA_COLS + c * 8, r);
         }
         PROF(2);
         // packed activations of the unit (8 chunks per token) -> two int8 atoms [npl][128 B], SW128 (PAIR: this CTA's half of the tokens)
-        unsigned char* bt0 = sm_b + (size_t)sl.idx * (npl * 128);
-        unsigned char* bt1 = sm_b + (size_t)s1.idx * (npl * 128);
+        unsigned char* bt0 = sm_b + (size_t)sl.idx * (npl * 256);
+        unsigned char* bt1 = bt0 + npl * 128;
         {
           const int cc = ac & 3;
           unsigned char* bt = ac < 4 ? bt0 : bt1;
@@ -722,22 +722,21 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         __syncwarp();
         if (lane == 0) {
           arrive_a_full(sl.idx);
-          arrive_a_full(s1.idx);
           mbar_arrive(smem_u32(&w_empty[st.idx]));
         }
         PROF(6);
       } else {
         Ring sq = sl;
 #pragma unroll
-        for (int sub = 0; sub < 4; ++sub) {
+        for (int sub = 0; sub < SPU; ++sub) {
           mbar_wait(smem_u32(&a_empty[sq.idx]), sq.phase ^ 1u);
           tc_fence_after();
           PROF(1);
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
+          for (int cc = 0; cc < 4; ++cc) {
             uint32_t r[16];
-            dequant32<MODE == MODE_BF16>(pk[2 * sub + cc], r);
-            tmem_st16(lane_base + sq.idx * 32 + cc * 16, r);
+            dequant32<MODE == MODE_BF16>(pk[(4 * sub + cc) & 7], r);
+            tmem_st16(lane_base + sq.idx * TA_COLS + cc * 16, r);
           }
           PROF(2);
           tmem_wait_st();
@@ -746,7 +745,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
           __syncwarp();
           if (lane == 0) {
             arrive_a_full(sq.idx);
-            if (sub == 3) mbar_arrive(smem_u32(&w_empty[st.idx]));
+            if (sub == SPU - 1) mbar_arrive(smem_u32(&w_empty[st.idx]));
           }
           sq.next();
           PROF(6);
@@ -1232,11 +1231,11 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   pl.dcols = pl.np <= 32 ? 32 : pl.np <= 64 ? 64 : pl.np <= 128 ? 128 : 256;
   pl.dbufs = pl.dcols <= 128 ? 2 : 1;
   pl.tmem_cols = small ? 256 : 512;
-  pl.ta = (pl.tmem_cols - pl.dbufs * pl.dcols) / 32;
+  pl.ta = (pl.tmem_cols - pl.dbufs * pl.dcols) / TA_COLS;
   if (pl.ta > MAX_TA) pl.ta = MAX_TA;
   const int npl = pl.pair ? pl.np / 2 : pl.np;              // token rows per CTA
   const size_t act_stage = mode == MODE_I8 ? (size_t)npl * 128 : mode == MODE_A8 ? (size_t)npl * 256 : (size_t)npl * 512;
-  const size_t fixed = 1024 + (mode == MODE_I8 ? (size_t)pl.ta * npl * 128 : 0);
+  const size_t fixed = 1024 + (mode == MODE_I8 ? (size_t)pl.ta * npl * 256 : 0);
   const size_t budget = small ? (size_t)110 * 1024 : (size_t)(227 * 1024 - 2048);
   int st = (int)((budget - fixed) / (W_STAGE + act_stage));
   if (st > MAX_STAGES) st = MAX_STAGES;
