@@ -298,6 +298,7 @@ struct Params {
   int dcols, ta, tmem_cols;   // accumulator buffer width, operand slots, TMEM allocation (columns)
   int dbufs;                  // accumulator buffers: 2 (the epilogue of tile i overlaps the main loop of tile i + 1), or 1 for 256-token tiles
   int out_bf16;
+  int stage_at;          // LONG: offset of the epilogue's stage in shared memory
   int debug_exit;        // debug: 1 = exit after setup, 2 = no TMEM alloc + exit after setup, 3 = exit at entry
   int trace_cta;         // debug: second CTA whose marks are recorded
   int trigger;           // when to release the dependent grid: 0 after setup, 1 when the weight stream has been issued, 2 at the end
@@ -332,6 +333,41 @@ __device__ __forceinline__ void finalize_store(const Params& p, uint32_t raw, in
     if (p.bias) f = __fadd_rn(f, bs);
     if (MODE == MODE_BF16) ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(f);
     else ((__half*)p.out)[o] = __float2half_rn(f);
+  }
+}
+
+// What the LONG form (below) stores with, eight channels (ch % 8 == 0) of a token as one 16-byte piece. Same arithmetic, same rounding.
+template <int MODE>
+__device__ __forceinline__ void finalize_store8(const Params& p, const uint32_t (&raw)[8], int tok_g, int ch, float sa, const float* sw, const float* bs) {
+  constexpr bool INT = MODE == MODE_I8 || MODE == MODE_A8;
+  const bool bf = INT ? p.out_bf16 != 0 : MODE == MODE_BF16;
+  uint32_t h[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    float f = INT ? __fmul_rn(__fmul_rn(__int2float_rn(((int32_t)raw[e]) >> (MODE == MODE_A8 ? 4 : 8)), sa), sw[e]) : __fmul_rn(__uint_as_float(raw[e]), sw[e]);
+    if (p.bias) f = __fadd_rn(f, bs[e]);
+    h[e] = bf ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
+  }
+  *reinterpret_cast<uint4*>((uint16_t*)p.out + (size_t)tok_g * p.N + ch) = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
+}
+// A warp's stage: [8][36] words, then scales and bias of its 32 channels. The 16 tokens of a tcgen05.ld group (tokens tok0 + j, j < nt) cross it
+// eight at a time, so that a lane finishes eight channels of one token.
+constexpr int STAGE_LD = 36, STAGE_WORDS = 8 * STAGE_LD + 64, STAGE_BYTES = NEPI * STAGE_WORDS * 4;
+template <int MODE>
+__device__ __forceinline__ void finalize16_staged(const Params& p, const uint32_t (&r)[16], int nt, int tok0, int ch0, const float* sa, uint32_t* stage) {
+  const int lane = threadIdx.x & 31, c = (lane & 3) * 8, tok = lane >> 2;
+  const float* s_sw = reinterpret_cast<const float*>(stage + 8 * STAGE_LD);
+#pragma unroll 1
+  for (int h8 = 0; h8 < 16 && h8 < nt; h8 += 8) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) stage[j * STAGE_LD + lane] = h8 ? r[8 + j] : r[j];
+    __syncwarp();
+    if (h8 + tok < nt && ch0 + c < p.N) {
+      const uint4 lo = *reinterpret_cast<const uint4*>(stage + tok * STAGE_LD + c), hi = *reinterpret_cast<const uint4*>(stage + tok * STAGE_LD + c + 4);
+      const uint32_t raw[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      finalize_store8<MODE>(p, raw, tok0 + h8 + tok, ch0 + c, sa[h8 + tok], s_sw + c, s_sw + 32 + c);
+    }
+    __syncwarp();                                        // read before the next eight are written
   }
 }
 
@@ -413,7 +449,13 @@ __device__ __forceinline__ unsigned long long gtimer_ns() {
 // activation tile in its shared memory. The leader (rank 0) issues every tcgen05.mma for both; its a_full / d_empty
 // barriers collect the arrivals of both CTAs (the follower arrives remotely), its commits are multicast to both.
 // p.U / p.G then count pair-units and pairs; blockIdx.x >> 1 is the pair.
-template <int MODE, bool PAIR>
+// LONG: the form for products whose CTAs have a tile's length or more to do each (the rule is in run()). What ends such a launch is an epilogue
+// that nothing hides, of up to 256 tokens: it runs once or twice, at the speed at which its instructions are fetched, so it is short here. Values
+// leave eight channels at a time through a stage in shared memory (16 stores of two bytes a lane, unrolled, took 4 us for a tile of 64 tokens), and a
+// shared tile that only waits for this CTA's part is finished from the accumulator. Outputs have to be 16-byte aligned, N a multiple of 8; no
+// deferred sums, clusters or raw int32 results. One kernel for both would be slower on either side: what an epilogue does not run lies between
+// what it does (tried: M = 100, 4096 x 4096, 10 to 15 % slower).
+template <int MODE, bool PAIR, bool LONG>
 __global__ void __launch_bounds__(THREADS, 1)
 w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_act, const Params p) {
   constexpr bool I8 = MODE == MODE_I8 || MODE == MODE_A8; // integer accumulate, per-token activation scale in the epilogue
@@ -427,6 +469,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   __shared__ __align__(8) uint64_t d_full[2], d_empty[2];
   __shared__ uint32_t tmem_base_smem;
   __shared__ unsigned s_is_last[2];
+  __shared__ uint32_t s_all_here;
   __shared__ __align__(8) uint64_t red_full;             // cluster reduction: every pushing thread of the other CTAs arrives here
   __shared__ float s_sa[128];
 
@@ -771,6 +814,8 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (p.bias) bs_ = p.out_bf16 ? __bfloat162float(__ldg((const __nv_bfloat16*)p.bias + ch_)) : __half2float(__ldg((const __half*)p.bias + ch_));
       }
     };
+    // LONG: behind the operand rings
+    uint32_t* const stage = reinterpret_cast<uint32_t*>(base + p.stage_at) + q * STAGE_WORDS;
     int npf = 0, pf_t[2] = {0, 0}, pf_cf[2] = {0, 0}, pf_cl[2] = {0, 0};   // this CTA's tiles that are shared with other CTAs
     // ---- stream-K tiles shared with other CTAs (at most two per CTA: its first and its last tile). The protocol is
     // runs right after the tile's accumulator has been drained (overlapping the main loop unless it is the CTA's last
@@ -813,7 +858,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
             if (p.bias) bse[e] = p.out_bf16 ? __bfloat162float(__ldg((const __nv_bfloat16*)p.bias + chq + e)) : __half2float(__ldg((const __half*)p.bias + chq + e));
           }
         }
-        if (m_here <= 4) {
+        if (!LONG && m_here <= 4) {
           // decode (one item per thread): four CONTRIBUTORS per round trip instead (a 4-token tile shared by 4 CTAs is one round)
           const int tok = tok_base;
           if (tok < m_here) {
@@ -895,8 +940,22 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                 const int tok = tok0 + 4 * k;
                 if (tok < m_here) {
                   const uint32_t a4[4] = {acc4[k].x, acc4[k].y, acc4[k].z, acc4[k].w};
+                  if (LONG) {
+                    constexpr bool INT = MODE == MODE_I8 || MODE == MODE_A8;
+                    const bool bf = INT ? p.out_bf16 != 0 : MODE == MODE_BF16;
+                    uint32_t h[4];
   #pragma unroll
-                  for (int e = 0; e < 4; ++e) finalize_store<MODE>(p, a4[e], m0 + tok, chq + e, sa[k], swe[e], bse[e]);
+                    for (int e = 0; e < 4; ++e) {
+                      float f = INT ? __fmul_rn(__fmul_rn(__int2float_rn(((int32_t)a4[e]) >> (MODE == MODE_A8 ? 4 : 8)), sa[k]), swe[e])
+                                    : __fmul_rn(__uint_as_float(a4[e]), swe[e]);
+                      if (p.bias) f = __fadd_rn(f, bse[e]);
+                      h[e] = bf ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
+                    }
+                    *reinterpret_cast<uint2*>((uint16_t*)p.out + (size_t)(m0 + tok) * p.N + chq) = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+                  } else {
+  #pragma unroll
+                    for (int e = 0; e < 4; ++e) finalize_store<MODE>(p, a4[e], m0 + tok, chq + e, sa[k], swe[e], bse[e]);
+                  }
                 }
               }
             }
@@ -922,6 +981,12 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       // everything a tile needs from global memory is requested one tile ahead of its use
       const float sw = sw_next, bs = bs_next;
       load_scale(u + (kb_end - ka), sw_next, bs_next);
+      if (LONG) {                                          // this warp's channels: written and read by this warp alone
+        __syncwarp();
+        stage[8 * STAGE_LD + lane] = __float_as_uint(sw);
+        stage[8 * STAGE_LD + 32 + lane] = __float_as_uint(bs);
+        __syncwarp();
+      }
       if (I8 && p.out && !p.split_out && sa_tile != tile_m) {   // decode (one token tile): loaded once per kernel
         named_bar_sync(1, NEPI * 32);                    // previous tile's readers are done with s_sa
         if (etid < m_here)
@@ -938,7 +1003,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       if (etid == 0) MARK(6 + 3 * min(f, 2));
       const uint32_t d_addr = tmem + ((uint32_t)(q * 32) << 16) + (db ? (uint32_t)p.dcols : 0u);
       const int split_rank = full ? 0 : cta - c_first;     // deferred reduction: this CTA's slice of the tile's k range
-      const bool clus = !PAIR && p.cs > 1;                 // the tile is shared by exactly this cluster; rank 0 owns it
+      const bool clus = !PAIR && !LONG && p.cs > 1;        // the tile is shared by exactly this cluster; rank 0 owns it
       const uint32_t crank = clus ? (uint32_t)(blockIdx.x % p.cs) : 0u;
       uint32_t push_base = 0;
       if (clus) {
@@ -953,15 +1018,50 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                          : "=r"(done) : "r"(smem_u32(&red_full)) : "memory");
         }
       }
+      // LONG: a shared tile whose other contributors have all arrived is finished from the accumulator, which spares this CTA's own part the way
+      // through the workspace and back: at the end of a launch nothing hides it. Asked only where it is likely, of the tile at the end of a CTA's
+      // range, whose rest the next CTA began with.
+      bool direct = false;
+      if (LONG && !full && u0 < t * KB) {
+        if (etid == 0) {
+          unsigned seen;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(p.counters + phys(c_first)) : "memory");
+          s_all_here = seen == (unsigned)(c_last - c_first) ? 1u : 0u;   // (written once: a range has one such tile)
+        }
+        named_bar_sync(1, NEPI * 32);
+        direct = s_all_here != 0;
+      }
+      if (LONG && direct) {
+        const size_t slot_words = (size_t)(np * TM);
+#pragma unroll 1
+        for (int c0 = 0; c0 < m_here; c0 += 16) {
+          uint32_t r[16], acc[16];
+          tmem_ld16(d_addr + c0, r);
+          bool have = false;
+          for (int c = c_first; c <= c_last; ++c) {        // ascending CTA order, as in resolve_shared
+            uint32_t v[16];
+            const uint32_t* src = p.ws_part + (size_t)(2 * phys(c) + (c == c_first && cta_start(c_first, p.U, p.G) < t * KB ? 1 : 0)) * slot_words +
+                                  (size_t)c0 * TM + chl;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = c == cta ? r[j] : c0 + j < m_here ? __ldcg(src + (size_t)j * TM) : 0u;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              acc[j] = !have ? v[j] : I8 ? acc[j] + v[j] : __float_as_uint(__fadd_rn(__uint_as_float(acc[j]), __uint_as_float(v[j])));
+            have = true;
+          }
+          finalize16_staged<MODE>(p, acc, m_here - c0, m0 + c0, n0 + q * 32, s_sa + c0, stage);
+        }
+        if (etid == 0) p.counters[phys(c_first)] = 0u;     // self-cleaning; this CTA never counted itself
+      }
       // What happens to the accumulators is chosen per TILE, outside the token loop. With the five-way choice inside it every
       // token carried ~330 instructions and one 16-token group spanned ~80 KB of code: the epilogue ran at instruction-fetch
       // speed (profiling build, gate_up W4A4: 3.4 us per 16-token group on an otherwise idle SM, 12-17 us per tile at M = 64).
-      const int variant = (p.debug_exit & 64) ? -1 : p.split_out ? 0 : full ? 1 : !clus ? 2 : crank != 0 ? 3 : 4;
-      for (int c0 = 0; c0 < m_here; c0 += 16) {
+      const int variant = (p.debug_exit & 64) ? -1 : !LONG && p.split_out ? 0 : full ? 1 : !clus ? 2 : crank != 0 ? 3 : 4;
+      for (int c0 = 0; c0 < m_here && !direct; c0 += 16) {
         uint32_t r[16];
         tmem_ld16(d_addr + c0, r);                       // warp-collective: never skipped per thread
         const int nt = m_here - c0;                      // this group's tokens are c0 + jj, jj < nt
-        if (variant == 0) {                              // deferred reduction: raw k-slice partial sums
+        if (!LONG && variant == 0) {                     // deferred reduction: raw k-slice partial sums
           if (ch_ok) {
             uint32_t* dst = p.split_out + ((size_t)split_rank * p.M + m0 + c0) * p.N + ch;
             const size_t ld = (size_t)p.N;
@@ -970,17 +1070,18 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
               if (jj < nt) dst[jj * ld] = r[jj];
           }
         } else if (variant == 1) {                       // whole tile in this CTA: epilogue and store
-          if (ch_ok) finalize16<MODE>(p, r, nt, m0 + c0, ch, s_sa + c0, sw, bs);
+          if (LONG) finalize16_staged<MODE>(p, r, nt, m0 + c0, n0 + q * 32, s_sa + c0, stage);
+          else if (ch_ok) finalize16<MODE>(p, r, nt, m0 + c0, ch, s_sa + c0, sw, bs);
         } else if (variant == 2) {                       // stream-K partial tile through the workspace
           uint32_t* dst = my_slot + (size_t)c0 * TM + chl;
 #pragma unroll
           for (int jj = 0; jj < 16; ++jj)
             if (jj < nt) dst[jj * TM] = r[jj];
-        } else if (variant == 3) {                       // cluster reduction, non-owner: push to the owner's shared memory
+        } else if (!LONG && variant == 3) {                       // cluster reduction, non-owner: push to the owner's shared memory
 #pragma unroll
           for (int jj = 0; jj < 16; ++jj)
             if (jj < nt) st_dsmem_u32(push_base + (uint32_t)((c0 + jj) * TM) * 4u, r[jj]);
-        } else if (variant == 4) {                       // cluster reduction, owner
+        } else if (!LONG && variant == 4) {                       // cluster reduction, owner
 #pragma unroll
           for (int jj = 0; jj < 16; ++jj) {
             const int tok = c0 + jj;
@@ -1006,7 +1107,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         else mbar_arrive(smem_u32(&d_empty[db]));
       }
       if (etid == 0) MARK(7 + 3 * min(f, 2));
-      if (!full && !clus && !p.split_out && !(p.debug_exit & 32)) {   // remember the shared tile; the protocol runs after the loop
+      if (!full && !direct && !clus && !p.split_out && !(p.debug_exit & 32)) {   // remember the shared tile; the protocol runs after the loop
         pf_t[npf] = t; pf_cf[npf] = c_first; pf_cl[npf] = c_last;
         ++npf;
         resolve_shared(npf - 1, npf);
@@ -1104,9 +1205,10 @@ static int env_int(const char* name, int dflt) {
   return v ? atoi(v) : dflt;
 }
 
+constexpr int SMEM_MOST = 227 * 1024 - 2048;   // dynamic: the static part is below 2 KB
 // pair = 1: CTA pairs (cta_group::2). tiles_n, U and G then count PAIR-tiles (two adjacent 128-channel tiles), pair-units
 // (2 x 16 KB of weights) and pairs; the launch has 2 G CTAs in clusters of two.
-struct Plan { int np, tiles_m, tiles_n, KB, U, G, cs, split, stages, dcols, dbufs, ta, tmem_cols, pair; size_t smem, slot_bytes; };
+struct Plan { int np, tiles_m, tiles_n, KB, U, G, cs, split, stages, dcols, dbufs, ta, tmem_cols, pair; size_t smem, slot_bytes, stage_bytes; };
 
 // QSPEC_GEMM_PAIR: 1 (default) = CTA pairs whenever the shape allows it, 0 = never (the round-1 kernel; kept for A/B runs).
 // QSPEC_GEMM_PAIR_MIN_M: smallest token count that uses pairs (default below). Read at every call: A/B runs in one process.
@@ -1236,7 +1338,7 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   const int npl = pl.pair ? pl.np / 2 : pl.np;              // token rows per CTA
   const size_t act_stage = mode == MODE_I8 ? (size_t)npl * 128 : mode == MODE_A8 ? (size_t)npl * 256 : (size_t)npl * 512;
   const size_t fixed = 1024 + (mode == MODE_I8 ? (size_t)pl.ta * npl * 256 : 0);
-  const size_t budget = small ? (size_t)110 * 1024 : (size_t)(227 * 1024 - 2048);
+  const size_t budget = small ? (size_t)110 * 1024 : (size_t)(SMEM_MOST);
   int st = (int)((budget - fixed) / (W_STAGE + act_stage));
   if (st > MAX_STAGES) st = MAX_STAGES;
   if (!small && st > env_int("QSPEC_GEMM_STAGES", 6)) st = env_int("QSPEC_GEMM_STAGES", 6);
@@ -1244,6 +1346,7 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   pl.stages = st;
   pl.smem = fixed + (size_t)st * (W_STAGE + act_stage) + (pl.cs > 1 ? (size_t)(pl.cs - 1) * pl.np * TM * 4 : 0);
   pl.slot_bytes = (size_t)pl.np * TM * 4;
+  pl.stage_bytes = W_STAGE + act_stage;
   return pl;
 }
 
@@ -1252,12 +1355,12 @@ static size_t workspace_bytes(const Plan& pl) {
 }
 static size_t workspace_bytes(int mode, int M, int N, int K) { return M <= 0 || N <= 0 || K <= 0 ? 0 : workspace_bytes(make_plan(mode, M, N, K)); }
 
-template <int MODE, bool PAIR>
+template <int MODE, bool PAIR, bool LONG>
 static int launch(const CUtensorMap& mw, const CUtensorMap& ma, const Params& p, const Plan& pl, cudaStream_t st) {
-  auto kern = w4_stream_kernel<MODE, PAIR>;
+  auto kern = w4_stream_kernel<MODE, PAIR, LONG>;
   static bool configured = false;
   if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 2048));
+    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST));
     configured = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -1390,7 +1493,7 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
                   (size_t)M * N * 4);
     return rows_run(mode, act, w, RowsArgs{sA, sW, bias, out, acc_out, split_out, M, N, (K + ROWS_UK - 1) / ROWS_UK, (N + ROWS_R - 1) / ROWS_R, 0, out_bf16}, K, st);
   }
-  const Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
+  Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
   const size_t need = split_out ? workspace_bytes(mode, M, N, K) : workspace_bytes(pl);
   QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
   if (split_out) {
@@ -1416,19 +1519,49 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   p.trace = g_trace ? g_trace + (size_t)(g_trace_seq++ % 8u) * 4096 : nullptr;
   p.M = M; p.N = N; p.K = K; p.np = pl.np; p.tiles_m = pl.tiles_m; p.KB = pl.KB; p.U = pl.U; p.G = pl.G; p.cs = pl.cs;
   p.stages = pl.stages; p.dcols = pl.dcols; p.dbufs = pl.dbufs; p.ta = pl.ta; p.tmem_cols = pl.tmem_cols; p.out_bf16 = out_bf16;
+  // The LONG form wherever it can run and a CTA's range is at least a tile long, so that whole tiles and ends of ranges are what a launch waits
+  // for. us, without | with it:  W4A16 28672 x 4096: 64 tokens 27.8 | 26.2, 256: 59.2 | 54.6, 1000: 198 | 186   10240 x 8192, 256 tokens: 46.9 | 43.7
+  //   W4A4 28672 x 4096: 65 tokens 24.6 | 22.9, 256: 49.4 | 38.9   W4A4 bytes 28672 x 4096: 64 tokens 20.5 | 18.2, 256: 47.5 | 35.8
+  // Shorter ranges, whose tiles are all shared, gain nothing: 4096 x 14336, 256 tokens, W4A4 30.1 | 31.4, W4A4 bytes 28.6 | 29.4, W4A16 34.6 | 34.6.
+  // Its stage may cost a ring its fifth stage, not its fourth (W4A16 27648 x 5120, 80 tokens, with three: 32.9 | 33.5).
+  if (out && !acc_out && !split_out && ((uintptr_t)out & 15) == 0 && N % 8 == 0 && pl.cs == 1 && pl.U >= pl.G * pl.KB && p.debug_exit == 0) {
+    if (pl.smem + STAGE_BYTES > (size_t)SMEM_MOST && pl.stages > 4) {
+      pl.stages -= 1;
+      pl.smem -= pl.stage_bytes;
+      p.stages = pl.stages;
+    }
+    if (pl.smem + STAGE_BYTES <= (size_t)SMEM_MOST) {
+      p.stage_at = (int)(pl.smem - 1024);
+      pl.smem += STAGE_BYTES;
+      if (pl.pair) {
+        switch (mode) {
+          case MODE_I8: return launch<MODE_I8, true, true>(mw, ma, p, pl, st);
+          case MODE_F16: return launch<MODE_F16, true, true>(mw, ma, p, pl, st);
+          case MODE_A8: return launch<MODE_A8, true, true>(mw, ma, p, pl, st);
+          default: return launch<MODE_BF16, true, true>(mw, ma, p, pl, st);
+        }
+      }
+      switch (mode) {
+        case MODE_I8: return launch<MODE_I8, false, true>(mw, ma, p, pl, st);
+        case MODE_F16: return launch<MODE_F16, false, true>(mw, ma, p, pl, st);
+        case MODE_A8: return launch<MODE_A8, false, true>(mw, ma, p, pl, st);
+        default: return launch<MODE_BF16, false, true>(mw, ma, p, pl, st);
+      }
+    }
+  }
   if (pl.pair) {
     switch (mode) {
-      case MODE_I8: return launch<MODE_I8, true>(mw, ma, p, pl, st);
-      case MODE_F16: return launch<MODE_F16, true>(mw, ma, p, pl, st);
-      case MODE_A8: return launch<MODE_A8, true>(mw, ma, p, pl, st);
-      default: return launch<MODE_BF16, true>(mw, ma, p, pl, st);
+      case MODE_I8: return launch<MODE_I8, true, false>(mw, ma, p, pl, st);
+      case MODE_F16: return launch<MODE_F16, true, false>(mw, ma, p, pl, st);
+      case MODE_A8: return launch<MODE_A8, true, false>(mw, ma, p, pl, st);
+      default: return launch<MODE_BF16, true, false>(mw, ma, p, pl, st);
     }
   }
   switch (mode) {
-    case MODE_I8: return launch<MODE_I8, false>(mw, ma, p, pl, st);
-    case MODE_F16: return launch<MODE_F16, false>(mw, ma, p, pl, st);
-    case MODE_A8: return launch<MODE_A8, false>(mw, ma, p, pl, st);
-    default: return launch<MODE_BF16, false>(mw, ma, p, pl, st);
+    case MODE_I8: return launch<MODE_I8, false, false>(mw, ma, p, pl, st);
+    case MODE_F16: return launch<MODE_F16, false, false>(mw, ma, p, pl, st);
+    case MODE_A8: return launch<MODE_A8, false, false>(mw, ma, p, pl, st);
+    default: return launch<MODE_BF16, false, false>(mw, ma, p, pl, st);
   }
 }
 
