@@ -333,42 +333,70 @@ hadamard_k28_kernel(const uint4* __restrict__ x, const uint4* __restrict__ gate_
 // ------------------------------------------------------------------------------------------
 // Cluster version of the down_proj rotation for n = 256 / 512 / 1024: one thread-block CLUSTER of 7 CTAs per
 // token row instead of one CTA, so that a 4-token decode step uses 28 SMs and every phase is 7x shorter.
-// All exchange is PUSHED over distributed shared memory (remote stores are fire-and-forget; remote loads would
+// All exchange is PUSHED over distributed shared memory (remote loads would
 // put a DSMEM round trip on the critical path after every barrier). CTA c of the cluster
-//   phase 1: SiLU*up + FHT_n of n-blocks 4c..4c+3 (one warp per block), f16, stored into EVERY CTA's copy of
-//            the [28][n] rotated row; one cluster barrier;
+//   phase 1: SiLU*up + FHT_n of n-blocks 4c..4c+3 (one or two warps per block), f16, copied into EVERY CTA's
+//            [28][n] rotated row;
 //   phase 2: outputs o = 4c..4c+3 of the 28x28 +-1 mix for all n columns from local shared memory, fp32
 //            accumulate in ascending k;
-//   quant:   CTA amax stored into every CTA, second barrier, row amax locally, quantiser on its 4 x n outputs.
+//   quant:   CTA amax stored into every CTA, row amax locally, quantiser on its 4 x n outputs.
 // The arithmetic (order included) is that of hadamard_k28_kernel, so the two are bit-identical.
 // ------------------------------------------------------------------------------------------
 constexpr int K28_CLUSTER = 7;
 constexpr int K28_BPC = 4;                           // n-blocks (and mix outputs) per CTA
 
-template <int SLOTS>
-__global__ void __launch_bounds__(128)
+// WPB = 2 warps share an n-block (the last butterfly stage crosses through shared memory): 24 warps an SM at 64 rows instead of 12, and half the
+// work in each of the chain's steps; one warp a block where there are rows enough to fill the SMs and the exchange only costs (see the dispatch).
+// Blocks reach the other CTAs as bulk copies of the CTA's four blocks, the maxima as single words, both counted by an mbarrier in the CTA that
+// receives them: stores of every thread into seven CTAs, with a release and acquire of the whole cluster after them, were the largest stall.
+// SiLU and quantiser, before -> now: n = 512, 1 row 5.7 -> 4.8 us, 64 rows 11.6 -> 9.2, 512 rows 44.5 -> 39.8; n = 1024, 64 rows 24.3 -> 17.7,
+// 512 rows 128 -> 98; n = 256, 64 rows 8.2 -> 7.3 (1 row 3.8 -> 3.9: a bulk copy of 2 KB takes a little longer than stores).
+// A wait that is given up (it is bounded) leaves NaN outputs and scales.
+__device__ __forceinline__ bool k28_wait(uint32_t bar) {
+  for (uint32_t spins = 0; spins < (1u << 20); ++spins) {
+    uint32_t done;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(bar) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+template <int SLOTS, int WPB>
+__global__ void __launch_bounds__(128 * WPB)
 hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict__ gate_up,
                             __half* __restrict__ out_f, uint8_t* __restrict__ out_q,
                             __half* __restrict__ scale_out, int n, float scale, float clip, int c8) {
+  constexpr int S1 = SLOTS / WPB, THR = 128 * WPB;   // vectors of 8 per lane, threads
   pdl_enter();
-  cluster_arrive_relaxed();                           // "this CTA runs": waited for before the first remote store
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __half* sm = reinterpret_cast<__half*>(smem_raw);   // [28][n] f16: ALL rotated blocks of the row (pushed by the cluster)
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __half* sm = reinterpret_cast<__half*>(smem_raw);   // [28][n] f16: ALL rotated blocks of the row
+  __shared__ __align__(16) float xbuf[WPB == 2 ? 8 * S1 * 256 : 4];
+  __shared__ __align__(8) uint64_t s_blocks, s_amax;  // the other CTAs' blocks / every CTA's maximum have landed
   __shared__ float red[8];
-  __shared__ float amax_all[K28_CLUSTER];
+  __shared__ float amax_all[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x % K28_CLUSTER;             // rank in cluster (cluster dims = (7,1,1))
   const size_t row = blockIdx.x / K28_CLUSTER;
   const int L = 28 * n, inter_v = L >> 3, nv = n >> 3;
   const uint32_t sm_base = (uint32_t)__cvta_generic_to_shared(sm);
+  const uint32_t bar_blocks = (uint32_t)__cvta_generic_to_shared(&s_blocks), bar_amax = (uint32_t)__cvta_generic_to_shared(&s_amax);
+  const uint32_t own_bytes = (uint32_t)(K28_BPC * n * 2);
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_blocks));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_amax));
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar_blocks), "r"((K28_CLUSTER - 1) * own_bytes) : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar_amax), "r"(K28_CLUSTER * 4) : "memory");
+  }
+  __syncthreads();                                    // the barriers are there, for this CTA's waits
+  cluster_arrive_release();                           // ... and for the other CTAs' copies: waited for before the first one
 
-  // ---- phase 1: warp w rotates n-block 4c + w and pushes it into every CTA of the cluster
+  // ---- phase 1: WPB warps rotate n-block 4c + warp / WPB
   {
-    const int blk = K28_BPC * c + warp;
-    float v[SLOTS][8];
+    const int blk = K28_BPC * c + warp / WPB, half = warp % WPB;
+    float v[S1][8];
 #pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
-      const int vi = blk * nv + lane + s * 32;
+    for (int s = 0; s < S1; ++s) {
+      const int vi = blk * nv + lane + (half * S1 + s) * 32;
       if (gate_up) {
         float up[8], g[8];
         unpack_h8(__ldg(gate_up + row * 2 * inter_v + vi), up);
@@ -379,28 +407,46 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
         unpack_h8(__ldg(x + row * inter_v + vi), v[s]);
       }
     }
-    warp_fht<SLOTS>(v, lane, 5);
-    uint4 pk[SLOTS];
+    warp_fht<S1>(v, lane, 5);
+    if (WPB == 2) {                                   // the last stage, stride n / 2: the block's other warp holds the other operand
+      float* mine = xbuf + warp * (S1 * 256);
+      const float* theirs = xbuf + (warp ^ 1) * (S1 * 256);
 #pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
+      for (int s = 0; s < S1; ++s)
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(mine + s * 256 + i * 32 + lane * 4) = make_float4(v[s][i], v[s][i + 1], v[s][i + 2], v[s][i + 3]);
+      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + warp / 2) : "memory");
+#pragma unroll
+      for (int s = 0; s < S1; ++s)
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+          const float4 o = *reinterpret_cast<const float4*>(theirs + s * 256 + i * 32 + lane * 4);
+          const float ov[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[s][i + e] = half ? __fsub_rn(ov[e], v[s][i + e]) : __fadd_rn(v[s][i + e], ov[e]);
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < S1; ++s) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[s][i] = __fmul_rn(v[s][i], scale);
-      pk[s] = pack_h8(v[s]);
-    }
-    cluster_wait_acquire();                           // every CTA of the cluster has started
-#pragma unroll
-    for (int r = 0; r < K28_CLUSTER; ++r) {
-      const uint32_t dst = mapa_shared(sm_base + (uint32_t)(blk * n * 2), (uint32_t)r);
-#pragma unroll
-      for (int s = 0; s < SLOTS; ++s) st_dsmem_v4(dst + (uint32_t)(lane + s * 32) * 16u, pk[s]);
+      reinterpret_cast<uint4*>(sm)[blk * nv + lane + (half * S1 + s) * 32] = pack_h8(v[s]);
     }
   }
-  cluster_arrive_release();
-  cluster_wait_acquire();
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  __syncthreads();
+  cluster_wait_acquire();                             // every CTA of the cluster has started
+  if (threadIdx.x < K28_CLUSTER && (int)threadIdx.x != c) {
+    const uint32_t src = sm_base + (uint32_t)c * own_bytes;
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(mapa_shared(src, threadIdx.x)), "r"(src),
+                 "r"(own_bytes), "r"(mapa_shared(bar_blocks, threadIdx.x)) : "memory");
+  }
+  bool ok = k28_wait(bar_blocks);
+  if (out_q == nullptr) cluster_arrive_relaxed();     // (before the end: no CTA leaves while another may still copy from or into it)
 
-  // ---- phase 2: outputs o0..o0+3, column pairs jp = tid, tid + 128, ...; all 28 blocks are local now
+  // ---- phase 2: outputs o0..o0+3, column pairs jp = tid, tid + THR, ...; all 28 blocks are local now
   const int o0 = K28_BPC * c;
-  constexpr int PPT = SLOTS;                          // pairs per thread: n/2/128 = 1 (n=256), 2 (n=512), 4 (n=1024)
+  constexpr int PPT = S1;                             // pairs per thread: n / 2 / THR
   float keep[PPT][K28_BPC][2];
   {
     // one FFMA2 per (pair, o, k) with the sign as a +-1 multiplier from constant memory: the fp32 add / subtract in ascending k
@@ -418,7 +464,7 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
       for (int o = 0; o < K28_BPC; ++o) sg[o] = d_had28_sign.v[(o0 + o) * 28 + k];
 #pragma unroll
       for (int pp = 0; pp < PPT; ++pp) {
-        const float2 y = __half22float2(reinterpret_cast<const __half2*>(sm)[((k * n) >> 1) + threadIdx.x + pp * 128]);
+        const float2 y = __half22float2(reinterpret_cast<const __half2*>(sm)[((k * n) >> 1) + threadIdx.x + pp * THR]);
         const unsigned long long y2 = pack_f2(y.x, y.y);
 #pragma unroll
         for (int o = 0; o < K28_BPC; ++o) k2[pp][o] = ffma2_rn(y2, pack_f2(sg[o], sg[o]), k2[pp][o]);
@@ -433,26 +479,32 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
         keep[pp][o][1] = r.y;
       }
   }
+  const float nan = __uint_as_float(0x7fffffffu);
   float amax = 0.f;
 #pragma unroll
   for (int pp = 0; pp < PPT; ++pp) {
-    const int jp = threadIdx.x + pp * 128;
+    const int jp = threadIdx.x + pp * THR;
 #pragma unroll
     for (int o = 0; o < K28_BPC; ++o) {
       keep[pp][o][0] = __half2float(__float2half_rn(keep[pp][o][0]));
       keep[pp][o][1] = __half2float(__float2half_rn(keep[pp][o][1]));
       amax = fmaxf(amax, fmaxf(fabsf(keep[pp][o][0]), fabsf(keep[pp][o][1])));
       if (out_f)
-        reinterpret_cast<__half2*>(out_f + row * L)[(((o0 + o) * n) >> 1) + jp] = __floats2half2_rn(keep[pp][o][0], keep[pp][o][1]);
+        reinterpret_cast<__half2*>(out_f + row * L)[(((o0 + o) * n) >> 1) + jp] =
+            ok ? __floats2half2_rn(keep[pp][o][0], keep[pp][o][1]) : __floats2half2_rn(nan, nan);
     }
   }
-  if (out_q == nullptr) return;                       // uniform over the cluster; nothing remote is outstanding
-  // ---- quantiser: CTA amax pushed to every CTA, one more barrier, row amax from local shared memory
+  if (out_q == nullptr) {                             // uniform over the cluster
+    cluster_wait_acquire();
+    return;
+  }
+  // ---- quantiser: CTA amax to every CTA, row amax from local shared memory
   amax = block_max(amax, red);
   if (threadIdx.x < K28_CLUSTER)
-    st_dsmem_u32(mapa_shared((uint32_t)__cvta_generic_to_shared(&amax_all[c]), (uint32_t)threadIdx.x), __float_as_uint(amax));
-  cluster_arrive_release();
-  cluster_wait_acquire();
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(mapa_shared((uint32_t)__cvta_generic_to_shared(&amax_all[c]), threadIdx.x)),
+                 "r"(__float_as_uint(amax)), "r"(mapa_shared(bar_amax, threadIdx.x)) : "memory");
+  ok = k28_wait(bar_amax) && ok;
+  cluster_arrive_relaxed();                           // (as above)
   float row_amax = 0.f;
 #pragma unroll
   for (int r = 0; r < K28_CLUSTER; ++r) row_amax = fmaxf(row_amax, amax_all[r]);
@@ -460,7 +512,7 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
   const float sc = __half2float(sh);
 #pragma unroll
   for (int pp = 0; pp < PPT; ++pp) {
-    const int jp = threadIdx.x + pp * 128;
+    const int jp = threadIdx.x + pp * THR;
 #pragma unroll
     for (int o = 0; o < K28_BPC; ++o) {
       const int q0 = max(-8, min(7, __half2int_rn(__float2half_rn(__fdiv_rn(keep[pp][o][0], sc)))));
@@ -470,7 +522,8 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
       else out_q[qi] = (uint8_t)((q0 & 0xF) | ((q1 & 0xF) << 4));
     }
   }
-  if (c == 0 && threadIdx.x == 0) scale_out[row] = sh;
+  if ((c == 0 || !ok) && threadIdx.x == 0) scale_out[row] = ok ? sh : __float2half_rn(nan);
+  cluster_wait_acquire();
 }
 
 }  // namespace qspec
@@ -569,13 +622,17 @@ static int launch_k28(const void* x, const void* gu, void* of, int8_t* oq, void*
   return QSPEC_OK;
 }
 
-template <int SLOTS>
+// n = 512: two warps a block up to here, one above. us with SiLU and quantiser, one | two warps: 1 row 5.7 | 4.8, 64: 10.9 | 9.2, 96: 13.7 | 12.1,
+// 112: 13.7 | 13.7, 128: 13.6 | 14.8, 512: 39.8 | 47.5 (the SMs are full either way, and the exchange between the warps is extra). n = 1024 always two (a lane
+// holds 16 values instead of 32), n = 256 always one (a lane has one vector).
+constexpr int K28_TWO_WARP_ROWS = 112;
+template <int SLOTS, int WPB>
 static int launch_k28_cluster(const void* x, const void* gu, void* of, int8_t* oq, void* so, int rows, int n,
                               float scale, float clip, cudaStream_t st, int c8) {
-  auto kern = hadamard_k28_cluster_kernel<SLOTS>;
+  auto kern = hadamard_k28_cluster_kernel<SLOTS, WPB>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)rows * K28_CLUSTER);
-  cfg.blockDim = dim3(128);
+  cfg.blockDim = dim3(128 * WPB);
   cfg.dynamicSmemBytes = (size_t)28 * n * sizeof(__half);
   static bool attr_set = false;                        // per instantiation (n = 1024 needs 56 KB)
   if (!attr_set) {
@@ -615,9 +672,12 @@ static int hadamard_k28_impl(const void* x, const void* gate_up, void* out_f16, 
   // neighbouring GEMMs' heads and tails. QSPEC_K28_CLUSTER_ROWS caps the row count that takes it (experiment knob).
   static const int cluster_rows = getenv("QSPEC_K28_CLUSTER_ROWS") ? atoi(getenv("QSPEC_K28_CLUSTER_ROWS")) : 65536;
   const bool few_rows = rows <= cluster_rows;
-  if (use_cluster && few_rows && n == 256) return launch_k28_cluster<1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
-  if (use_cluster && few_rows && n == 512) return launch_k28_cluster<2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
-  if (use_cluster && few_rows && n == 1024) return launch_k28_cluster<4>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
+  if (use_cluster && few_rows && n == 256) return launch_k28_cluster<1, 1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
+  if (use_cluster && few_rows && n == 512) {
+    if (rows <= K28_TWO_WARP_ROWS) return launch_k28_cluster<2, 2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
+    return launch_k28_cluster<2, 1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
+  }
+  if (use_cluster && few_rows && n == 1024) return launch_k28_cluster<4, 2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
   switch (n) {
     case 1024: return launch_k28<4, 28, true>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
     case 512:  return launch_k28<2, 28, true>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);

@@ -1,0 +1,32 @@
+"""The cluster form of the 28 x n rotation (csrc/hadamard_kernels.cu) on both sides of the rule that gives a block one warp or two, and as part
+of a larger batch: bit for bit the oracle, and the same row whatever stands around it."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [256, 512, 1024])
+@pytest.mark.parametrize("rows", [1, 2, 112, 113, 300])
+def test_rotation_is_the_oracle_and_batch_invariant(n, rows):
+    from oracle import qspec_oracle as O
+    from qspec_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + n)
+    x = torch.randn(rows, 28 * n, generator=g, device="cuda").half()
+    x[rows - 1, 5] = 300.0                                               # a row maximum that one CTA of the seven holds
+    scale = 0.00835418701171875
+
+    def run(part):
+        m = part.shape[0]
+        o, q, s = torch.empty_like(part), torch.empty(m, 14 * n, dtype=torch.int8, device="cuda"), torch.empty(m, dtype=torch.float16, device="cuda")
+        ops.hadamard_k28(part, n, scale, out=o, out_q=q, scale_out=s)
+        plain = torch.empty_like(part)
+        ops.hadamard_k28(part, n, scale, out=plain)
+        assert torch.equal(o, plain)
+        return o, q, s
+    o, q, s = run(x)
+    for i in sorted({0, rows - 1}):
+        for a, b in zip((o, q, s), run(x[i:i + 1].contiguous())):
+            assert torch.equal(a[i:i + 1], b)
+        np.testing.assert_array_equal(o[i:i + 1].cpu().numpy(), O.hadamard_k28(x[i:i + 1].cpu().numpy(), n, scale))
