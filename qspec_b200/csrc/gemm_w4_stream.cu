@@ -1392,9 +1392,11 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& ma, const Params& p,
 // Which calls the few-token kernel takes (gemm_w4_rows.cuh). Its time grows with the tokens (mma.sync, and for W4A16 the widening, which every
 // CTA does for its tokens at half the tensor rate), that of the tcgen05 form hardly: the line lies where they meet, later for products whose
 // time is mostly latency (up to 2^26 weights). us, few-token | tcgen05 form, on both sides of the lines:
-//   W4A4              28672 x 4096: 32 tokens 19.6 | 19.9, 48: 24.4 | 21.2   8192 x 8192: 64 tokens 18.5 | 19.1   10240 x 8192: 64: 31.0 | 21.7
-//   W4A4 bytes, W4A8  28672 x 4096: 24 tokens 16.6 | 17.6, 32: 27.1 | 17.8   8192 x 8192: 32 tokens 15.3 | 15.3   10240 x 8192: 32: 25.0 | 16.7
-//   W4A16             28672 x 4096: 16 tokens 20.0 | 26.1, 24: 31.1 | 27.0   8192 x 8192: 32 tokens 19.1 | 19.3   10240 x 8192: 24: 29.6 | 22.5
+//   W4A4              28672 x 4096: 32 tokens 20.0 | 18.1, 24: 15.9 | 17.9   27648 x 5120: 32: 19.4 | 20.9, 48: 25.2 | 22.3   8192 x 8192: 64: 19.0 | 18.8
+//   W4A4 bytes, W4A8  28672 x 4096: 24 tokens 17.1 | 16.3, 16: 14.5 | 15.7   27648 x 5120: 24: 16.4 | 18.5, 32: 28.6 | 18.8   8192 x 8192: 32: 15.6 | 14.9
+//   W4A16             28672 x 4096: 16 tokens 20.5 | 24.1, 24: 30.9 | 24.5   10240 x 8192: 16: 17.6 | 20.1, 24: 29.3 | 21.4   8192 x 8192: 32: 19.5 | 18.3
+// (the sizes differ by a few percent at one token count: the line is one for all), and well inside: 6144 x 4096, 64 tokens W4A4 11.5 | 12.6, 32 tokens
+// bytes 7.9 | 10.9, W4A16 10.7 | 12.6.
 // QSPEC_GEMM_ROWS, read at every call, for measurements and tests: 0 = none, 2 = all that it can run.
 static bool rows_wanted(int mode, int M, int N, int K) {
   const int want = env_int("QSPEC_GEMM_ROWS", 1);
