@@ -93,6 +93,10 @@ int qspec_gemm_split_factor(int w4a16, int M, int N, int K);
  * f16, 2 = W4A16 bf16, 3 = W4A8. out[0..7] = {token tile, CTA pairs?, grid (CTAs or CTA pairs), cluster size, deferred
  * split, ring stages, token tiles, (pair-)tiles along N}. */
 int qspec_debug_gemm_plan(int mode, int M, int N, int K, int deferred, int* out);
+/* For tests: the product of mode (0 W4A4, 1 W4A16 f16, 2 W4A16 bf16, 3 W4A8) into out, or the raw integer sums into acc. give_up 1: the first waits
+ * are given up at once, and what depends on them is NaN (raw sums: the lowest integer). */
+int qspec_debug_gemm_give_up(int mode, const void* act, const void* sA, const int8_t* w, const void* sW, const void* bias, void* out, int32_t* acc,
+                             int M, int N, int K, int dtype, void* workspace, size_t workspace_bytes, int give_up, void* stream);
 int qspec_gemm_w4a4_split(const int8_t* a, const int8_t* w, void* partials, size_t partial_bytes, int M, int N, int K,
                           void* workspace, size_t workspace_bytes, void* stream);
 int qspec_gemm_w4a16_split(const void* x, const int8_t* w, void* partials, size_t partial_bytes, int M, int N, int K,

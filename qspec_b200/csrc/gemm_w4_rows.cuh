@@ -22,8 +22,8 @@
 //   W4A16  4096 x 4096  3.9 / 4.9 |  9.6 / 10.4    28672 x 4096 14.8 / 20.5 | 23.5 / 24.1    4096 x 14336 9.2 / 10.9 | 15.4 / 16.3
 // Errors of the raw W4A16 sums against 64 bits: 9.3e-8 of their norm at K = 14336, 8.3e-8 at 4096 (tcgen05 form: 9.5e-7, 2.1e-7), for the tensor
 // cores cut at the accumulator's last bit and an accumulator takes only an item's 256 products; at K <= 512 both are off by 2e-8 to 8e-8.
-// Every wait is bounded. A CTA that gives one up stops loading, waits (with the same limit) for the copies under way, writes NaN (raw sums:
-// the lowest integer or NaN) and counts itself in rows_timeouts.
+// Every wait is bounded. A warp gives one up as a whole, stops loading and waits (up to the full limit) for its copies under way; its CTA writes NaN
+// (raw sums: the lowest integer or NaN) and counts itself in rows_timeouts.
 #pragma once
 
 constexpr int ROWS_R = 32, ROWS_UK = 256;          // channels of a tile, k of an item
@@ -36,14 +36,17 @@ struct RowsArgs {
   const void* sA; const void* sW; const void* bias;
   void* out; int32_t* acc_out; uint32_t* split_out;
   int M, N, items, tiles, depth, out_bf16;         // items of a tile; slots of a warp
+  int give_up;                                     // tests: every warp gives its first wait up at once
 };
 
+// By a whole warp, which goes on or gives up as one: what follows (mma.sync, elect) takes all its lanes. (The vote inside the loop costs nothing, for the
+// loop then needs no reconvergence; behind it, W4A16 28672 x 4096, 4 tokens 15.6 -> 16.3 us.)
 __device__ __forceinline__ bool rows_wait(uint32_t bar, uint32_t parity) {
   for (uint32_t spins = 0; spins < ROWS_SPINS; ++spins) {
     uint32_t done;
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
                  : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
+    if (__all_sync(0xffffffffu, done)) return true;
   }
   return false;
 }
@@ -170,7 +173,8 @@ w4_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const int rho = row_of<MODE>(g);
   int slot = 0, under_way = pre;
   uint32_t parity = 0;
-  bool ok = true;
+  bool ok = p.give_up == 0;
+  if (!ok) s_fail = 1;
   for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
     const int ch = tile * ROWS_R + ch_in;
     float sw = 0.f, bs = 0.f;                        // requested before the tile's sums are there

@@ -1477,7 +1477,7 @@ static int rows_run(int mode, const void* act, const int8_t* w, const RowsArgs& 
 
 static int run(int mode, const void* act, const void* sA, const int8_t* w, const void* sW, const void* bias, void* out,
                int32_t* acc_out, int M, int N, int K, int out_bf16, void* workspace, size_t ws_bytes, cudaStream_t st,
-               const char* who, uint32_t* split_out = nullptr, size_t split_bytes = 0) {
+               const char* who, uint32_t* split_out = nullptr, size_t split_bytes = 0, int give_up = 0) {
   QSPEC_REQUIRE(act && w && (out || acc_out || split_out), QSPEC_ERR_INVALID_ARG, "%s: null pointer", who);
   QSPEC_REQUIRE(!out || sW, QSPEC_ERR_INVALID_ARG, "%s: null scale pointer", who);
   QSPEC_REQUIRE(!mode_is_int(mode) || !out || sA, QSPEC_ERR_INVALID_ARG, "%s: null activation-scale pointer", who);
@@ -1493,7 +1493,8 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
     QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
     QSPEC_REQUIRE(!split_out || split_bytes >= (size_t)M * N * 4, QSPEC_ERR_WORKSPACE, "%s: partial buffer too small (%zu < %zu)", who, split_bytes,
                   (size_t)M * N * 4);
-    return rows_run(mode, act, w, RowsArgs{sA, sW, bias, out, acc_out, split_out, M, N, (K + ROWS_UK - 1) / ROWS_UK, (N + ROWS_R - 1) / ROWS_R, 0, out_bf16}, K, st);
+    return rows_run(mode, act, w, RowsArgs{sA, sW, bias, out, acc_out, split_out, M, N, (K + ROWS_UK - 1) / ROWS_UK, (N + ROWS_R - 1) / ROWS_R, 0, out_bf16, give_up},
+                    K, st);
   }
   Plan pl = make_plan(mode, M, N, K, split_out != nullptr);
   const size_t need = split_out ? workspace_bytes(mode, M, N, K) : workspace_bytes(pl);
@@ -1627,6 +1628,14 @@ extern "C" int qspec_debug_gemm_plan(int mode, int M, int N, int K, int deferred
   const w4s::Plan pl = w4s::make_plan(mode, M, N, K, deferred != 0);
   out[0] = pl.np; out[1] = pl.pair; out[2] = pl.G; out[3] = pl.cs; out[4] = pl.split; out[5] = pl.stages; out[6] = pl.tiles_m; out[7] = pl.tiles_n;
   return QSPEC_OK;
+}
+
+// For tests: the product of `mode` (0 W4A4, 1 W4A16 f16, 2 W4A16 bf16, 3 W4A8) into out or acc; give_up 1: its first waits are given up at once.
+extern "C" int qspec_debug_gemm_give_up(int mode, const void* act, const void* sA, const int8_t* w, const void* sW, const void* bias, void* out, int32_t* acc,
+                                        int M, int N, int K, int dtype, void* workspace, size_t workspace_bytes, int give_up, void* stream) {
+  QSPEC_REQUIRE(mode >= 0 && mode <= 3 && (w4s::mode_is_int(mode) || !acc), QSPEC_ERR_INVALID_ARG, "debug_gemm_give_up: mode %d", mode);
+  return w4s::run(mode, act, sA, w, sW, bias, out, acc, M, N, K, dtype == QSPEC_DTYPE_BF16, workspace, workspace_bytes, (cudaStream_t)stream,
+                  "debug_gemm_give_up", nullptr, 0, give_up);
 }
 
 extern "C" int qspec_gemm_split_factor(int w4a16, int M, int N, int K) {

@@ -1,0 +1,72 @@
+"""Bounded waits that are given up (at once, while what they wait for is on its way): the result shows it, it is counted, nothing is left behind
+and the next call is right. Each scenario runs in a process of its own, for the counts hold for the life of a process."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _product(mode, act, sA, w, sW, out, acc, give_up):
+    import torch
+    from qspec_b200 import _lib
+    lib = _lib.load()
+    M, N, K = act.shape[0], w.shape[0], 2 * w.shape[1]
+    need = max(lib.qspec_gemm_w4a4_workspace_bytes(M, N, K), lib.qspec_gemm_w4a16_workspace_bytes(M, N, K), lib.qspec_gemm_w4a8_workspace_bytes(M, N, K))
+    ws = _product.__dict__.setdefault("ws", torch.zeros(1 << 28, dtype=torch.uint8, device="cuda"))      # one for all calls: it has to stay clean
+    assert ws.numel() >= need
+    p = lambda t: None if t is None else t.data_ptr()  # noqa: E731
+    _lib.check(lib.qspec_debug_gemm_give_up(mode, p(act), p(sA), p(w), p(sW), None, p(out), p(acc), M, N, K, int(mode == 2), p(ws), ws.numel(), give_up,
+                                            torch.cuda.current_stream().cuda_stream), "qspec_debug_gemm_give_up")
+
+
+def _products(shapes, modes):
+    """Give the waits of a product up, then run it as ever: NaN or the lowest integer, and a count; then the exact sums."""
+    import torch
+    from qspec_b200 import ops
+    for M, N, K in shapes:
+        g = torch.Generator(device="cuda").manual_seed(M + N + K)
+        w = torch.randint(-128, 128, (N, K // 2), generator=g, dtype=torch.int8, device="cuda")
+        wide = torch.stack(((w << 4) >> 4, w >> 4), -1).reshape(N, K).double()
+        q = torch.randint(-8, 8, (M, K), generator=g, dtype=torch.int8, device="cuda")
+        packed = ((q[:, 0::2] & 15) | (q[:, 1::2] << 4)).contiguous()
+        sums = q.double() @ wide.T
+        for mode in modes:
+            dt = torch.bfloat16 if mode == 2 else torch.float16
+            one = torch.ones(max(M, N), dtype=dt, device="cuda")
+            act = {0: packed, 3: q}.get(mode, q.to(dt))
+            for raw in (False, True) if mode in (0, 3) else (False,):
+                out = None if raw else torch.zeros(M, N, dtype=dt, device="cuda")
+                acc = torch.zeros(M, N, dtype=torch.int32, device="cuda") if raw else None
+                before = ops.attn_tile_timeouts()
+                _product(mode, act, one, w, one, out, acc, 1)
+                assert ops.attn_tile_timeouts() > before, (mode, M, N, K, raw)
+                assert bool((acc == -2 ** 31).all() if raw else out.isnan().all()), (mode, M, N, K, raw)
+                before = ops.attn_tile_timeouts()
+                _product(mode, act, one, w, one, out, acc, 0)
+                got = acc if raw else out
+                assert torch.equal(got, sums.int() if raw else sums.float().to(dt)), (mode, M, N, K, raw)      # whole numbers below 2^24: exact in float32
+                assert ops.attn_tile_timeouts() == before
+
+
+def few_tokens():
+    os.environ["QSPEC_GEMM_ROWS"] = "2"
+    _products([(1, 8, 128), (9, 4736, 640), (17, 9504, 256), (32, 776, 2176), (4, 28672, 1024)], (0, 1, 2, 3))
+    _products([(48, 4800, 256), (64, 9504, 512)], (0,))
+
+
+SCENARIOS = [few_tokens]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scenario", [s.__name__ for s in SCENARIOS])
+def test_given_up_waits(scenario):
+    run = subprocess.run([sys.executable, os.path.abspath(__file__), scenario], cwd=ROOT, capture_output=True, text=True, timeout=600)
+    assert run.returncode == 0, run.stdout[-2000:] + run.stderr[-4000:]
+
+
+if __name__ == "__main__":
+    sys.path.insert(0, ROOT)
+    {s.__name__: s for s in SCENARIOS}[sys.argv[1]]()
