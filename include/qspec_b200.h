@@ -126,6 +126,9 @@ int qspec_hadamard_heads_c8(const void* x, void* out_f16, int8_t* out_q, void* s
                             int rows, int H, int D, float scale, float clip_ratio, void* stream);
 int qspec_hadamard_k28_c8(const void* x, const void* gate_up, void* out_f16, int8_t* out_q,
                           void* scale_out, int rows, int n, float scale, float clip_ratio, void* stream);
+/* For tests: the cluster form (n = 256, 512, 1024); the CTAs of every row's cluster in the mask give_up (bits 0 .. 6) give their waits up at once. */
+int qspec_debug_hadamard_k28_give_up(const void* x, void* out_f16, int8_t* out_q, void* scale_out, int rows, int n, float scale, unsigned give_up,
+                                     void* stream);
 int qspec_gemm_w4a8_split(const int8_t* a, const int8_t* w, void* partials, size_t partial_bytes, int M, int N, int K,
                           void* workspace, size_t workspace_bytes, void* stream);
 
@@ -299,8 +302,9 @@ int qspec_seq_attention(const void* qkv, const void* cache_k, const void* cache_
                         void* stream);
 
 /* CTAs of qspec_seq_attention, of the tensor-core prompt form inside it and qspec_decode_attention, and of the few-token form of the
- * qspec_gemm_* calls that gave up a bounded wait since the library was loaded on the current device (what such a CTA would have written is
- * NaN, raw integer sums the lowest integer): 0 unless something is broken; -1 if it cannot be read. Synchronises. No counterpart. */
+ * qspec_gemm_* calls, and rows of qspec_hadamard_k28 with n >= 256, that gave up a bounded wait since the library was loaded on the current
+ * device (what depends on it is NaN, quantised rows their scale, raw integer sums the lowest integer): 0 unless something is broken; -1 if it
+ * cannot be read. Synchronises. No counterpart. */
 int qspec_attn_tile_timeouts(void);
 
 /* The attention block between qkv_proj and o_proj as one launch for decode-sized passes: rotary embedding and

@@ -1036,8 +1036,8 @@ extern "C" int qspec_decode_attention(const void* qkv, const void* cache_k, cons
 extern "C" int qspec_attn_tile_timeouts(void) {
   unsigned n = 0;
   if (cudaMemcpyFromSymbol(&n, atile::attn_tile_timeouts, sizeof(n)) != cudaSuccess) return -1;
-  const int rows = qspec::gemm_rows_timeouts();
-  return rows < 0 ? -1 : (int)(n & 0x3fffffffu) + rows;
+  const int rows = qspec::gemm_rows_timeouts(), rotations = qspec::rotation_timeouts();
+  return rows < 0 || rotations < 0 ? -1 : (int)(n & 0x1fffffffu) + (rows & 0x1fffffff) + rotations;
 }
 
 extern "C" int qspec_seq_attention_supported(int T, int Hq, int Hkv, int D, int S) {

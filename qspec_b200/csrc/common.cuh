@@ -17,6 +17,7 @@ void set_error(const char* fmt, ...);            // stores thread-local text for
 void count_launch(int n = 1);                    // bumps qspec_launch_count()
 int  sm_count();
 int  gemm_rows_timeouts();                         // CTAs of the few-token GEMM that gave a wait up; -1: not readable
+int  rotation_timeouts();                          // rows of the cluster rotation with a wait given up; -1: not readable
 
 #define QSPEC_REQUIRE(cond, code, ...)                                                       \
   do {                                                                                       \

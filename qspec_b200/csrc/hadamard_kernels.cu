@@ -351,9 +351,13 @@ constexpr int K28_BPC = 4;                           // n-blocks (and mix output
 // receives them: stores of every thread into seven CTAs, with a release and acquire of the whole cluster after them, were the largest stall.
 // SiLU and quantiser, before -> now: n = 512, 1 row 5.7 -> 4.8 us, 64 rows 11.6 -> 9.2, 512 rows 44.5 -> 39.8; n = 1024, 64 rows 24.3 -> 17.7,
 // 512 rows 128 -> 98; n = 256, 64 rows 8.2 -> 7.3 (1 row 3.8 -> 3.9: a bulk copy of 2 KB takes a little longer than stores).
-// A wait that is given up (it is bounded) leaves NaN outputs and scales.
-__device__ __forceinline__ bool k28_wait(uint32_t bar) {
-  for (uint32_t spins = 0; spins < (1u << 20); ++spins) {
+// Every wait is bounded. A thread that gives one up tells the row's first CTA, which alone writes the row's scale: NaN then, after the cluster's last
+// barrier, whatever it was before; outputs of such a thread are NaN, its copies under way are waited for (up to the limit), and the row is counted
+// in k28_timeouts. `give_up`: the CTAs of a cluster, a bit each, that give their waits up at once (tests).
+constexpr uint32_t K28_SPINS = 1u << 20;
+static __device__ unsigned k28_timeouts;              // rows with a wait given up since the library was loaded
+__device__ __forceinline__ bool k28_wait(uint32_t bar, uint32_t limit) {
+  for (uint32_t spins = 0; spins < limit; ++spins) {
     uint32_t done;
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(done) : "r"(bar) : "memory");
     if (done) return true;
@@ -364,7 +368,7 @@ template <int SLOTS, int WPB>
 __global__ void __launch_bounds__(128 * WPB)
 hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict__ gate_up,
                             __half* __restrict__ out_f, uint8_t* __restrict__ out_q,
-                            __half* __restrict__ scale_out, int n, float scale, float clip, int c8) {
+                            __half* __restrict__ scale_out, int n, float scale, float clip, int c8, unsigned give_up) {
   constexpr int S1 = SLOTS / WPB, THR = 128 * WPB;   // vectors of 8 per lane, threads
   pdl_enter();
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -373,6 +377,7 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
   __shared__ __align__(8) uint64_t s_blocks, s_amax;  // the other CTAs' blocks / every CTA's maximum have landed
   __shared__ float red[8];
   __shared__ float amax_all[8];
+  __shared__ uint32_t s_bad;                          // in the first CTA: a wait of the cluster has been given up
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x % K28_CLUSTER;             // rank in cluster (cluster dims = (7,1,1))
   const size_t row = blockIdx.x / K28_CLUSTER;
@@ -380,7 +385,9 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
   const uint32_t sm_base = (uint32_t)__cvta_generic_to_shared(sm);
   const uint32_t bar_blocks = (uint32_t)__cvta_generic_to_shared(&s_blocks), bar_amax = (uint32_t)__cvta_generic_to_shared(&s_amax);
   const uint32_t own_bytes = (uint32_t)(K28_BPC * n * 2);
+  const uint32_t limit = give_up >> c & 1u ? 0u : K28_SPINS;
   if (threadIdx.x == 0) {
+    s_bad = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_blocks));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_amax));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -441,8 +448,26 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(mapa_shared(src, threadIdx.x)), "r"(src),
                  "r"(own_bytes), "r"(mapa_shared(bar_blocks, threadIdx.x)) : "memory");
   }
-  bool ok = k28_wait(bar_blocks);
-  if (out_q == nullptr) cluster_arrive_relaxed();     // (before the end: no CTA leaves while another may still copy from or into it)
+  bool ok = k28_wait(bar_blocks, limit);
+  // Before the end every CTA arrives once more: none leaves while another may still copy from or into it.
+  auto last_arrive = [&]() {
+    if (!ok) {                                        // (a fence and a relaxed arrival: the word is there when the first CTA's wait is over)
+      st_dsmem_u32(mapa_shared((uint32_t)__cvta_generic_to_shared(&s_bad), 0), 1u);
+      asm volatile("fence.acq_rel.cluster;\n" ::: "memory");
+      k28_wait(bar_blocks, K28_SPINS);
+      if (out_q) k28_wait(bar_amax, K28_SPINS);
+    }
+    __syncwarp();                                     // the arrival takes whole warps
+    cluster_arrive_relaxed();
+  };
+  auto last_wait = [&]() {
+    cluster_wait_acquire();
+    if (c == 0 && threadIdx.x == 0 && *(volatile uint32_t*)&s_bad) {
+      if (out_q) scale_out[row] = __float2half_rn(__uint_as_float(0x7fffffffu));
+      atomicAdd(&k28_timeouts, 1u);
+    }
+  };
+  if (out_q == nullptr) last_arrive();
 
   // ---- phase 2: outputs o0..o0+3, column pairs jp = tid, tid + THR, ...; all 28 blocks are local now
   const int o0 = K28_BPC * c;
@@ -495,7 +520,7 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
     }
   }
   if (out_q == nullptr) {                             // uniform over the cluster
-    cluster_wait_acquire();
+    last_wait();
     return;
   }
   // ---- quantiser: CTA amax to every CTA, row amax from local shared memory
@@ -503,8 +528,8 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
   if (threadIdx.x < K28_CLUSTER)
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(mapa_shared((uint32_t)__cvta_generic_to_shared(&amax_all[c]), threadIdx.x)),
                  "r"(__float_as_uint(amax)), "r"(mapa_shared(bar_amax, threadIdx.x)) : "memory");
-  ok = k28_wait(bar_amax) && ok;
-  cluster_arrive_relaxed();                           // (as above)
+  ok = k28_wait(bar_amax, limit) && ok;
+  last_arrive();
   float row_amax = 0.f;
 #pragma unroll
   for (int r = 0; r < K28_CLUSTER; ++r) row_amax = fmaxf(row_amax, amax_all[r]);
@@ -522,8 +547,8 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
       else out_q[qi] = (uint8_t)((q0 & 0xF) | ((q1 & 0xF) << 4));
     }
   }
-  if ((c == 0 || !ok) && threadIdx.x == 0) scale_out[row] = ok ? sh : __float2half_rn(nan);
-  cluster_wait_acquire();
+  if (c == 0 && threadIdx.x == 0) scale_out[row] = sh;
+  last_wait();
 }
 
 }  // namespace qspec
@@ -628,7 +653,7 @@ static int launch_k28(const void* x, const void* gu, void* of, int8_t* oq, void*
 constexpr int K28_TWO_WARP_ROWS = 112;
 template <int SLOTS, int WPB>
 static int launch_k28_cluster(const void* x, const void* gu, void* of, int8_t* oq, void* so, int rows, int n,
-                              float scale, float clip, cudaStream_t st, int c8) {
+                              float scale, float clip, cudaStream_t st, int c8, unsigned give_up) {
   auto kern = hadamard_k28_cluster_kernel<SLOTS, WPB>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)rows * K28_CLUSTER);
@@ -650,13 +675,13 @@ static int launch_k28_cluster(const void* x, const void* gu, void* of, int8_t* o
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   QSPEC_CUDA(cudaLaunchKernelEx(&cfg, kern, (const uint4*)x, (const uint4*)gu, (__half*)of, (uint8_t*)oq, (__half*)so, n,
-                                scale, clip, c8));
+                                scale, clip, c8, give_up));
   count_launch(1);
   return QSPEC_OK;
 }
 
 static int hadamard_k28_impl(const void* x, const void* gate_up, void* out_f16, int8_t* out_q, void* scale_out, int rows,
-                             int n, float scale, float clip_ratio, void* stream, int c8) {
+                             int n, float scale, float clip_ratio, void* stream, int c8, unsigned give_up = 0) {
   QSPEC_REQUIRE((x || gate_up) && (out_f16 || out_q), QSPEC_ERR_INVALID_ARG,
                 "hadamard_k28: null pointer");
   QSPEC_REQUIRE(!out_q || scale_out, QSPEC_ERR_INVALID_ARG, "hadamard_k28: out_q needs scale_out");
@@ -672,12 +697,12 @@ static int hadamard_k28_impl(const void* x, const void* gate_up, void* out_f16, 
   // neighbouring GEMMs' heads and tails. QSPEC_K28_CLUSTER_ROWS caps the row count that takes it (experiment knob).
   static const int cluster_rows = getenv("QSPEC_K28_CLUSTER_ROWS") ? atoi(getenv("QSPEC_K28_CLUSTER_ROWS")) : 65536;
   const bool few_rows = rows <= cluster_rows;
-  if (use_cluster && few_rows && n == 256) return launch_k28_cluster<1, 1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
+  if (use_cluster && few_rows && n == 256) return launch_k28_cluster<1, 1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8, give_up);
   if (use_cluster && few_rows && n == 512) {
-    if (rows <= K28_TWO_WARP_ROWS) return launch_k28_cluster<2, 2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
-    return launch_k28_cluster<2, 1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
+    if (rows <= K28_TWO_WARP_ROWS) return launch_k28_cluster<2, 2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8, give_up);
+    return launch_k28_cluster<2, 1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8, give_up);
   }
-  if (use_cluster && few_rows && n == 1024) return launch_k28_cluster<4, 2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
+  if (use_cluster && few_rows && n == 1024) return launch_k28_cluster<4, 2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8, give_up);
   switch (n) {
     case 1024: return launch_k28<4, 28, true>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
     case 512:  return launch_k28<2, 28, true>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8);
@@ -687,10 +712,20 @@ static int hadamard_k28_impl(const void* x, const void* gate_up, void* out_f16, 
   }
 }
 
+int qspec::rotation_timeouts() {
+  unsigned n = 0;
+  return cudaMemcpyFromSymbol(&n, k28_timeouts, sizeof(n)) == cudaSuccess ? (int)(n & 0x1fffffffu) : -1;
+}
+
 extern "C" int qspec_hadamard_k28(const void* x, const void* gate_up, void* out_f16,
                                   int8_t* out_q, void* scale_out, int rows, int n, float scale,
                                   float clip_ratio, void* stream) {
   return hadamard_k28_impl(x, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, stream, 0);
+}
+// For tests: the cluster form (n = 256, 512, 1024), the CTAs of a row's cluster in the mask `give_up` giving their waits up at once.
+extern "C" int qspec_debug_hadamard_k28_give_up(const void* x, void* out_f16, int8_t* out_q, void* scale_out, int rows, int n, float scale, unsigned give_up,
+                                                void* stream) {
+  return hadamard_k28_impl(x, nullptr, out_f16, out_q, scale_out, rows, n, scale, 1.0f, stream, 0, give_up);
 }
 // Same, with out_q written one int4 value per byte ([rows, 28 n] int8): the operand of qspec_gemm_w4a8*.
 extern "C" int qspec_hadamard_k28_c8(const void* x, const void* gate_up, void* out_f16, int8_t* out_q, void* scale_out,

@@ -188,7 +188,7 @@ class QSpecEngine:
         if peers is not None and peers.timeouts():
             raise RuntimeError(f"tensor-parallel peer time-out: {peers.timeouts()} arrival flag(s) never came")
         if given_up := ops.attn_tile_timeouts():
-            raise RuntimeError(f"{given_up} CTA(s) gave up a wait for the operands or products of attention or of a linear layer; the outputs of "
+            raise RuntimeError(f"{given_up} CTA(s) or rows gave up a wait in attention, a linear layer or the rotation before one; the outputs of "
                                "those steps hold NaN")
         acc, draft, emitted = [int(v) for v in self.counters.tolist()]
         steps = draft // (self.B * self.k) if draft else 0

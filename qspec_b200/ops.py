@@ -689,8 +689,9 @@ def decode_attention(qkv: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Te
 
 
 def attn_tile_timeouts() -> int:
-    """CTAs of seq_attention, of the prompt forms inside it, decode_attention and seq_window_attention_mma, and of the few-token products,
-    that gave up a bounded wait (their rows are NaN): 0 unless something is broken. Counts those of the current device, synchronises."""
+    """CTAs of seq_attention, of the prompt forms inside it, decode_attention and seq_window_attention_mma, and of the few-token products, and rows
+    of the 28 x n rotation, that gave up a bounded wait (what depends on it is NaN): 0 unless something is broken. Counts those of the current
+    device, synchronises."""
     counts = []
     if _lib._lib is not None:
         counts.append(_lib._lib.qspec_attn_tile_timeouts())

@@ -57,7 +57,42 @@ def few_tokens():
     _products([(48, 4800, 256), (64, 9504, 512)], (0,))
 
 
-SCENARIOS = [few_tokens]
+def rotation():
+    """Any CTAs of a row's cluster give up: the row's scale is NaN whichever they are, their outputs are NaN, and the row is counted once."""
+    import math
+
+    import torch
+    from qspec_b200 import _lib, ops
+    lib = _lib.load()
+    for n, rows in [(256, 1), (256, 40), (512, 3), (512, 113), (1024, 2)]:
+        x = torch.randn(rows, 28 * n, generator=torch.Generator(device="cuda").manual_seed(n + rows), device="cuda").half()
+        scale = 1.0 / math.sqrt(28 * n)
+        want_o, want_q, want_s = torch.empty_like(x), torch.empty(rows, 14 * n, dtype=torch.int8, device="cuda"), torch.empty(rows, dtype=torch.float16, device="cuda")
+        ops.hadamard_k28(x, n, scale, out=want_o, out_q=want_q, scale_out=want_s)
+        assert want_s.isfinite().all()
+
+        def call(give_up, plain):
+            o, q, s = torch.zeros_like(want_o), torch.zeros_like(want_q), torch.zeros_like(want_s)
+            before = ops.attn_tile_timeouts()
+            _lib.check(lib.qspec_debug_hadamard_k28_give_up(x.data_ptr(), o.data_ptr(), None if plain else q.data_ptr(), None if plain else s.data_ptr(), rows, n,
+                                                            scale, give_up, torch.cuda.current_stream().cuda_stream), "qspec_debug_hadamard_k28_give_up")
+            return o, q, s, ops.attn_tile_timeouts() - before
+        for give_up in (1, 2, 8, 64, 127):
+            for plain in (False, True):
+                o, q, s, counted = call(give_up, plain)
+                assert counted == rows
+                assert plain or s.isnan().all()
+                for c in range(7):
+                    part = slice(4 * c * n, 4 * (c + 1) * n)
+                    if give_up >> c & 1:
+                        assert o[:, part].isnan().all()
+                    else:
+                        assert torch.equal(o[:, part], want_o[:, part])
+        o, q, s, counted = call(0, False)
+        assert counted == 0 and torch.equal(o, want_o) and torch.equal(q, want_q) and torch.equal(s, want_s)
+
+
+SCENARIOS = [few_tokens, rotation]
 
 
 @pytest.mark.gpu
