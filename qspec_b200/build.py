@@ -7,6 +7,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -70,11 +71,20 @@ def build_seq_library(force: bool = False, verbose: bool = False) -> str:
     return SEQ_LIB_PATH
 
 
+def fast_path() -> str:
+    """Where the linear layers' native call path for this Python and this torch lies. It uses both by their inline headers, so a file built for
+    others must not be loaded: their versions are part of its name."""
+    import sysconfig
+    import torch
+    return os.path.join(OUT_DIR, f"_fast-torch{torch.__version__}-abi{int(torch.compiled_with_cxx11_abi())}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
 def build_fast(force: bool = False) -> str:
-    """_C/_fast.so: the linear layers' call path (csrc/fast_call.cpp), against the headers of the torch that is installed."""
-    src, path = os.path.join(CSRC, "fast_call.cpp"), os.path.join(OUT_DIR, "_fast.so")
+    """The linear layers' call path (csrc/fast_call.cpp), against the headers of the torch that is installed."""
+    src, path = os.path.join(CSRC, "fast_call.cpp"), fast_path()
     os.makedirs(OUT_DIR, exist_ok=True)
-    if not force and os.path.exists(path) and os.path.getmtime(path) >= os.path.getmtime(src):
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(HERE, "..", "include", "qspec_b200.h")))
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= newest:
         return path
     import sysconfig
     import torch
@@ -87,6 +97,14 @@ def build_fast(force: bool = False) -> str:
         raise RuntimeError(f"g++ failed for fast_call.cpp:\n{r.stderr}")
     os.replace(tmp, path)
     return path
+
+
+def build_fast_if_possible(force: bool = False) -> None:
+    """The libraries do without it (ops.py then goes through ctypes), so where it cannot be built (no g++, no Python or torch headers) they still are."""
+    try:
+        build_fast(force=force)
+    except Exception as e:
+        warnings.warn(f"csrc/fast_call.cpp is not built, linear layers are called through ctypes: {type(e).__name__}: {e}")
 
 
 def build_variant(suffix: str, defines, verbose: bool = False) -> str:
@@ -116,7 +134,8 @@ def build_library(force: bool = False, verbose: bool = False, prof: bool = False
     """prof=True builds libqspec_b200_prof.so with the GEMM cycle counters compiled in (scripts/gpu_gemm_trace.py;
     select it with QSPEC_LIB=<path>); watchdog=True builds libqspec_b200_wd.so whose pipeline waits trap instead of
     hanging (for protocol changes). The product library carries neither."""
-    build_fast(force=force)
+    os.makedirs(OUT_DIR, exist_ok=True)
+    build_fast_if_possible(force=force)
     lib_path = LIB_PATH.replace(".so", "_prof.so") if prof else LIB_PATH.replace(".so", "_wd.so") if watchdog else LIB_PATH
     if not force and os.path.exists(lib_path) and os.path.getmtime(lib_path) >= _newest_source_mtime(SOURCES):
         build_seq_library(force=False, verbose=verbose)

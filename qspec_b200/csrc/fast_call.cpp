@@ -7,11 +7,13 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include "../../include/qspec_b200.h"
+
 namespace {
 
-typedef int (*Int4Fn)(const int8_t*, const void*, const int8_t*, const void*, const void*, void*, int, int, int, int, void*, size_t, void*);
-typedef int (*Fp16Fn)(const void*, const int8_t*, const void*, const void*, void*, int, int, int, int, void*, size_t, void*);
-constexpr int OK = 0, ERR_WORKSPACE = 4;                      // QSPEC_OK, QSPEC_ERR_WORKSPACE (include/qspec_b200.h)
+typedef decltype(&qspec_gemm_w4a4) Int4Fn;                    // (of qspec_gemm_w4a8, too)
+typedef decltype(&qspec_gemm_w4a16) Fp16Fn;
+static_assert(std::is_same<Int4Fn, decltype(&qspec_gemm_w4a8)>::value, "one call for both");
 
 PyTypeObject* parameter_type = nullptr;
 
@@ -79,7 +81,7 @@ PyObject* linear_(PyObject* const* a, Py_ssize_t n) {
   status = kind == 1 ? ((Fp16Fn)fn)(xp, (const int8_t*)wp, wsp, b, op, (int)M, (int)N, (int)K, dtype, rp, bytes, stream)
                      : ((Int4Fn)fn)((const int8_t*)xp, sp, (const int8_t*)wp, wsp, b, op, (int)M, (int)N, (int)K, dtype, rp, bytes, stream);
   Py_END_ALLOW_THREADS
-  if (status == ERR_WORKSPACE) Py_RETURN_NONE;
+  if (status == QSPEC_ERR_WORKSPACE) Py_RETURN_NONE;
   return PyLong_FromLong(status);
 }
 

@@ -18,6 +18,7 @@ from __future__ import annotations
 from typing import Optional
 
 import ctypes
+import importlib.util
 import os
 
 import torch
@@ -63,12 +64,24 @@ def _ptr(t: Optional[torch.Tensor]):
 _I4 = (torch.int8, torch.uint8)
 
 # csrc/fast_call.cpp: the linear layers' calls without the Python below them. It takes what the functions here take without an error and
-# returns None for everything else, which then goes the ordinary way (and so does everything where it has not been built).
-try:
-    from ._C import _fast
-except ImportError:
-    _fast = None
+# returns None for everything else, which then goes the ordinary way (and so does everything where it has not been built for this Python and torch).
+_fast = False                                             # loaded by the first call: False before it, None where there is none
 _addresses: dict = {}
+
+
+def _load_fast():
+    global _fast
+    from .build import fast_path
+    try:
+        path = fast_path()
+        spec = importlib.util.spec_from_file_location("_fast", path) if os.path.exists(path) else None
+        module = None if spec is None else importlib.util.module_from_spec(spec)
+        if module is not None:
+            spec.loader.exec_module(module)
+    except ImportError:
+        module = None
+    _fast = module
+    return module
 
 
 def _address(name: str) -> int:
@@ -82,9 +95,10 @@ def _address(name: str) -> int:
 
 def _fast_linear(name: str, kind: int, x, x_scale, weight, weight_scale, bias, out, what: str) -> bool:
     """True: the call has been made."""
-    if _fast is None or out is None:
+    fast = _load_fast() if _fast is False else _fast
+    if fast is None or out is None:
         return False
-    status = _fast.linear(_address(name), kind, x, x_scale, weight, weight_scale, bias, out, _workspaces, "w4a16" if kind == 1 else "w4a4")
+    status = fast.linear(_address(name), kind, x, x_scale, weight, weight_scale, bias, out, _workspaces, "w4a16" if kind == 1 else "w4a4")
     if status is None:
         return False
     if status:
