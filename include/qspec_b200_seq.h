@@ -97,7 +97,7 @@ int qspec_moe_expert_tokens(const void* h, const void* gate_up, const void* down
                             int W, int F, int E, int top, float limit, int dtype, void* stream);
 
 /* Grouped form for many tokens (bfloat16): the (token, choice) pairs are sorted by expert and every expert's rows go
- * through 128 x 128 tcgen05 tiles with the accumulator in tensor memory. Workspace: bytes from the query, zero-filled
+ * through tcgen05 tiles of up to 256 of them and 256 channels with the accumulator in tensor memory. Workspace: bytes from the query, zero-filled
  * once by the caller; its layout is internal except for the first int32, a status word that a CTA sets to 1 when a
  * bounded wait of its pipeline runs out (that CTA stores nothing); no call clears it. */
 size_t qspec_moe_grouped_workspace_bytes(int ntok, int top, int E, int F);
@@ -121,6 +121,9 @@ int qspec_moe_expert_tokens_act(const void* h, const void* up, const void* down,
 int qspec_moe_expert_grouped_act(const void* h, const void* up, const void* down, const int* idx, void* out, int ntok, int W,
                                  int F, int E, int top, float limit, int act, void* workspace, size_t workspace_bytes,
                                  void* stream);
+/* For tests: the roles of the pipeline in the mask give_up (1 products, 2 epilogue) give their first wait up at once. */
+int qspec_debug_moe_grouped_give_up(const void* h, const void* up, const void* down, const int* idx, void* out, int ntok, int W, int F, int E, int top,
+                                    float limit, int act, void* workspace, size_t workspace_bytes, unsigned give_up, void* stream);
 
 /* ---- mixers whose state outlives a chunk: token shift, windowed softmax attention with a sink (latent or grouped-query
  * keys), gated linear recurrence. Ring caches: row = position % cap; the step's own rows are written before they are read,

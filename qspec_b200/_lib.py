@@ -139,6 +139,8 @@ SEQ_SIGNATURES = {
                                             c_float, c_int, c_int, c_void_p]),
     "qspec_moe_expert_grouped_act": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                              c_float, c_int, c_void_p, c_size_t, c_void_p]),
+    "qspec_debug_moe_grouped_give_up": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                                c_float, c_int, c_void_p, c_size_t, ctypes.c_uint, c_void_p]),
     "qspec_seq_token_shift": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "qspec_seq_add_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_ll, c_ll, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                    c_int, c_int, c_float, c_int, c_int, c_void_p]),

@@ -445,6 +445,7 @@ struct GroupPlan {
   int* ntiles;       // [1]
   int4* tile;        // [max tiles] expert, first sorted row, end of its rows, rows it is made for (multiple of 16)
   int* perm;         // [npairs] sorted row -> pair index
+  unsigned give_up;  // tests: roles that give their waits up at once (1 products, 2 epilogue)
 };
 
 // One CTA: counts, prefix sums over the experts, then every pair takes the next row of its expert. The pairs' experts are read once, and the
@@ -690,8 +691,9 @@ grouped_gemm_kernel(const bf16* __restrict__ A, const bf16* __restrict__ B, bf16
 // from request to arrival). 128 x 128 tiles, with a barrier of the whole CTA each k-step and an epilogue on its own, took 131 / 80 us (gated / down product; 8192
 // rows of 16 experts, 2048 x 1024), 128 x 256 tiles of one CTA 85 / 39; this form 80 / 38
 // with cold caches, the whole call 227 -> 130 in a row of calls (the pass over pairs without an expert, 10.5, is gone).
-// Every wait is bounded: a role whose barrier does not complete raises the plan's status word, the others follow; copies and products under
-// way are waited for (with the same limit), the tile is not stored, and the tensor memory is freed.
+// Every wait is bounded: a role whose barrier does not complete raises the plan's status word, the others follow, and the tile is not stored. The
+// threads that issue copies and products wait for the last of their own (with the same limit) whether or not anyone gave up, so that nothing is
+// under way when the tensor memory is freed and the CTAs leave; where nobody did they have nothing else to do by then.
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int TC_STAGES = 3, TC_BK = 128, TC_ATOMS = TC_BK / 64;           // k of a stage, in atoms of 64
 constexpr int TC_ROWS = 256;                                               // rows of a tile, at most
@@ -840,14 +842,16 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
     __nv_bfloat16* swap = reinterpret_cast<__nv_bfloat16*>(tc_smem_raw + (base - tc_smem_u32(tc_smem_raw)) + (size_t)TC_STAGES * TC_STAGE + (size_t)group * TC_SWAP);
     auto meet = [&]() { asm volatile("bar.sync %0, 128;\n" ::"r"(1 + group) : "memory"); };
     int i = 0;
+    if (p.give_up & 2) s_fail = 1;
     Tile next = tile_at(pair);
-    for (int it = pair; it < count; it += pairs, ++i) {
+    for (int it = pair; it < count && !(p.give_up & 2); it += pairs, ++i) {
       const Tile t = next;
       next = tile_at(it + pairs);
       const int d = i & 1, rows = t.mend - t.m0, ch0 = t.n0 + rank * CH;
       // the four warps go on or leave together: they meet below
       const uint32_t given_up = tc_mbar_wait(tc_smem_u32(&s_done[d]), (uint32_t)(i >> 1) & 1, &s_fail) ? 0 : 1;
       uint32_t leave;
+      __syncwarp();                                      // (bar.red takes whole warps)
       asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, %2, 128, q;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(leave) : "r"(given_up),
                    "r"(1 + group) : "memory");
       if (leave) break;
@@ -1018,7 +1022,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
           if (++s == TC_STAGES) { s = 0; parity ^= 1u; }
         }
       }
-      if (!ok && rank == 0) {                            // the newest copies of the ring, of both CTAs (which leave together)
+      if (rank == 0) {                                   // the newest copies of the ring, of both CTAs (which leave together)
         for (int j = max(0, issued - TC_STAGES); j < issued; ++j) tc_drain(tc_smem_u32(&s_full[j % TC_STAGES]), (uint32_t)(j / TC_STAGES) & 1);
       }
     }
@@ -1028,7 +1032,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
       int s = 0, i = 0;
       uint32_t parity = 0;
       Tile next = tile_at(pair);
-      bool ok = true;
+      bool ok = !(p.give_up & 1);
+      if (!ok) s_fail = 1;
       for (int it = pair; it < count && ok; it += pairs, ++i) {
         const int d = i & 1;
         const uint32_t idesc = tc_idesc(next.rows);
@@ -1048,10 +1053,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_c
           if (++s == TC_STAGES) { s = 0; parity ^= 1u; }
         }
       }
-      if (!ok) {
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(tc_smem_u32(&s_last)) : "memory");
-        tc_drain(tc_smem_u32(&s_last), 0);
-      }
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(tc_smem_u32(&s_last)) : "memory");
+      tc_drain(tc_smem_u32(&s_last), 0);
     }
     __syncwarp();
   }
@@ -1158,9 +1161,8 @@ extern "C" size_t qspec_moe_grouped_workspace_bytes(int ntok, int top, int E, in
   return grouped_layout(ntok > 0 ? ntok : 0, top, E, F, off);
 }
 
-extern "C" int qspec_moe_expert_grouped_act(const void* h, const void* gate_up, const void* down, const int* idx, void* out, int ntok,
-                                            int W, int F, int E, int top, float limit, int act, void* workspace,
-                                            size_t workspace_bytes, void* stream) {
+static int moe_grouped(const void* h, const void* gate_up, const void* down, const int* idx, void* out, int ntok, int W, int F, int E, int top, float limit,
+                       int act, void* workspace, size_t workspace_bytes, void* stream, unsigned give_up) {
   QSPEC_REQUIRE(act == QSPEC_EXPERT_ACT_GATED || act == QSPEC_EXPERT_ACT_RELU2 || act == QSPEC_EXPERT_ACT_SILU, QSPEC_ERR_INVALID_ARG,
                 "moe_expert_grouped: unknown activation %d", act);
   QSPEC_REQUIRE(h && idx && out && workspace && (E == 0 || (gate_up && down)), QSPEC_ERR_INVALID_ARG, "moe_expert_grouped: null pointer");
@@ -1177,6 +1179,7 @@ extern "C" int qspec_moe_expert_grouped_act(const void* h, const void* gate_up, 
   GroupPlan p;
   p.offsets = (int*)(ws + off[0]); p.status = (int*)(ws + off[1]); p.ntiles = (int*)(ws + off[2]);
   p.tile = (int4*)(ws + off[3]); p.perm = (int*)(ws + off[5]);
+  p.give_up = give_up;
   bf16* Y = (bf16*)(ws + off[6]);
   const int npairs = ntok * top;
   const int max_tiles = npairs / 128 + E + 1;
@@ -1223,6 +1226,18 @@ extern "C" int qspec_moe_expert_grouped_act(const void* h, const void* gate_up, 
              p, F, W, top, limit);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
+}
+
+extern "C" int qspec_moe_expert_grouped_act(const void* h, const void* gate_up, const void* down, const int* idx, void* out, int ntok,
+                                            int W, int F, int E, int top, float limit, int act, void* workspace,
+                                            size_t workspace_bytes, void* stream) {
+  return moe_grouped(h, gate_up, down, idx, out, ntok, W, F, E, top, limit, act, workspace, workspace_bytes, stream, 0);
+}
+
+// For tests: the roles in the mask `give_up` (1 products, 2 epilogue) of the tcgen05 form give their first wait up at once.
+extern "C" int qspec_debug_moe_grouped_give_up(const void* h, const void* gate_up, const void* down, const int* idx, void* out, int ntok, int W, int F, int E,
+                                               int top, float limit, int act, void* workspace, size_t workspace_bytes, unsigned give_up, void* stream) {
+  return moe_grouped(h, gate_up, down, idx, out, ntok, W, F, E, top, limit, act, workspace, workspace_bytes, stream, give_up);
 }
 
 extern "C" int qspec_moe_expert_grouped(const void* h, const void* gate_up, const void* down, const int* idx, void* out, int ntok,

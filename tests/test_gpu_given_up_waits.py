@@ -92,7 +92,34 @@ def rotation():
         assert counted == 0 and torch.equal(o, want_o) and torch.equal(q, want_q) and torch.equal(s, want_s)
 
 
-SCENARIOS = [few_tokens, rotation]
+def experts():
+    """Products that stop while every copy of a short k range has been issued, and an epilogue that leaves the products to themselves: the status
+    word says so, and after it has been cleared the next call is right."""
+    import torch
+    from qspec_b200 import _lib, ops
+    lib = _lib.load_seq()
+    for T, top, E, W, F in [(5, 1, 1, 128, 128), (40, 2, 3, 256, 264), (700, 4, 8, 1024, 512), (3000, 2, 4, 384, 256)]:
+        g = torch.Generator(device="cuda").manual_seed(T + W)
+        h = torch.randn(T, W, generator=g, device="cuda").bfloat16()
+        gate_up = (torch.randn(E, 2 * F, W, generator=g, device="cuda") * W ** -0.5).bfloat16()
+        down = (torch.randn(E, W, F, generator=g, device="cuda") * F ** -0.5).bfloat16()
+        idx = torch.randint(-1, E, (T, top), generator=g, device="cuda").int()
+        want = torch.empty(T, top, W, dtype=torch.bfloat16, device="cuda")
+        ops.moe_expert_grouped(h, gate_up, down, idx, want, E, F, 7.0, act="silu")
+        assert ops.moe_grouped_status() == 0
+        ws = torch.zeros(lib.qspec_moe_grouped_workspace_bytes(T, top, E, F), dtype=torch.uint8, device="cuda")
+        out = torch.empty_like(want)
+        for give_up in (1, 2, 3, 0):
+            ws[:4].zero_()
+            _lib.check(lib.qspec_debug_moe_grouped_give_up(h.data_ptr(), gate_up.data_ptr(), down.data_ptr(), idx.data_ptr(), out.data_ptr(), T, W, F, E, top, 7.0,
+                                                           ops.EXPERT_ACTS["silu"], ws.data_ptr(), ws.numel(), give_up, torch.cuda.current_stream().cuda_stream),
+                       "qspec_debug_moe_grouped_give_up")
+            assert int(ws[:4].view(torch.int32).item()) == (give_up != 0)
+            ops.moe_expert_grouped(h, gate_up, down, idx, out, E, F, 7.0, act="silu")
+            assert torch.equal(out, want) and ops.moe_grouped_status() == 0
+
+
+SCENARIOS = [few_tokens, rotation, experts]
 
 
 @pytest.mark.gpu
