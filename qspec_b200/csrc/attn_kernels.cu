@@ -510,10 +510,11 @@ static int launch_attn_block(const void* qkv, const void* cos_sin, const int* po
   QSPEC_REQUIRE(stage_bytes >= 0, QSPEC_ERR_UNSUPPORTED, "attn_block: T=%d tokens x cache length %d does not fit in shared memory", T, S);
   const size_t dyn = attn_block_fixed_smem(G, T, S) + (size_t)stage_bytes;
   const int kcap = (int)stage_bytes;
-  static bool attr_set = false;                        // per instantiation
-  if (!attr_set) {
-    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_block_smem_budget()));
-    attr_set = true;
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(kern, attn_block_smem_budget()));
+  static bool told = false;
+  if (!told) {
+    told = true;
     if (getenv("QSPEC_ATTN_DEBUG")) {
       cudaLaunchConfig_t c2 = {};
       c2.gridDim = dim3((unsigned)T * HKV); c2.blockDim = dim3(128); c2.dynamicSmemBytes = dyn;
@@ -880,13 +881,8 @@ static int launch_seq_attention_st(const void* qkv, const void* ck, const void* 
   constexpr size_t dyn = (size_t)NW * ST * SEQ_BLOCK;
   static_assert(SEQ_BLOCK >= 16 * (128 + 4) * (int)sizeof(float), "the partial outputs lie in the blocks");
   auto kern = seq_attention_kernel<G, ST, NW>;
-  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
-  int dev = 0;
-  QSPEC_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
-    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(kern, dyn));
   // T <= SEQ_CHUNKS: sequences with a token and whole chunks bound the number of chunks
   const int units = T <= SEQ_CHUNKS ? min(T, min(B, T) + T / (16 / G)) : B;
   launch_pdl(kern, dim3(units * Hkv), dim3(NW * 32), dyn, st, (const __half*)qkv, (const __half*)ck, (const __half*)cv,

@@ -809,13 +809,8 @@ inline int cache_map(CUtensorMap* map, const void* p, long long ss, int rs, int 
 template <bool BF, bool QF32>
 inline int launch(const Args& a, int kv_heads, cudaStream_t stream) {
   auto kern = attn_tile_kernel<BF, QF32>;
-  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
-  int dev = 0;
-  QSPEC_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
-    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
-    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(kern, SMEM));
   CUtensorMap mk, mv;
   const int nseq = a.nseq < (1 << 20) ? a.nseq : 1 << 20;     // (a caller that does not know their number: nothing is cut off)
   int rc = cache_map<BF>(&mk, a.k, a.k_ss, a.k_rs, a.k_hs, kv_heads, a.cap, nseq);

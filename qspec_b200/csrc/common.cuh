@@ -9,6 +9,7 @@
 #include <atomic>
 
 #include "../../include/qspec_b200.h"
+#include "smem_limit.h"
 
 namespace qspec {
 

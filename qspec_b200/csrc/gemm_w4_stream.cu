@@ -1358,11 +1358,8 @@ static size_t workspace_bytes(int mode, int M, int N, int K) { return M <= 0 || 
 template <int MODE, bool PAIR, bool LONG>
 static int launch(const CUtensorMap& mw, const CUtensorMap& ma, const Params& p, const Plan& pl, cudaStream_t st) {
   auto kern = w4_stream_kernel<MODE, PAIR, LONG>;
-  static bool configured = false;
-  if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST));
-    configured = true;
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(kern, SMEM_MOST));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(PAIR ? 2 * pl.G : pl.G);
   cfg.blockDim = dim3(THREADS);
@@ -1416,13 +1413,8 @@ static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, RowsArgs p,
   const int grid = p.tiles < sms * CTAS ? p.tiles : sms * CTAS;
   const int most = (p.tiles + grid - 1) / grid * ((p.items + NW - 1) / NW);      // items of a warp
   p.depth = most < DEPTH ? most : DEPTH;
-  static std::atomic<uint64_t> raised{0};                   // devices on which the kernel's shared-memory limit has been raised
-  int dev = 0;
-  QSPEC_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !(raised.load(std::memory_order_relaxed) >> dev & 1)) {
-    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BUDGET));
-    if (dev < 64) raised.fetch_or(1ull << dev);
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(kern, BUDGET));
   QSPEC_CUDA(launch_pdl(kern, dim3(grid), dim3(NW * 32), FIXED + (size_t)p.depth * NW * Sh::SLOT, st, mw, ma, p));
   count_launch(1);
   return QSPEC_OK;

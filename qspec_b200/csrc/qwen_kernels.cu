@@ -250,11 +250,8 @@ extern "C" int qspec_hadamard_k108(const void* x, const void* gate_up, int gate_
   QSPEC_REQUIRE(n == QN, QSPEC_ERR_UNSUPPORTED, "hadamard_k108: n=%d, only 108 x 128 (intermediate size 13824) is built", n);
   if (rows == 0) return QSPEC_OK;
   constexpr size_t K108_SMEM = (size_t)QK * QN * sizeof(__half) + (size_t)QK * 4 * 7 * sizeof(float4);   // 27 KB + 47 KB
-  static bool attr_set = false;
-  if (!attr_set) {
-    QSPEC_CUDA(cudaFuncSetAttribute(hadamard_k108_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K108_SMEM));
-    attr_set = true;
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(hadamard_k108_kernel, K108_SMEM));
   launch_pdl(hadamard_k108_kernel, dim3(rows), dim3(256), K108_SMEM, (cudaStream_t)stream, (const uint4*)(gate_up ? nullptr : x),
              (const uint4*)gate_up, gate_first, (__half*)out_f16, (uint8_t*)out_q, (__half*)scale_out, scale, clip_ratio);
   QSPEC_CHECK_LAUNCH(1);

@@ -846,11 +846,8 @@ extern "C" int qspec_seq_softcap_f32(float* a, long long n, float cap, void* str
 template <typename T, int VEC, int NCV>
 static int launch_head_prep(const qspec_head_prep_args& a, cudaStream_t st) {
   const size_t smem = a.rot_dims ? (size_t)8 * (a.D + a.rot_dims) * sizeof(float) : 0;
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(head_prep_kernel<T, VEC, NCV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(head_prep_kernel<T, VEC, NCV>, smem));
   // heads of a token go round grid y: enough CTAs to fill the GPU, few enough that a token's angles serve several heads
   const int nh = a.H + a.G + (a.v_off >= 0 ? a.G : 0), rows = (a.ntok + 7) / 8;
   int gy = (148 * 16 + rows - 1) / rows;
@@ -927,11 +924,8 @@ template <typename T, int KT>
 static int launch_delta_block(const qspec_delta_channel_args& a, const int* block_rows, int nblocks, float* blocks, cudaStream_t st) {
   const int DP = delta_padded(a.D), VS = (a.DV + 15) / 16 * 16;
   const size_t smem = ((size_t)3 * DBLK * (DP + 4) + (size_t)DBLK * VS + 4 * 256 + 16) * sizeof(float);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(delta_channel_block_kernel<T, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(delta_channel_block_kernel<T, KT>, smem));
   launch_pdl(delta_channel_block_kernel<T, KT>, dim3(nblocks, a.H), dim3(256), smem, st, a, block_rows, blocks, DP);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
@@ -941,11 +935,8 @@ template <int NHR>
 static int launch_delta_scan_blocks(const qspec_delta_channel_args& a, const int* long_starts, const int* long_block0, int nlong,
                                     const float* blocks, float* o, cudaStream_t st) {
   constexpr size_t smem = (size_t)2 * (49 * 64 * NHR + 512) * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(delta_channel_scan_kernel<NHR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(delta_channel_scan_kernel<NHR>, smem));
   launch_pdl(delta_channel_scan_kernel<NHR>, dim3(nlong, a.H, (a.DV + 15) / 16), dim3(256), smem, st, a, long_starts, long_block0, blocks, o);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;

@@ -832,11 +832,8 @@ static int launch_norm_conv(const float* x_in, float* x_out, const void* y, int 
                             float eps, cudaStream_t st) {
   const size_t smem = (size_t)taps * W * sizeof(float);
   QSPEC_REQUIRE(smem <= 200 * 1024, QSPEC_ERR_UNSUPPORTED, "seq_norm_conv: %d taps x width %d exceed shared memory", taps, W);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA((cudaFuncSetAttribute(norm_conv_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(norm_conv_kernel<T, VEC>, smem));
   // tokens per CTA: one while the batch is small (latency), a run of four once there are CTAs to spare
   const int run = ntok >= 1024 ? 4 : 1;
   launch_pdl(norm_conv_kernel<T, VEC>, dim3((ntok + run - 1) / run), dim3(256), smem, st, x_in, x_out, (const T*)y, y_parts,
@@ -968,12 +965,8 @@ extern "C" int qspec_seq_chunk_attention(const void* qkv, int ld, const void* ca
     const size_t smem = (size_t)(rep * D + rep * ATT_KB) * sizeof(float) + (size_t)ATT_KB * (kst + DV / wpe) * 4 +
                         (nsplit > 1 ? (size_t)rep * (DV / wpe) * 2 * sizeof(float) : 0);
     QSPEC_REQUIRE(smem <= 200 * 1024, QSPEC_ERR_UNSUPPORTED, "seq_chunk_attention: %d query heads of size %d per key/value head do not fit shared memory", rep, D);
-    static size_t configured[2] = {0, 0};
-    if (smem > 48 * 1024 && smem > configured[w]) {
-      if (w == 0) QSPEC_CUDA(cudaFuncSetAttribute(chunk_attn_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      else QSPEC_CUDA(cudaFuncSetAttribute(chunk_attn_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      configured[w] = smem;
-    }
+    static SmemLimit limit[2];
+    if (smem > 48 * 1024) QSPEC_CUDA(w == 0 ? limit[0].raise(chunk_attn_kernel<float>, smem) : limit[1].raise(chunk_attn_kernel<__nv_bfloat16>, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ntok, G, nsplit);
     cfg.blockDim = dim3(128);
@@ -1007,12 +1000,8 @@ extern "C" int qspec_seq_chunk_attention(const void* qkv, int ld, const void* ca
   }
   const size_t smem = (size_t)(D + size) * sizeof(float);
   QSPEC_REQUIRE(smem <= 200 * 1024, QSPEC_ERR_UNSUPPORTED, "seq_chunk_attention: chunk of %d keys does not fit shared memory", size);
-  static size_t configured_plain[2] = {0, 0};
-  if (smem > 48 * 1024 && smem > configured_plain[w]) {
-    if (w == 0) QSPEC_CUDA(cudaFuncSetAttribute(chunk_attn_plain_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else QSPEC_CUDA(cudaFuncSetAttribute(chunk_attn_plain_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured_plain[w] = smem;
-  }
+  static SmemLimit limit[2];
+  if (smem > 48 * 1024) QSPEC_CUDA(w == 0 ? limit[0].raise(chunk_attn_plain_kernel<float>, smem) : limit[1].raise(chunk_attn_plain_kernel<__nv_bfloat16>, smem));
   if (w == 0)
     launch_pdl(chunk_attn_plain_kernel<float>, dim3(ntok, H), dim3(128), smem, st, (const float*)qkv, ld, (const float*)cache_k,
                (const float*)cache_v, bias, (float*)out, meta, ntok, H, G, D, DV, size, scale, softcap);
@@ -1111,13 +1100,9 @@ extern "C" int qspec_moe_expert_tokens_act(const void* h, const void* gate_up, c
   if (ntok == 0) return QSPEC_OK;
   const size_t smem = (size_t)(W + F) * sizeof(float);
   QSPEC_REQUIRE(smem <= 200 * 1024, QSPEC_ERR_UNSUPPORTED, "moe_expert_tokens: width %d + expert size %d exceed shared memory", W, F);
-  static size_t configured[2] = {0, 0};
+  static SmemLimit room[2];
   const int w = dtype == QSPEC_DTYPE_F32 ? 0 : 1;
-  if (smem > 48 * 1024 && smem > configured[w]) {
-    if (w == 0) QSPEC_CUDA(cudaFuncSetAttribute(expert_tokens_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else QSPEC_CUDA(cudaFuncSetAttribute(expert_tokens_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured[w] = smem;
-  }
+  if (smem > 48 * 1024) QSPEC_CUDA(w == 0 ? room[0].raise(expert_tokens_kernel<float>, smem) : room[1].raise(expert_tokens_kernel<__nv_bfloat16>, smem));
   if (w == 0)
     launch_pdl(expert_tokens_kernel<float>, dim3(ntok, top), dim3(256), smem, (cudaStream_t)stream, (const float*)h,
                (const float*)gate_up, (const float*)down, idx, (float*)out, W, F, E, top, limit, act);

@@ -881,11 +881,8 @@ static int launch_add_norm(const float* x_in, float* x_out, const void* y, int y
                            const float* y_w, const float* w, const float* b, int kind, void* out, int ntok, int W, float eps,
                            cudaStream_t st) {
   const size_t smem = (size_t)W * sizeof(float);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(add_norm_kernel<T, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(add_norm_kernel<T, YT>, smem));
   launch_pdl(add_norm_kernel<T, YT>, dim3(ntok), dim3(256), smem, st, x_in, x_out, (const YT*)y, y_parts, y_part_stride, y_tok_stride,
              y_w, w, b, kind, (T*)out, W, eps);
   QSPEC_CHECK_LAUNCH(1);
@@ -984,11 +981,8 @@ template <typename T, int NACC, int VEC>
 static int launch_window_attn(const qspec_window_attn_args* a, cudaStream_t st) {
   const int DK = a->DA + a->DB;
   const size_t smem = ((size_t)((DK + 3) & ~3) + (size_t)4 * a->DV) * sizeof(float);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(window_attn_kernel<T, NACC, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(window_attn_kernel<T, NACC, VEC>, smem));
   launch_pdl(window_attn_kernel<T, NACC, VEC>, dim3(a->ntok, a->H), dim3(128), smem, st, a->qa, a->qa_tok_stride, a->qa_head_stride, a->DA,
              a->qb, a->qb_tok_stride, a->qb_head_stride, a->DB, (const T*)a->k, a->k_slot_stride, a->k_row_stride, a->k_head_stride,
              (const T*)a->v, a->v_slot_stride, a->v_row_stride, a->v_head_stride, a->DV, a->sink, (const T*)a->gate, a->gate_ld, a->gate_per_head, (T*)a->out,
@@ -1055,13 +1049,8 @@ static int launch_recurrence_chunks_d(const T* p, int ld, const float* gates, fl
   float* P = ws + (size_t)chunks * H * D * DV;
   const dim3 grid(chunks, H), block((D / 16) * (DV / 4));
   constexpr size_t smem_e = (size_t)RC_BT * (4 * D + 4 * DV) * sizeof(float), smem_o = smem_e + (size_t)RC_BT * (2 * D + (D / 16) * DV) * sizeof(float);
-  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
-  int dev = 0;
-  QSPEC_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
-    QSPEC_CUDA(cudaFuncSetAttribute(recurrence_chunk_kernel<T, D, DV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o));
-    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(recurrence_chunk_kernel<T, D, DV, true>, smem_o));
   launch_pdl(recurrence_chunk_kernel<T, D, DV, false>, grid, block, smem_e, st, p, ld, gates, E, P, state, o, out, norm_w, eps, meta, seg_starts, nseg, ntok, H, C, decay);
   QSPEC_CHECK_LAUNCH(1);
   launch_pdl(recurrence_carry_kernel, dim3(nseg, H, (D * DV + 1023) / 1024), dim3(256), 0, st, E, (const float*)P, (const float*)state, meta, seg_starts, nseg,
@@ -1176,11 +1165,8 @@ static int launch_residual_norm_v(const float* x_in, float* x_out, const void* y
                                   const float* y_w, const void* y2, const float* y2_w, int y2_w_stride, float mult, const float* w,
                                   float w_offset, void* out, int ntok, int W, float eps, const float* y_scale, cudaStream_t st) {
   const size_t smem = (size_t)W * sizeof(float);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(residual_norm_kernel<T, YT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(residual_norm_kernel<T, YT, VEC>, smem));
   launch_pdl(residual_norm_kernel<T, YT, VEC>, dim3(ntok), dim3(256), smem, st, x_in, x_out, (const YT*)y, y_parts, y_part_stride,
              y_tok_stride, y_w, (const YT*)y2, y2_w, y2_w_stride, mult, w, w_offset, (T*)out, W, eps, y_scale);
   QSPEC_CHECK_LAUNCH(1);

@@ -208,11 +208,8 @@ template <int D, int DV>
 static int launch_attn_mma(const void* qkv, int ld, const void* ck, const void* cv, const float* bias, void* out, const int* meta,
                            int ntok, int H, int G, int size, float scale, float softcap, cudaStream_t st) {
   constexpr size_t smem = (size_t)(2 * 64 * (D + 8) + DV * 72) * sizeof(bf16) + 5 * 64 * sizeof(int);
-  static bool configured = false;
-  if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(chunk_attn_mma_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(chunk_attn_mma_kernel<D, DV>, smem));
   launch_pdl(chunk_attn_mma_kernel<D, DV>, dim3((ntok + 63) / 64, H), dim3(128), smem, st, (const bf16*)qkv, ld, (const bf16*)ck,
              (const bf16*)cv, bias, (bf16*)out, meta, ntok, H, G, size, scale, softcap);
   QSPEC_CHECK_LAUNCH(1);
@@ -385,11 +382,8 @@ static int launch_attn_token_mma(const void* qkv, int ld, const void* ck, const 
   int nsplit = 1;
   while (nsplit < 8 && 4 * nsplit < blocks && (long long)ntok * G * nsplit * 2 <= 296) nsplit *= 2;
   const size_t smem = (size_t)16 * (D / 2 + 4) * 4 + (size_t)(4 + (nsplit > 1 ? 1 : 0)) * rep * DV * sizeof(float);
-  static size_t configured = 0;                          // per instantiation
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(chunk_attn_token_mma_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(chunk_attn_token_mma_kernel<D, DV>, smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ntok, G, nsplit);
   cfg.blockDim = dim3(128);
@@ -1087,13 +1081,8 @@ template <int MODE>
 static int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mb, const bf16* A, bf16* C, const GroupPlan& p, int tiles, int K, int N, int top, int npairs,
                           int E, float limit, const int* idx, bf16* whole, cudaStream_t st) {
   auto kern = grouped_gemm_tc_kernel<MODE>;
-  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
-  int dev = 0;
-  QSPEC_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
-    QSPEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM));
-    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
-  }
+  static SmemLimit room;
+  QSPEC_CUDA(room.raise(kern, TC_SMEM));
   constexpr int BN = MODE & 1 ? 128 : 256;
   const long long most = (long long)tiles * ((N + BN - 1) / BN);
   const int pairs = (sm_count() > 0 ? sm_count() : 148) / 2;
@@ -1190,13 +1179,8 @@ static int moe_grouped(const void* h, const void* gate_up, const void* down, con
     QSPEC_CHECK_LAUNCH(1);
   }
   if (E == 0) return QSPEC_OK;
-  static std::atomic<unsigned long long> ready{0};            // devices whose limit is raised
-  int dev = 0;
-  QSPEC_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64 || !(ready.load(std::memory_order_relaxed) >> dev & 1ull)) {
-    QSPEC_CUDA(cudaFuncSetAttribute(moe_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)moe_group_smem(MOE_KEEP * 1024, 8192)));
-    if (dev < 64) ready.fetch_or(1ull << dev, std::memory_order_relaxed);
-  }
+  static SmemLimit room;
+  QSPEC_CUDA(room.raise(moe_group_kernel, moe_group_smem(MOE_KEEP * 1024, 8192)));
   launch_pdl(moe_group_kernel, dim3(1), dim3(1024), moe_group_smem(npairs, E), st, idx, npairs, E, warp_level ? GG_BM : 0, moe_group_kept(npairs) ? 1 : 0, p);
   QSPEC_CHECK_LAUNCH(1);
   QSPEC_REQUIRE(!warp_level || act == QSPEC_EXPERT_ACT_GATED, QSPEC_ERR_UNSUPPORTED,
@@ -1213,12 +1197,9 @@ static int moe_grouped(const void* h, const void* gate_up, const void* down, con
     if (rc != QSPEC_OK) return rc;
     return launch_grouped<0>(my, md, nullptr, (bf16*)out, p, max_tiles, F, W, top, npairs, E, limit, idx, nullptr, st);
   }
-  static bool configured = false;
-  if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(grouped_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM));
-    QSPEC_CUDA(cudaFuncSetAttribute(grouped_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GG_SMEM));
-    configured = true;
-  }
+  static SmemLimit gated, down_product;
+  QSPEC_CUDA(gated.raise(grouped_gemm_kernel<true>, GG_SMEM));
+  QSPEC_CUDA(down_product.raise(grouped_gemm_kernel<false>, GG_SMEM));
   launch_pdl(grouped_gemm_kernel<true>, dim3(max_tiles, (F + 63) / 64), dim3(256), GG_SMEM, st, (const bf16*)h, (const bf16*)gate_up, Y, p, W,
              F, top, limit);
   QSPEC_CHECK_LAUNCH(1);
@@ -1731,11 +1712,8 @@ static int launch_latent_absorbed(const WinMma& a, cudaStream_t st) {
   int nsplit = 1;
   while (nsplit < 4 && (long long)a.ntok * a.G * nsplit * 2 <= 148 && a.window >= 128 * nsplit * 2) nsplit *= 2;
   const size_t smem = (size_t)16 * ((DA + 64) / 2 + 4) * 4 + (size_t)2 * 16 * 36 * 4 + (nsplit > 1 ? (size_t)(32 + 16 * DA) * 4 : 0);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(latent_absorbed_mma_kernel<DA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(latent_absorbed_mma_kernel<DA>, smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.ntok, a.G, nsplit);
   cfg.blockDim = dim3(256);
@@ -1969,11 +1947,8 @@ template <int DA, int DB, int DV, int NW>
 static int launch_prompt_attn_w(const WinMma& a, int slot, int pos0, cudaStream_t st) {
   constexpr int BM = 16 * NW;
   constexpr size_t smem = ((size_t)(BM + 2 * 64) * (DA + DB + 8) + (size_t)2 * 64 * (DV + 8)) * sizeof(bf16);
-  static bool configured = false;
-  if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(prompt_attn_mma_kernel<DA, DB, DV, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(prompt_attn_mma_kernel<DA, DB, DV, NW>, smem));
   launch_pdl(prompt_attn_mma_kernel<DA, DB, DV, NW>, dim3((a.ntok + BM - 1) / BM, a.H), dim3(32 * NW), smem, st, a, slot, pos0);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
@@ -2020,11 +1995,8 @@ int prompt_attention_mma(const qspec_window_attn_args* p, const void* kB, long l
 template <int DA, int DB, int DV, bool STREAM>
 static int launch_window_mma(const WinMma& a, int slices, cudaStream_t st) {
   constexpr size_t smem = (size_t)16 * ((DA + DB) / 2 + 4) * 4 + (size_t)4 * 16 * DV * sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(window_attn_mma_kernel<DA, DB, DV, STREAM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
-  }
+  static SmemLimit limit;
+  QSPEC_CUDA(limit.raise(window_attn_mma_kernel<DA, DB, DV, STREAM>, smem));
   const dim3 grid = a.token_rows ? dim3((a.ntok + 15) / 16, a.H, slices) : dim3(a.ntok, a.G, slices);
   launch_pdl(window_attn_mma_kernel<DA, DB, DV, STREAM>, grid, dim3(128), smem, st, a);
   QSPEC_CHECK_LAUNCH(1);

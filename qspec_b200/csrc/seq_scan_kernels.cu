@@ -756,12 +756,9 @@ static int launch_sd_chunks(const qspec_scalar_decay_args& a, const int* chunk_r
                             float* add, float* total, cudaStream_t st) {
   constexpr int KS = DP + CPAD, VS = 64 + CPAD;
   constexpr size_t smem_add = (size_t)(CHK * KS + 2 * CHK * VS) * 2, smem_out = (size_t)(2 * CHK * KS + CHK * VS + 2 * DP * VS) * 2;
-  static bool configured = false;
-  if (!configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(scalar_decay_chunk_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_add));
-    QSPEC_CUDA(cudaFuncSetAttribute(scalar_decay_out_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_out));
-    configured = true;
-  }
+  static SmemLimit limit_add, limit_out;
+  QSPEC_CUDA(limit_add.raise(scalar_decay_chunk_kernel<DP>, smem_add));
+  QSPEC_CUDA(limit_out.raise(scalar_decay_out_kernel<DP>, smem_out));
   const dim3 grid(nchunks, a.H, (a.DV + 63) / 64);
   launch_pdl(scalar_decay_chunk_kernel<DP>, grid, dim3(128), smem_add, st, a, chunk_rows, add, total);
   QSPEC_CHECK_LAUNCH(1);

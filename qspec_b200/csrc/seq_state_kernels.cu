@@ -1098,11 +1098,8 @@ static size_t talking_smem_bytes(const qspec_talking_attn_args* a, int nq, int r
 template <typename T, int REP, int NQ>
 static int launch_talking(const qspec_talking_attn_args* a, int nsplit, int tc_gc, int pv_tc, cudaStream_t st) {
   const size_t smem = talking_smem_bytes(a, NQ, REP, tc_gc, pv_tc);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    QSPEC_CUDA(cudaFuncSetAttribute(talking_attn_kernel<T, REP, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (smem > 48 * 1024) QSPEC_CUDA(limit.raise(talking_attn_kernel<T, REP, NQ>, smem));
   // 16-byte pieces of a key row, two value columns per load: only where every row starts on such a boundary
   const size_t es = sizeof(T);
   const int kv = 16 / (int)es;
