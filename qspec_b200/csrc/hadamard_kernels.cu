@@ -350,12 +350,12 @@ constexpr int K28_BPC = 4;                           // n-blocks (and mix output
 // Blocks reach the other CTAs as bulk copies of the CTA's four blocks, the maxima as single words, both counted by an mbarrier in the CTA that
 // receives them: stores of every thread into seven CTAs, with a release and acquire of the whole cluster after them, were the largest stall.
 // SiLU and quantiser, before -> now: n = 512, 1 row 5.7 -> 4.8 us, 64 rows 11.6 -> 9.2, 512 rows 44.5 -> 39.8; n = 1024, 64 rows 24.3 -> 17.7,
-// 512 rows 128 -> 98; n = 256, 64 rows 8.2 -> 7.3 (1 row 3.8 -> 3.9: a bulk copy of 2 KB takes a little longer than stores).
+// 512 rows 128 -> 98; n = 256, 64 rows 8.2 -> 7.3.
 // Every wait is bounded. A thread that gives one up tells the row's first CTA, which alone writes the row's scale: NaN then, after the cluster's last
 // barrier, whatever it was before; outputs of such a thread are NaN, its copies under way are waited for (up to the limit), and the row is counted
 // in k28_timeouts. `give_up`: the CTAs of a cluster, a bit each, that give their waits up at once (tests).
 constexpr uint32_t K28_SPINS = 1u << 20;
-static __device__ unsigned k28_timeouts;              // rows with a wait given up since the library was loaded
+static __device__ unsigned k28_timeouts;              // rows (or CTAs that stand alone) with a wait given up since the library was loaded
 __device__ __forceinline__ bool k28_wait(uint32_t bar, uint32_t limit) {
   for (uint32_t spins = 0; spins < limit; ++spins) {
     uint32_t done;
@@ -364,11 +364,15 @@ __device__ __forceinline__ bool k28_wait(uint32_t bar, uint32_t limit) {
   }
   return false;
 }
-template <int SLOTS, int WPB>
+// STORES (n = 256, few rows): blocks leave as asynchronous stores from the registers. Without a quantiser nothing is on its way to a CTA then that has its
+// blocks, nor read from it, and it leaves without the last barrier. us at 1 / 8 rows, bulk copies | stores: without quantiser 3.06 / 3.27 | 2.92 / 3.12, with it
+// 3.90 / 4.02 | 3.81 / 4.01; 32 rows 4.68 | 4.51 and 5.64 | 5.58, 64 with quantiser 7.43 | 7.76. (`stores` is 1 where STORES is: with the bulk copies left out
+// of this instantiation it is 0.3 us slower, 1 row 4.08 and 3.18, which nothing but the compiler's order of instructions was found to explain.)
+template <int SLOTS, int WPB, bool STORES>
 __global__ void __launch_bounds__(128 * WPB)
 hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict__ gate_up,
                             __half* __restrict__ out_f, uint8_t* __restrict__ out_q,
-                            __half* __restrict__ scale_out, int n, float scale, float clip, int c8, unsigned give_up) {
+                            __half* __restrict__ scale_out, int n, float scale, float clip, int c8, int stores, unsigned give_up) {
   constexpr int S1 = SLOTS / WPB, THR = 128 * WPB;   // vectors of 8 per lane, threads
   pdl_enter();
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -386,6 +390,7 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
   const uint32_t bar_blocks = (uint32_t)__cvta_generic_to_shared(&s_blocks), bar_amax = (uint32_t)__cvta_generic_to_shared(&s_amax);
   const uint32_t own_bytes = (uint32_t)(K28_BPC * n * 2);
   const uint32_t limit = give_up >> c & 1u ? 0u : K28_SPINS;
+  const bool alone = STORES && stores && out_q == nullptr;
   if (threadIdx.x == 0) {
     s_bad = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar_blocks));
@@ -394,8 +399,9 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar_blocks), "r"((K28_CLUSTER - 1) * own_bytes) : "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar_amax), "r"(K28_CLUSTER * 4) : "memory");
   }
-  __syncthreads();                                    // the barriers are there, for this CTA's waits
-  cluster_arrive_release();                           // ... and for the other CTAs' copies: waited for before the first one
+  __syncwarp();
+  cluster_arrive_release();                           // the barriers are there for the other CTAs' copies, before the first one (and for this CTA's waits after
+                                                      // the next barrier of the block)
 
   // ---- phase 1: WPB warps rotate n-block 4c + warp / WPB
   {
@@ -440,15 +446,32 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
       reinterpret_cast<uint4*>(sm)[blk * nv + lane + (half * S1 + s) * 32] = pack_h8(v[s]);
     }
   }
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  __syncthreads();
-  cluster_wait_acquire();                             // every CTA of the cluster has started
-  if (threadIdx.x < K28_CLUSTER && (int)threadIdx.x != c) {
-    const uint32_t src = sm_base + (uint32_t)c * own_bytes;
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(mapa_shared(src, threadIdx.x)), "r"(src),
-                 "r"(own_bytes), "r"(mapa_shared(bar_blocks, threadIdx.x)) : "memory");
+  if (STORES && stores) {
+    cluster_wait_acquire();                           // every CTA of the cluster has started
+    const uint32_t at = (uint32_t)((K28_BPC * c + warp) * nv + lane) * 16u;
+    const uint4 v = reinterpret_cast<const uint4*>(sm)[at / 16];       // this thread's own
+#pragma unroll
+    for (int r = 1; r < K28_CLUSTER; ++r) {
+      const uint32_t to = (uint32_t)(c + r < K28_CLUSTER ? c + r : c + r - K28_CLUSTER), dst = mapa_shared(sm_base + at, to);
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w),
+                   "r"(mapa_shared(bar_blocks, to)) : "memory");
+    }
+    __syncthreads();
+  } else {
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    cluster_wait_acquire();                           // every CTA of the cluster has started
+    if (threadIdx.x < K28_CLUSTER && (int)threadIdx.x != c) {
+      const uint32_t src = sm_base + (uint32_t)c * own_bytes;
+      asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(mapa_shared(src, threadIdx.x)), "r"(src),
+                   "r"(own_bytes), "r"(mapa_shared(bar_blocks, threadIdx.x)) : "memory");
+    }
   }
   bool ok = k28_wait(bar_blocks, limit);
+  if (alone && !ok) {
+    k28_wait(bar_blocks, K28_SPINS);
+    if (atomicExch(&s_bad, 1u) == 0) atomicAdd(&k28_timeouts, 1u);
+  }
   // Before the end every CTA arrives once more: none leaves while another may still copy from or into it.
   auto last_arrive = [&]() {
     if (!ok) {                                        // (a fence and a relaxed arrival: the word is there when the first CTA's wait is over)
@@ -467,7 +490,7 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
       atomicAdd(&k28_timeouts, 1u);
     }
   };
-  if (out_q == nullptr) last_arrive();
+  if (out_q == nullptr && !alone) last_arrive();
 
   // ---- phase 2: outputs o0..o0+3, column pairs jp = tid, tid + THR, ...; all 28 blocks are local now
   const int o0 = K28_BPC * c;
@@ -520,7 +543,7 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
     }
   }
   if (out_q == nullptr) {                             // uniform over the cluster
-    last_wait();
+    if (!alone) last_wait();
     return;
   }
   // ---- quantiser: CTA amax to every CTA, row amax from local shared memory
@@ -651,10 +674,13 @@ static int launch_k28(const void* x, const void* gu, void* of, int8_t* oq, void*
 // 112: 13.7 | 13.7, 128: 13.6 | 14.8, 512: 39.8 | 47.5 (the SMs are full either way, and the exchange between the warps is extra). n = 1024 always two (a lane
 // holds 16 values instead of 32), n = 256 always one (a lane has one vector).
 constexpr int K28_TWO_WARP_ROWS = 112;
-template <int SLOTS, int WPB>
+// n = 256: stores from the registers up to here, bulk copies above (figures beside the kernel: a copy's own latency counts while few rows are under
+// way, the number of stores later).
+constexpr int K28_STORE_ROWS = 32;
+template <int SLOTS, int WPB, bool STORES = false>
 static int launch_k28_cluster(const void* x, const void* gu, void* of, int8_t* oq, void* so, int rows, int n,
                               float scale, float clip, cudaStream_t st, int c8, unsigned give_up) {
-  auto kern = hadamard_k28_cluster_kernel<SLOTS, WPB>;
+  auto kern = hadamard_k28_cluster_kernel<SLOTS, WPB, STORES>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)rows * K28_CLUSTER);
   cfg.blockDim = dim3(128 * WPB);
@@ -672,7 +698,7 @@ static int launch_k28_cluster(const void* x, const void* gu, void* of, int8_t* o
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   QSPEC_CUDA(cudaLaunchKernelEx(&cfg, kern, (const uint4*)x, (const uint4*)gu, (__half*)of, (uint8_t*)oq, (__half*)so, n,
-                                scale, clip, c8, give_up));
+                                scale, clip, c8, STORES ? 1 : 0, give_up));
   count_launch(1);
   return QSPEC_OK;
 }
@@ -694,6 +720,8 @@ static int hadamard_k28_impl(const void* x, const void* gate_up, void* out_f16, 
   // neighbouring GEMMs' heads and tails. QSPEC_K28_CLUSTER_ROWS caps the row count that takes it (experiment knob).
   static const int cluster_rows = getenv("QSPEC_K28_CLUSTER_ROWS") ? atoi(getenv("QSPEC_K28_CLUSTER_ROWS")) : 65536;
   const bool few_rows = rows <= cluster_rows;
+  if (use_cluster && few_rows && n == 256 && rows <= K28_STORE_ROWS)
+    return launch_k28_cluster<1, 1, true>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8, give_up);
   if (use_cluster && few_rows && n == 256) return launch_k28_cluster<1, 1>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8, give_up);
   if (use_cluster && few_rows && n == 512) {
     if (rows <= K28_TWO_WARP_ROWS) return launch_k28_cluster<2, 2>(xx, gate_up, out_f16, out_q, scale_out, rows, n, scale, clip_ratio, st, c8, give_up);

@@ -80,7 +80,8 @@ def rotation():
         for give_up in (1, 2, 8, 64, 127):
             for plain in (False, True):
                 o, q, s, counted = call(give_up, plain)
-                assert counted == rows
+                alone = plain and n == 256 and rows <= 32                                # each CTA counts itself
+                assert counted == rows * (bin(give_up).count("1") if alone else 1)
                 assert plain or s.isnan().all()
                 for c in range(7):
                     part = slice(4 * c * n, 4 * (c + 1) * n)

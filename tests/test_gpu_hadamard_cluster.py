@@ -30,3 +30,23 @@ def test_rotation_is_the_oracle_and_batch_invariant(n, rows):
         for a, b in zip((o, q, s), run(x[i:i + 1].contiguous())):
             assert torch.equal(a[i:i + 1], b)
         np.testing.assert_array_equal(o[i:i + 1].cpu().numpy(), O.hadamard_k28(x[i:i + 1].cpu().numpy(), n, scale))
+
+
+@pytest.mark.parametrize("rows", [1, 7, 32, 33])
+@pytest.mark.parametrize("gated", [False, True])
+def test_256_wide_rows_by_stores_and_by_bulk_copies(rows, gated):
+    """Both sides of the row count up to which the blocks of n = 256 leave as stores, with and without the quantiser: a row is the same in any batch."""
+    from qspec_b200 import ops
+    n, scale = 256, 0.0118
+    x = torch.randn(300, (2 if gated else 1) * 28 * n, generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda").half()
+
+    def run(part, quant, plain):
+        m = part.shape[0]
+        o = torch.empty(m, 28 * n, dtype=torch.float16, device="cuda") if plain else None
+        q = torch.empty(m, 14 * n, dtype=torch.int8, device="cuda") if quant else None
+        s = torch.empty(m, dtype=torch.float16, device="cuda") if quant else None
+        ops.hadamard_k28(None if gated else part, n, scale, gate_up=part if gated else None, out=o, out_q=q, scale_out=s)
+        return [t for t in (o, q, s) if t is not None]
+    for quant, plain in ((True, False), (False, True), (True, True)):
+        for a, b in zip(run(x[:rows].contiguous(), quant, plain), run(x, quant, plain)):
+            assert torch.equal(a, b[:rows])
