@@ -93,6 +93,9 @@ int qspec_gemm_split_factor(int w4a16, int M, int N, int K);
  * f16, 2 = W4A16 bf16, 3 = W4A8. out[0..7] = {token tile, CTA pairs?, grid (CTAs or CTA pairs), cluster size, deferred
  * split, ring stages, token tiles, (pair-)tiles along N}. */
 int qspec_debug_gemm_plan(int mode, int M, int N, int K, int deferred, int* out);
+/* For tests: the form that a call of these sizes takes: 1 few tokens, 2 the tcgen05 form for long ranges (outputs on 16 bytes), 0 the other tcgen05
+ * form; -1: sizes that no call takes. No launch. */
+int qspec_debug_gemm_form(int mode, int M, int N, int K);
 /* For tests: the product of mode (0 W4A4, 1 W4A16 f16, 2 W4A16 bf16, 3 W4A8) into out, or the raw integer sums into acc. give_up 1: the first waits
  * are given up at once, and what depends on them is NaN (raw sums: the lowest integer). */
 int qspec_debug_gemm_give_up(int mode, const void* act, const void* sA, const int8_t* w, const void* sW, const void* bias, void* out, int32_t* acc,

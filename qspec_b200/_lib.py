@@ -56,6 +56,7 @@ SIGNATURES = {
     "qspec_gemm_w4a8_split": (c_int, [c_void_p, c_void_p, c_void_p, c_size_t, c_int, c_int, c_int, c_void_p, c_size_t,
                                       c_void_p]),
     "qspec_debug_gemm_plan": (c_int, [c_int, c_int, c_int, c_int, c_int, c_void_p]),
+    "qspec_debug_gemm_form": (c_int, [c_int, c_int, c_int, c_int]),
     "qspec_debug_gemm_give_up": (c_int, [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                          c_void_p, c_size_t, c_int, c_void_p]),
     "qspec_debug_hadamard_k28_give_up": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, ctypes.c_uint, c_void_p]),

@@ -1386,20 +1386,74 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& ma, const Params& p,
   return QSPEC_OK;
 }
 
-// Which calls the few-token kernel takes (gemm_w4_rows.cuh). Its time grows with the tokens (mma.sync, and for W4A16 the widening, which every
-// CTA does for its tokens at half the tensor rate), that of the tcgen05 form hardly: the line lies where they meet, later for products whose
-// time is mostly latency (up to 2^26 weights). us, few-token | tcgen05 form, on both sides of the lines:
-//   W4A4              28672 x 4096: 32 tokens 20.0 | 18.1, 24: 15.9 | 17.9   27648 x 5120: 32: 19.4 | 20.9, 48: 25.2 | 22.3   8192 x 8192: 64: 19.0 | 18.8
-//   W4A4 bytes, W4A8  28672 x 4096: 24 tokens 17.1 | 16.3, 16: 14.5 | 15.7   27648 x 5120: 24: 16.4 | 18.5, 32: 28.6 | 18.8   8192 x 8192: 32: 15.6 | 14.9
-//   W4A16             28672 x 4096: 16 tokens 20.5 | 24.1, 24: 30.9 | 24.5   10240 x 8192: 16: 17.6 | 20.1, 24: 29.3 | 21.4   8192 x 8192: 32: 19.5 | 18.3
-// (the sizes differ by a few percent at one token count: the line is one for all), and well inside: 6144 x 4096, 64 tokens W4A4 11.5 | 12.6, 32 tokens
-// bytes 7.9 | 10.9, W4A16 10.7 | 12.6.
+// Which calls the few-token kernel takes (gemm_w4_rows.cuh): those that it is the faster form for, by an estimate of both times (us; fitted to 41 sizes from
+// 512 x 512 to 128000 x 2048, 12 to 64 tokens, root of the mean squared error 4 to 9 %).
+//  * Few-token form: a constant, a share for each round of tiles (the sums that meet in shared memory), and one for each item that a warp of the
+//    busiest SM goes through; all grow with the tokens (mma.sync, and for W4A16 the widening, which every CTA does for its tokens at half the rate).
+//  * tcgen05 form: a constant, its units per CTA, what a tile costs that is shared between CTAs, by their number, and the stream of the weights.
+// Up to 16 tokens the few-token form is kept unless the other one is the faster by an eighth and more, which the estimates' error does not reach.
+// With the line N x K <= 2^26 or M <= 32 / 24 / 16 (W4A4 / W4A8 / W4A16) that was here before, 12288 x 4096 took 20.7 us at 64 tokens (now 13.2), 11008 x 4096
+// W4A8 15.4 at 32 (10.6), 12288 x 4096 W4A16 20.0 at 32 (15.0).
+// us, few-token | tcgen05 form, on both sides of the line:
+//   W4A4              28672 x 4096: 24 tokens 16.2 | 18.2, 32: 20.2 | 18.4   12288 x 4096: 24: 9.0 | 11.4, 64: 20.7 | 13.1   8192 x 8192: 64: 18.8 | 19.0   32000 x 1024: 24: 8.3 | 8.9, 32: 10.6 | 9.3
+//   W4A4 bytes, W4A8  28672 x 4096: 16 tokens 14.5 | 16.0, 24: 17.2 | 16.4   11008 x 4096: 24: 9.8 | 10.3, 32: 15.4 | 10.5   4096 x 14336: 32: 13.3 | 14.8
+//   W4A16             28672 x 4096: 16 tokens 20.4 | 24.0, 24: 31.4 | 24.5   12288 x 4096: 16: 11.5 | 14.4, 24: 17.5 | 14.8   5120 x 5120: 32: 12.6 | 12.8   5120 x 27648: 16: 32.6 | 26.7
 // QSPEC_GEMM_ROWS, read at every call, for measurements and tests: 0 = none, 2 = all that it can run.
+static bool rows_faster(int mode, int M, int N, int K, const Plan& pl) {
+  struct Rows { double base, round, item; };
+  static const Rows rows_i8[6] = {{1.4, 0.07, 0.59}, {1.2, 0.54, 0.66}, {1.3, 0.75, 0.76}, {0.8, 1.24, 0.97}, {0.8, 1.36, 1.28}, {0.9, 1.69, 1.95}};
+  static const Rows rows_a8[4] = {{1.4, 0.22, 0.63}, {1.1, 0.55, 0.72}, {1.3, 0.70, 0.84}, {1.1, 0.98, 1.57}};
+  static const Rows rows_f16[4] = {{1.1, 0.31, 0.90}, {1.0, 0.45, 1.17}, {1.0, 0.12, 2.00}, {1.9, 0.24, 2.25}};
+  struct Stream { double base, unit, shared, contributor, mb; };
+  static const Stream stream_i8[4] = {{4.5, 0.21, 2.5, 0.17, 0.074}, {4.9, 0.31, 3.2, 0.43, 0.053}, {5.4, 0.33, 3.9, 0.59, 0.053}, {6.1, 0.35, 4.5, 0.75, 0.055}};
+  static const Stream stream_a8[2] = {{4.6, 0.18, 2.5, 0.16, 0.092}, {4.9, 0.21, 3.2, 0.43, 0.084}};
+  static const Stream stream_f16[2] = {{4.5, 0.50, 2.6, 0.12, 0.055}, {5.1, 0.46, 2.9, 0.29, 0.077}};
+  const int sms = sm_count() > 0 ? sm_count() : 148, tiles = (N + ROWS_R - 1) / ROWS_R, items = (K + ROWS_UK - 1) / ROWS_UK, groups = (M + 7) / 8;
+  const int rounds = tiles <= sms ? 1 : (tiles + 2 * sms - 1) / (2 * sms);
+  const int last = tiles % (2 * sms);                                       // a last round of few tiles has the SMs nearly to itself
+  const double full = rounds > 1 && last > 0 && last <= sms / 4 ? rounds - 0.25 : rounds;
+  const double per_warp = tiles <= sms ? (items + 7) / 8 : full * (mode == MODE_I8 && groups == 1 ? 2 * ((items + 7) / 8) : (items + 3) / 4);   // (NW, CTAS of rows_launch)
+  const int g = groups <= 4 ? groups - 1 : groups <= 6 ? 4 : 5, m = M <= 16 ? 0 : M <= 32 ? 1 : M <= 48 ? 2 : 3;
+  const Rows r = mode == MODE_I8 ? rows_i8[g] : mode == MODE_A8 ? rows_a8[g] : rows_f16[g];
+  const Stream s = mode == MODE_I8 ? stream_i8[m] : mode == MODE_A8 ? stream_a8[m] : stream_f16[m];
+  const int units = (pl.U + pl.G - 1) / pl.G;
+  const bool whole = pl.U % pl.G == 0 && units % pl.KB == 0;
+  const double each = (double)pl.G * pl.KB / pl.U;             // CTAs of a tile
+  const double few = r.base + r.round * rounds + r.item * per_warp;
+  const double other = s.base + s.unit * units + (whole ? 0.0 : s.shared + s.contributor * (each > 1.0 ? each - 1.0 : 0.0)) + s.mb * ((double)N * K / 2e6);
+  return M <= 16 ? 0.87 * few <= other : few < other;
+}
+// What a size's plan says, remembered for the sizes asked for last: the plan takes a microsecond of a call of three
+struct Known { int mode, M, N, K; size_t bytes; bool rows; };
+static Known known_size(int mode, int M, int N, int K) {
+  static thread_local Known known[64];                        // (bytes 0: nothing known)
+  Known& k = known[((unsigned)N * 31u + (unsigned)K * 7u + (unsigned)M * 3u + (unsigned)mode) >> 3 & 63u];
+  if (!k.bytes || k.mode != mode || k.M != M || k.N != N || k.K != K) {
+    const Plan pl = make_plan(mode, M, N, K);
+    k = Known{mode, M, N, K, workspace_bytes(pl), rows_faster(mode, M, N, K, pl)};
+  }
+  return k;
+}
 static bool rows_wanted(int mode, int M, int N, int K) {
   const int want = env_int("QSPEC_GEMM_ROWS", 1);
   const int most = mode == MODE_I8 ? ROWS_MAX_M : ROWS_MAX_M / 2;         // what is instantiated
   if (want == 0 || M > most) return false;
-  return want == 2 || (long long)N * K <= (1ll << 26) || M <= (mode == MODE_I8 ? 32 : mode == MODE_A8 ? 24 : 16);
+  return want == 2 || known_size(mode, M, N, K).rows;
+}
+// Whether the tcgen05 form runs as LONG: wherever it can and a CTA's range is at least a tile long, so that whole tiles and ends of ranges are what a
+// launch waits for. us, without | with it:  W4A16 28672 x 4096: 64 tokens 27.8 | 26.2, 256: 59.2 | 54.6, 1000: 198 | 186   10240 x 8192, 256 tokens: 46.9 | 43.7
+//   W4A4 28672 x 4096: 65 tokens 24.6 | 22.9, 256: 49.4 | 38.9   W4A4 bytes 28672 x 4096: 64 tokens 20.5 | 18.2, 256: 47.5 | 35.8
+// Shorter ranges, whose tiles are all shared, gain nothing: 4096 x 14336, 256 tokens, W4A4 30.1 | 31.4, W4A4 bytes 28.6 | 29.4, W4A16 34.6 | 34.6.
+// Its stage may cost a ring its fifth stage, not its fourth (W4A16 27648 x 5120, 80 tokens, with three: 32.9 | 33.5).
+static bool long_wanted(Plan& pl) {
+  if (pl.cs != 1 || pl.U < pl.G * pl.KB) return false;
+  const bool fits = pl.smem + STAGE_BYTES <= (size_t)SMEM_MOST;
+  if (!fits && (pl.stages <= 4 || pl.smem - pl.stage_bytes + STAGE_BYTES > (size_t)SMEM_MOST)) return false;
+  if (!fits) {
+    pl.stages -= 1;
+    pl.smem -= pl.stage_bytes;
+  }
+  return true;
 }
 
 template <int MODE, int NT, int NW, int CTAS>
@@ -1441,14 +1495,6 @@ static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, const RowsA
   if constexpr (MODE == MODE_I8) return p.M <= 48 ? rows_launch<MODE, 6>(mw, ma, p, st) : rows_launch<MODE, 8>(mw, ma, p, st);
   return QSPEC_ERR_UNSUPPORTED;
 }
-// workspace_bytes(mode, M, N, K), remembered for the sizes asked for last: the plan behind it takes a microsecond of a call of three
-static size_t rows_workspace_bytes(int mode, int M, int N, int K) {
-  struct Known { int mode, M, N, K; size_t bytes; };
-  static thread_local Known known[16];                        // (bytes 0: nothing known)
-  Known& k = known[((unsigned)N * 31u + (unsigned)K * 7u + (unsigned)M * 3u + (unsigned)mode) >> 3 & 15u];
-  if (!k.bytes || k.mode != mode || k.M != M || k.N != N || k.K != K) k = Known{mode, M, N, K, workspace_bytes(mode, M, N, K)};
-  return k.bytes;
-}
 static int rows_run(int mode, const void* act, const int8_t* w, const RowsArgs& a, int K, cudaStream_t st) {
   CUtensorMap mw, ma;
   int rc = get_map(w, (uint64_t)a.N, (uint64_t)K / 2, ROWS_R, 1, &mw);
@@ -1481,7 +1527,7 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   if (M == 0) return QSPEC_OK;
   if (rows_wanted(mode, M, N, K)) {
     // (it needs no workspace, but asks for the one of the stream form all the same: which form runs is not the caller's business)
-    const size_t need = rows_workspace_bytes(mode, M, N, K);
+    const size_t need = known_size(mode, M, N, K).bytes;
     QSPEC_REQUIRE(workspace && ws_bytes >= need, QSPEC_ERR_WORKSPACE, "%s: workspace too small (%zu < %zu)", who, ws_bytes, need);
     QSPEC_REQUIRE(!split_out || split_bytes >= (size_t)M * N * 4, QSPEC_ERR_WORKSPACE, "%s: partial buffer too small (%zu < %zu)", who, split_bytes,
                   (size_t)M * N * 4);
@@ -1514,34 +1560,23 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   p.trace = g_trace ? g_trace + (size_t)(g_trace_seq++ % 8u) * 4096 : nullptr;
   p.M = M; p.N = N; p.K = K; p.np = pl.np; p.tiles_m = pl.tiles_m; p.KB = pl.KB; p.U = pl.U; p.G = pl.G; p.cs = pl.cs;
   p.stages = pl.stages; p.dcols = pl.dcols; p.dbufs = pl.dbufs; p.ta = pl.ta; p.tmem_cols = pl.tmem_cols; p.out_bf16 = out_bf16;
-  // The LONG form wherever it can run and a CTA's range is at least a tile long, so that whole tiles and ends of ranges are what a launch waits
-  // for. us, without | with it:  W4A16 28672 x 4096: 64 tokens 27.8 | 26.2, 256: 59.2 | 54.6, 1000: 198 | 186   10240 x 8192, 256 tokens: 46.9 | 43.7
-  //   W4A4 28672 x 4096: 65 tokens 24.6 | 22.9, 256: 49.4 | 38.9   W4A4 bytes 28672 x 4096: 64 tokens 20.5 | 18.2, 256: 47.5 | 35.8
-  // Shorter ranges, whose tiles are all shared, gain nothing: 4096 x 14336, 256 tokens, W4A4 30.1 | 31.4, W4A4 bytes 28.6 | 29.4, W4A16 34.6 | 34.6.
-  // Its stage may cost a ring its fifth stage, not its fourth (W4A16 27648 x 5120, 80 tokens, with three: 32.9 | 33.5).
-  if (out && !acc_out && !split_out && ((uintptr_t)out & 15) == 0 && N % 8 == 0 && pl.cs == 1 && pl.U >= pl.G * pl.KB && p.debug_exit == 0) {
-    if (pl.smem + STAGE_BYTES > (size_t)SMEM_MOST && pl.stages > 4) {
-      pl.stages -= 1;
-      pl.smem -= pl.stage_bytes;
-      p.stages = pl.stages;
-    }
-    if (pl.smem + STAGE_BYTES <= (size_t)SMEM_MOST) {
-      p.stage_at = (int)(pl.smem - 1024);
-      pl.smem += STAGE_BYTES;
-      if (pl.pair) {
-        switch (mode) {
-          case MODE_I8: return launch<MODE_I8, true, true>(mw, ma, p, pl, st);
-          case MODE_F16: return launch<MODE_F16, true, true>(mw, ma, p, pl, st);
-          case MODE_A8: return launch<MODE_A8, true, true>(mw, ma, p, pl, st);
-          default: return launch<MODE_BF16, true, true>(mw, ma, p, pl, st);
-        }
-      }
+  if (out && !acc_out && !split_out && ((uintptr_t)out & 15) == 0 && N % 8 == 0 && p.debug_exit == 0 && long_wanted(pl)) {
+    p.stages = pl.stages;
+    p.stage_at = (int)(pl.smem - 1024);
+    pl.smem += STAGE_BYTES;
+    if (pl.pair) {
       switch (mode) {
-        case MODE_I8: return launch<MODE_I8, false, true>(mw, ma, p, pl, st);
-        case MODE_F16: return launch<MODE_F16, false, true>(mw, ma, p, pl, st);
-        case MODE_A8: return launch<MODE_A8, false, true>(mw, ma, p, pl, st);
-        default: return launch<MODE_BF16, false, true>(mw, ma, p, pl, st);
+        case MODE_I8: return launch<MODE_I8, true, true>(mw, ma, p, pl, st);
+        case MODE_F16: return launch<MODE_F16, true, true>(mw, ma, p, pl, st);
+        case MODE_A8: return launch<MODE_A8, true, true>(mw, ma, p, pl, st);
+        default: return launch<MODE_BF16, true, true>(mw, ma, p, pl, st);
       }
+    }
+    switch (mode) {
+      case MODE_I8: return launch<MODE_I8, false, true>(mw, ma, p, pl, st);
+      case MODE_F16: return launch<MODE_F16, false, true>(mw, ma, p, pl, st);
+      case MODE_A8: return launch<MODE_A8, false, true>(mw, ma, p, pl, st);
+      default: return launch<MODE_BF16, false, true>(mw, ma, p, pl, st);
     }
   }
   if (pl.pair) {
@@ -1628,6 +1663,14 @@ extern "C" int qspec_debug_gemm_give_up(int mode, const void* act, const void* s
   QSPEC_REQUIRE(mode >= 0 && mode <= 3 && (w4s::mode_is_int(mode) || !acc), QSPEC_ERR_INVALID_ARG, "debug_gemm_give_up: mode %d", mode);
   return w4s::run(mode, act, sA, w, sW, bias, out, acc, M, N, K, dtype == QSPEC_DTYPE_BF16, workspace, workspace_bytes, (cudaStream_t)stream,
                   "debug_gemm_give_up", nullptr, 0, give_up);
+}
+
+// For tests: which form a call takes: 1 few tokens, 2 tcgen05 LONG (outputs on 16 bytes), 0 tcgen05 without it.
+extern "C" int qspec_debug_gemm_form(int mode, int M, int N, int K) {
+  if (mode < 0 || mode > 3 || M <= 0 || N <= 0 || K <= 0 || K % 128 || N % 8) return -1;
+  if (w4s::rows_wanted(mode, M, N, K)) return 1;
+  w4s::Plan pl = w4s::make_plan(mode, M, N, K);
+  return w4s::long_wanted(pl) ? 2 : 0;
 }
 
 extern "C" int qspec_gemm_split_factor(int w4a16, int M, int N, int K) {

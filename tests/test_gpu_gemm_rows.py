@@ -63,18 +63,27 @@ def test_rows_products_are_the_exact_sums(ops, monkeypatch, M, N, K, dt, with_bi
     assert ops.attn_tile_timeouts() == 0
 
 
-@pytest.mark.parametrize("mode,M,N,K", [("w4a4", 32, 28672, 4096), ("w4a4", 33, 28672, 4096), ("w4a4", 64, 8192, 8192), ("w4a4", 65, 8192, 8192),
-                                        ("w4a8", 24, 10240, 8192), ("w4a8", 25, 10240, 8192), ("w4a8", 32, 8192, 8192), ("w4a8", 33, 8192, 8192),
-                                        ("w4a16", 16, 10240, 8192), ("w4a16", 17, 10240, 8192), ("w4a16", 32, 8192, 8192), ("w4a16", 33, 8192, 8192)])
-def test_both_sides_of_the_rule(ops, monkeypatch, mode, M, N, K):
-    """Which form runs shows in the deferred split (the few-token form leaves one slice); both agree, run twice in a row on two inputs."""
+FORM = {"w4a4": 0, "w4a16": 1, "w4a8": 3}                    # the debug entries' modes
+
+
+# the last token count that the few-token form takes, and the next group
+@pytest.mark.parametrize("mode,M,N,K,few", [
+    ("w4a4", 24, 28672, 4096, True), ("w4a4", 25, 28672, 4096, False), ("w4a4", 32, 12288, 4096, True), ("w4a4", 33, 12288, 4096, False), ("w4a4", 64, 8192, 8192, True),
+    ("w4a4", 65, 8192, 8192, False), ("w4a4", 24, 32000, 1024, True), ("w4a4", 25, 32000, 1024, False), ("w4a8", 16, 28672, 4096, True), ("w4a8", 17, 28672, 4096, False),
+    ("w4a8", 24, 11008, 4096, True), ("w4a8", 25, 11008, 4096, False), ("w4a8", 32, 4096, 14336, True), ("w4a8", 33, 4096, 14336, False), ("w4a16", 16, 28672, 4096, True),
+    ("w4a16", 17, 28672, 4096, False), ("w4a16", 16, 12288, 4096, True), ("w4a16", 17, 12288, 4096, False), ("w4a16", 24, 8192, 8192, True), ("w4a16", 25, 8192, 8192, False),
+    ("w4a16", 8, 5120, 27648, True), ("w4a16", 9, 5120, 27648, False)])
+def test_both_sides_of_the_rule(ops, monkeypatch, mode, M, N, K, few):
+    """The form that runs is the one expected (the deferred split of the few-token form is one slice), and both agree, run twice in a row on two inputs."""
+    from qspec_b200 import _lib
     w, sW, _, sA, q, x = _operands(M, N, K, torch.float16, M + N)
     kind = {"w4a4": 0, "w4a16": 1, "w4a8": 2}[mode]
-    rows = M <= {0: 64, 1: 32, 2: 32}[kind] if N * K <= 2 ** 26 else M <= {0: 32, 1: 16, 2: 24}[kind]
     packed = ((q[:, 0::2] & 15) | (q[:, 1::2] << 4)).contiguous()
+    assert (_lib.load().qspec_debug_gemm_form(FORM[mode], M, N, K) == 1) == few
 
     def call(form, flip):
         monkeypatch.setenv("QSPEC_GEMM_ROWS", form)
+        assert (_lib.load().qspec_debug_gemm_form(FORM[mode], M, N, K) == 1) == (few if form == "1" else form == "2")
         out = torch.empty(M, N, dtype=torch.float16, device="cuda")
         if mode == "w4a4":
             ops.rowwise_scaled_linear_cutlass_s4s4_unified(packed.flip(0).contiguous() if flip else packed, sA, w, sW, None, out)
@@ -84,14 +93,41 @@ def test_both_sides_of_the_rule(ops, monkeypatch, mode, M, N, K):
             ops.gemm_w4a16(x.flip(0).contiguous() if flip else x, w, sW, None, out)
         return out
 
-    if rows:
+    if few:
         assert ops.gemm_split_factor(kind, M, N, K) == 1
+    can = M <= (64 if mode == "w4a4" else 32)
     for flip in (False, True, False):
-        a, b = call("1", flip), call("0", flip)
+        a, b = call("0" if few or not can else "2", flip), call("1", flip)                 # the other form, and the rule's
         if mode == "w4a16":                                               # another order of float32 sums, then a rounding to 11 bits
             assert (a.float() - b.float()).norm() <= 1e-4 * b.float().norm()
         else:
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 128), (4, 4096, 4096), (5, 776, 2176), (9, 40, 384), (16, 4736, 640), (17, 4768, 384), (32, 14336, 512)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_few_tokens_through_the_tcgen05_form(ops, monkeypatch, M, N, K, dt):
+    """What the rule leaves to the few-token form: the tcgen05 form takes it all the same, where it is asked to."""
+    from qspec_b200 import _lib
+    w, sW, bias, sA, q, x = _operands(M, N, K, dt, M * 131 + N + K)
+    packed = ((q[:, 0::2] & 15) | (q[:, 1::2] << 4)).contiguous()
+    monkeypatch.setenv("QSPEC_GEMM_ROWS", "0")
+    assert all(_lib.load().qspec_debug_gemm_form(mode, M, N, K) != 1 for mode in range(4))
+    sums = q.double() @ _int4(w).T
+    want = ((sums.float() * sA.float()[:, None]) * sW.float()[None, :] + bias.float()).to(dt)
+    for call, act in ((ops.rowwise_scaled_linear_cutlass_s4s4_unified, packed), (ops.rowwise_scaled_linear_cutlass_s8s4, q)):
+        out = torch.full((M, N), float("nan"), dtype=dt, device="cuda")
+        call(act, sA, w, sW, bias, out)
+        assert torch.equal(out, want)
+    assert torch.equal(ops.gemm_w4a4_acc_i32(packed, w), sums.int()) and torch.equal(ops.gemm_w4a8_acc_i32(q, w), sums.int())
+    out = torch.full((M, N), float("nan"), dtype=dt, device="cuda")
+    ops.gemm_w4a16(x, w, sW, bias, out)
+    exact = x.double() @ _int4(w).T * sW.double() + bias.double()
+    # float32: a partial sum of K products stays below 6 of its standard deviations; every 16 of them lose at most 2^-23 of it, as do the joins of a
+    # tile's parts and the epilogue's two operations. Then one rounding to 8 or 11 bits.
+    mag = (x.double().square().sum(1, keepdim=True) * 21.5).sqrt() * 6 * sW.double()
+    tol = mag * (K / 16 + 8) * 2.0 ** -23 + (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11) * exact.abs() + 2.0 ** -24
+    assert bool(((out.double() - exact).abs() <= tol).all())
 
 
 def test_capture_and_two_streams(ops):
