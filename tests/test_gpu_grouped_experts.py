@@ -1,5 +1,5 @@
-"""The grouped expert feed-forward (tcgen05 form) at the edges of its tiles: rows of an expert around 128, widths and expert sizes that are not
-multiples of a tile or a k-step, pairs without an expert, experts without a pair, more pairs and experts than the grouping keeps in registers."""
+"""The grouped expert feed-forward (tcgen05 form) at the edges of its tiles: rows of an expert around 128, around 256 and at multiples of 16, widths and
+expert sizes that are not multiples of a tile or a k-step, pairs without an expert, experts without a pair, more pairs and experts than the grouping keeps in registers."""
 import pytest
 import torch
 
@@ -52,4 +52,24 @@ def test_grouped_experts_match_64_bits(T, top, E, W, F, act):
     # each moving the result by at most 2^-7 (square) * sqrt(share); the rounding of the result is 2^-9 of its own value. 2^-8 covers both in the 2-norm.
     assert torch.isfinite(out).all()
     assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm()
+    assert ops.moe_grouped_status() == 0
+
+
+@pytest.mark.parametrize("rows", [[255], [256], [257], [272, 16, 1], [512, 513, 15], [240, 0, 496, 17], [769]])
+@pytest.mark.parametrize("act", ["silu", "relu2"])
+def test_rows_of_an_expert_around_its_tiles(rows, act):
+    """Experts with exactly these rows: tiles of up to 256 rows, evenly divided, in multiples of 16."""
+    from qspec_b200 import ops
+    E, W, F, T = len(rows), 264, 136, sum(rows)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    h = torch.randn(T, W, generator=g, device="cuda").bfloat16()
+    gate_up = (torch.randn(E, F if act == "relu2" else 2 * F, W, generator=g, device="cuda") * W ** -0.5).bfloat16()
+    down = (torch.randn(E, W, F, generator=g, device="cuda") * F ** -0.5).bfloat16()
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(rows))[torch.randperm(T, generator=torch.Generator().manual_seed(T))].int().cuda()[:, None].contiguous()
+    out = torch.full((T, 1, W), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.moe_expert_grouped(h, gate_up, down, idx, out, E, F, 7.0, act=act)
+    want = _expected(h, gate_up, down, idx, E, F, act, 7.0)
+    assert torch.isfinite(out).all()
+    assert ((out.double() - want).norm(dim=2) <= 2.0 ** -6 * want.norm(dim=2)).all()     # each row by itself: a few projections beside a rounding edge in 136
+    assert (out.double() - want).norm() <= 2.0 ** -8 * want.norm()                         # (the bound of the test above)
     assert ops.moe_grouped_status() == 0
