@@ -117,7 +117,7 @@ int qspec_split_add_norm_f16(void* x, const void* partials, int split, int w4a16
  * them through its int8-activation instantiation (qspec_gemm_w4a8 / qspec_gemm_w4a8_split: TMA delivers the operand as it
  * lies) and does not widen the activation tile again for every weight tile. Outputs are bit-identical to the packed route:
  * acc = 16 * sum(a * w) >> 4 instead of 256 * sum(a * w) >> 8. Worth it from ~64 token rows (12.8 vs 14.5 us for the 8B qkv
- * GEMM, profiles/r02y); the packed format stays the interchange format of the plugin API. In qspec_gemm_split_factor and
+ * GEMM); the packed format stays the interchange format of the plugin API. In qspec_gemm_split_factor and
  * qspec_split_add_norm_* the kind argument (`w4a16`) takes 2 for partials produced by qspec_gemm_w4a8_split. */
 int qspec_split_add_norm_quant_i4_c8(void* x, const void* partials, int split, int w4a16, const void* sA, const void* sW,
                                      const void* bias, int8_t* out_q, void* scale, void* input_sum, int rows, int K,
@@ -271,7 +271,7 @@ int qspec_gemm_w4a16(const void* x, const int8_t* w, const void* sW, const void*
                      int M, int N, int K, int dtype, void* workspace, size_t workspace_bytes,
                      void* stream);
 
-/* ---- neighbours of the path used by the decode loop (SURVEY 8(f)) -------------------------------
+/* ---- neighbours of the path used by the decode loop -------------------------------
  * out = a + b elementwise (residual add, quarot_llama.py:380,389). n elements of dtype. */
 int qspec_add(const void* a, const void* b, void* out, size_t n, int dtype, void* stream);
 /* out[r,i] = f16(f16(silu(gate[r,i])) * up[r,i]) with gate_up [rows, 2*inter] = [up ; gate]
@@ -343,7 +343,7 @@ int qspec_argmax_rows_static_max_rows(void);
 int qspec_argmax_rows_static(const void* logits, int rows, int V, long long row_stride, long long* out_idx, float* out_val,
                              void* stream);
 
-/* ---- Qwen2.5-14B variant of the path (SURVEY 8(f) rank 4; vllm/model_executor/models/qwen2_quarot.py) -------------
+/* ---- Qwen2.5-14B variant of the path (vllm/model_executor/models/qwen2_quarot.py) -------------
  * hidden 5120 = 40 heads x 128, intermediate 13824 = 108 x 128, bias in qkv_proj (the `bias` argument of both GEMMs).
  *
  * down_proj rotation had108 (x) H_128, optionally fused with SiLU*mul in front and the Quantizer behind. Replaces

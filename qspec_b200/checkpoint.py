@@ -1,4 +1,4 @@
-"""Weight-format loader for the published QSpec / QuaRot int4 checkpoint (SURVEY 8(f) rank 3); host-side logic only.
+"""Weight-format loader for the published QSpec / QuaRot int4 checkpoint; host-side logic only.
 
 What the reference does at load time, restated once here so that the decode engine can take real weights:
 
@@ -10,7 +10,7 @@ What the reference does at load time, restated once here so that the decode engi
   `down_proj.2.` -> `down_proj.`; two safetensors shards merged into one state dict.
 * fusion (vllm/model_executor/models/quarot_llama.py:152-173, 301-314): qkv = [q ; k ; v] rows, gate_up = [up ; gate] rows, weights
   and scales alike.
-* tensor parallelism (SURVEY 8(e)): qkv / gate_up column-sharded by heads / by co-located up+gate slices, o / down row-sharded
+* tensor parallelism: qkv / gate_up column-sharded by heads / by co-located up+gate slices, o / down row-sharded
   along the packed K dimension with replicated scales, lm_head vocab-sharded (`qspec_b200.parallel`).
 
 Both kernels read the checkpoint bytes as they are: no repacking, no offset-binary copy.
@@ -158,7 +158,7 @@ def load_state_dict(model, state_dict: Mapping[str, torch.Tensor], reference_key
 
 
 # ----------------------------------------------------------------------------------------------
-# TP-aware re-rotation of the row-parallel weights (SURVEY 7 hard part 5, 8(f) rank 3)
+# TP-aware re-rotation of the row-parallel weights
 #
 # The checkpoint's o_proj / down_proj weights were folded with the GLOBAL online rotation R (o_proj: H_heads (x) I_d / sqrt(heads),
 # quarot_llama.py:230-234; down_proj: (had28 (x) H_n) / sqrt(inter), hadamard.py:109-113): y = W_ckpt . (R x). At TP = t every rank

@@ -15,7 +15,7 @@ namespace qspec {
 // (thread t owns vectors t, t+256, ...), so HBM is read exactly once.
 // ------------------------------------------------------------------------------------------
 //
-// Tensor-parallel form (TP=true), SURVEY 8(e): the row-parallel GEMM that precedes this norm leaves one partial
+// Tensor-parallel form (TP=true): the row-parallel GEMM that precedes this norm leaves one partial
 // sum per rank. Instead of an all-reduce launch between the two (RowParallelLinear.forward,
 // layers/linear.py:1143-1144) the norm reads every rank's partial over NVLink peer memory, adds them in rank
 // order in fp32 (one rounding to the storage type: the value the all-reduce would have left in `out`) and goes
@@ -433,7 +433,7 @@ sym_quant_i8_kernel(const uint4* __restrict__ x, __half* __restrict__ scale_out,
 }
 
 // ------------------------------------------------------------------------------------------
-// element-wise neighbours (SURVEY 8(f) rank 2): residual add, SiLU(gate)*up
+// element-wise neighbours: residual add, SiLU(gate)*up
 // ------------------------------------------------------------------------------------------
 template <bool BF16>
 __global__ void add_kernel(const uint4* a, const uint4* b, uint4* out, size_t nvec) {
@@ -795,7 +795,7 @@ extern "C" int qspec_sym_quant_i4(const void* x, void* scale, int8_t* out_q, int
   return QSPEC_OK;
 }
 
-// ---- W4A8 activation side (SURVEY 8(f) rank 4) ----------------------------------------------
+// ---- W4A8 activation side ----------------------------------------------
 extern "C" int qspec_norm_quant_i8(const void* x, int8_t* out_q, void* scale, void* input_sum,
                                    int rows, int K, float eps, void* stream) {
   QSPEC_REQUIRE(x && out_q && scale, QSPEC_ERR_INVALID_ARG, "norm_quant_i8: null pointer");

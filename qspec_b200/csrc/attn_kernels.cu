@@ -1,5 +1,5 @@
 // Neighbours of the dual-mode linear path that the QSpec decode loop needs between qkv_proj and
-// the o_proj rotation (SURVEY 8(f) rank 2; vllm ops.rotary_embedding + reshape_and_cache +
+// the o_proj rotation (vllm ops.rotary_embedding + reshape_and_cache +
 // flash-attn in the reference, quarot_llama.py:207-221). Not part of the parity contract of the
 // linear path: fp32 math, compared against a torch fp32 reference with a tolerance. sm_100a.
 #include "common.cuh"

@@ -7,7 +7,7 @@
 // rowwise_scaled_linear_cutlass/rowwise_scaled_linear_cutlass_unified.cuh:240-488, an SM80 mma.sync.s4
 // kernel) and the BitBLAS Matmul + per-call `weight ^ 0x88` pass (quarot_nn/linear.py:102-124,156-211).
 //
-// Products of few tokens take another kernel (gemm_w4_rows.cuh; rule: rows_wanted below).
+// Products of few tokens take another kernel (gemm_w4_rows.cuh; rule: rows_faster below); what is said of decode sizes here counts where it does not.
 //
 // Design (nothing here follows the reference's kernels):
 //  * swap-AB: the 128 output channels of a tile are the UMMA M dimension, tokens are UMMA N (16..128).
@@ -99,8 +99,7 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
 // arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster. Default semantics (release, cta
 // scope) like CUTLASS's ClusterBarrier::arrive(cta_id): what the arrival orders -- tcgen05.st results and async-proxy
 // visible shared memory -- is fenced explicitly (tcgen05.wait::st + fence::before_thread_sync, fence.proxy.async) before it.
-// A cluster-scope release / acquire on these barriers costs a full fence (L1 invalidate) per slot hand-over: measured 2x
-// slower kernels (profiles/r02b_pair_first.md).
+// A cluster-scope release / acquire on these barriers costs a full fence (L1 invalidate) per slot hand-over: kernels twice as slow, measured.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t rank) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(mapa_shared(bar, rank)) : "memory");
 }
@@ -160,8 +159,8 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 // D[tmem] (+)= A[tmem] * B[smem]; A is 128 lanes x 8 columns (32 bytes of K per row).
 // PAIR (cta_group::2): ONE instruction, issued by the leader CTA, drives both SMs' tensor cores: M = 256 = the 128 weight
 // channels in EACH CTA's tensor memory (same columns), the token tile B split between the two CTAs' shared memory (each
-// holds N/2 rows at the same offset), D = 128 lanes x N columns in each CTA. Measured on B200 (scripts/umma_probe.cu,
-// profiles/r02_umma_probe.md): ~58 cycles per instruction for N <= 64 in BOTH forms, so the pair halves the tensor-pipe
+// holds N/2 rows at the same offset), D = 128 lanes x N columns in each CTA. Measured on B200
+// (scripts/umma_probe.cu): ~58 cycles per instruction for N <= 64 in BOTH forms, so the pair halves the tensor-pipe
 // issue time per weight byte.
 template <int MODE, bool PAIR>
 __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -692,8 +691,8 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         const unsigned char* act = sm_act + (size_t)st.idx * act_stage;
         // Decode tiles (<= 16 token rows per CTA): one chunk per thread. Larger tiles: up to AB chunks per thread (64 tokens per
         // group), loaded together so that their shared-memory latencies overlap -- one chunk per loop iteration cost ~200 cycles
-        // per iteration, 830 cycles per unit at 64 tokens (profiles/r02c_gemm_trace.txt). Kept apart: the batched form costs
-        // the decode-sized kernels ~10 % (16 more live registers across the weight widening; r02o bench, configs[1]).
+        // per iteration, 830 cycles per unit at 64 tokens. Kept apart: the batched form costs
+        // the decode-sized kernels ~10 % (16 more live registers across the weight widening). The few-token form takes calls of that size by default.
         constexpr int AB = 4;
         const bool a_small = npl <= 16;
         const int ac = gtid & 7;                         // a thread's chunks: tokens (gtid >> 3) + 16 j, the same 16-byte column
@@ -846,7 +845,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         // A thread's items are tokens tok_base + 4 j of ONE channel quad (128 threads = 4 tokens x 32 quads): the per-channel
         // scales are loaded once, and RB items are reduced together so that RB x 2 partial-tile loads are in flight per L2
         // round trip. (One item per iteration made the reduction a chain of m_here / 4 dependent round trips: ~8 us for a
-        // 64-token tile, ~16 us for 128 tokens -- profiles/r02m_gsweep_tp.md -- against ~2.5 us at decode sizes.)
+        // 64-token tile, ~16 us for 128 tokens, against ~2.5 us at decode sizes.)
         constexpr int RB = 4;
         const int quad = etid & 31, tok_base = etid >> 5;
         const int chq = n0 + 4 * quad;
@@ -1210,10 +1209,10 @@ constexpr int SMEM_MOST = 227 * 1024 - 2048;   // dynamic: the static part is be
 // (2 x 16 KB of weights) and pairs; the launch has 2 G CTAs in clusters of two.
 struct Plan { int np, tiles_m, tiles_n, KB, U, G, cs, split, stages, dcols, dbufs, ta, tmem_cols, pair; size_t smem, slot_bytes, stage_bytes; };
 
-// QSPEC_GEMM_PAIR: 1 (default) = CTA pairs whenever the shape allows it, 0 = never (the round-1 kernel; kept for A/B runs).
+// QSPEC_GEMM_PAIR: 1 (default) = CTA pairs whenever the shape allows it, 0 = never (for A/B runs).
 // QSPEC_GEMM_PAIR_MIN_M: smallest token count that uses pairs (default below). Read at every call: A/B runs in one process.
 static bool pair_wanted(int M, int N) {
-  // measured (profiles/r02d_pair_ab.md): pairs win from one full 128-token tile on (M = 256: -9 .. -20 %), and lose 10-35 %
+  // measured: pairs win from one full 128-token tile on (M = 256: -9 .. -20 %), and lose 10-35 %
   // at decode sizes, where the cluster launch and the remote hand-overs add to an already latency-bound kernel
   return env_int("QSPEC_GEMM_PAIR", 1) != 0 && N % (2 * TM) == 0 && M >= env_int("QSPEC_GEMM_PAIR_MIN_M", 128);
 }
@@ -1226,14 +1225,14 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   // 256-token tiles (CTA pairs, W4A16 only): ONE pass over the weights for M in (128, 256] -- each weight unit is converted
   // once and multiplied with tcgen05.mma N = 256 (128 cycles per instruction = the dense rate, scripts/umma_probe.cu) instead
   // of twice with N = 128. The accumulator then takes 256 of the 512 tensor-memory columns, single-buffered.
-  // Measured (profiles/r02j_np256_ab.md): -7 % where every pair owns whole tiles (gate_up 75.7 -> 70.3 us, the 70B gate_up
+  // Measured: -7 % where every pair owns whole tiles (gate_up 75.7 -> 70.3 us, the 70B gate_up
   // 250.5 -> 244.6 us); shapes with fewer pair tiles than SM pairs, whose tiles are shared between pairs, got SLOWER in
   // isolation (qkv 23.8 -> 54.9 us, down 46.5 -> 70.4 us; cause not isolated: the 256 KB shared-tile reduction with a
   // single accumulator buffer is the suspect) => only for N / 256 >= 2 x SM pairs (see below). QSPEC_GEMM_NP256: 0 = never, 2 = always.
   {
     const int want = env_int("QSPEC_GEMM_NP256", 1);
     const int pairs = (sm_count() > 0 ? sm_count() : 148) / 2;
-    // (r03c, after the shared-tile reduction was batched and the scheduler refitted: the two-pass form is ahead again on the 8B
+    // (After the shared-tile reduction was batched and the scheduler refitted: the two-pass form is ahead again on the 8B
     // gate_up, 67.7 vs 70.1 us -- 112 pair tiles leave 18 of 74 pairs idle in the one-pass form -- and behind on the 70B gate_up,
     // 246 vs 228 us => one-pass tiles from two full waves of pair tiles)
     if (pl.pair && !mode_is_int(mode) && M > 128 && (want == 2 || (want == 1 && N / (2 * TM) >= 2 * pairs)))
@@ -1244,18 +1243,20 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   pl.KB = (K + UK - 1) / UK;
   pl.U = pl.tiles_m * pl.tiles_n * pl.KB;
   const int sms = (sm_count() > 0 ? sm_count() : 148) / (pl.pair ? 2 : 1);   // schedulable units: SMs, or SM pairs
-  // measured on B200 (scripts/umma_probe.cu): a tcgen05.mma of this kernel's shape issues every ~58 cycles (N <= 64) in both
+  // The unit, reduction and tile-width figures below were fitted before operand slots of eight instructions and the LONG form, and have not been since:
+  // whether they still choose the best grids has not been measured again, and they are no times of the present kernel (rows_faster has those).
+  // Measured on B200 (scripts/umma_probe.cu): a tcgen05.mma of this kernel's shape issues every ~58 cycles (N <= 64) in both
   // cta_group forms => per (pair-)unit 8 (int) / 16 (f16) instructions = 0.25 / 0.49 us at 1.9 GHz, plus the converters'
   // share; a pair-unit carries twice the bytes
   // ... and grows with the token tile (the converters widen np activation rows per unit, the MMAs get longer from N = 128):
-  // measured slopes of the grid sweeps at 64 / 256 tokens (profiles/r02m_gsweep_tp.md): W4A4 0.46 us per unit at np = 64,
+  // measured slopes of the grid sweeps at 64 / 256 tokens: W4A4 0.46 us per unit at np = 64,
   // W4A16 0.93 (0.75 per pair-unit) at np = 128
   const double tu_np = pl.np > 16 ? (double)(pl.np - 16) : 0.0;
   // (256-token pair tiles: 1.9 us per pair-unit -- 55 % of the MMA rate: every pair pulls 128 KB of activations per unit from L2)
   const double tu_cta = mode_is_int(mode) ? (pl.pair ? 0.27 : 0.316) + 0.003 * tu_np
                         : pl.pair ? (pl.np > 128 ? 1.9 : 0.50 + 0.0022 * tu_np) : 0.606 + 0.0029 * tu_np;
   // every further contributor of a shared tile adds np x 128 words to the last arriver's reduction: us per token row
-  // (decode tiles: fitted in round 1; larger tiles: r02m sweep, 3.7 us for 2 and 6.0 us for 4 contributors at np = 64)
+  // (larger tiles: 3.7 us for 2 and 6.0 us for 4 contributors at np = 64)
   const double red_row = pl.np <= 32 ? 0.00512 : 0.02;
   const double tu_hbm = pl.pair ? 0.00512 : 0.00256;
   // Grid size. Default: every SM, units split evenly (stream-K). When a CTA's range is shorter than a tile it then
@@ -1628,7 +1629,7 @@ extern "C" int qspec_gemm_w4a4_acc_i32(const int8_t* a, const int8_t* w, int32_t
                   (cudaStream_t)stream, "gemm_w4a4_acc_i32");
 }
 
-// W4A8 (SURVEY 8(f) rank 4): int8 activations [M, K] x the same packed int4 weights, exact int32 accumulation, the W4A4 epilogue.
+// W4A8: int8 activations [M, K] x the same packed int4 weights, exact int32 accumulation, the W4A4 epilogue.
 // Replaces torchao's rowwise_scaled_linear_cutlass_s8s4 as called by Linear4bit.forward_w4a8 (quarot_nn/linear.py:86-99).
 extern "C" size_t qspec_gemm_w4a8_workspace_bytes(int M, int N, int K) { return w4s::workspace_bytes(w4s::MODE_A8, M, N, K); }
 

@@ -715,8 +715,8 @@ static int hadamard_k28_impl(const void* x, const void* gate_up, void* out_f16, 
   cudaStream_t st = (cudaStream_t)stream;
   const void* xx = gate_up ? nullptr : x;
   static const bool use_cluster = !(getenv("QSPEC_K28_CLUSTER") && getenv("QSPEC_K28_CLUSTER")[0] == '0');
-  // The 7-CTA cluster form serves every row count: with many rows (64 / 256-token passes of configs[2]) it still wins in the
-  // decode loop (19.9 vs 20.8 ms per 64-sequence step, profiles/r02f_notes.md) because its short CTAs overlap the
+  // The 7-CTA cluster form serves every row count: with many rows (64 / 256-token passes of 64 sequences) it still wins in the
+  // decode loop (19.9 vs 20.8 ms per 64-sequence step) because its short CTAs overlap the
   // neighbouring GEMMs' heads and tails. QSPEC_K28_CLUSTER_ROWS caps the row count that takes it (experiment knob).
   static const int cluster_rows = getenv("QSPEC_K28_CLUSTER_ROWS") ? atoi(getenv("QSPEC_K28_CLUSTER_ROWS")) : 65536;
   const bool few_rows = rows <= cluster_rows;

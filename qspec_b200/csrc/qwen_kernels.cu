@@ -1,4 +1,4 @@
-// Activation-side kernels of the Qwen2.5-14B variant of the QSpec path (SURVEY 8(f) rank 4; reference
+// Activation-side kernels of the Qwen2.5-14B variant of the QSpec path (reference
 // vllm/model_executor/models/qwen2_quarot.py): hidden 5120 = 40 heads x 128, intermediate 13824 = 108 x 128.
 //   * down_proj rotation had108 (x) H_128 (qwen2_quarot.py:114-127 -> hadamard_utils.matmul_hadU_cuda, K = 108:
 //     FHT_128 * 1/sqrt(13824) rounded to f16, then had108 @ . with fp32 accumulation, f16 out), optional SiLU*up prologue
@@ -40,7 +40,7 @@ hadamard_k108_kernel(const uint4* __restrict__ x, const uint4* __restrict__ gate
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t row = blockIdx.x;
   constexpr int L = QK * QN, inter_v = L >> 3, nv = QN >> 3;      // 16 vectors per block
-  // the sign table into shared memory (from constant memory it cost a scoreboard stall per k-step, profiles/r03i_qwen_notes.md);
+  // the sign table into shared memory (from constant memory it cost a scoreboard stall per k-step);
   // it does not depend on the predecessor kernel, and is consumed after the __syncthreads() that closes phase 1
   for (int i = threadIdx.x; i < QK * 4 * 7; i += 256) s_sign[i] = __ldg(&d_had108_sign[0][0][0] + i);
   const uint4* xrow = x ? x + row * inter_v : nullptr;

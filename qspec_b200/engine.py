@@ -8,7 +8,7 @@ rejection (draft token accepted iff it equals the target argmax), and the metric
 spec_decode/metrics.py:171-179 (draft_acceptance_rate, system_efficiency).
 
 The whole step (3 x 32 draft layers + 32 verify layers + sampling + acceptance + state update)
-is captured once into a CUDA graph (SURVEY 8(f) rank 1: the reference runs ~550 eager launches
+is captured once into a CUDA graph (the reference runs ~550 eager launches
 per draft step with --enforce_eager); all per-step state lives on the device.
 """
 from __future__ import annotations

@@ -9,7 +9,7 @@ One `nn.Module` instance and ONE packed int4 weight per linear serve both modes;
 the `w4a4` flag of `forward`, the reference's ExecuteModelRequest.w4a4 -> kwargs["w4a4"]
 switch (spec_decode_worker.py:797-812, worker_base.py:416).
 
-Tensor parallelism (SURVEY 8(e)): column-parallel qkv / gate_up, row-parallel o / down. The all-reduce of
+Tensor parallelism: column-parallel qkv / gate_up, row-parallel o / down. The all-reduce of
 RowParallelLinear.forward (layers/linear.py:1143-1144) is fused into the norm that follows (peer-mapped partial
 sums, `parallel.PeerPartials`; QSPEC_TP_FUSED=0 restores one NCCL all-reduce per row-parallel GEMM); online
 rotations are shard-local.
@@ -40,7 +40,7 @@ class QSpecLlamaConfig:
     rope_theta: float = 500000.0
     max_seq_len: int = 1024          # KV-cache length per sequence
     name: str = "llama-3-8b"
-    # Qwen2.5-14B variant of the path (SURVEY 8(f) rank 4, vllm/model_executor/models/qwen2_quarot.py):
+    # Qwen2.5-14B variant of the path (vllm/model_executor/models/qwen2_quarot.py):
     qkv_bias: bool = False           # bias in qkv_proj (:172-178)
     had_k: int = 28                  # down_proj rotation had_k (x) H_{inter/had_k}: 28 (Llama-3) or 108 (13824 = 108 * 128)
     heads_rotation: str = "sylvester"   # o_proj rotation across heads: Sylvester FHT (2^k heads) or "had40" (:269-277)
@@ -72,7 +72,7 @@ class QSpecLlamaConfig:
         return QSpecLlamaConfig(**d)
 
     def linear_shapes(self, tp: int = 1):
-        """(N, K) per rank of the four linears (SURVEY 8: qkv, o, gate_up, down)."""
+        """(N, K) per rank of the four linears (qkv, o, gate_up, down)."""
         D = self.head_dim
         hq, hkv = self.num_attention_heads // tp, max(self.num_key_value_heads // tp, 1)
         return {"qkv": ((hq + 2 * hkv) * D, self.hidden_size), "o": (self.hidden_size, hq * D),
@@ -81,7 +81,7 @@ class QSpecLlamaConfig:
 
 
 def random_int4_linear(N: int, K: int, seed: int, device, bias: bool = False) -> Linear4bit:
-    """Random-init packed weights + scales as SURVEY 8(d): q ~ U{-8..7}, sW = (0.5+U)*2^-7 (bias ~ N(0, 0.1^2))."""
+    """Random-init packed weights + scales: q ~ U{-8..7}, sW = (0.5+U)*2^-7 (bias ~ N(0, 0.1^2))."""
     device = torch.device(device)
     g = torch.Generator(device=device).manual_seed(seed)
     lin = Linear4bit(K, N, bias=False, dtype=torch.float16, device=device, empty_init=True)
@@ -152,7 +152,7 @@ class QSpecLlamaModel(torch.nn.Module):
         self.lm_head = (torch.randn(vs, cfg.hidden_size, generator=g2) * 0.02).to(torch.float16).to(self.device)
         self.vocab_shard = vs
         self.cos_sin = build_cos_sin_cache(D, cfg.max_seq_len, cfg.rope_theta, self.device)
-        # shard-local rotation scales (SURVEY 7 hard part 5): 1/sqrt(local heads), 1/sqrt(local inter), evaluated the way the
+        # shard-local rotation scales: 1/sqrt(local heads), 1/sqrt(local inter), evaluated the way the
         # reference's run time evaluates them (float16: nn.reference_hadamard_scale)
         self.scale_heads = reference_hadamard_scale(self.hq)
         if cfg.heads_rotation == "had40":
@@ -163,7 +163,7 @@ class QSpecLlamaModel(torch.nn.Module):
         L, S = cfg.num_hidden_layers, cfg.max_seq_len
         self.cache_k = torch.zeros(L, max_batch, S, self.hkv, D, dtype=torch.float16, device=self.device)
         self.cache_v = torch.zeros_like(self.cache_k)
-        # scratch arena, allocated once (SURVEY a11)
+        # scratch arena, allocated once
         T, H = max_tokens, cfg.hidden_size
         f16 = dict(dtype=torch.float16, device=self.device)
         i8 = dict(dtype=torch.int8, device=self.device)

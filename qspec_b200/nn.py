@@ -200,7 +200,7 @@ def get_matmul_op_w4a16(in_features, out_features, with_scaling=True, enable_tun
 
 
 # ----------------------------------------------------------------------------------------------
-# RMSNorm  (quarot_nn/normalization.py:5-82) -- mean-subtracting, no gamma (SURVEY 0.5)
+# RMSNorm  (quarot_nn/normalization.py:5-82) -- mean-subtracting, no gamma
 # ----------------------------------------------------------------------------------------------
 
 class RMSNorm(torch.nn.Module):

@@ -1,7 +1,7 @@
 """Tensor-level operators over the C-ABI library.
 
 The function names and argument meaning mirror the reference's native entry points
- so `quarot_nn`-style callers can switch by changing the import:
+so `quarot_nn`-style callers can switch by changing the import:
 
   layernorm_ops.rms_norm_general_fuse_sum_i4   third-party/kernels/csrc/layernorm.cpp:32-38
   layernorm_ops.rms_norm_general_fuse_sum_fp16 third-party/kernels/csrc/layernorm.cpp:40-42
@@ -205,7 +205,7 @@ def add_rms_norm_fuse_sum_fp16(out: torch.Tensor, x: torch.Tensor, delta: torch.
 def tp_two_step(peers, rows: int) -> bool:
     """Which form of the fused all-reduce an exchange of `rows` token rows uses -- a function of (rows, world) only, so every
     rank decides alike. Two-step (row r summed by rank r % world, pushed to the peers) when (world - 1) * rows >=
-    QSPEC_TP_SCATTER_MIN. OFF by default: measured on 8 x B200 (profiles/r02s_two_step_ab.md) the one-step form is not bound by
+    QSPEC_TP_SCATTER_MIN. OFF by default: measured on 8 x B200 the one-step form is not bound by
     the (world - 1) x rows x K x 2 bytes every rank reads but by the hand-over latency between GPUs, and the second hand-over of
     the two-step form costs more than its smaller traffic saves (TP = 8: -1 % on the 256-token verify exchanges alone, +10 % with
     the 64-token draft exchanges too; TP = 4: +4 %). Kept as a tested option for larger exchanges (prefill-sized passes)."""
@@ -454,7 +454,7 @@ def gemm_w4a16(x: torch.Tensor, weight: torch.Tensor, weight_scale: torch.Tensor
 
 
 # ---------------------------------------------------------------------------------------------
-# W4A8 mode (kwargs["w4a8"], off by default in the reference; SURVEY 8(f) rank 4)
+# W4A8 mode (kwargs["w4a8"], off by default in the reference)
 #   layernorm_ops.rms_norm_general_fuse_sum_i8   third-party/kernels/csrc/layernorm.cpp:44-50
 #   quarot._CUDA.fuse_sym_quant_i8               third-party/QuaRot/quarot/kernels/bindings.cpp:148-164
 #   rowwise_scaled_linear_cutlass_s8s4           torchao, as called at quarot_nn/linear.py:98

@@ -1,4 +1,4 @@
-"""Tensor-parallel sharding of the dual-mode layer (SURVEY 8(e)); host-side logic only.
+"""Tensor-parallel sharding of the dual-mode layer; host-side logic only.
 
 Column-parallel (qkv, gate_up): shard N; scales shard with N; no collective.
 Row-parallel (o, down): shard K (packed dim: k columns -> k/2 bytes); scales replicated; the
