@@ -1428,7 +1428,8 @@ static bool rows_faster(int mode, int M, int N, int K, const Plan& pl) {
 struct Known { int mode, M, N, K; size_t bytes; bool rows; };
 static Known known_size(int mode, int M, int N, int K) {
   static thread_local Known known[64];                        // (bytes 0: nothing known)
-  Known& k = known[((unsigned)N * 31u + (unsigned)K * 7u + (unsigned)M * 3u + (unsigned)mode) >> 3 & 63u];
+  // (sizes are multiples of large powers of two: the upper bits of a product tell them apart, the lower ones do not)
+  Known& k = known[((((unsigned)N * 0x9E3779B1u ^ (unsigned)K) * 0x9E3779B1u ^ ((unsigned)M << 2 | (unsigned)mode)) * 0x9E3779B1u) >> 26];
   if (!k.bytes || k.mode != mode || k.M != M || k.N != N || k.K != K) {
     const Plan pl = make_plan(mode, M, N, K);
     k = Known{mode, M, N, K, workspace_bytes(pl), rows_faster(mode, M, N, K, pl)};
