@@ -685,8 +685,8 @@ static int launch_k28_cluster(const void* x, const void* gu, void* of, int8_t* o
   cfg.gridDim = dim3((unsigned)rows * K28_CLUSTER);
   cfg.blockDim = dim3(128 * WPB);
   cfg.dynamicSmemBytes = (size_t)28 * n * sizeof(__half);
-  static SmemLimit limit;                              // n = 1024 needs 56 KB
-  QSPEC_CUDA(limit.raise(kern, 28 * 1024 * sizeof(__half)));
+  static SmemLimit limit;                              // n = 1024 needs 56 KB; below, 28 KB and up to 9 KB of static memory need no asking for
+  if (SLOTS == 4) QSPEC_CUDA(limit.raise(kern, 28 * 1024 * sizeof(__half)));
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
