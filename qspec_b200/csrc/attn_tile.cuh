@@ -62,6 +62,7 @@ struct Args {
   int min_run, ring, skip_outside;             // skip_outside: a token whose position is outside the cache is not stored
   void* out; long long out_ts; int out_hs;
   const float* sink; const void* gate; int gate_ld, gate_per_head; float out_scale;
+  uint32_t rep_inv;                            // set by launch(): r * rep_inv >> 16 = r / rep for r < 128
 };
 
 // Tokens t and t + 1 of the batch are of one run.
@@ -158,10 +159,17 @@ __device__ __forceinline__ void st32(uint32_t addr, const uint32_t* r) {
                "%25,%26,%27,%28,%29,%30,%31,%32};\n"
                ::"r"(addr), QSPEC_W8(r, 0), QSPEC_W8(r, 8), QSPEC_W8(r, 16), QSPEC_W8(r, 24) : "memory");
 }
+__device__ __forceinline__ void ld8(uint32_t addr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n" : QSPEC_R8(r, 0) : "r"(addr));
+}
 __device__ __forceinline__ void st16(uint32_t addr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(addr), QSPEC_W8(r, 0),
                QSPEC_W8(r, 8) : "memory");
 }
+#define QSPEC_T8(r, o) "+r"(r[o]), "+r"(r[o + 1]), "+r"(r[o + 2]), "+r"(r[o + 3]), "+r"(r[o + 4]), "+r"(r[o + 5]), "+r"(r[o + 6]), "+r"(r[o + 7])
+// Behind wait_ld(): nothing that is done with these registers is moved in front of it.
+__device__ __forceinline__ void landed8(uint32_t* r) { asm volatile("" : QSPEC_T8(r, 0)); }
+#undef QSPEC_T8
 #undef QSPEC_R8
 #undef QSPEC_W8
 __device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
@@ -173,23 +181,15 @@ __device__ __forceinline__ void unpair(uint64_t v, uint32_t& a, uint32_t& b) { a
 __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t r; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b)); return r; }
 
-// lead(): the leading bits of two weights (bits of float32, 0 <= weight < 2^15), rounded and packed, and their values; rest(): two
-// remainders, packed. Mostly on the integer units: the conversion instruction shares the special-function unit with the exponentials (with
-// conversions for both terms that unit was 95 % busy and the kernel waited for it). ZEROS: whether lead() and rest() give zero for a weight
-// of zero; lead_zero() does in any case.
+// lead(): the leading bits of two weights (bits of float32), rounded and packed, and their values; rest(): two remainders, packed. float16: conversions
+// (a scheduler issues one in two cycles; the integer form, seven instructions of which five take two, made a block of 128 keys 1.43 us instead of
+// 1.37). bfloat16: integer instructions, of which it takes few (with conversions for the remainders 1.53 us instead of 1.51).
 template <bool BF> struct Elem;
 template <> struct Elem<false> {
   using T = __half;
   static __device__ __forceinline__ uint32_t pack(float a, float b) { const __half2 h = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
   static __device__ __forceinline__ float2 unpack(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
-  static constexpr bool ZEROS = false;
-  // weights below 2^-14, the smallest normal number, give 2^-14: their remainder is negative
   static __device__ __forceinline__ uint32_t lead(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
-    h0 = __viaddmax_u32(p0, 0x1000u, 0x38800000u) & 0xffffe000u;
-    h1 = __viaddmax_u32(p1, 0x1000u, 0x38800000u) & 0xffffe000u;
-    return (h0 >> 13) + (h1 << 3) - 0xc001c000u;           // exponent bias 127 -> 15 in both halves
-  }
-  static __device__ __forceinline__ uint32_t lead_zero(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
     const uint32_t w = pack(__uint_as_float(p0), __uint_as_float(p1));
     const float2 f = unpack(w);
     h0 = __float_as_uint(f.x);
@@ -202,7 +202,6 @@ template <> struct Elem<true> {
   using T = __nv_bfloat16;
   static __device__ __forceinline__ uint32_t pack(float a, float b) { const __nv_bfloat162 h = __floats2bfloat162_rn(a, b); return *reinterpret_cast<const uint32_t*>(&h); }
   static __device__ __forceinline__ float2 unpack(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
-  static constexpr bool ZEROS = true;
   static __device__ __forceinline__ uint32_t lead(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) {
     p0 += 0x8000u;
     p1 += 0x8000u;
@@ -210,7 +209,6 @@ template <> struct Elem<true> {
     h1 = p1 & 0xffff0000u;
     return __byte_perm(p0, p1, 0x7632);
   }
-  static __device__ __forceinline__ uint32_t lead_zero(uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) { return lead(p0, p1, h0, h1); }
   static __device__ __forceinline__ uint32_t rest(uint32_t q0, uint32_t q1) { return __byte_perm(q0 + 0x8000u, q1 + 0x8000u, 0x7632); }   // rounded
 };
 
@@ -376,12 +374,11 @@ template <bool BF, bool QF32>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const Args a) {
   using T = typename Elem<BF>::T;
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
   extern __shared__ __align__(16) unsigned char at_raw[];
   __shared__ int pos[TOKENS_MAX], seq[TOKENS_MAX];
   __shared__ int s_rs[TOKENS_MAX], s_re[TOKENS_MAX];
   __shared__ uint32_t s_start[TOKENS_MAX / 32];
-  __shared__ __align__(8) uint64_t b_kfull[KS], b_kempty[KS], b_vfull[VS], b_vempty[VS], b_s[2], b_p[2][2], b_o, b_done, b_part, b_mx[4];
+  __shared__ __align__(8) uint64_t b_kfull[KS], b_kempty[KS], b_vfull[VS], b_vempty[VS], b_q, b_s[2], b_p[2][2], b_o, b_done, b_part, b_mx[4];
   __shared__ float s_mx[2][2][128];                         // [block & 1][half][row]
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_fail;
@@ -391,51 +388,23 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   const int kvh = blockIdx.x;
   const int n2 = min(tok, a.ntok - c0);
 
-  // ---- the runs among this CTA's tokens
-  bool start = false, end = false;
-  if (tid < TOKENS_MAX) {
-    bool before, after;
-    bool in = attn_in_run(a.pos, a.seq, a.ntok, c0 + warp * 32, a.min_run, before, after) && tid < n2;
-    if (a.seg && tid < n2) {
-      const int t = c0 + tid, s0 = a.seg[t], s1 = a.seg[a.ntok + t];
-      in = s1 - s0 >= a.min_run;
-      before = before && t > s0;
-      after = after && t + 1 < s1;
-    }
-    if (in) {
-      pos[tid] = a.pos[c0 + tid];
-      seq[tid] = a.seq[c0 + tid];
-      in = (unsigned)seq[tid] < (unsigned)a.nseq;
-    }
-    start = in && (tid == 0 || !before);
-    end = in && (tid == n2 - 1 || !after);
-    const uint32_t bits = __ballot_sync(0xffffffffu, start);
-    if (lane == 0) s_start[warp] = bits;
-  }
-  if (tid == 0) s_fail = 0;
-  __syncthreads();
-  int nruns = 0, before = 0;
-  for (int w = 0; w < TOKENS_MAX / 32; ++w) {
-    if (w < warp) before += __popc(s_start[w]);
-    nruns += __popc(s_start[w]);
-  }
-  if (nruns == 0) return;                                    // nothing for this form here
-  if (tid < TOKENS_MAX) {                                    // a run's end has as many starts at or before it as its start has
-    const int rank = before + __popc(s_start[warp] & ((2u << lane) - 1u)) - 1;
-    if (start) s_rs[rank] = tid;
-    if (end) s_re[rank] = tid;
-  }
+  // ---- what needs nothing from the kernel before
   if (warp == WARP_MMA) {
+    // (Kernels with tensor memory let their dependents start only when all their CTAs hold theirs: whoever this waits for goes on without it.)
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  if (tid == 0) {
+  if (tid == WARP_K * 32) {
+    asm volatile("prefetch.tensormap [%0];\n" ::"l"(&map_k) : "memory");
+    asm volatile("prefetch.tensormap [%0];\n" ::"l"(&map_v) : "memory");
+    s_fail = 0;
     for (int i = 0; i < KS; ++i) { bar_init(smem_addr(&b_kfull[i]), 1); bar_init(smem_addr(&b_kempty[i]), 1); }
     for (int i = 0; i < VS; ++i) { bar_init(smem_addr(&b_vfull[i]), 1); bar_init(smem_addr(&b_vempty[i]), 1); }
     for (int i = 0; i < 2; ++i) {
       bar_init(smem_addr(&b_s[i]), 1);
       bar_init(smem_addr(&b_p[i][0]), 8); bar_init(smem_addr(&b_p[i][1]), 4);
     }
+    bar_init(smem_addr(&b_q), WARP_K);
     bar_init(smem_addr(&b_o), 1);
     bar_init(smem_addr(&b_done), 1);
     bar_init(smem_addr(&b_part), 1);
@@ -444,27 +413,84 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   }
   const uint32_t base = (smem_addr(at_raw) + 1023u) & ~1023u;
   unsigned char* gbase = at_raw + (base - smem_addr(at_raw));
-  // ---- queries
-  for (int i = tid; i < 128 * 16; i += THREADS) {
-    const int r = i >> 4, c = i & 15, tl = r / rep;
-    uint4 val = make_uint4(0u, 0u, 0u, 0u);
-    if (r < tok * rep && tl < n2) {
-      const size_t o = (size_t)(c0 + tl) * a.q_ts + (size_t)(kvh * rep + r % rep) * a.q_hs + c * 8;
-      if (QF32) {
-        const float4 x = *reinterpret_cast<const float4*>((const float*)a.q + o), y = *reinterpret_cast<const float4*>((const float*)a.q + o + 4);
-        val = make_uint4(Elem<BF>::pack(x.x, x.y), Elem<BF>::pack(x.z, x.w), Elem<BF>::pack(y.x, y.y), Elem<BF>::pack(y.z, y.w));
-      } else {
-        val = *reinterpret_cast<const uint4*>((const T*)a.q + o);
-      }
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  // ---- the runs among this CTA's tokens
+  bool start = false, end = false;
+  if (tid < TOKENS_MAX) {
+    const int t = c0 + tid;
+    int p = 0, q = 0, s0 = 0, s1 = 0;
+    if (tid < n2) {
+      p = a.pos[t];
+      q = a.seq[t];
+      if (a.seg) { s0 = a.seg[t]; s1 = a.seg[a.ntok + t]; }
     }
-    *reinterpret_cast<uint4*>(gbase + (c >> 3) * HALF + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = val;
+    bool before, after;
+    bool in = attn_in_run(a.pos, a.seq, a.ntok, c0 + warp * 32, a.min_run, before, after) && tid < n2;
+    if (a.seg && tid < n2) {
+      in = s1 - s0 >= a.min_run;
+      before = before && t > s0;
+      after = after && t + 1 < s1;
+    }
+    if (in) {
+      pos[tid] = p;
+      seq[tid] = q;
+      in = (unsigned)q < (unsigned)a.nseq;
+    }
+    start = in && (tid == 0 || !before);
+    end = in && (tid == n2 - 1 || !after);
+    const uint32_t bits = __ballot_sync(0xffffffffu, start);
+    if (lane == 0) s_start[warp] = bits;
   }
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem = s_tmem;
+  int nruns = 0, before = 0;
+  for (int w = 0; w < TOKENS_MAX / 32; ++w) {
+    if (w < warp) before += __popc(s_start[w]);
+    nruns += __popc(s_start[w]);
+  }
+  if (nruns == 0) {                                          // nothing for this form here
+    if (warp == WARP_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
+    return;
+  }
+  // ---- queries: asked for here, stored while the first keys are on their way
+  constexpr int QP = 128 * 16 / (WARP_K * 32), QW = QF32 ? 2 : 1;   // 16-byte pieces of a thread; loads of each
+  uint4 qv[QP][QW];
+  if (warp < WARP_K) {
+#pragma unroll
+    for (int j = 0; j < QP; ++j) {
+      const int r = (tid >> 4) + j * (WARP_K * 2), tl = (int)(r * a.rep_inv >> 16);
+      const size_t o = (size_t)(c0 + min(tl, n2 - 1)) * a.q_ts + (size_t)(kvh * rep + r - tl * rep) * a.q_hs + (tid & 15) * 8;   // (rows of no token: any)
+#pragma unroll
+      for (int e = 0; e < QW; ++e) qv[j][e] = *reinterpret_cast<const uint4*>((const unsigned char*)a.q + o * (QF32 ? 4 : 2) + e * 16);
+    }
+  }
+  if (tid < TOKENS_MAX) {                                    // a run's end has as many starts at or before it as its start has
+    const int rank = before + __popc(s_start[warp] & ((2u << lane) - 1u)) - 1;
+    if (start) s_rs[rank] = tid;
+    if (end) s_re[rank] = tid;
+  }
+  __syncthreads();
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // tensor memory is held: a dependent that waits for this grid cannot take it first
+
+  if (warp < WARP_K) {
+#pragma unroll
+    for (int j = 0; j < QP; ++j) {
+      const int r = (tid >> 4) + j * (WARP_K * 2), c = tid & 15, tl = (int)(r * a.rep_inv >> 16);
+      uint4 val = qv[j][0];
+      if (QF32) {
+        const uint4 y = qv[j][QW - 1];
+        val = make_uint4(Elem<BF>::pack(__uint_as_float(val.x), __uint_as_float(val.y)), Elem<BF>::pack(__uint_as_float(val.z), __uint_as_float(val.w)),
+                         Elem<BF>::pack(__uint_as_float(y.x), __uint_as_float(y.y)), Elem<BF>::pack(__uint_as_float(y.z), __uint_as_float(y.w)));
+      }
+      if (tl >= n2 || r >= tok * rep) val = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(gbase + (c >> 3) * HALF + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = val;
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncwarp();
+    if (lane == 0) bar_arrive(smem_addr(&b_q));
+  }
 
   Items items{s_rs, s_re, pos, seq, nruns, a.window, a.ring ? 0x7fffffff - 256 : a.cap - 1, a.ring ? a.cap : 0};
   Item it;
@@ -491,7 +517,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         if (++ks == KS) { ks = 0; kphase ^= 1u; }
         return true;
       };
-      bool ok = blocks == 0 || scores(0), over = blocks == 0;
+      bool ok = blocks == 0 || (bar_wait(smem_addr(&b_q), 0, &s_fail) && scores(0)), over = blocks == 0;
       for (uint32_t n = 0; ok && n < blocks; ++n) {
         if (n + 1 < blocks && !scores(n + 1)) break;
         if (!bar_wait(smem_addr(&b_vfull[n % VS]), (n / VS) & 1, &s_fail)) break;
@@ -568,13 +594,14 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   } else if (warp < WARP_K) {
     // ---- softmax: thread = 64 columns (half h) of row r
     const int h = warp >> 2, r = (warp & 3) * 32 + lane;
-    const int tl = r / rep, head = kvh * rep + r % rep;
+    const int tl = (int)(r * a.rep_inv >> 16), head = kvh * rep + r - tl * rep;
     const bool row_in = r < tok * rep && tl < n2;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t ot = tmem + lanes + 256 + h * 64;
     const uint32_t bmx = smem_addr(&b_mx[warp & 3]);
     const float c2 = a.scale * 1.4426950408889634f;
     const int last = a.ring ? 0x7fffffff : a.cap - 1;
+    const float sink = a.sink && row_in ? a.sink[head] * 1.4426950408889634f : 0.f;
     float m = -INFINITY, l = 0.f;                             // maximum in units of log2; sum of this half's weights relative to it
     int n = 0, my_lo = 0, my_hi = -1, my_seq = 0;
     bool ok = true, mine = false;
@@ -653,28 +680,24 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       const uint64_t minus2 = pair(0xbf800000u, 0xbf800000u);
       uint64_t l2[2] = {0ull, 0ull};
       // weight = hi + lo: hi = the leading bits that the type keeps, rounded, lo = the rest, rounded
-      auto weights = [&](auto lead) {
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          uint32_t hi[16], lo[16];
+      for (int g = 0; g < 2; ++g) {
+        uint32_t hi[16], lo[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            uint32_t p0, p1, h0, h1, q0, q1;
-            unpair(fma2(pair(x[g * 32 + 2 * j], x[g * 32 + 2 * j + 1]), c22, mu2), p0, p1);
-            p0 = __float_as_uint(ex2(__uint_as_float(p0)));
-            p1 = __float_as_uint(ex2(__uint_as_float(p1)));
-            const uint64_t pp = pair(p0, p1);
-            l2[j & 1] = add2(l2[j & 1], pp);
-            hi[j] = lead(p0, p1, h0, h1);
-            unpair(fma2(pair(h0, h1), minus2, pp), q0, q1);
-            lo[j] = Elem<BF>::rest(q0, q1);
-          }
-          st16(st + g * 16, hi);
-          st16(st + 32 + g * 16, lo);
+        for (int j = 0; j < 16; ++j) {
+          uint32_t p0, p1, h0, h1, q0, q1;
+          unpair(fma2(pair(x[g * 32 + 2 * j], x[g * 32 + 2 * j + 1]), c22, mu2), p0, p1);
+          p0 = __float_as_uint(ex2(__uint_as_float(p0)));
+          p1 = __float_as_uint(ex2(__uint_as_float(p1)));
+          const uint64_t pp = pair(p0, p1);
+          l2[j & 1] = add2(l2[j & 1], pp);
+          hi[j] = Elem<BF>::lead(p0, p1, h0, h1);
+          unpair(fma2(pair(h0, h1), minus2, pp), q0, q1);
+          lo[j] = Elem<BF>::rest(q0, q1);
         }
-      };
-      if (Elem<BF>::ZEROS || plain) weights([](uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) { return Elem<BF>::lead(p0, p1, h0, h1); });
-      else weights([](uint32_t p0, uint32_t p1, uint32_t& h0, uint32_t& h1) { return Elem<BF>::lead_zero(p0, p1, h0, h1); });   // some are hidden
+        st16(st + g * 16, hi);
+        st16(st + 32 + g * 16, lo);
+      }
       wait_st();
       fence_before();
       __syncwarp();
@@ -686,7 +709,26 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       }
       ++n;
     }
-    // ---- the last product is done: add the halves' sums, divide, gate, store
+    // ---- the last product is done: add the halves' sums, divide, gate, store. Rows leave through shared memory, eight lanes a row: a lane per row
+    // touched 32 rows with every instruction (2 us a tile, 5 with a gate's loads). The loops are short: what runs once per tile runs at the speed at
+    // which its instructions are fetched. This, and queries that are on their way beside the first keys: 1000 tokens after 1000,
+    // 32 / 8 heads 63.5 -> 56.5 us, window of 1024, 2000 tokens, 16 / 4 heads, with gate and sink 66.8 -> 55.5.
+    const int pc8 = lane & 7;                                 // this lane's rows of the warp's 32 are lane / 8 + 4 k, its eight columns of 64 from 8 pc8 on
+    auto row_at = [&](int k, size_t ts, int hs) {             // where that row's half lies in a [token][head][..] tensor
+      const int rr = (warp & 3) * 32 + (lane >> 3) + 4 * k, t = (int)(rr * a.rep_inv >> 16);
+      return (size_t)(c0 + min(t, n2 - 1)) * ts + (size_t)(kvh * rep + rr - t * rep) * hs + h * 64 + pc8 * 8;
+    };
+    constexpr int LD = 68;                                    // floats of a row, so that neither side meets bank conflicts
+    float* const rows = reinterpret_cast<float*>(gbase) + warp * 32 * LD;   // (queries and keys are done with, the gates lie behind the rows)
+    unsigned char* const gates = gbase + 3 * TILE + warp * 4096;
+    static_assert(8 * 32 * LD * 4 <= 3 * TILE && 8 * 4096 <= TILE && KS >= 3, "rows and gates on their way");
+    const bool gate = a.gate && !a.gate_per_head && ok;
+    if (gate) {
+#pragma unroll 1
+      for (int k = 0; k < 8; ++k)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(gates + k * 512 + lane * 16)), "l"((const T*)a.gate + row_at(k, a.gate_ld, a.out_hs)) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
     // (A barrier of its own: a warp may get here two products ahead, where the parity of b_o's phase n - 3 reads like that of n - 1.)
     if (ok && n) ok = bar_wait(smem_addr(&b_done), 0, &s_fail);
     ok = __all_sync(0xffffffffu, ok);
@@ -712,47 +754,57 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     if (!dead) {
       float mm = m, ls = l;
       if (a.sink && row_in) {
-        const float s2 = a.sink[head] * 1.4426950408889634f;
-        mm = fmaxf(m, s2);
-        ls = l * ex2(m - mm) + ex2(s2 - mm);
+        mm = fmaxf(m, sink);
+        ls = l * ex2(m - mm) + ex2(sink - mm);
       }
       f = ex2(m - mm) / ls * a.out_scale;
     }
     if (a.gate && a.gate_per_head && store)
       f *= __fdividef(1.f, 1.f + __expf(-(float)((const T*)a.gate)[(size_t)(c0 + tl) * a.gate_ld + head]));
-    T* dst = (T*)a.out + (size_t)(c0 + tl) * a.out_ts + (size_t)head * a.out_hs + h * 64;
-    const T* gt = a.gate && !a.gate_per_head ? (const T*)a.gate + (size_t)(c0 + tl) * a.gate_ld + (size_t)head * a.out_hs + h * 64 : nullptr;
-    uint64_t bad = 0;                                         // columns that are not finite
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     if (ok) {
+      float spoilt = 0.f;                                     // not a number where a column is not finite
 #pragma unroll 1
-      for (int q = 0; q < 2; ++q) {
-        uint32_t o[32], low[32];
-        ld32(ot + q * 32, o);
-        ld32(ot + 128 + q * 32, low);
+      for (int q = 0; q < 8; ++q) {
+        uint32_t o[8], low[8];
+        ld8(ot + q * 8, o);
+        ld8(ot + 128 + q * 8, low);
         wait_ld();
-        if (store) {
+        landed8(o);
+        landed8(low);
+        float v[8];
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            float v[8];
+        for (int e = 0; e < 8; ++e) {
+          v[e] = dead ? none : (__uint_as_float(o[e]) + __uint_as_float(low[e])) * f;
+          spoilt = fmaf(v[e], 0.f, spoilt);
+        }
+        *reinterpret_cast<float4*>(rows + lane * LD + q * 8) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(rows + lane * LD + q * 8 + 4) = make_float4(v[4], v[5], v[6], v[7]);
+      }
+      const uint32_t stored = __ballot_sync(0xffffffffu, store);   // (and the rows are there; every lane reads the gates that it asked for)
+#pragma unroll 1
+      for (int k = 0; k < 8; ++k) {
+        const int rr = (lane >> 3) + 4 * k;
+        const float4 x = *reinterpret_cast<const float4*>(rows + rr * LD + pc8 * 8), y = *reinterpret_cast<const float4*>(rows + rr * LD + pc8 * 8 + 4);
+        float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        if (gate) {
+          const uint4 gw = *reinterpret_cast<const uint4*>(gates + k * 512 + lane * 16);
+          const uint32_t ww[4] = {gw.x, gw.y, gw.z, gw.w};
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              v[e] = dead ? none : (__uint_as_float(o[g * 8 + e]) + __uint_as_float(low[g * 8 + e])) * f;
-              if (!(fabsf(v[e]) < INFINITY)) bad |= 1ull << (q * 32 + g * 8 + e);
-            }
-            if (gt) {
-              const uint4 gw = *reinterpret_cast<const uint4*>(gt + q * 32 + g * 8);
-              const uint32_t ww[4] = {gw.x, gw.y, gw.z, gw.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 z = Elem<BF>::unpack(ww[e]);
-                v[2 * e] *= __fdividef(1.f, 1.f + __expf(-z.x));
-                v[2 * e + 1] *= __fdividef(1.f, 1.f + __expf(-z.y));
-              }
-            }
-            *reinterpret_cast<uint4*>(dst + q * 32 + g * 8) =
-                make_uint4(Elem<BF>::pack(v[0], v[1]), Elem<BF>::pack(v[2], v[3]), Elem<BF>::pack(v[4], v[5]), Elem<BF>::pack(v[6], v[7]));
+          for (int e = 0; e < 4; ++e) {
+            const float2 z = Elem<BF>::unpack(ww[e]);
+            v[2 * e] *= __fdividef(1.f, 1.f + __expf(-z.x));
+            v[2 * e + 1] *= __fdividef(1.f, 1.f + __expf(-z.y));
           }
         }
+        if (stored >> rr & 1)
+          *reinterpret_cast<uint4*>((T*)a.out + row_at(k, a.out_ts, a.out_hs)) =
+              make_uint4(Elem<BF>::pack(v[0], v[1]), Elem<BF>::pack(v[2], v[3]), Elem<BF>::pack(v[4], v[5]), Elem<BF>::pack(v[6], v[7]));
+      }
+      uint64_t bad = 0;                                       // columns that are not finite
+      if (__any_sync(0xffffffffu, !(spoilt == 0.f) && store)) {
+        for (int q = 0; q < 64; ++q)
+          if (!(fabsf(rows[lane * LD + q]) < INFINITY)) bad |= 1ull << q;
       }
       // (a sum of weights that is not a number makes every column so: nothing to do again)
       const uint32_t again = __ballot_sync(0xffffffffu, bad != 0 && store && !dead && l == l);
@@ -807,7 +859,8 @@ inline int cache_map(CUtensorMap* map, const void* p, long long ss, int rs, int 
 }
 
 template <bool BF, bool QF32>
-inline int launch(const Args& a, int kv_heads, cudaStream_t stream) {
+inline int launch(Args a, int kv_heads, cudaStream_t stream) {
+  a.rep_inv = (65536u + (uint32_t)a.rep - 1u) / (uint32_t)a.rep;   // (rep <= 64: the quotient is off by less than 128 / 65536, which no r reaches the next one by)
   auto kern = attn_tile_kernel<BF, QF32>;
   static SmemLimit limit;
   QSPEC_CUDA(limit.raise(kern, SMEM));
