@@ -204,7 +204,7 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory");
 }
 constexpr uint64_t POLICY_EVICT_NORMAL = 0x1000000000000000ull;
-constexpr uint64_t POLICY_EVICT_FIRST = 0x12F0000000000000ull;   // streamed-once weights
+constexpr uint64_t POLICY_EVICT_FIRST = 0x12F0000000000000ull;   // weights that are streamed once
 constexpr uint64_t POLICY_EVICT_LAST = 0x14F0000000000000ull;    // activations re-read by every CTA
 
 // K-major SWIZZLE_128B shared-memory matrix descriptor (see cute::UMMA::SmemDescriptor):
@@ -499,10 +499,15 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   auto step_unit = [&]() {
     if (++kb == KB) { kb = 0; if (++tile_m == p.tiles_m) { tile_m = 0; ++tile_n; } }
   };
+  // Weights are read once, or, by a CTA whose range is longer than a tile, once for every token tile: with three and more of these they stay in L2. W4A16, 1999
+  // tokens, 10240 x 8192: 590 MB came from memory for 75, and the GPU runs at its power limit there: 318 -> 296 us; 509 tokens, 28672 x 4096: 117 -> 112.
+  // Two token tiles gain nothing (256 tokens, 28672 x 4096: 63.4 | 63.8), nor do ranges within a tile, which other CTAs read at the same time
+  // (509 tokens, 4096 x 14336: 54.0 | 54.7).
+  const uint64_t w_policy = (LONG && p.tiles_m > 2) || (p.debug_exit & 16) ? POLICY_EVICT_NORMAL : POLICY_EVICT_FIRST;
   auto load_w = [&](int s) {
     if (elect_one()) {
       mbar_expect_tx(smem_u32(&w_full[s]), stage_tx);
-      tma_load_2d(smem_u32(sm_w + (size_t)s * W_STAGE), &map_w, kb * UB, ptile(tile_n) * TM, smem_u32(&w_full[s]), (p.debug_exit & 16) ? POLICY_EVICT_NORMAL : POLICY_EVICT_FIRST);
+      tma_load_2d(smem_u32(sm_w + (size_t)s * W_STAGE), &map_w, kb * UB, ptile(tile_n) * TM, smem_u32(&w_full[s]), w_policy);
     }
     __syncwarp();
   };
