@@ -263,6 +263,9 @@ int qspec_seq_lightning(const void* p, int ld, const float* decay, const float* 
  * with more segments and heads than the walk leaves room for), as they are without a workspace or without seg_starts. */
 size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV);
 size_t qspec_seq_lightning_chunk_bytes(int nseg, int ntok, int H, int D, int DV);
+/* What qspec_seq_hgrn2_chunked takes of this element type: bfloat16 rows (16-byte boundaries, ld a multiple of 8) go to a form on the tensor cores,
+ * which takes shorter segments too. With the smaller workspace of qspec_seq_recurrence_chunk_bytes they go where float32 rows go. */
+size_t qspec_seq_hgrn2_chunk_bytes(int nseg, int ntok, int H, int D, int DV, int dtype);
 int qspec_seq_hgrn2_chunked(const void* p, int ld, const float* f_b, const float* lower, const float* norm_w, float* state,
                             float* scratch, void* out, const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D,
                             int DV, float eps, int dtype, void* workspace, size_t workspace_bytes, void* stream);

@@ -156,6 +156,7 @@ SEQ_SIGNATURES = {
     "qspec_seq_attn_tile_timeouts": (c_int, []),
     "qspec_seq_recurrence_chunk_bytes": (c_size_t, [c_int] * 5),
     "qspec_seq_lightning_chunk_bytes": (c_size_t, [c_int] * 5),
+    "qspec_seq_hgrn2_chunk_bytes": (c_size_t, [c_int] * 6),
     "qspec_seq_hgrn2_chunked": (c_int, [c_void_p, c_int] + [c_void_p] * 8 + [c_int] * 5 + [c_float, c_int, c_void_p, c_size_t, c_void_p]),
     "qspec_seq_lightning_chunked": (c_int, [c_void_p, c_int] + [c_void_p] * 7 + [c_int] * 5 + [c_float, c_int, c_void_p, c_size_t, c_void_p]),
     "qspec_seq_window_attention_mma_supported": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int]),

@@ -32,7 +32,7 @@ def _nvcc() -> str:
 
 
 def _newest_source_mtime(sources=None) -> float:
-    names = [f for f in os.listdir(CSRC) if f != "fast_call.cpp"] if sources is None else list(sources) + ["common.cuh", "seq_common.cuh", "attn_tile.cuh", "gemm_w4_rows.cuh", "smem_limit.h"]
+    names = [f for f in os.listdir(CSRC) if f != "fast_call.cpp"] if sources is None else list(sources) + ["common.cuh", "seq_common.cuh", "attn_tile.cuh", "gemm_w4_rows.cuh", "recurrence_mma.cuh", "smem_limit.h"]
     paths = [os.path.join(CSRC, f) for f in names]
     paths.append(os.path.join(HERE, "..", "include", "qspec_b200.h"))
     paths.append(os.path.join(HERE, "..", "include", "qspec_b200_seq.h"))

@@ -822,6 +822,10 @@ recurrence_carry_kernel(float* __restrict__ E, const float* __restrict__ P, cons
   }
 }
 
+}  // namespace qspec
+#include "recurrence_mma.cuh"
+namespace qspec {
+
 // Per-head unit-RMS norm with one weight vector shared by the heads: one warp per (token, head); src float32.
 template <typename T>
 __global__ void __launch_bounds__(128)
@@ -1072,6 +1076,47 @@ static int launch_recurrence_chunks(const void* p, int ld, const float* gates, f
 #undef RC_ARGS
 }
 
+// ---- the gated recurrence of bfloat16 rows on the tensor cores (recurrence_mma.cuh) ----
+// Tokens of a chunk: as many as let the chunks of all heads fill the GPU once, at least two blocks. 0: these sizes are not taken.
+// Three launches and the first blocks take what the walk (launch_hgrn2 without a workspace) takes for 130 tokens, so it keeps short segments. Estimates,
+// us: here 31 (25 where a head's state is smaller than 128 x 128) and 2.5 for 1000 tokens of a head; the walk 8 and 0.18 (0.13) a token of a segment,
+// more where its CTAs (a segment, a head, 16 columns each) fill the GPU several times over. Measured, walk | here, 128 x 128, segments x tokens x heads:
+// 1 x 100 x 16 27 | 35, 1 x 150 x 32 38 | 41, 5 x 60 x 16 40 | 45, 2 x 150 x 32 70 | 55, 1 x 300 x 16 60 | 39, 5 x 300 x 16 175 | 104; 64 x 64, 1 x 300 x 16
+// 46 | 28, 2 x 33 x 8 15 | 20. The form of float32 rows: 1 x 1500 x 16, 128 x 128 143 | 93, 1 x 600 x 8, 64 x 64 40 | 28.
+static int rm_chunk_tokens(int nseg, int ntok, int H, int D, int DV) {
+  if (!((D == 64 || D == 128) && (DV == 64 || DV == 128)) || nseg < 1 || ntok < nseg || sm_count() < 1) return 0;
+  const bool large = D * DV == 128 * 128;
+  const double walkers = (double)nseg * H * (DV / 16) / 210;
+  const double walk = 8 + (large ? 0.18 : 0.13) * ((double)ntok / nseg) * (walkers > 1 ? walkers : 1);
+  if ((large ? 31 : 25) + 0.0025 * ntok * H * (D * DV / 16384.0) > walk) return 0;
+  const long long slots = (long long)sm_count() * (DV == 128 ? 2 : 4);
+  const long long c = (((long long)ntok * H + slots - 1) / slots + rmma::BT - 1) / rmma::BT * rmma::BT;
+  return (int)(c < 2 * rmma::BT ? 2 * rmma::BT : c);
+}
+static size_t rm_bytes(int nseg, int ntok, int H, int D, int DV) {
+  const int C = ntok < 1 || H < 1 || D < 1 || DV < 1 ? 0 : rm_chunk_tokens(nseg, ntok, H, D, DV);
+  return C ? (size_t)(ntok / C + nseg) * H * ((size_t)D * DV + D) * sizeof(float) : 0;
+}
+template <int D, int DV>
+static int launch_rm_d(rmma::Args a, cudaStream_t st) {
+  const int chunks = a.ntok / a.C + a.nseg;
+  using Sh = rmma::Shape<D, DV>;
+  constexpr size_t smem_e = rmma::smem_bytes<D, DV, false>(), smem_o = rmma::smem_bytes<D, DV, true>();
+  static SmemLimit limit_e, limit_o;
+  QSPEC_CUDA(limit_e.raise(rmma::chunk_kernel<D, DV, false>, smem_e));
+  QSPEC_CUDA(limit_o.raise(rmma::chunk_kernel<D, DV, true>, smem_o));
+  a.P = a.E + (size_t)chunks * a.H * D * DV;
+  if (a.ntok - a.nseg + 1 > a.C) {                            // a segment may be longer than a chunk
+    launch_pdl(rmma::chunk_kernel<D, DV, false>, dim3(chunks, a.H), dim3(Sh::THREADS), smem_e, st, a);
+    QSPEC_CHECK_LAUNCH(1);
+    launch_pdl(rmma::carry_kernel<D, DV>, dim3(a.nseg, a.H, D * DV / 1024), dim3(256), 0, st, a);
+    QSPEC_CHECK_LAUNCH(1);
+  }
+  launch_pdl(rmma::chunk_kernel<D, DV, true>, dim3(chunks, a.H), dim3(Sh::THREADS), smem_o, st, a);
+  QSPEC_CHECK_LAUNCH(1);
+  return QSPEC_OK;
+}
+
 template <typename T>
 static int launch_hgrn2(const void* p, int ld, const float* f_b, const float* lower, float* state, float* o, float* gates, const int* meta,
                         const int* seg_starts, int nseg, int ntok, int H, int D, int DV, cudaStream_t st, const float* decay, void* ws, void* out,
@@ -1100,6 +1145,10 @@ static size_t rc_bytes(int nseg, int ntok, int H, int D, int DV, bool scalar_dec
 }
 
 extern "C" size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV) { return rc_bytes(nseg, ntok, H, D, DV, false); }
+extern "C" size_t qspec_seq_hgrn2_chunk_bytes(int nseg, int ntok, int H, int D, int DV, int dtype) {
+  const size_t walk = rc_bytes(nseg, ntok, H, D, DV, false), mma = dtype == QSPEC_DTYPE_BF16 ? rm_bytes(nseg, ntok, H, D, DV) : 0;
+  return walk > mma ? walk : mma;                             // (rows that are not on 16-byte boundaries take the other form)
+}
 extern "C" size_t qspec_seq_lightning_chunk_bytes(int nseg, int ntok, int H, int D, int DV) { return rc_bytes(nseg, ntok, H, D, DV, true); }
 
 // The chunk form's buffer, if these sizes take it and the caller brought one that fits (rows are read 16 bytes at a time).
@@ -1120,6 +1169,15 @@ extern "C" int qspec_seq_hgrn2_chunked(const void* p, int ld, const float* f_b, 
   if (ntok == 0) return QSPEC_OK;
   cudaStream_t st = (cudaStream_t)stream;
   void* ws = chunk_workspace(workspace, workspace_bytes, seg_starts, nseg, ntok, H, D, DV, scratch, state, false);
+  if (dtype == QSPEC_DTYPE_BF16 && seg_starts && workspace && ld % 8 == 0 && (((uintptr_t)p | (uintptr_t)workspace) & 15) == 0 && ((uintptr_t)out & 3) == 0) {
+    const size_t need = rm_bytes(nseg, ntok, H, D, DV);
+    if (need && workspace_bytes >= need) {
+      const rmma::Args a{(const bf16_t*)p, ld, f_b, lower, (float*)workspace, nullptr, state, (bf16_t*)out, norm_w, eps, meta, seg_starts, nseg, ntok, H,
+                         rm_chunk_tokens(nseg, ntok, H, D, DV)};
+      if (D == 128) return DV == 128 ? launch_rm_d<128, 128>(a, st) : launch_rm_d<128, 64>(a, st);
+      return DV == 128 ? launch_rm_d<64, 128>(a, st) : launch_rm_d<64, 64>(a, st);
+    }
+  }
   float* gates = scratch + (size_t)ntok * H * DV;          // scratch: un-normalised outputs, then the gates
   int s = dtype == QSPEC_DTYPE_F32
               ? launch_hgrn2<float>(p, ld, f_b, lower, state, scratch, gates, meta, seg_starts, nseg, ntok, H, D, DV, st, nullptr, ws, out, norm_w, eps)

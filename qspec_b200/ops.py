@@ -1175,10 +1175,10 @@ def seq_window_attention_mma(q: torch.Tensor, cache_k: torch.Tensor, k_shared: O
          "seq_window_attention_mma")
 
 
-def _chunk_workspace(need, nseg: int, ntok: int, H: int, D: int, DV: int, device) -> Optional[torch.Tensor]:
+def _chunk_workspace(need, nseg: int, ntok: int, H: int, D: int, DV: int, device, *dtype: int) -> Optional[torch.Tensor]:
     """Room for the states between the chunks of a recurrence over long segments: of the call's own (the caching allocator ties it to
     the current stream), so that calls on several streams do not meet in it."""
-    nbytes = need(nseg, ntok, H, D, DV) if nseg else 0
+    nbytes = need(nseg, ntok, H, D, DV, *dtype) if nseg else 0
     return torch.empty(nbytes, dtype=torch.uint8, device=device) if nbytes else None
 
 
@@ -1196,7 +1196,7 @@ def seq_hgrn2(p: torch.Tensor, f_b: torch.Tensor, lower: torch.Tensor, norm_w: t
             or f_b.numel() != H * D or lower.numel() != H * D:
         raise ValueError("seq_hgrn2: shapes do not match")
     lib, nseg = _lib.load_seq(), 0 if seg_starts is None else seg_starts.numel()
-    ws = _chunk_workspace(lib.qspec_seq_recurrence_chunk_bytes, nseg, ntok, H, D, DV, p.device)
+    ws = _chunk_workspace(lib.qspec_seq_hgrn2_chunk_bytes, nseg, ntok, H, D, DV, p.device, _sdt(p))
     _seq(lib.qspec_seq_hgrn2_chunked(_ptr(p), p.shape[1], _ptr(f_b), _ptr(lower), _ptr(norm_w), _ptr(state), _ptr(scratch), _ptr(out),
                                      _ptr(meta), _ptr(seg_starts), nseg, ntok, H, D, DV, float(eps), _sdt(p), _ptr(ws),
                                      0 if ws is None else ws.numel(), _stream()), "seq_hgrn2")
