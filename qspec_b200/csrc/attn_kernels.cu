@@ -558,13 +558,14 @@ static int launch_attn_block(const void* qkv, const void* cos_sin, const int* po
 //   * 16 query rows per chunk = R tokens x G heads (R = 16 / G). In passes of up to SEQ_CHUNKS tokens a CTA takes one chunk, so that a
 //     prompt portion spreads over the GPU as well as many sequences do, in one launch. The 4 or 8 warps split the keys; every warp runs a
 //     flash-decoding loop over 16-key blocks with an online softmax, then the warps' (max, sum, O) are merged in shared memory.
-//   * Keys and values come by bulk copies, one per 256-byte row, into a ring of ST 16-key blocks per warp: a block's successor in its place
+//   * Keys and values come by asynchronous copies, 16 lanes a row, into a ring of ST 16-key blocks per warp: a block's successor in its place
 //     is asked for as soon as its keys (values) are multiplied. Loaded straight into the fragments, 16-byte pieces of 32 different sectors
-//     per instruction kept the L1 at 71 % and a warp waited for every block; prefetching into the L2 made that slower. ST = 1 leaves room for
+//     per instruction kept the L1 at 71 % and a warp waited for every block; bulk copies, one per 256-byte row, take their operands from uniform
+//     registers, so that a warp issues its lanes' one after the other: more instructions than the rest of a block's work. ST = 1 leaves room for
 //     four CTAs per SM, so that 64 sequences x 8 heads fit the GPU at once; ST = 2 (two CTAs) is for fewer, whose loads have to hide behind
-//     their own work, with eight warps per CTA instead of four once an SM each is left for them (us; before = loads into the fragments;
-//     32 query heads): 64 x 4 tokens after 900 51 (ST 2: 61; before: 54), 20 x 4 after 2000 69 (ST 1: 73; before: 88), 33 x 1 after 1000
-//     39 (41; 50), 8 x 5 after 1900 72 (ST 1: 125, ST 2 with four warps: 118; before: 104).
+//     their own work, with eight warps per CTA instead of four once an SM each is left for them. us, 32 query heads, bulk copies -> now (the other
+//     forms now: ST 2 with eight warps, ST 2, ST 1): 64 x 4 tokens after 900 50.3 -> 43.3 (55, 43, 43), 64 x 1 after 100 10.9 -> 10.5 (23, 14, 10), 20 x 4
+//     after 2000 69 -> 37 (40, 37, 47), 33 x 1 after 1000 37 -> 23 (30, 23, 33), 8 x 5 after 1900 34 -> 22 (22, 30, 37), 16 x 4 after 500 13.8 -> 11.6 (12, 15, 21).
 //     The rows are padded so that the fragment reads are free of bank conflicts, and the fragments are met without a transposition by
 //     permuting the reduction index (QK^T: lane (gid, tig) takes dims [32 i + 8 tig, + 8), i < 4, of key row gid -- both operands use the same
 //     permutation) and the output index (P.V: n-tiles t and 8 + t of lane gid are dims 8 gid + t and 64 + 8 gid + t).
@@ -605,8 +606,6 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   __shared__ int s_ntok, s_seq;
   __shared__ float s_m[NW][16], s_l[NW][16];
   __shared__ __align__(16) uint4 s_qf[8][32];                // Q fragments of the chunk in mma order: [k-step][lane] = (a0, a1, a2, a3)
-  __shared__ __align__(8) uint64_t s_full[NW][2][ST];         // keys, values of a warp's blocks
-  __shared__ volatile int s_fail;                            // a bounded wait ran out: NaN is stored
   extern __shared__ __align__(16) unsigned char seq_dyn[];   // [NW][ST] blocks; after the keys:
   constexpr int OS = D + 4;                                  // (row stride of the partial outputs: the rows of a store fall on different banks)
   float (*s_o)[16][OS] = reinterpret_cast<float (*)[16][OS]>(seq_dyn);   // [NW][16][OS] fp32: per-warp partial outputs
@@ -614,14 +613,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   const int hk = blockIdx.x % Hkv;                            // the heads of a sequence side by side: their rows are neighbours in the cache
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
-  if (tid == 0) {
-    s_ntok = 0;
-    s_fail = 0;
-  }
-  if (tid < NW * 2 * ST) {
-    atile::bar_init(atile::smem_addr(&s_full[0][0][0] + tid), 1);
-    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-  }
+  if (tid == 0) s_ntok = 0;
   if (T <= SEQ_CHUNKS) {
     // chunk c of the pass: R tokens of one sequence, in batch order; the chunks are numbered by their first tokens
     const int chunk = seq;
@@ -696,23 +688,26 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   const __half* vbase = cache_v + ((size_t)seq * S * Hkv + hk) * D;
   const size_t kv_stride = (size_t)Hkv * D;                  // elements between consecutive positions
   unsigned char* ring = seq_dyn + (size_t)warp * ST * SEQ_BLOCK;   // this warp's blocks: 16 key rows, 16 value rows each
-  uint32_t blocks = 0;                                       // blocks this warp has consumed: place and phase in the ring
-  // rows kb .. of the keys or of the values into place `at` of the ring, one row per lane
-  auto fetch = [&](bool values, uint32_t at, int kb, int nkeys) {
-    const uint32_t bar = atile::smem_addr(&s_full[warp][values][at]);
-    const int n = min(16, nkeys - kb);
-    if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"((uint32_t)n * 256u) : "memory");
-    __syncwarp();
-    if (lane < n)
-      bulk_row_256(atile::smem_addr(ring) + at * SEQ_BLOCK + (values ? 16 * SEQ_KS + lane * SEQ_VS : lane * SEQ_KS),
-                   (values ? vbase : kbase) + (size_t)(kb + lane) * kv_stride, bar);
+  // rows kb .. of the keys or of the values into place `at` of the ring: 16 lanes a row, zeros past the last key (weights there are zero, values must be
+  // finite). A group of its own, empty without rows, so that what is under way can be counted.
+  auto fetch = [&](bool values, int at, int kb, int nkeys) {
+    const int pitch = values ? SEQ_VS : SEQ_KS, r0 = lane >> 4, n = nkeys - kb;
+    uint32_t dst = atile::smem_addr(ring) + at * SEQ_BLOCK + (values ? 16 * SEQ_KS : 0) + r0 * pitch + (lane & 15) * 16;
+    const __half* src = (values ? vbase : kbase) + (size_t)kb * kv_stride + (lane & 15) * 8;
+    if (n >= 16) {
+      src += r0 * kv_stride;
+#pragma unroll
+      for (int j = 0; j < 8; ++j, src += 2 * kv_stride) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 2 * j * pitch), "l"(src) : "memory");
+    } else if (n > 0) {
+#pragma unroll 1
+      for (int r = r0; r < 16; r += 2, dst += 2 * pitch)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src + (r < n ? r * kv_stride : 0)), "r"(r < n ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  // before giving up at block kb: the keys of the blocks from `keys` places on (0: itself), the values from itself on, if they were asked for
-  auto drain = [&](uint32_t keys, int kb, int nkeys) {
-    for (uint32_t i = keys; i < ST + keys; ++i)
-      if (kb + (int)i * NW * 16 < nkeys) atile::bar_drain(atile::smem_addr(&s_full[warp][0][(blocks + i) % ST]), ((blocks + i) / ST) & 1);
-    for (uint32_t i = 0; i < ST; ++i)
-      if (kb + (int)i * NW * 16 < nkeys) atile::bar_drain(atile::smem_addr(&s_full[warp][1][(blocks + i) % ST]), ((blocks + i) / ST) & 1);
+  auto landed = [&]() {                                      // all but the newest 2 ST - 1 groups: the next keys or values to be used are there
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(2 * ST - 1) : "memory");
+    __syncwarp();
   };
   for (int c0 = 0; c0 < ntok; c0 += R) {
     const int nr = min(R, ntok - c0);
@@ -728,14 +723,10 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
     // ---- Q fragments: dims [32 i + 8 tig, + 8) of rows gid / gid + 8 (zero for padding rows). Identical for every warp:
     // warp 0 loads them and leaves them in shared memory in mma order (registers are needed for the accumulators).
     __syncthreads();                                         // the previous chunk is done with s_qf and with its partial outputs
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
 #pragma unroll
-    for (uint32_t i = 0; i < ST; ++i) {
-      const int kb = (warp + (int)i * NW) * 16;
-      if (kb < nkeys) {
-        fetch(false, (blocks + i) % ST, kb, nkeys);
-        fetch(true, (blocks + i) % ST, kb, nkeys);
-      }
+    for (int i = 0; i < ST; ++i) {
+      fetch(false, i, (warp + i * NW) * 16, nkeys);
+      fetch(true, i, (warp + i * NW) * 16, nkeys);
     }
     if (warp == 0) {
       const uint4 z = make_uint4(0, 0, 0, 0);
@@ -754,12 +745,12 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
     for (int t = 0; t < 16; ++t) { o[t][0] = 0.f; o[t][1] = 0.f; o[t][2] = 0.f; o[t][3] = 0.f; }
     float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;
     // this warp's keys: blocks of 16, interleaved over the warps
-    for (int kb = warp * 16; kb < nkeys; kb += NW * 16) {
+    int at = 0;                                              // this block's place in the ring
+    for (int kb = warp * 16; kb < nkeys; kb += NW * 16, at = at + 1 == ST ? 0 : at + 1) {
       const int next = kb + ST * NW * 16;                    // the block that takes this one's place
-      const uint32_t at = blocks % ST, phase = (blocks / ST) & 1;
       const unsigned char* blk = ring + at * SEQ_BLOCK;
-      unsigned char* blv = ring + at * SEQ_BLOCK + 16 * SEQ_KS;
-      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][0][at]), phase, &s_fail))) { drain(0, kb, nkeys); break; }
+      const unsigned char* blv = blk + 16 * SEQ_KS;
+      landed();
       // ---- S = Q K^T for the two 8-key tiles
       float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -773,7 +764,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
         mma16816(s1, c.x, c.y, c.z, c.w, k1.z, k1.w);
       }
       __syncwarp();
-      if (next < nkeys) fetch(false, at, next, nkeys);
+      fetch(false, at, next, nkeys);
       // ---- scale, mask (key j <= position of the row), online softmax
       const int j00 = kb + 2 * tig, j10 = kb + 8 + 2 * tig;
       float pA[4], pB[4];                                    // row gid: keys j00, j00 + 1, j10, j10 + 1; row gid + 8 likewise
@@ -801,11 +792,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
       uint32_t ah[4], al[4];
       split_h2(pA[0], pA[1], ah[0], al[0]); split_h2(pB[0], pB[1], ah[1], al[1]);
       split_h2(pA[2], pA[3], ah[2], al[2]); split_h2(pB[2], pB[3], ah[3], al[3]);
-      if (!__all_sync(0xffffffffu, atile::bar_wait(atile::smem_addr(&s_full[warp][1][at]), phase, &s_fail))) { drain(1, kb, nkeys); break; }
-      if (kb + 16 > nkeys) {                                 // rows past the last key: their weights are zero, their values must be finite
-        for (int i = (nkeys - kb) * 16 + lane; i < 256; i += 32) *reinterpret_cast<uint4*>(blv + (i >> 4) * SEQ_VS + (i & 15) * 16) = make_uint4(0u, 0u, 0u, 0u);
-        __syncwarp();                                        // (a warp's last block: the barrier before the next chunk's copies follows)
-      }
+      landed();
 #pragma unroll
       for (int h = 0; h < 2; ++h) {                          // value rows 2 tig, + 1, + 8, + 9: dims 8 gid .. + 7, and 64 further
         uint4 v[4];
@@ -822,9 +809,8 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
           mma16816(o[h * 8 + t], al[0], al[1], al[2], al[3], b0, b1);
         }
       }
-      ++blocks;
       __syncwarp();
-      if (next < nkeys) fetch(true, at, next, nkeys);
+      fetch(true, at, next, nkeys);
     }
     // ---- quad-reduce the row sums, publish this warp's (m, l, O)
     lA += __shfl_xor_sync(0xffffffffu, lA, 1); lA += __shfl_xor_sync(0xffffffffu, lA, 2);
@@ -838,13 +824,6 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
       s_o[warp][gid + 8][d] = o[t][2];  s_o[warp][gid + 8][d + 8] = o[t][3];
     }
     __syncthreads();
-    if (s_fail) {                                            // (written before the barrier: uniform)
-      if (tid == 0) atomicAdd(&atile::attn_tile_timeouts, 1u);
-      for (int i = tid; i < (ntok - c0) * G * 16; i += NW * 32)   // nobody takes what the buffer held for a result
-        *reinterpret_cast<uint4*>(out + ((size_t)s_tok[c0 + i / (G * 16)] * Hq + hk * G + i / 16 % G) * D + (i & 15) * 8) =
-            make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
-      return;
-    }
     // ---- merge the warps: thread = (row r, 16 dims); out = sum_w e^{m_w - m} O_w / sum_w e^{m_w - m} l_w
     for (int item = tid; item < 16 * 8; item += NW * 32) {
       const int r = item >> 3, dq = item & 7;
