@@ -335,39 +335,44 @@ __device__ __forceinline__ void finalize_store(const Params& p, uint32_t raw, in
   }
 }
 
-// What the LONG form (below) stores with, eight channels (ch % 8 == 0) of a token as one 16-byte piece. Same arithmetic, same rounding.
+// What the LONG form (below) stores with: the 16 tokens of a tcgen05.ld group (tokens tok0 + j, j < nt), finished by the lanes that hold them (a channel each),
+// cross a warp's stage [16][32] of 16-bit values and leave as 16-byte pieces, eight channels of two tokens a lane. Same arithmetic, same rounding as
+// finalize_store. (float32 values through a stage of eight tokens took 6.8 us for a tile of 128 tokens beside
+// the products and 3.7 alone, now 3.6 and 1.9; finishing in the lanes with the output type asked for every value took the integer modes 15 % longer.)
+constexpr int STAGE_HALVES = 16 * 32, STAGE_BYTES = NEPI * STAGE_HALVES * 2;
 template <int MODE>
-__device__ __forceinline__ void finalize_store8(const Params& p, const uint32_t (&raw)[8], int tok_g, int ch, float sa, const float* sw, const float* bs) {
+__device__ __forceinline__ void finalize16_staged(const Params& p, const uint32_t (&r)[16], int nt, int tok0, int ch0, const float* sa, float sw, float bs,
+                                                  uint16_t* stage) {
   constexpr bool INT = MODE == MODE_I8 || MODE == MODE_A8;
-  const bool bf = INT ? p.out_bf16 != 0 : MODE == MODE_BF16;
-  uint32_t h[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    float f = INT ? __fmul_rn(__fmul_rn(__int2float_rn(((int32_t)raw[e]) >> (MODE == MODE_A8 ? 4 : 8)), sa), sw[e]) : __fmul_rn(__uint_as_float(raw[e]), sw[e]);
-    if (p.bias) f = __fadd_rn(f, bs[e]);
-    h[e] = bf ? __bfloat16_as_ushort(__float2bfloat16_rn(f)) : __half_as_ushort(__float2half_rn(f));
-  }
-  *reinterpret_cast<uint4*>((uint16_t*)p.out + (size_t)tok_g * p.N + ch) = make_uint4(h[0] | h[1] << 16, h[2] | h[3] << 16, h[4] | h[5] << 16, h[6] | h[7] << 16);
-}
-// A warp's stage: [8][36] words, then scales and bias of its 32 channels. The 16 tokens of a tcgen05.ld group (tokens tok0 + j, j < nt) cross it
-// eight at a time, so that a lane finishes eight channels of one token.
-constexpr int STAGE_LD = 36, STAGE_WORDS = 8 * STAGE_LD + 64, STAGE_BYTES = NEPI * STAGE_WORDS * 4;
-template <int MODE>
-__device__ __forceinline__ void finalize16_staged(const Params& p, const uint32_t (&r)[16], int nt, int tok0, int ch0, const float* sa, uint32_t* stage) {
   const int lane = threadIdx.x & 31, c = (lane & 3) * 8, tok = lane >> 2;
-  const float* s_sw = reinterpret_cast<const float*>(stage + 8 * STAGE_LD);
-#pragma unroll 1
-  for (int h8 = 0; h8 < 16 && h8 < nt; h8 += 8) {
+  float f[16];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) stage[j * STAGE_LD + lane] = h8 ? r[8 + j] : r[j];
-    __syncwarp();
-    if (h8 + tok < nt && ch0 + c < p.N) {
-      const uint4 lo = *reinterpret_cast<const uint4*>(stage + tok * STAGE_LD + c), hi = *reinterpret_cast<const uint4*>(stage + tok * STAGE_LD + c + 4);
-      const uint32_t raw[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-      finalize_store8<MODE>(p, raw, tok0 + h8 + tok, ch0 + c, sa[h8 + tok], s_sw + c, s_sw + 32 + c);
-    }
-    __syncwarp();                                        // read before the next eight are written
+  for (int j4 = 0; j4 < 16; j4 += 4) {
+    const float4 a4 = INT ? *reinterpret_cast<const float4*>(sa + j4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      f[j4 + e] = INT ? __fmul_rn(__fmul_rn(__int2float_rn(((int32_t)r[j4 + e]) >> (MODE == MODE_A8 ? 4 : 8)), a[e]), sw) : __fmul_rn(__uint_as_float(r[j4 + e]), sw);
   }
+  if (p.bias) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) f[j] = __fadd_rn(f[j], bs);
+  }
+  if (INT ? p.out_bf16 != 0 : MODE == MODE_BF16) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) stage[j * 32 + lane] = __bfloat16_as_ushort(__float2bfloat16_rn(f[j]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) stage[j * 32 + lane] = __half_as_ushort(__float2half_rn(f[j]));
+  }
+  __syncwarp();
+  if (ch0 + c < p.N) {
+#pragma unroll
+    for (int h = 0; h < 16; h += 8)
+      if (h + tok < nt)
+        *reinterpret_cast<uint4*>((uint16_t*)p.out + (size_t)(tok0 + h + tok) * p.N + ch0 + c) = *reinterpret_cast<const uint4*>(stage + (h + tok) * 32 + c);
+  }
+  __syncwarp();                                        // read before the next group is written
 }
 
 // finalize_store for the 16 tokens of one tcgen05.ld group (tokens tok0 + j, j < nt), with everything that does not depend
@@ -451,7 +456,9 @@ __device__ __forceinline__ unsigned long long gtimer_ns() {
 // LONG: the form for products whose CTAs have a tile's length or more to do each (the rule is in run()). What ends such a launch is an epilogue
 // that nothing hides, of up to 256 tokens: it runs once or twice, at the speed at which its instructions are fetched, so it is short here. Values
 // leave eight channels at a time through a stage in shared memory (16 stores of two bytes a lane, unrolled, took 4 us for a tile of 64 tokens), and a
-// shared tile that only waits for this CTA's part is finished from the accumulator. Outputs have to be 16-byte aligned, N a multiple of 8; no
+// shared tile that only waits for this CTA's part is finished from the accumulator. Its epilogues also bound the last two tiles of a CTA, which the products
+// finish before them: with the two made shorter, and weights kept in L2 (w_policy), W4A16 28672 x 4096 256 tokens 65 -> 59 us, 509 118 -> 104, 10240 x 8192
+// 1999 tokens 325 -> 277 (at the power limit), W4A4 28672 x 4096 256 tokens 38.6 -> 36.9, one value per byte 64 tokens 17.9 -> 17.2. Outputs have to be 16-byte aligned, N a multiple of 8; no
 // deferred sums, clusters or raw int32 results. One kernel for both would be slower on either side: what an epilogue does not run lies between
 // what it does (tried: M = 100, 4096 x 4096, 10 to 15 % slower).
 template <int MODE, bool PAIR, bool LONG>
@@ -468,9 +475,9 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   __shared__ __align__(8) uint64_t d_full[2], d_empty[2];
   __shared__ uint32_t tmem_base_smem;
   __shared__ unsigned s_is_last[2];
-  __shared__ uint32_t s_all_here;
+  __shared__ uint32_t s_all_here[2];
   __shared__ __align__(8) uint64_t red_full;             // cluster reduction: every pushing thread of the other CTAs arrives here
-  __shared__ float s_sa[128];
+  __shared__ __align__(16) float s_sa[128];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) { MARK(0); MARK_CTA(512); }
@@ -819,7 +826,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       }
     };
     // LONG: behind the operand rings
-    uint32_t* const stage = reinterpret_cast<uint32_t*>(base + p.stage_at) + q * STAGE_WORDS;
+    uint16_t* const stage = reinterpret_cast<uint16_t*>(base + p.stage_at) + q * STAGE_HALVES;
     int npf = 0, pf_t[2] = {0, 0}, pf_cf[2] = {0, 0}, pf_cl[2] = {0, 0};   // this CTA's tiles that are shared with other CTAs
     // ---- stream-K tiles shared with other CTAs (at most two per CTA: its first and its last tile). The protocol is
     // runs right after the tile's accumulator has been drained (overlapping the main loop unless it is the CTA's last
@@ -985,12 +992,6 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       // everything a tile needs from global memory is requested one tile ahead of its use
       const float sw = sw_next, bs = bs_next;
       load_scale(u + (kb_end - ka), sw_next, bs_next);
-      if (LONG) {                                          // this warp's channels: written and read by this warp alone
-        __syncwarp();
-        stage[8 * STAGE_LD + lane] = __float_as_uint(sw);
-        stage[8 * STAGE_LD + 32 + lane] = __float_as_uint(bs);
-        __syncwarp();
-      }
       if (I8 && p.out && !p.split_out && sa_tile != tile_m) {   // decode (one token tile): loaded once per kernel
         named_bar_sync(1, NEPI * 32);                    // previous tile's readers are done with s_sa
         if (etid < m_here)
@@ -1002,9 +1003,37 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       const int c_first = full ? 0 : cta_of_unit(t * KB, p.U, p.G);
       const int c_last = full ? 0 : cta_of_unit(t * KB + KB - 1, p.U, p.G);
       uint32_t* my_slot = p.ws_part + (size_t)(2 * blockIdx.x + (u0 < t * KB ? 1 : 0)) * (size_t)(np * TM);
+      // LONG: a shared tile whose other contributor has arrived is finished from the accumulator, which spares this CTA's own part the way
+      // through the workspace and back: at the end of a launch nothing hides it. Asked only where it is likely, of the tile at the end of a CTA's
+      // range (of a tile's length or more, so that there is one other contributor), whose rest the next CTA began with. It has mostly arrived long before:
+      // then its part is asked for in front of the wait, and 32 tokens ahead from there on (loads of 16 tokens at a time, waited for one after the
+      // other, took 9 us for a tile of 128, now 3).
+      constexpr int AHEAD = 32;
+      const bool ask = LONG && !full && u0 < t * KB;
+      uint32_t theirs[LONG ? AHEAD : 1];
+      auto all_here = [&](int i) {
+        if (etid == 0) {
+          unsigned seen;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(p.counters + phys(c_first)) : "memory");
+          s_all_here[i] = seen == (unsigned)(c_last - c_first) ? 1u : 0u;   // (written once each: a range has one such tile)
+        }
+        named_bar_sync(1, NEPI * 32);
+        return s_all_here[i] != 0;
+      };
+      auto fetch_theirs = [&](int c0, uint32_t (&v)[LONG ? AHEAD : 1]) {
+        const uint32_t* src = p.ws_part + (size_t)(2 * phys(c_last)) * (size_t)(np * TM) + (size_t)c0 * TM + chl;
+#pragma unroll
+        for (int j = 0; j < (LONG ? AHEAD : 1); ++j) v[j] = c0 + j < m_here ? __ldcg(src + (size_t)j * TM) : 0u;
+      };
+      bool direct = ask && all_here(0);
+      if (LONG && direct) fetch_theirs(0, theirs);
       mbar_wait(smem_u32(&d_full[db]), ((uint32_t)(dbl ? f >> 1 : f)) & 1u);
       tc_fence_after();
       if (etid == 0) MARK(6 + 3 * min(f, 2));
+      if (ask && !direct) {
+        direct = all_here(1);
+        if (LONG && direct) fetch_theirs(0, theirs);
+      }
       const uint32_t d_addr = tmem + ((uint32_t)(q * 32) << 16) + (db ? (uint32_t)p.dcols : 0u);
       const int split_rank = full ? 0 : cta - c_first;     // deferred reduction: this CTA's slice of the tile's k range
       const bool clus = !PAIR && !LONG && p.cs > 1;        // the tile is shared by exactly this cluster; rank 0 owns it
@@ -1022,38 +1051,24 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
                          : "=r"(done) : "r"(smem_u32(&red_full)) : "memory");
         }
       }
-      // LONG: a shared tile whose other contributors have all arrived is finished from the accumulator, which spares this CTA's own part the way
-      // through the workspace and back: at the end of a launch nothing hides it. Asked only where it is likely, of the tile at the end of a CTA's
-      // range, whose rest the next CTA began with.
-      bool direct = false;
-      if (LONG && !full && u0 < t * KB) {
-        if (etid == 0) {
-          unsigned seen;
-          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(p.counters + phys(c_first)) : "memory");
-          s_all_here = seen == (unsigned)(c_last - c_first) ? 1u : 0u;   // (written once: a range has one such tile)
-        }
-        named_bar_sync(1, NEPI * 32);
-        direct = s_all_here != 0;
-      }
       if (LONG && direct) {
-        const size_t slot_words = (size_t)(np * TM);
 #pragma unroll 1
-        for (int c0 = 0; c0 < m_here; c0 += 16) {
-          uint32_t r[16], acc[16];
-          tmem_ld16(d_addr + c0, r);
-          bool have = false;
-          for (int c = c_first; c <= c_last; ++c) {        // ascending CTA order, as in resolve_shared
-            uint32_t v[16];
-            const uint32_t* src = p.ws_part + (size_t)(2 * phys(c) + (c == c_first && cta_start(c_first, p.U, p.G) < t * KB ? 1 : 0)) * slot_words +
-                                  (size_t)c0 * TM + chl;
+        for (int c0 = 0; c0 < m_here; c0 += AHEAD) {
+          uint32_t next[LONG ? AHEAD : 1];
+          fetch_theirs(c0 + AHEAD, next);
+#pragma unroll 1
+          for (int h = 0; h < AHEAD && c0 + h < m_here; h += 16) {
+            uint32_t r[16];
+            tmem_ld16(d_addr + c0 + h, r);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = c == cta ? r[j] : c0 + j < m_here ? __ldcg(src + (size_t)j * TM) : 0u;
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              acc[j] = !have ? v[j] : I8 ? acc[j] + v[j] : __float_as_uint(__fadd_rn(__uint_as_float(acc[j]), __uint_as_float(v[j])));
-            have = true;
+            for (int j = 0; j < 16; ++j) {                   // ascending CTA order, as in resolve_shared
+              const uint32_t v = theirs[h ? (LONG ? 16 + j : 0) : (LONG ? j : 0)];
+              r[j] = I8 ? r[j] + v : __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(v)));
+            }
+            finalize16_staged<MODE>(p, r, m_here - c0 - h, m0 + c0 + h, n0 + q * 32, s_sa + c0 + h, sw, bs, stage);
           }
-          finalize16_staged<MODE>(p, acc, m_here - c0, m0 + c0, n0 + q * 32, s_sa + c0, stage);
+#pragma unroll
+          for (int j = 0; j < (LONG ? AHEAD : 1); ++j) theirs[j] = next[j];
         }
         if (etid == 0) p.counters[phys(c_first)] = 0u;     // self-cleaning; this CTA never counted itself
       }
@@ -1074,7 +1089,7 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
               if (jj < nt) dst[jj * ld] = r[jj];
           }
         } else if (variant == 1) {                       // whole tile in this CTA: epilogue and store
-          if (LONG) finalize16_staged<MODE>(p, r, nt, m0 + c0, n0 + q * 32, s_sa + c0, stage);
+          if (LONG) finalize16_staged<MODE>(p, r, nt, m0 + c0, n0 + q * 32, s_sa + c0, sw, bs, stage);
           else if (ch_ok) finalize16<MODE>(p, r, nt, m0 + c0, ch, s_sa + c0, sw, bs);
         } else if (variant == 2) {                       // stream-K partial tile through the workspace
           uint32_t* dst = my_slot + (size_t)c0 * TM + chl;
@@ -1448,9 +1463,10 @@ static bool rows_wanted(int mode, int M, int N, int K) {
   return want == 2 || known_size(mode, M, N, K).rows;
 }
 // Whether the tcgen05 form runs as LONG: wherever it can and a CTA's range is at least a tile long, so that whole tiles and ends of ranges are what a
-// launch waits for. us, without | with it:  W4A16 28672 x 4096: 64 tokens 27.8 | 26.2, 256: 59.2 | 54.6, 1000: 198 | 186   10240 x 8192, 256 tokens: 46.9 | 43.7
-//   W4A4 28672 x 4096: 65 tokens 24.6 | 22.9, 256: 49.4 | 38.9   W4A4 bytes 28672 x 4096: 64 tokens 20.5 | 18.2, 256: 47.5 | 35.8
-// Shorter ranges, whose tiles are all shared, gain nothing: 4096 x 14336, 256 tokens, W4A4 30.1 | 31.4, W4A4 bytes 28.6 | 29.4, W4A16 34.6 | 34.6.
+// launch waits for. us, without | with it:  W4A16 28672 x 4096: 64 tokens 27.5 | 25.8, 256: 69 | 59, 1000: 240 | 193   10240 x 8192, 256 tokens: 50 | 43
+//   W4A4 28672 x 4096: 65 tokens 24.3 | 21.6, 256: 48.7 | 36.3   W4A4 bytes 28672 x 4096: 64 tokens 20.0 | 17.1, 256: 47.1 | 34.7
+// Shorter ranges, whose tiles are all shared (by more than two CTAs, which the form's way with shared tiles rules out), gained nothing with the earlier
+// epilogue: 4096 x 14336, 256 tokens, W4A4 30.1 | 31.4, W4A4 bytes 28.6 | 29.4, W4A16 34.6 | 34.6.
 // Its stage may cost a ring its fifth stage, not its fourth (W4A16 27648 x 5120, 80 tokens, with three: 32.9 | 33.5).
 static bool long_wanted(Plan& pl) {
   if (pl.cs != 1 || pl.U < pl.G * pl.KB) return false;
