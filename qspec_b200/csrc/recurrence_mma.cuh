@@ -14,12 +14,12 @@
 // pass of their own over memory), decays' products, the scores a_ij (summed over the rows by exchanges that halve the number of values a lane holds) and
 // the split operands, which go to shared memory (16-byte pieces c of row r at c ^ (r & 7)). With warps of their own for the preparation, four beside eight, the
 // kernel waited for these (outputs of 1500 tokens, 16 heads of 128 x 128, 100 us instead of 75).
-// What bounds it is the number of instructions (2700 a warp and block where outputs are computed: gates 640, scores 660, splitting and products 650) at two
-// a cycle and SM; the tensor cores are busy a fifth of the time. 1500 tokens, 16 heads of 128 x 128, all launches: 143 -> 93 us (each by itself: states 27,
-// carry 10, outputs 75); 600 tokens, 8 heads of 64 x 64: 40 -> 28.
+// What bounds it is the number of instructions (about 2500 a warp and block where outputs are computed: gates, scores, splitting and products a quarter each) at two
+// a cycle and SM; the tensor cores are busy a fifth of the time. A launch of its own for the gates takes as long as it saves here (11 us; outputs 70 -> 62,
+// states 25 -> 21). 1500 tokens, 16 heads of 128 x 128, all launches: 143 -> 91 us; 600 tokens, 8 heads of 64 x 64: 40 -> 27.
 //
-// Values that are not finite would turn into NaN in the lower terms (infinity - infinity) and reach rows that the walk spares; a chunk that meets one is
-// walked again token by token (rm_walk).
+// Values that are not finite would turn into NaN in the lower terms (infinity - infinity) and reach rows that the walk spares. They show in the chunk's
+// outputs or in its last state, which no later token makes finite again; such a chunk is walked once more token by token (rm_walk).
 namespace qspec {
 namespace rmma {
 
@@ -287,7 +287,6 @@ __global__ void __launch_bounds__(Shape<D, DV>::THREADS, Shape<D, DV>::CTAS) chu
         q0 = z0 / (1.0f + expf(-z0));
         q1 = z1 / (1.0f + expf(-z1));
       }
-      odd |= !(finite(f0) && finite(f1) && finite(o0) && finite(o1) && finite(q0) && finite(q1));
       *reinterpret_cast<uint64_t*>(dec + i * D) = in ? rc_pair(f0, f1) : rc_pair(1.f, 1.f);
       const uint64_t om = in ? rc_pair(o0, o1) : 0ull, q = in ? rc_pair(q0, q1) : 0ull;
       mine[k] = OUT ? q : om;
@@ -302,8 +301,6 @@ __global__ void __launch_bounds__(Shape<D, DV>::THREADS, Shape<D, DV>::CTAS) chu
     for (int k = 0; k < BT * DV / 8 / Sh::THREADS; ++k) {
       const int i = tid + k * Sh::THREADS, r = i / (DV / 8), pc = i % (DV / 8);
       const uint4 x = r < nb ? zv[k] : make_uint4(0u, 0u, 0u, 0u);
-      odd |= (__vcmpeq2(x.x & 0x7f807f80u, 0x7f807f80u) | __vcmpeq2(x.y & 0x7f807f80u, 0x7f807f80u) | __vcmpeq2(x.z & 0x7f807f80u, 0x7f807f80u) |
-              __vcmpeq2(x.w & 0x7f807f80u, 0x7f807f80u)) != 0u;
       *reinterpret_cast<uint4*>(rm_smem + vbuf + r * DV * 2 + ((pc ^ (r & 7)) << 4)) = x;
     }
     const float diag = OUT ? lane_sums<TT>(own) : 0.f;
@@ -316,9 +313,10 @@ __global__ void __launch_bounds__(Shape<D, DV>::THREADS, Shape<D, DV>::CTAS) chu
         sa[i * 20 + i] = diag;
       }
       // columns j = t and 15 - t: fifteen scores below the diagonal, those of t (rows t + 1 .. 15) first
-#pragma unroll 1
+#pragma unroll
       for (int k = 0; k < TT / 2; ++k) {
         const int t = grp * (TT / 2) + k, turn = 15 - t;
+        const float* row = dec + (t + 1) * D;                 // decays of row i = v + t + 1, then of v + 1; the queries lie QF_AT - DEC_AT further
         uint64_t r = two(som + t * D);
         float val[16];
 #pragma unroll
@@ -326,10 +324,10 @@ __global__ void __launch_bounds__(Shape<D, DV>::THREADS, Shape<D, DV>::CTAS) chu
           if (v == turn) {
             put(Sh::K_AT, t, r);                              // at the block's end: what multiplies v_t in the state
             r = two(som + turn * D);
+            row = dec + D;
           }
-          const int i = v < turn ? v + t + 1 : v + 1;
-          r = rc_mul(r, two(dec + i * D));
-          const float2 x = rc_unpair(rc_mul(two(sqf + i * D), r));
+          r = rc_mul(r, two(row + v * D));
+          const float2 x = rc_unpair(rc_mul(two(row + v * D + (Sh::QF_AT - Sh::DEC_AT) / 4), r));
           val[v] = x.x + x.y;
         }
         val[15] = 0.f;
@@ -408,6 +406,7 @@ __global__ void __launch_bounds__(Shape<D, DV>::THREADS, Shape<D, DV>::CTAS) chu
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           o[j][e] = ((hi[0][j][e] + hi[1][j][e]) + x[e]) + lo[j][e];
+          odd |= !finite(o[j][e]);
           ss[e >> 1] += o[j][e] * o[j][e];
         }
       }

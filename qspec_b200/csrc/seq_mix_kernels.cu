@@ -1082,7 +1082,7 @@ static int launch_recurrence_chunks(const void* p, int ld, const float* gates, f
 // us: here 31 (25 where a head's state is smaller than 128 x 128) and 2.5 for 1000 tokens of a head; the walk 8 and 0.18 (0.13) a token of a segment,
 // more where its CTAs (a segment, a head, 16 columns each) fill the GPU several times over. Measured, walk | here, 128 x 128, segments x tokens x heads:
 // 1 x 100 x 16 27 | 35, 1 x 150 x 32 38 | 41, 5 x 60 x 16 40 | 45, 2 x 150 x 32 70 | 55, 1 x 300 x 16 60 | 39, 5 x 300 x 16 175 | 104; 64 x 64, 1 x 300 x 16
-// 46 | 28, 2 x 33 x 8 15 | 20. The form of float32 rows: 1 x 1500 x 16, 128 x 128 143 | 93, 1 x 600 x 8, 64 x 64 40 | 28.
+// 46 | 28, 2 x 33 x 8 15 | 20. The form of float32 rows: 1 x 1500 x 16, 128 x 128 143 | 91, 1 x 600 x 8, 64 x 64 40 | 28.
 static int rm_chunk_tokens(int nseg, int ntok, int H, int D, int DV) {
   if (!((D == 64 || D == 128) && (DV == 64 || DV == 128)) || nseg < 1 || ntok < nseg || sm_count() < 1) return 0;
   const bool large = D * DV == 128 * 128;
