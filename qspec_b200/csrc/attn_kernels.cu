@@ -586,7 +586,8 @@ __global__ void __launch_bounds__(NW * 32, ST == 1 ? 4 : NW == 4 ? 2 : 1)
 seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ cache_k, const __half* __restrict__ cache_v,
                      const int* __restrict__ positions, const int* __restrict__ seq_ids, __half* __restrict__ out,
                      int T, int B, int Hq, int Hkv, int S, float sm_scale, int min_run) {
-  pdl_enter();
+  if (min_run) atile::attn_beside_tiles();                   // (launched behind attn_tile_kernel)
+  else pdl_enter();
   constexpr int D = 128, R = 16 / G;                         // R tokens x G heads <= 16 query rows per chunk
   __shared__ int s_tok[1024];                                // tokens of this sequence in the pass (T <= 1024)
   __shared__ int s_pos[1024];                                // ... and their positions (loaded in the same round trip as the scan)
@@ -643,7 +644,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
   } else {
     __syncthreads();
     for (int t = tid; t < T; t += NW * 32) {
-      const int sq = __ldg(seq_ids + t), ps = __ldg(positions + t);
+      const int sq = __ldcg(seq_ids + t), ps = __ldcg(positions + t);
       if (sq == seq) {
         const int i = atomicAdd(&s_ntok, 1);
         s_tok[i] = t;
@@ -660,15 +661,16 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
     for (int t0 = warp * 32; t0 < T; t0 += NW * 32) {
       const int t = t0 + lane;
       bool before, after;
-      if (!atile::attn_in_run(positions, seq_ids, T, t0, min_run, before, after) && t < T && seq_ids[t] == seq) {
+      if (!atile::attn_in_run(positions, seq_ids, T, t0, min_run, before, after) && t < T && __ldcg(seq_ids + t) == seq) {
         const int i = atomicAdd(&s_ntok, 1);
         s_tok[i] = t;
-        s_pos[i] = positions[t];
+        s_pos[i] = __ldcg(positions + t);
       }
     }
     __syncthreads();
     ntok = s_ntok;
   }
+  if (min_run) atile::attn_tiles_done();
   if (ntok == 0) return;
   const size_t row_elems = (size_t)(Hq + 2 * Hkv) * D;
   const __half* kbase = cache_k + ((size_t)seq * S * Hkv + hk) * D;

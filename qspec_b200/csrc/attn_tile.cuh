@@ -65,10 +65,16 @@ struct Args {
   uint32_t rep_inv;                            // set by launch(): r * rep_inv >> 16 = r / rep for r < 128
 };
 
-// Tokens t and t + 1 of the batch are of one run.
+// Tokens t and t + 1 of the batch are of one run. (Read from L2: see attn_beside_tiles.)
 __device__ __forceinline__ bool attn_link(const int* pos, const int* seq, int ntok, int t) {
-  return t >= 0 && t + 1 < ntok && seq[t] == seq[t + 1] && pos[t + 1] == pos[t] + 1;
+  return t >= 0 && t + 1 < ntok && __ldcg(seq + t) == __ldcg(seq + t + 1) && __ldcg(pos + t + 1) == __ldcg(pos + t) + 1;
 }
+// The kernel launched behind attn_tile_kernel for the other tokens starts with this instead of waiting: it looks for its tokens (positions and
+// sequences, or the table of segments, from L2) while the tiles run, and calls attn_tiles_done() before it reads anything else, writes, or leaves. The
+// tiles let it start only behind their own wait, so what lies in front of them is over by then, and nothing of theirs is read; that it waits at
+// all is for the kernels behind it, which wait for it alone.
+__device__ __forceinline__ void attn_beside_tiles() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void attn_tiles_done() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 // For the 32 tokens t0 .. t0 + 31 of a whole warp, token t0 + lane: is it in a run of at least min_run (<= 16) tokens? `before`, `after`: is
 // it linked to its neighbours?
 __device__ __forceinline__ bool attn_in_run(const int* pos, const int* seq, int ntok, int t0, int min_run, bool& before, bool& after) {

@@ -1489,8 +1489,10 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_kernel(const WinMma a)
 // batch without short segments costs a launch and little more.
 constexpr int WIN_RUN = 16;
 template <int DA, int DV>
-__global__ void __launch_bounds__(128, 2) window_attn_mma_short_kernel(const WinMma a) {
-  pdl_enter();
+__global__ void __launch_bounds__(128, 2) window_attn_mma_short_kernel(const WinMma a, int beside) {   // beside: launched behind attn_tile_kernel
+  if (beside) atile::attn_beside_tiles();
+  else pdl_enter();
+  bool wait = beside != 0;
   __shared__ uint32_t s_short;
   const int most = 16 / (a.H / a.G);                          // tokens of a piece
   for (int t0 = blockIdx.x; t0 < a.ntok; t0 += 32 * (int)gridDim.x) {
@@ -1498,7 +1500,7 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_short_kernel(const Win
       const int t = t0 + (int)threadIdx.x * (int)gridDim.x;
       bool begins = false;
       if (t < a.ntok) {
-        const int s0 = a.meta[2 * a.ntok + t], s1 = a.meta[3 * a.ntok + t];
+        const int s0 = __ldcg(a.meta + 2 * a.ntok + t), s1 = __ldcg(a.meta + 3 * a.ntok + t);
         begins = s1 - s0 < WIN_RUN && (t - s0) % most == 0;
       }
       const uint32_t bits = __ballot_sync(0xffffffffu, begins);
@@ -1506,6 +1508,10 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_short_kernel(const Win
     }
     __syncthreads();
     uint32_t left = s_short;
+    if (left && wait) {
+      atile::attn_tiles_done();
+      wait = false;
+    }
     for (; left; left &= left - 1u) {
       const int t = t0 + (__ffs(left) - 1) * (int)gridDim.x;
       window_attn_mma_rows<DA, 0, DV, false>(a, t, min(most, a.meta[3 * a.ntok + t] - t));
@@ -1513,6 +1519,7 @@ __global__ void __launch_bounds__(128, 2) window_attn_mma_short_kernel(const Win
     }
     __syncthreads();
   }
+  if (wait) atile::attn_tiles_done();
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -2004,12 +2011,12 @@ static int launch_window_mma(const WinMma& a, int slices, cudaStream_t st) {
 }
 
 // Tokens of segments shorter than WIN_RUN, beside attn_tile_kernel.
-static int launch_window_short(WinMma a, cudaStream_t st) {
+static int launch_window_short(WinMma a, bool beside, cudaStream_t st) {
   constexpr size_t smem = (size_t)16 * (128 / 2 + 4) * 4 + (size_t)4 * 16 * 128 * sizeof(float);   // below the limit that needs no asking for
   static_assert(smem <= 48 * 1024, "dynamic shared memory");
   a.token_rows = 0;
   const int per = (2 * sm_count() / a.G) | 1;                 // two CTAs per SM; odd, so that pieces of 2, 4, .. tokens go to all of them
-  launch_pdl(window_attn_mma_short_kernel<128, 128>, dim3(min(a.ntok, per), a.G), dim3(128), smem, st, a);
+  launch_pdl(window_attn_mma_short_kernel<128, 128>, dim3(min(a.ntok, per), a.G), dim3(128), smem, st, a, beside ? 1 : 0);
   QSPEC_CHECK_LAUNCH(1);
   return QSPEC_OK;
 }
@@ -2064,7 +2071,7 @@ int window_attention_mma(const qspec_window_attn_args* p, const void* kB, long l
         const int rc = atile::launch<true, true>(t, p->G, st);
         if (rc != QSPEC_OK) return rc;
       }
-      return mixed ? launch_window_short(a, st) : QSPEC_OK;
+      return mixed ? launch_window_short(a, p->ntok >= WIN_RUN, st) : QSPEC_OK;
     }
   }
   // a latent cache read in the absorbed form (keys and values are the same rows): the CTA-level kernel; QSPEC_SEQ_LATENT=sliced
