@@ -349,8 +349,8 @@ constexpr int K28_BPC = 4;                           // n-blocks (and mix output
 // work in each of the chain's steps; one warp a block where there are rows enough to fill the SMs and the exchange only costs (see the dispatch).
 // Blocks reach the other CTAs as bulk copies of the CTA's four blocks, the maxima as single words, both counted by an mbarrier in the CTA that
 // receives them: stores of every thread into seven CTAs, with a release and acquire of the whole cluster after them, were the largest stall.
-// SiLU and quantiser, before -> now: n = 512, 1 row 5.7 -> 4.8 us, 64 rows 11.6 -> 9.2, 512 rows 44.5 -> 39.8; n = 1024, 64 rows 24.3 -> 17.7,
-// 512 rows 128 -> 98; n = 256, 64 rows 8.2 -> 7.3.
+// SiLU and quantiser, before -> now (the quantiser's quotients included): n = 512, 1 row 5.7 -> 4.5 us, 64 rows 11.6 -> 8.9, 512 rows 44.5 -> 36.0;
+// n = 1024, 64 rows 24.3 -> 17.0, 512 rows 128 -> 88; n = 256, 64 rows 8.2 -> 7.1.
 // Every wait is bounded. A thread that gives one up tells the row's first CTA, which alone writes the row's scale: NaN then, after the cluster's last
 // barrier, whatever it was before; outputs of such a thread are NaN, its copies under way are waited for (up to the limit), and the row is counted
 // in k28_timeouts. `give_up`: the CTAs of a cluster, a bit each, that give their waits up at once (tests).
@@ -363,6 +363,16 @@ __device__ __forceinline__ bool k28_wait(uint32_t bar, uint32_t limit) {
     if (done) return true;
   }
   return false;
+}
+// x / s, correctly rounded, from the correctly rounded reciprocal r of s, for quotients far from the ends of the range: the remainder of the product
+// x r is exact in a fused multiply-add, and one step with it rounds as the division does (P. Markstein, Computation of elementary functions on the
+// IBM RISC System/6000 processor, 1990). One reciprocal serves a row. s = 0: x r is what the division gives; s infinite
+// or NaN: NaN, which quantises to 0 as the quotient does.
+// us with division | now: n = 256, 4 rows 3.89 | 3.65, n = 512, 64 rows 9.15 | 8.87, 512 rows 38.1 | 36.0, n = 1024, 64 rows 17.6 | 17.0. (The mix with its
+// signs in the instructions, a copy for every rank instead of constants: 64 rows the same, 512 rows 3 % slower.)
+__device__ __forceinline__ float k28_quotient(float x, float s, float r) {
+  const float q = __fmul_rn(x, r);
+  return s == 0.f ? q : __fmaf_rn(__fmaf_rn(-q, s, x), r, q);
 }
 // STORES (n = 256, few rows): blocks leave as asynchronous stores from the registers. Without a quantiser nothing is on its way to a CTA then that has its
 // blocks, nor read from it, and it leaves without the last barrier. us at 1 / 8 rows, bulk copies | stores: without quantiser 3.06 / 3.27 | 2.92 / 3.12, with it
@@ -557,14 +567,14 @@ hadamard_k28_cluster_kernel(const uint4* __restrict__ x, const uint4* __restrict
 #pragma unroll
   for (int r = 0; r < K28_CLUSTER; ++r) row_amax = fmaxf(row_amax, amax_all[r]);
   const __half sh = sym_scale(row_amax, clip);
-  const float sc = __half2float(sh);
+  const float sc = __half2float(sh), inv = __frcp_rn(sc);
 #pragma unroll
   for (int pp = 0; pp < PPT; ++pp) {
     const int jp = threadIdx.x + pp * THR;
 #pragma unroll
     for (int o = 0; o < K28_BPC; ++o) {
-      const int q0 = max(-8, min(7, __half2int_rn(__float2half_rn(__fdiv_rn(keep[pp][o][0], sc)))));
-      const int q1 = max(-8, min(7, __half2int_rn(__float2half_rn(__fdiv_rn(keep[pp][o][1], sc)))));
+      const int q0 = max(-8, min(7, __half2int_rn(__float2half_rn(k28_quotient(keep[pp][o][0], sc, inv)))));
+      const int q1 = max(-8, min(7, __half2int_rn(__float2half_rn(k28_quotient(keep[pp][o][1], sc, inv)))));
       const size_t qi = row * (L >> 1) + (((o0 + o) * n) >> 1) + jp;
       if (c8) reinterpret_cast<uint16_t*>(out_q)[qi] = (uint16_t)((q0 & 0xFF) | ((q1 & 0xFF) << 8));     // one value per byte
       else out_q[qi] = (uint8_t)((q0 & 0xF) | ((q1 & 0xF) << 4));
@@ -670,7 +680,7 @@ static int launch_k28(const void* x, const void* gu, void* of, int8_t* oq, void*
   return QSPEC_OK;
 }
 
-// n = 512: two warps a block up to here, one above. us with SiLU and quantiser, one | two warps: 1 row 5.7 | 4.8, 64: 10.9 | 9.2, 96: 13.7 | 12.1,
+// n = 512: two warps a block up to here, one above. us with SiLU and quantiser (and divisions in it), one | two warps: 1 row 5.7 | 4.8, 64: 10.9 | 9.2, 96: 13.7 | 12.1,
 // 112: 13.7 | 13.7, 128: 13.6 | 14.8, 512: 39.8 | 47.5 (the SMs are full either way, and the exchange between the warps is extra). n = 1024 always two (a lane
 // holds 16 values instead of 32), n = 256 always one (a lane has one vector).
 constexpr int K28_TWO_WARP_ROWS = 112;

@@ -50,3 +50,23 @@ def test_256_wide_rows_by_stores_and_by_bulk_copies(rows, gated):
     for quant, plain in ((True, False), (False, True), (True, True)):
         for a, b in zip(run(x[:rows].contiguous(), quant, plain), run(x, quant, plain)):
             assert torch.equal(a, b[:rows])
+
+
+@pytest.mark.parametrize("n", [256, 512, 1024])
+def test_quantised_values_are_the_quotients(n):
+    """Rows from subnormal scales to the largest, a row of zeros, rows with infinite values and NaN: every value is that of the rounded division."""
+    from qspec_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(40, 28 * n, generator=g, device="cuda")
+    x = (x * torch.logspace(-7.5, 2.5, 40, device="cuda")[:, None]).half()
+    x[3] = 0.0
+    x[5, 77] = float("inf")
+    x[7, 99] = float("nan")
+    out = torch.empty_like(x)
+    q = torch.empty(40, 14 * n, dtype=torch.int8, device="cuda")
+    s = torch.empty(40, dtype=torch.float16, device="cuda")
+    ops.hadamard_k28(x, n, 0.0118, out=out, out_q=q, scale_out=s)
+    quotient = (out.float() / s.float()[:, None]).half().float()                       # an IEEE division, rounded to float16
+    want = torch.where(quotient.isnan(), 0.0, quotient.round().clamp(-8, 7)).to(torch.int8)
+    got = torch.stack(((q << 4) >> 4, q >> 4), -1).view(40, -1)
+    assert torch.equal(got, want)
