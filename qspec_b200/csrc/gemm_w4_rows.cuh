@@ -18,8 +18,8 @@
 //    that the lanes of a read meet different banks (ROW_OF). The nibbles of a word leave in the order (0, 4) (1, 5) (2, 6) (3, 7).
 //  * The weights of the first items are requested before the preceding kernel's end is waited for, as in the stream form.
 // us at 4 / 16 tokens, graph of calls on three to six weights in turn, this form | tcgen05 form:
-//   W4A4   4096 x 4096  2.7 / 3.4 |  8.1 /  9.3    28672 x 4096 10.3 / 13.2 | 15.0 / 15.3    4096 x 14336 6.9 /  7.7 | 11.6 / 12.7
-//   W4A16  4096 x 4096  3.9 / 4.9 |  9.6 / 10.4    28672 x 4096 14.8 / 20.5 | 23.5 / 24.1    4096 x 14336 9.2 / 10.9 | 15.4 / 16.3
+//   W4A4   4096 x 4096  2.7 / 3.4 |  8.1 /  9.3    28672 x 4096 10.3 / 13.2 | 15.0 / 15.3    4096 x 14336 6.6 /  7.6 | 11.6 / 12.7
+//   W4A16  4096 x 4096  3.9 / 4.9 |  9.6 / 10.4    28672 x 4096 14.8 / 20.5 | 23.5 / 24.1    4096 x 14336 8.7 / 10.9 | 15.4 / 16.3
 // Errors of the raw W4A16 sums against 64 bits: 9.3e-8 of their norm at K = 14336, 8.3e-8 at 4096 (tcgen05 form: 9.5e-7, 2.1e-7), for the tensor
 // cores cut at the accumulator's last bit and an accumulator takes only an item's 256 products; at K <= 512 both are off by 2e-8 to 8e-8.
 // Every wait is bounded. A warp gives one up as a whole, stops loading and waits (up to the full limit) for its copies under way; its CTA writes NaN

@@ -1433,7 +1433,7 @@ static bool rows_faster(int mode, int M, int N, int K, const Plan& pl) {
   const int rounds = tiles <= sms ? 1 : (tiles + 2 * sms - 1) / (2 * sms);
   const int last = tiles % (2 * sms);                                       // a last round of few tiles has the SMs nearly to itself
   const double full = rounds > 1 && last > 0 && last <= sms / 4 ? rounds - 0.25 : rounds;
-  const double per_warp = tiles <= sms ? (items + 7) / 8 : full * (mode == MODE_I8 && groups == 1 ? 2 * ((items + 7) / 8) : (items + 3) / 4);   // (NW, CTAS of rows_launch)
+  const double per_warp = tiles <= sms ? (items + 7) / 8 : full * (mode == MODE_I8 && groups == 1 ? 2 * ((items + 7) / 8) : (items + 3) / 4);   // (eight warps also where rows_launch takes twelve, W4A8 as it was with four)
   const int g = groups <= 4 ? groups - 1 : groups <= 6 ? 4 : 5, m = M <= 16 ? 0 : M <= 32 ? 1 : M <= 48 ? 2 : 3;
   const Rows r = mode == MODE_I8 ? rows_i8[g] : mode == MODE_A8 ? rows_a8[g] : rows_f16[g];
   const Stream s = mode == MODE_I8 ? stream_i8[m] : mode == MODE_A8 ? stream_a8[m] : stream_f16[m];
@@ -1498,13 +1498,27 @@ static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, RowsArgs p,
 }
 
 // One CTA of eight warps where every tile gets an SM of its own; otherwise two CTAs per SM, of four warps, or of eight where the slots are
-// small (W4A4, up to 8 tokens): the second CTA loads while the first one adds its sums up. 28672 x 4096, one | two CTAs per SM: W4A4, 4 tokens
-// 12.4 | 10.3 us, W4A16, 16 tokens 23.4 | 20.4.
+// small (up to 8 tokens, W4A4, and W4A8 of at most 16 items): the second CTA loads while the first one adds its sums up. 28672 x 4096, one | two CTAs per
+// SM: W4A4, 4 tokens 12.4 | 10.3 us, W4A16, 16 tokens 23.4 | 20.4. W4A8, 4 tokens, two CTAs of four | eight warps: 28672 x 4096 11.7 | 11.4, 12288 x 4096
+// 6.15 | 5.64, 6144 x 4096 3.84 | 3.58; longer tiles 8192 x 8192 7.16 | 7.25, 27648 x 5120 13.0 | 13.2.
+// A CTA alone on its SM has twelve warps where its slots are small and its tile has more than 16 items: a warp's way from its fragments to the sums is a
+// chain, and eight leave two a scheduler to hide it, with the same bytes under way (24 slots of 8 KB). Eight | twelve: 4 tokens, 4096 x 14336 W4A4
+// 7.0 | 6.6, W4A16 9.0 | 8.7; 4096 x 5120 3.3 | 3.1, 4.3 | 4.1; 16 items 2.8 | 2.9, 3.9 | 4.1, for two rounds of items either way. W4A16, 16 tokens, whose ring holds
+// one slot a warp then, 10.7 | 12.8; W4A8 6.6 | 6.9.
 template <int MODE, int NT>
 static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, const RowsArgs& p, cudaStream_t st) {
   const int sms = sm_count() > 0 ? sm_count() : 148;
-  if (p.tiles <= sms) return rows_launch<MODE, NT, 8, 1>(mw, ma, p, sms, st);
-  return rows_launch<MODE, NT, (MODE == MODE_I8 && NT == 1) ? 8 : 4, 2>(mw, ma, p, sms, st);
+  if (p.tiles <= sms) {
+    if constexpr ((MODE == MODE_I8 && NT <= 2) || (!mode_is_int(MODE) && NT == 1)) {
+      if (p.items > 16) return rows_launch<MODE, NT, 12, 1>(mw, ma, p, sms, st);
+    }
+    return rows_launch<MODE, NT, 8, 1>(mw, ma, p, sms, st);
+  }
+  if constexpr (mode_is_int(MODE) && NT == 1) {
+    if (MODE == MODE_I8 || p.items <= 16) return rows_launch<MODE, NT, 8, 2>(mw, ma, p, sms, st);
+  }
+  if constexpr (MODE != MODE_I8 || NT > 1) return rows_launch<MODE, NT, 4, 2>(mw, ma, p, sms, st);
+  return QSPEC_ERR_UNSUPPORTED;                      // (not reached)
 }
 template <int MODE>
 static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, const RowsArgs& p, cudaStream_t st) {

@@ -63,6 +63,13 @@ def test_rows_products_are_the_exact_sums(ops, monkeypatch, M, N, K, dt, with_bi
     assert ops.attn_tile_timeouts() == 0
 
 
+# twelve warps of a CTA alone (more than 16 items of 256 k, up to 8 tokens, W4A4 up to 16) and eight or four warps a CTA of W4A8 on more tiles than SMs
+@pytest.mark.parametrize("M,N,K", [(1, 8, 4352), (8, 40, 6144), (9, 776, 6272), (16, 4736, 4352), (4, 4736, 14336), (4, 4744, 4096), (8, 9504, 256), (5, 4744, 4352)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+def test_more_warps_for_long_tiles(ops, monkeypatch, M, N, K, dt):
+    test_rows_products_are_the_exact_sums(ops, monkeypatch, M, N, K, dt, True)
+
+
 FORM = {"w4a4": 0, "w4a16": 1, "w4a8": 3}                    # the debug entries' modes
 
 
