@@ -787,7 +787,8 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
         *reinterpret_cast<float4*>(rows + lane * LD + q * 8) = make_float4(v[0], v[1], v[2], v[3]);
         *reinterpret_cast<float4*>(rows + lane * LD + q * 8 + 4) = make_float4(v[4], v[5], v[6], v[7]);
       }
-      const uint32_t stored = __ballot_sync(0xffffffffu, store);   // (and the rows are there; every lane reads the gates that it asked for)
+      const uint32_t stored = __ballot_sync(0xffffffffu, store);
+      __syncwarp();                                           // the rows are there (a vote orders no memory); every lane reads the gates that it asked for
 #pragma unroll 1
       for (int k = 0; k < 8; ++k) {
         const int rr = (lane >> 3) + 4 * k;

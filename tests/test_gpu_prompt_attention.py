@@ -279,6 +279,23 @@ def test_the_maximum_moves_in_every_block(ops, Hq, Hkv, segments):
     check(first, reference(qkv, ck, cv, pos, seq, Hq, Hkv, scale))
 
 
+def test_rows_leave_through_shared_memory_the_same_every_time(ops):
+    """Every lane stores pieces of rows that other lanes of its warp have finished, repaired ones among them: the same bits in every call."""
+    Hq, Hkv = 32, 8
+    qkv, ck, cv, pos, seq = batch([(0, 100, 200), (1, 3, 90)], Hq, Hkv, 320, 2, seed=16)
+    cv[0, 30, :, 5] = float("inf")
+    cv[0, 250:, 1, 64:] = float("nan")
+    first = None
+    for _ in range(100):
+        out = torch.full((len(pos), Hq * 128), 7.0, dtype=torch.float16, device="cuda")
+        ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, Hkv, 128, 0.1)
+        if first is None:
+            first = out
+        assert torch.equal(first.view(torch.int16), out.view(torch.int16))
+    assert torch.isinf(first[:200].view(200, Hq, 128)[..., 5]).sum() >= 150 * Hq
+    check(first[200:], reference(qkv[200:], ck, cv, pos[200:], seq[200:], Hq, Hkv, 0.1))
+
+
 def test_positions_outside_the_cache(ops):
     """seq_attention shows such a token every row of the cache (past its end) or none (before its start: zeros), decode_attention does
     not store it; neither reads outside."""
