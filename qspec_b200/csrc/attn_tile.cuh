@@ -736,7 +736,8 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     // (A barrier of its own: a warp may get here two products ahead, where the parity of b_o's phase n - 3 reads like that of n - 1.)
-    if (ok && n) ok = bar_wait(smem_addr(&b_done), 0, &s_fail);
+    // Without a block nothing has read the queries, and other warps may still be storing theirs where the rows go: then those are waited for.
+    if (ok) ok = bar_wait(n ? smem_addr(&b_done) : smem_addr(&b_q), 0, &s_fail);
     ok = __all_sync(0xffffffffu, ok);
     fence_after();
     s_mx[n & 1][h][r] = l;

@@ -315,6 +315,34 @@ def test_positions_outside_the_cache(ops):
         assert (out[~seen] == 0).all()
 
 
+@pytest.mark.parametrize("Hq", [16, 32])
+@pytest.mark.parametrize("others", [[], [(1, 0, 150)]])
+def test_tiles_without_a_key(ops, Hq, others):
+    """Whole tiles whose tokens all stand before the cache's start, by themselves and beside tiles with keys: no query may be left in the rows that such a
+    tile stores, however late a warp's queries come."""
+    from qspec_b200 import _lib
+    qkv, ck, cv, pos, seq = batch([(0, -200, 200)] + others, Hq, 8, 256, 2, seed=21)
+    want = reference(qkv[200:], ck, cv, pos[200:], seq[200:], Hq, 8, 0.1)
+    for _ in range(50):
+        out = torch.full((len(pos), Hq * 128), 7.0, dtype=torch.float16, device="cuda")
+        ops.seq_attention(qkv, ck, cv, pos, seq, out, Hq, 8, 128, 0.1)
+        assert (out[:200] == 0).all()
+        check(out[200:], want)
+    # the window form: 0 / 0 without a sink, zeros with one, gated or not
+    q = qkv[:, :Hq * 128].float().reshape(len(pos), Hq, 128)
+    start = torch.tensor([0] * 200 + [200] * (len(pos) - 200), dtype=torch.int32, device="cuda")
+    end = torch.tensor([200] * 200 + [len(pos)] * (len(pos) - 200), dtype=torch.int32, device="cuda")
+    meta = torch.stack([seq, pos, start, end, 0 * pos]).contiguous()
+    gate, sink = torch.randn(len(pos), Hq * 128, device="cuda").bfloat16(), torch.randn(Hq, device="cuda")
+    for g, s in ((None, None), (gate, None), (None, sink), (gate, sink)):
+        out = torch.full((len(pos), Hq, 128), 7.0, dtype=torch.bfloat16, device="cuda")
+        before = _lib.load_seq().qspec_launch_count()
+        ops.seq_window_attention_mma(q, ck.bfloat16(), None, cv.bfloat16(), out, meta, 1000, 0.1, True, sink=s, gate=g)
+        assert _lib.load_seq().qspec_launch_count() - before == 2                       # tiles, and the kernel beside them
+        assert torch.isnan(out[:200]).all() if s is None else (out[:200] == 0).all()
+        assert torch.isfinite(out[200:]).all()
+
+
 def test_far_apart_scores(ops):
     """Scores that grow along the sequence (the running maximum moves in every block) and a first key that outweighs all others."""
     qkv, ck, cv, pos, seq = batch([(0, 0, 300)], 8, 8, 300, 1, seed=3)
