@@ -395,11 +395,6 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   const int n2 = min(tok, a.ntok - c0);
 
   // ---- what needs nothing from the kernel before
-  if (warp == WARP_MMA) {
-    // (Kernels with tensor memory let their dependents start only when all their CTAs hold theirs: whoever this waits for goes on without it.)
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-  }
   if (tid == WARP_K * 32) {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&map_k) : "memory");
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(&map_v) : "memory");
@@ -420,6 +415,12 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   const uint32_t base = (smem_addr(at_raw) + 1023u) & ~1023u;
   unsigned char* gbase = at_raw + (base - smem_addr(at_raw));
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  // Tensor memory only now: a kernel of another library some launches ahead (a product in front of the one that prepares the queries) may have let its
+  // dependents start before it held its own, and would wait for columns of a CTA that waits for it. Beside the search for runs it takes no time.
+  if (warp == WARP_MMA) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
   // ---- the runs among this CTA's tokens
   bool start = false, end = false;
   if (tid < TOKENS_MAX) {
