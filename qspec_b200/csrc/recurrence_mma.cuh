@@ -478,6 +478,8 @@ __global__ void __launch_bounds__(256) carry_kernel(const __grid_constant__ Args
   __shared__ RcChunk s_chunk;
   __shared__ bool s_found;
   if (!rc_find(a.meta, a.seg_starts, a.nseg, a.ntok, a.C, -1, blockIdx.x, &s_chunk, &s_found)) return;
+  const int n = s_chunk.chunks;
+  if (n == 1) return;                                         // the outputs read and write the state itself
   const int h = blockIdx.y, e = blockIdx.z * 256 + threadIdx.x, lane = e & 31, g = e >> 5 & 1, rt = e >> 6 & (D / 16 - 1), ct = e / (4 * D);
   if (e >= D * DV / 4) return;
   const int d = 16 * rt + 2 * (lane & 3);
@@ -490,8 +492,7 @@ __global__ void __launch_bounds__(256) carry_kernel(const __grid_constant__ Args
     s = make_float4(src[0], src[DV], src[8 * DV], src[9 * DV]);
   }
   constexpr int AHEAD = 8;
-  const int n = s_chunk.chunks;
-  if (n > 1) at[0] = s;
+  at[0] = s;
   for (int c = 1; c < n; c += AHEAD) {
     float4 x[AHEAD];
     float2 f[AHEAD], f8[AHEAD];

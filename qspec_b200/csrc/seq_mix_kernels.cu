@@ -1079,23 +1079,40 @@ static int launch_recurrence_chunks(const void* p, int ld, const float* gates, f
 // ---- the gated recurrence of bfloat16 rows on the tensor cores (recurrence_mma.cuh) ----
 // Tokens of a chunk: as many as let the chunks of all heads fill the GPU once, at least two blocks. 0: these sizes are not taken.
 // Three launches and the first blocks take what the walk (launch_hgrn2 without a workspace) takes for 130 tokens, so it keeps short segments. Estimates,
-// us: here 31 (25 where a head's state is smaller than 128 x 128) and 2.5 for 1000 tokens of a head; the walk 8 and 0.18 (0.13) a token of a segment,
-// more where its CTAs (a segment, a head, 16 columns each) fill the GPU several times over. Measured, walk | here, 128 x 128, segments x tokens x heads:
-// 1 x 100 x 16 27 | 35, 1 x 150 x 32 38 | 41, 5 x 60 x 16 40 | 45, 2 x 150 x 32 70 | 55, 1 x 300 x 16 60 | 39, 5 x 300 x 16 175 | 104; 64 x 64, 1 x 300 x 16
-// 46 | 28, 2 x 33 x 8 15 | 20. The form of float32 rows: 1 x 1500 x 16, 128 x 128 143 | 91, 1 x 600 x 8, 64 x 64 40 | 28.
+// us: here 32.5 and 2.6 for 1000 tokens of a head (states smaller than 128 x 128: 25.5 and their share of 2.5); the walk 8 and 0.18 (0.13) a token of a
+// segment, more where its CTAs (a segment, a head, 16 columns each) fill the GPU several times over. Measured, walk | here, 128 x 128, segments x tokens x
+// heads: 1 x 100 x 16 27 | 33, 1 x 200 x 16 45 | 36, 1 x 300 x 16 60 | 39, 5 x 100 x 16 62 | 51, 5 x 300 x 16 175 | 104, 64 x 32 x 32 464 | 249; 64 x 64,
+// 1 x 300 x 16 46 | 28, 2 x 33 x 8 15 | 20; decoding tokens beside a prompt portion, 64 x 1 + 2000, 32 heads 783 | 480, 32 x 1 + 1000, 16 heads 248 | 130.
+// The estimate counts tokens, the kernel whole blocks of 16, and every segment's state goes through a CTA: many short segments are the walk's. Where they
+// would have been taken: 64 x 4 x 32 108 | 275, 256 x 1 x 16 180 | 262, 64 x 16 x 16 143 | 153, 64 x 1 + 256, 32 heads 180 | 260; from 24 tokens a segment
+// on 3200 measured sizes, even and ragged, are within 5 % of the walk at the worst, but one (1 + 1 + 98 tokens, 64 heads, 62 | 68), and twice as fast in the
+// mean. (Key size 128 with 64 columns: from
+// 200 tokens on, 24 x 100 x 16 154 | 164, and up to 20000 token-heads, above which the form of float32 rows is the faster one: 1 x 1000 x 16 70 | 68,
+// 1 x 2000 x 16 109 | 121, 1 x 1000 x 32 106 | 117.)
+// A chunk a little shorter than the segments would make two of each. Where these fill the GPU twice, segments of up to 64 tokens stay whole (128 x 128,
+// 12 x 33 x 16: 65 -> 47, the walk 56); where they do not, small states gain nothing from so short segments (64 x 64, 9 x 64 x 16 25 | 28).
 static int rm_chunk_tokens(int nseg, int ntok, int H, int D, int DV) {
-  if (!((D == 64 || D == 128) && (DV == 64 || DV == 128)) || nseg < 1 || ntok < nseg || sm_count() < 1) return 0;
+  if (!((D == 64 || D == 128) && (DV == 64 || DV == 128)) || nseg < 1 || sm_count() < 1) return 0;
   const bool large = D * DV == 128 * 128;
-  const double walkers = (double)nseg * H * (DV / 16) / 210;
+  if (ntok < (D > DV ? 200 : 24) * (long long)nseg || (D > DV && (long long)ntok * H > 20000)) return 0;
+  const double share = D * DV / 16384.0, walkers = (double)nseg * H * (DV / 16) / 210;
   const double walk = 8 + (large ? 0.18 : 0.13) * ((double)ntok / nseg) * (walkers > 1 ? walkers : 1);
-  if ((large ? 31 : 25) + 0.0025 * ntok * H * (D * DV / 16384.0) > walk) return 0;
-  const long long slots = (long long)sm_count() * (DV == 128 ? 2 : 4);
-  const long long c = (((long long)ntok * H + slots - 1) / slots + rmma::BT - 1) / rmma::BT * rmma::BT;
-  return (int)(c < 2 * rmma::BT ? 2 * rmma::BT : c);
+  if ((large ? 32.5 : 25.5) + (large ? 0.0026 : 0.0025) * ntok * H * share > walk) return 0;
+  const long long slots = (long long)sm_count() * (DV == 128 ? 2 : 4), each = (ntok + (long long)nseg - 1) / nseg;
+  long long c = (((long long)ntok * H + slots - 1) / slots + rmma::BT - 1) / rmma::BT * rmma::BT;
+  if (c < 2 * rmma::BT) c = 2 * rmma::BT;
+  if (c < each && each <= 64) {
+    if (2LL * nseg * H > slots) c = (each + rmma::BT - 1) / rmma::BT * rmma::BT;
+    else if (!large && each <= 56) return 0;
+  }
+  return (int)c;
 }
+// Whether a segment may be longer than a chunk, so that states between chunks are needed (every segment has a token).
+static bool rm_splits(int nseg, int ntok, int C) { return ntok - nseg + 1 > C; }
+// 16 bytes: taken, and nothing is kept between chunks.
 static size_t rm_bytes(int nseg, int ntok, int H, int D, int DV) {
   const int C = ntok < 1 || H < 1 || D < 1 || DV < 1 ? 0 : rm_chunk_tokens(nseg, ntok, H, D, DV);
-  return C ? (size_t)(ntok / C + nseg) * H * ((size_t)D * DV + D) * sizeof(float) : 0;
+  return !C ? 0 : rm_splits(nseg, ntok, C) ? (size_t)(ntok / C + nseg) * H * ((size_t)D * DV + D) * sizeof(float) : 16;
 }
 template <int D, int DV>
 static int launch_rm_d(rmma::Args a, cudaStream_t st) {
@@ -1106,7 +1123,7 @@ static int launch_rm_d(rmma::Args a, cudaStream_t st) {
   QSPEC_CUDA(limit_e.raise(rmma::chunk_kernel<D, DV, false>, smem_e));
   QSPEC_CUDA(limit_o.raise(rmma::chunk_kernel<D, DV, true>, smem_o));
   a.P = a.E + (size_t)chunks * a.H * D * DV;
-  if (a.ntok - a.nseg + 1 > a.C) {                            // a segment may be longer than a chunk
+  if (rm_splits(a.nseg, a.ntok, a.C)) {
     launch_pdl(rmma::chunk_kernel<D, DV, false>, dim3(chunks, a.H), dim3(Sh::THREADS), smem_e, st, a);
     QSPEC_CHECK_LAUNCH(1);
     launch_pdl(rmma::carry_kernel<D, DV>, dim3(a.nseg, a.H, D * DV / 1024), dim3(256), 0, st, a);

@@ -100,3 +100,42 @@ def test_both_sides_of_the_rule(ops, H, D, DV, segments, mma):
     ops.seq_hgrn2(p, bias, lower, norm, state, torch.empty(T * H * (DV + 3 * D), device="cuda"), out, meta, H, D, DV, 1e-5, seg_starts=starts)
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()
     assert (state.double() - want_state).abs().max() <= 2e-5 * want_state.abs().max()
+
+
+def lengths(lens):
+    return [(k, 0 if k % 2 else 70, n) for k, n in enumerate(lens)]             # every other segment starts from a state
+
+
+@pytest.mark.parametrize("H,D,DV,lens", [
+    (32, 128, 128, [4] * 64), (16, 128, 128, [1] * 64), (16, 128, 128, [1] * 512), (32, 128, 128, [1] * 256), (64, 128, 128, [5] * 16 + [9]),
+    (32, 128, 128, [1] * 64 + [256]), (16, 128, 128, [17] * 64), (8, 64, 64, [5] * 400), (32, 64, 64, [8] * 256), (16, 64, 128, [16] * 128), (16, 128, 64, [100] * 24), (32, 128, 64, [150] * 5),
+    (16, 128, 128, [33] * 4), (8, 64, 64, [40] * 24)])
+def test_many_short_segments_keep_the_walk_and_no_workspace(ops, H, D, DV, lens):
+    from qspec_b200 import _lib
+    lib = _lib.load_seq()
+    assert lib.qspec_seq_hgrn2_chunk_bytes(len(lens), sum(lens), H, D, DV, _lib.DTYPE_BF16) == lib.qspec_seq_recurrence_chunk_bytes(len(lens), sum(lens), H, D, DV) == 0
+
+
+@pytest.mark.parametrize("H,D,DV,lens,nbytes", [
+    (16, 128, 128, [24, 1, 300, 2, 16, 60], None),                              # one long, others shorter than a block
+    (16, 128, 128, [1] * 32 + [1000], None),                                    # decoding sequences beside a prompt
+    (16, 128, 128, [33] * 12, None),                                            # segments a little longer than the smallest chunk stay whole
+    (200, 128, 128, [60], 16),                                                  # nothing is kept between chunks
+    (4, 128, 64, [220, 200], None),
+    (32, 64, 64, [1] * 16 + [512], None),
+])
+def test_segments_of_all_lengths(ops, H, D, DV, lens, nbytes):
+    from qspec_b200 import _lib
+    T = sum(lens)
+    need = _lib.load_seq().qspec_seq_hgrn2_chunk_bytes(len(lens), T, H, D, DV, _lib.DTYPE_BF16)
+    assert need == nbytes or nbytes is None and need > 16
+    segments = lengths(lens)
+    meta, starts = table(segments)
+    p, bias, lower, norm, state = inputs(T, H, D, DV, len(lens), 17)
+    bias = bias / 8 + 2                                                         # a memory of some ten tokens
+    want, want_state = want_of(p, bias, lower, norm, state, segments, H, D, DV)
+    out = torch.empty(T, H * DV, dtype=torch.bfloat16, device="cuda")
+    ops.seq_hgrn2(p, bias, lower, norm, state, torch.empty(T * H * (DV + 3 * D), device="cuda"), out, meta, H, D, DV, 1e-5, seg_starts=starts)
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()
+    for s in range(len(lens)):                                                  # float32 sums with such a memory: 1.2e-7 to 1.6e-7 of the state in every form
+        assert (state[s].double() - want_state[s]).norm() <= 6e-7 * want_state[s].norm()
