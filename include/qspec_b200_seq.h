@@ -257,14 +257,19 @@ int qspec_seq_lightning(const void* p, int ld, const float* decay, const float* 
                         void* stream);
 
 /* The two recurrences over long segments in chunks that run side by side (the walk through a segment's tokens is a chain): same arguments
- * and results (float32 throughout; another order of products of decays), and a workspace of qspec_seq_recurrence_chunk_bytes(..) bytes
+ * and results (float32 throughout, another order of products of decays; for bfloat16 rows of the gated recurrence see qspec_seq_hgrn2_chunk_bytes), and a
+ * workspace of qspec_seq_recurrence_chunk_bytes(..) bytes
  * (qspec_seq_lightning_chunk_bytes for the scalar decay) on a 16-byte boundary, which the call may leave anything in. 0 bytes: these sizes
  * are walked token by token (segments shorter than 256 to 336 tokens on average, key or value sizes other than 64 and 128, a scalar decay
  * with more segments and heads than the walk leaves room for), as they are without a workspace or without seg_starts. */
 size_t qspec_seq_recurrence_chunk_bytes(int nseg, int ntok, int H, int D, int DV);
 size_t qspec_seq_lightning_chunk_bytes(int nseg, int ntok, int H, int D, int DV);
-/* What qspec_seq_hgrn2_chunked takes of this element type: bfloat16 rows (16-byte boundaries, ld a multiple of 8) go to a form on the tensor cores,
- * which takes shorter segments too. With the smaller workspace of qspec_seq_recurrence_chunk_bytes they go where float32 rows go. */
+/* The workspace of qspec_seq_hgrn2_chunked for rows of this element type. Sizes and alignment choose the form: bfloat16 rows (p and workspace on 16-byte
+ * boundaries, ld a multiple of 8) go to one on the tensor cores by a rule of its own, which asks for 24 tokens a segment on average, other rows go by the
+ * rule above. Where qspec_seq_recurrence_chunk_bytes is not 0 its bytes are enough for both; with less than a form needs the next one is taken, the walk in
+ * the end. On the tensor cores the state is held and updated in float32 from exact products; queries and state meet as sums of two terms of 11 bits each
+ * (off by 2^-23 of an operand at most), all four products taken and summed in float32. Errors of the state against 64 bits are the other forms' (1.74e-7
+ * of its norm, the float32 form 1.75e-7), those of the outputs before they are rounded to bfloat16 the walk's (1.16e-7; the float32 form 1.10e-7). */
 size_t qspec_seq_hgrn2_chunk_bytes(int nseg, int ntok, int H, int D, int DV, int dtype);
 int qspec_seq_hgrn2_chunked(const void* p, int ld, const float* f_b, const float* lower, const float* norm_w, float* state,
                             float* scratch, void* out, const int* meta, const int* seg_starts, int nseg, int ntok, int H, int D,

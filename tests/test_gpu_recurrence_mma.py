@@ -139,3 +139,28 @@ def test_segments_of_all_lengths(ops, H, D, DV, lens, nbytes):
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()
     for s in range(len(lens)):                                                  # float32 sums with such a memory: 1.2e-7 to 1.6e-7 of the state in every form
         assert (state[s].double() - want_state[s]).norm() <= 6e-7 * want_state[s].norm()
+
+
+@pytest.mark.parametrize("H,D,DV,lens", [(16, 128, 128, [300]), (4, 64, 64, [257, 256]), (8, 128, 64, [600]), (32, 64, 128, [500, 300]), (16, 128, 128, [150] * 3), (200, 128, 128, [60])])
+def test_every_workspace_size(ops, H, D, DV, lens):
+    """The bytes of both queries, one less of each, and none: whichever form that leads to, the same results."""
+    from qspec_b200 import _lib
+    lib, T = _lib.load_seq(), sum(lens)
+    segments = lengths(lens)
+    meta, starts = table(segments)
+    p, bias, lower, norm, start = inputs(T, H, D, DV, len(lens), 23)
+    bias = bias / 8 + 2
+    want, want_state = want_of(p, bias, lower, norm, start, segments, H, D, DV)
+    old, new = lib.qspec_seq_recurrence_chunk_bytes(len(lens), T, H, D, DV), lib.qspec_seq_hgrn2_chunk_bytes(len(lens), T, H, D, DV, _lib.DTYPE_BF16)
+    assert new >= old and new > 0                                               # (the larger of both forms': rows may be unaligned)
+    scratch = torch.empty(T * H * (DV + 3 * D), device="cuda")
+    for nbytes in sorted({0, max(0, old - 1), old, new - 1, new}):
+        ws = torch.full((nbytes + 64,), 255, dtype=torch.uint8, device="cuda")
+        state, out = start.clone(), torch.full((T, H * DV), float("nan"), dtype=torch.bfloat16, device="cuda")
+        rc = lib.qspec_seq_hgrn2_chunked(p.data_ptr(), p.shape[1], bias.data_ptr(), lower.data_ptr(), norm.data_ptr(), state.data_ptr(), scratch.data_ptr(), out.data_ptr(),
+                                         meta.data_ptr(), starts.data_ptr(), len(lens), T, H, D, DV, 1e-5, _lib.DTYPE_BF16, ws.data_ptr() if nbytes else None, nbytes,
+                                         torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and bool((ws[nbytes:] == 255).all())
+        assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()
+        for s in range(len(lens)):
+            assert (state[s].double() - want_state[s]).norm() <= 6e-7 * want_state[s].norm()
