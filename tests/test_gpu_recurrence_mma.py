@@ -3,7 +3,7 @@ out, decays next to 0 and 1, values that are not finite, and the rule that takes
 import pytest
 import torch
 
-from test_gpu_recurrence_chunks import ops, table, walk  # noqa: F401
+from test_gpu_recurrence_chunks import CASES, ops, table, walk  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -85,6 +85,26 @@ def test_rows_that_are_not_aligned_take_the_other_form(ops):
     out = torch.empty(320, H * DV, dtype=torch.bfloat16, device="cuda")
     ops.seq_hgrn2(wide, bias, lower, norm, state, torch.empty(320 * H * (DV + 3 * D), device="cuda"), out, meta, H, D, DV, 1e-5, seg_starts=starts)
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()
+    assert (state.double() - want_state).abs().max() <= 2e-5 * want_state.abs().max()
+
+
+@pytest.mark.parametrize("H,D,DV,segments", CASES)
+def test_rows_of_the_other_form_that_are_not_aligned(ops, H, D, DV, segments):
+    meta, starts = table(segments)
+    T = meta.shape[1]
+    p, bias, lower, norm, state = inputs(T, H, D, DV, 3, 6)
+    bias = bias * 3 / 8                                                         # decays from nearly 0 to nearly 1
+    for slot, p0, _ in segments:
+        if p0 == 0:
+            state[slot] = float("nan")                                          # a slot's leftovers do not matter at position 0
+    wide = torch.zeros(T * (p.shape[1] + 3) + 1, dtype=torch.bfloat16, device="cuda")[1:].view(T, -1)       # 2-byte boundaries, rows of an odd number of elements
+    wide[:, :p.shape[1]] = p
+    want, want_state = want_of(p, bias, lower, norm, state, segments, H, D, DV)
+    out = torch.empty(T, H * DV, dtype=torch.bfloat16, device="cuda")
+    ops.seq_hgrn2(wide, bias, lower, norm, state, torch.empty(T * H * (DV + 3 * D), device="cuda"), out, meta, H, D, DV, 1e-5, seg_starts=starts)
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()
+    for slot, _, _ in segments:
+        assert (state[slot].double() - want_state[slot]).abs().max() <= 2e-5 * want_state[slot].abs().max()
 
 
 @pytest.mark.parametrize("H,D,DV,segments,mma", [
