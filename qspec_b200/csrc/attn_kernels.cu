@@ -661,7 +661,7 @@ seq_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict__ 
     for (int t0 = warp * 32; t0 < T; t0 += NW * 32) {
       const int t = t0 + lane;
       bool before, after;
-      if (!atile::attn_in_run(positions, seq_ids, T, t0, min_run, before, after) && t < T && __ldcg(seq_ids + t) == seq) {
+      if (!atile::attn_in_run<true>(positions, seq_ids, T, t0, min_run, before, after) && t < T && __ldcg(seq_ids + t) == seq) {
         const int i = atomicAdd(&s_ntok, 1);
         s_tok[i] = t;
         s_pos[i] = __ldcg(positions + t);

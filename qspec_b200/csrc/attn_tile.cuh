@@ -65,9 +65,12 @@ struct Args {
   uint32_t rep_inv;                            // set by launch(): r * rep_inv >> 16 = r / rep for r < 128
 };
 
-// Tokens t and t + 1 of the batch are of one run. (Read from L2: see attn_beside_tiles.)
+// Tokens t and t + 1 of the batch are of one run. L2: read past the L1, which only who runs beside the tiles needs (see attn_beside_tiles); the CTAs of
+// decode_attention, one per token and head, ask for the same few lines, and waited for each other at the L2 (64 tokens, 32 / 32 heads 20.0 us for 13.9).
+template <bool L2>
 __device__ __forceinline__ bool attn_link(const int* pos, const int* seq, int ntok, int t) {
-  return t >= 0 && t + 1 < ntok && __ldcg(seq + t) == __ldcg(seq + t + 1) && __ldcg(pos + t + 1) == __ldcg(pos + t) + 1;
+  auto at = [](const int* p) { return L2 ? __ldcg(p) : *p; };
+  return t >= 0 && t + 1 < ntok && at(seq + t) == at(seq + t + 1) && at(pos + t + 1) == at(pos + t) + 1;
 }
 // The kernel launched behind attn_tile_kernel for the other tokens starts with this instead of waiting: it looks for its tokens (positions and
 // sequences, or the table of segments, from L2) while the tiles run, and calls attn_tiles_done() before it reads anything else, writes, or leaves. The
@@ -77,10 +80,11 @@ __device__ __forceinline__ void attn_beside_tiles() { asm volatile("griddepcontr
 __device__ __forceinline__ void attn_tiles_done() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 // For the 32 tokens t0 .. t0 + 31 of a whole warp, token t0 + lane: is it in a run of at least min_run (<= 16) tokens? `before`, `after`: is
 // it linked to its neighbours?
+template <bool L2>
 __device__ __forceinline__ bool attn_in_run(const int* pos, const int* seq, int ntok, int t0, int min_run, bool& before, bool& after) {
   const int lane = threadIdx.x & 31;
-  const uint64_t links = (uint64_t)__ballot_sync(0xffffffffu, attn_link(pos, seq, ntok, t0 - 16 + lane)) |
-                         (uint64_t)__ballot_sync(0xffffffffu, attn_link(pos, seq, ntok, t0 + 16 + lane)) << 32;   // bit i: token t0 - 16 + i
+  const uint64_t links = (uint64_t)__ballot_sync(0xffffffffu, attn_link<L2>(pos, seq, ntok, t0 - 16 + lane)) |
+                         (uint64_t)__ballot_sync(0xffffffffu, attn_link<L2>(pos, seq, ntok, t0 + 16 + lane)) << 32;   // bit i: token t0 - 16 + i
   const uint64_t left = ~(links << (48 - lane)), right = ~(links >> (16 + lane));
   before = links >> (15 + lane) & 1;
   after = links >> (16 + lane) & 1;
@@ -89,7 +93,7 @@ __device__ __forceinline__ bool attn_in_run(const int* pos, const int* seq, int 
 // One token, asked by a whole warp.
 __device__ __forceinline__ bool attn_token_in_run(const int* pos, const int* seq, int ntok, int t, int min_run) {
   bool x, y;
-  return __shfl_sync(0xffffffffu, attn_in_run(pos, seq, ntok, t, min_run, x, y), 0);
+  return __shfl_sync(0xffffffffu, attn_in_run<false>(pos, seq, ntok, t, min_run, x, y), 0);
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -432,7 +436,7 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
       if (a.seg) { s0 = a.seg[t]; s1 = a.seg[a.ntok + t]; }
     }
     bool before, after;
-    bool in = attn_in_run(a.pos, a.seq, a.ntok, c0 + warp * 32, a.min_run, before, after) && tid < n2;
+    bool in = attn_in_run<false>(a.pos, a.seq, a.ntok, c0 + warp * 32, a.min_run, before, after) && tid < n2;
     if (a.seg && tid < n2) {
       in = s1 - s0 >= a.min_run;
       before = before && t > s0;
