@@ -419,12 +419,6 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
   const uint32_t base = (smem_addr(at_raw) + 1023u) & ~1023u;
   unsigned char* gbase = at_raw + (base - smem_addr(at_raw));
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
-  // Tensor memory only now: a kernel of another library some launches ahead (a product in front of the one that prepares the queries) may have let its
-  // dependents start before it held its own, and would wait for columns of a CTA that waits for it. Beside the search for runs it takes no time.
-  if (warp == WARP_MMA) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-  }
   // ---- the runs among this CTA's tokens
   bool start = false, end = false;
   if (tid < TOKENS_MAX) {
@@ -452,18 +446,18 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     const uint32_t bits = __ballot_sync(0xffffffffu, start);
     if (lane == 0) s_start[warp] = bits;
   }
-  fence_before();
   __syncthreads();
-  fence_after();
-  const uint32_t tmem = s_tmem;
   int nruns = 0, before = 0;
   for (int w = 0; w < TOKENS_MAX / 32; ++w) {
     if (w < warp) before += __popc(s_start[w]);
     nruns += __popc(s_start[w]);
   }
-  if (nruns == 0) {                                          // nothing for this form here
-    if (warp == WARP_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
-    return;
+  if (nruns == 0) return;                                    // nothing for this form here
+  // Tensor memory only now: a kernel of another library some launches ahead (a product in front of the one that prepares the queries) may have let its
+  // dependents start before it held its own, and would wait for columns of a CTA that waits for it. Beside the queries' way here it takes no time.
+  if (warp == WARP_MMA) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   // ---- queries: asked for here, stored while the first keys are on their way
   constexpr int QP = 128 * 16 / (WARP_K * 32), QW = QF32 ? 2 : 1;   // 16-byte pieces of a thread; loads of each
@@ -482,7 +476,10 @@ attn_tile_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constan
     if (start) s_rs[rank] = tid;
     if (end) s_re[rank] = tid;
   }
+  fence_before();
   __syncthreads();
+  fence_after();
+  const uint32_t tmem = s_tmem;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");   // tensor memory is held: a dependent that waits for this grid cannot take it first
 
   if (warp < WARP_K) {
