@@ -141,8 +141,8 @@ decode_attention_kernel(const __half* __restrict__ qkv, const __half* __restrict
 // Grid = T x Hkv CTAs of 128 threads, two CTAs per SM; the Hkv CTAs of a token form a thread-block cluster.
 // CTA (token, kv head):
 //   0. one round trip for the positions, then everything that only depends on them is put in flight at once:
-//      the key rows of the first 128 positions (one per thread, registers), bulk copies of the remaining key rows
-//      and of the value rows into shared memory (cp.async.bulk, one 256-byte copy per row), the rotary inputs;
+//      the key rows of the first 128 positions (one per thread, registers), copies of the remaining key rows and of
+//      the value rows into shared memory (cp.async, 16 bytes a lane, 16 lanes a row), the rotary inputs;
 //      rotates the token's G = Hq/Hkv query heads (-> shared memory, qkv is not written) and the key of EVERY
 //      token of this pass that belongs to the same sequence at a position <= its own (keys/values written to the
 //      cache by other CTAs of this launch are not visible yet, so they are recomputed: same arithmetic, same

@@ -1502,9 +1502,10 @@ static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, RowsArgs p,
 // SM: W4A4, 4 tokens 12.4 | 10.3 us, W4A16, 16 tokens 23.4 | 20.4. W4A8, 4 tokens, two CTAs of four | eight warps: 28672 x 4096 11.7 | 11.4, 12288 x 4096
 // 6.15 | 5.64, 6144 x 4096 3.84 | 3.58; longer tiles 8192 x 8192 7.16 | 7.25, 27648 x 5120 13.0 | 13.2.
 // A CTA alone on its SM has twelve warps where its slots are small and its tile has more than 16 items: a warp's way from its fragments to the sums is a
-// chain, and eight leave two a scheduler to hide it, with the same bytes under way (24 slots of 8 KB). Eight | twelve: 4 tokens, 4096 x 14336 W4A4
-// 7.0 | 6.6, W4A16 9.0 | 8.7; 4096 x 5120 3.3 | 3.1, 4.3 | 4.1; 16 items 2.8 | 2.9, 3.9 | 4.1, for two rounds of items either way. W4A16, 16 tokens, whose ring holds
-// one slot a warp then, 10.7 | 12.8; W4A8 6.6 | 6.9.
+// chain, and eight leave two a scheduler to hide it. The bytes under way are the same for W4A16 (8 x 3 or 12 x 2 slots of 8 KB) and fewer for W4A4 (8 x 5
+// or 12 x 3 of 5 KB, at 16 tokens 8 x 4 or 12 x 2 of 6 KB). Eight | twelve: 4 tokens, 4096 x 14336 W4A4 7.0 | 6.6, W4A16 9.0 | 8.7; 4096 x 5120 3.3 | 3.1,
+// 4.3 | 4.1; 16 items 2.8 | 2.9, 3.9 | 4.1, for two rounds of items either way. W4A16, 16 tokens, whose ring holds one slot a warp then, 10.7 | 12.8;
+// W4A8 6.6 | 6.9.
 template <int MODE, int NT>
 static int rows_launch(const CUtensorMap& mw, const CUtensorMap& ma, const RowsArgs& p, cudaStream_t st) {
   const int sms = sm_count() > 0 ? sm_count() : 148;
