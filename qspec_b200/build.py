@@ -131,8 +131,8 @@ def build_variant(suffix: str, defines, verbose: bool = False) -> str:
 
 
 def build_library(force: bool = False, verbose: bool = False, prof: bool = False, watchdog: bool = False) -> str:
-    """prof=True builds libqspec_b200_prof.so with the GEMM cycle counters compiled in (scripts/gpu_gemm_trace.py;
-    select it with QSPEC_LIB=<path>); watchdog=True builds libqspec_b200_wd.so whose pipeline waits trap instead of
+    """prof=True builds libqspec_b200_prof.so with the GEMM cycle counters compiled in
+    (select it with QSPEC_LIB=<path>); watchdog=True builds libqspec_b200_wd.so whose pipeline waits trap instead of
     hanging (for protocol changes). The product library carries neither."""
     os.makedirs(OUT_DIR, exist_ok=True)
     build_fast_if_possible(force=force)

@@ -160,7 +160,7 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 // PAIR (cta_group::2): ONE instruction, issued by the leader CTA, drives both SMs' tensor cores: M = 256 = the 128 weight
 // channels in EACH CTA's tensor memory (same columns), the token tile B split between the two CTAs' shared memory (each
 // holds N/2 rows at the same offset), D = 128 lanes x N columns in each CTA. Measured on B200
-// (scripts/umma_probe.cu): ~58 cycles per instruction for N <= 64 in BOTH forms, so the pair halves the tensor-pipe
+// with chains of these instructions alone: ~58 cycles per instruction for N <= 64 in BOTH forms, so the pair halves the tensor-pipe
 // issue time per weight byte.
 template <int MODE, bool PAIR>
 __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -1243,7 +1243,7 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   pl.np = mp < 128 ? mp : 128;
   pl.pair = pair_wanted(M, N) ? 1 : 0;
   // 256-token tiles (CTA pairs, W4A16 only): ONE pass over the weights for M in (128, 256] -- each weight unit is converted
-  // once and multiplied with tcgen05.mma N = 256 (128 cycles per instruction = the dense rate, scripts/umma_probe.cu) instead
+  // once and multiplied with tcgen05.mma N = 256 (128 cycles per instruction = the dense rate) instead
   // of twice with N = 128. The accumulator then takes 256 of the 512 tensor-memory columns, single-buffered.
   // Measured: -7 % where every pair owns whole tiles (gate_up 75.7 -> 70.3 us, the 70B gate_up
   // 250.5 -> 244.6 us); shapes with fewer pair tiles than SM pairs, whose tiles are shared between pairs, got SLOWER in
@@ -1265,7 +1265,7 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   const int sms = (sm_count() > 0 ? sm_count() : 148) / (pl.pair ? 2 : 1);   // schedulable units: SMs, or SM pairs
   // The unit, reduction and tile-width figures below were fitted before operand slots of eight instructions and the LONG form, and have not been since:
   // whether they still choose the best grids has not been measured again, and they are no times of the present kernel (rows_faster has those).
-  // Measured on B200 (scripts/umma_probe.cu): a tcgen05.mma of this kernel's shape issues every ~58 cycles (N <= 64) in both
+  // Measured on B200: a tcgen05.mma of this kernel's shape issues every ~58 cycles (N <= 64) in both
   // cta_group forms => per (pair-)unit 8 (int) / 16 (f16) instructions = 0.25 / 0.49 us at 1.9 GHz, plus the converters'
   // share; a pair-unit carries twice the bytes
   // ... and grows with the token tile (the converters widen np activation rows per unit, the MMAs get longer from N = 128):
@@ -1283,7 +1283,7 @@ static Plan make_plan(int mode, int M, int N, int K, bool deferred = false) {
   // usually straddles two tiles and ends with TWO shared-tile reductions back to back (~2.5 us each, measured), which
   // for the small decode GEMMs costs more than it saves: prefer a slightly smaller grid whose ranges are aligned to the
   // tiles (q units per CTA with q | KB: one shared tile per CTA; q a multiple of KB: whole tiles, no reduction).
-  // Cost model (us, measured on B200 with scripts/gpu_gemm_gsweep.py): a CTA needs tu per unit -- the tensor pipe's
+  // Cost model (us, measured on B200 by forcing grids with QSPEC_GEMM_G): a CTA needs tu per unit -- the tensor pipe's
   // 8 (W4A4) / 16 (W4A16) minimum-latency MMAs per unit, or its share of HBM when every SM streams --; a trailing
   // reduction of a shared tile through the workspace costs tp, through distributed shared memory (the CTAs of a
   // tile launched as a thread-block cluster, decode-sized M only) tc.

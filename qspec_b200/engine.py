@@ -147,8 +147,8 @@ class QSpecEngine:
     def _join_caller_stream(self) -> None:
         """self.stream is a non-blocking stream: work the caller queued on ITS stream (prefill, state edits) is ordered before
         the step only by an explicit wait. Without it the step can read seq_len / cur_tok before prefill has written them and
-        append draft K/V rows at the wrong cache positions (found by scripts/gpu_determinism.py: intermittently different
-        tokens when capture() followed prefill() without a synchronize)."""
+        append draft K/V rows at the wrong cache positions (seen as intermittently
+        different tokens when capture() followed prefill() without a synchronize)."""
         cur = torch.cuda.current_stream(self.model.device)
         if cur != self.stream:
             self.stream.wait_stream(cur)

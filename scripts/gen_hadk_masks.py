@@ -1,6 +1,6 @@
 """Emit qspec_b200/csrc/hadk_masks.inc and qspec_b200/_hadk.py from tests/golden/had108.npy / had40.npy (the reference's
 get_had108 / get_had40 matrices, third-party/QuaRot/quarot/functional/hadamard.py, exported by tests/golden/make_golden.py):
-the Qwen2.5-14B variant's rotations (SURVEY 8(f) rank 4). Bit k of word k >> 5 of mask[o] is set iff H[o][k] == -1."""
+the Qwen2.5-14B variant's rotations. Bit k of word k >> 5 of mask[o] is set iff H[o][k] == -1."""
 import os
 import numpy as np
 

@@ -385,7 +385,7 @@ def test_engine_is_deterministic_without_caller_synchronisation(cuda, monkeypatc
     """Size-independent property at BASELINE configs[2] width (64 sequences, k = 3, Llama-3-8B layer shapes, 2 layers): decoding
     the same prompts twice -- prefill, capture and steps queued back to back with NO synchronize in between, under the CUDA graph
     and eagerly -- emits the same tokens. (The engine's stream is non-blocking: before QSpecEngine._join_caller_stream the first
-    step could overtake prefill() and append draft K/V rows at stale cache positions; scripts/gpu_determinism.py.)"""
+    step could overtake prefill() and append draft K/V rows at stale cache positions.)"""
     from qspec_b200.engine import QSpecEngine
     from qspec_b200.model import QSpecLlamaConfig, QSpecLlamaModel
     B, k, steps = 64, 3, 6
