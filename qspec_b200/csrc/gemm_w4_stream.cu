@@ -298,6 +298,7 @@ struct Params {
   int dbufs;                  // accumulator buffers: 2 (the epilogue of tile i overlaps the main loop of tile i + 1), or 1 for 256-token tiles
   int out_bf16;
   int stage_at;          // LONG: offset of the epilogue's stage in shared memory
+  int keep_w;            // weights stay in L2 (see w_policy)
   int debug_exit;        // debug: 1 = exit after setup, 2 = no TMEM alloc + exit after setup, 3 = exit at entry
   int trace_cta;         // debug: second CTA whose marks are recorded
   int trigger;           // when to release the dependent grid: 0 after setup, 1 when the weight stream has been issued, 2 at the end
@@ -509,8 +510,9 @@ w4_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   // Weights are read once, or, by a CTA whose range is longer than a tile, once for every token tile: with three and more of these they stay in L2. W4A16, 1999
   // tokens, 10240 x 8192: 590 MB came from memory for 75, and the GPU runs at its power limit there: 318 -> 296 us; 509 tokens, 28672 x 4096: 117 -> 112.
   // Two token tiles gain nothing (256 tokens, 28672 x 4096: 63.4 | 63.8), nor do ranges within a tile, which other CTAs read at the same time
-  // (509 tokens, 4096 x 14336: 54.0 | 54.7).
-  const uint64_t w_policy = (LONG && p.tiles_m > 2) || (p.debug_exit & 16) ? POLICY_EVICT_NORMAL : POLICY_EVICT_FIRST;
+  // (509 tokens, 4096 x 14336: 54.0 | 54.7), nor operands that do not fit beside each other (streamed | kept: W4A16 8192 x 28672, 700 tokens 255 | 268, 1000
+  // tokens 341 | 375; 16384 x 16384, 1500 tokens 574 | 649; 57344 x 8192, 2000 tokens 1475 | 1549; 5120 x 27648, 1000 tokens 212 | 218).
+  const uint64_t w_policy = p.keep_w || (p.debug_exit & 16) ? POLICY_EVICT_NORMAL : POLICY_EVICT_FIRST;
   auto load_w = [&](int s) {
     if (elect_one()) {
       mbar_expect_tx(smem_u32(&w_full[s]), stage_tx);
@@ -1462,6 +1464,7 @@ static bool rows_wanted(int mode, int M, int N, int K) {
   if (want == 0 || M > most) return false;
   return want == 2 || known_size(mode, M, N, K).rows;
 }
+constexpr size_t L2_KEEPS = 112 << 20;   // of the L2's 126 MB, for a product's weights and activations (see w_policy)
 // Whether the tcgen05 form runs as LONG: wherever it can and a CTA's range is at least a tile long, so that whole tiles and ends of ranges are what a
 // launch waits for. us, without | with it:  W4A16 28672 x 4096: 64 tokens 27.5 | 25.8, 256: 69 | 59, 1000: 240 | 193   10240 x 8192, 256 tokens: 50 | 43
 //   W4A4 28672 x 4096: 65 tokens 24.3 | 21.6, 256: 48.7 | 36.3   W4A4 bytes 28672 x 4096: 64 tokens 20.0 | 17.1, 256: 47.1 | 34.7
@@ -1593,6 +1596,7 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   p.counters = (unsigned*)workspace;
   p.ws_part = (uint32_t*)((unsigned char*)workspace + COUNTER_BYTES);
   p.trigger = env_int("QSPEC_GEMM_TRIGGER", 2);
+  p.keep_w = 0;
   p.debug_exit = env_int("QSPEC_GEMM_DEBUG_EXIT", 0);
   p.trace_cta = env_int("QSPEC_GEMM_TRACE_CTA", pl.G - 1);
   p.trace = g_trace ? g_trace + (size_t)(g_trace_seq++ % 8u) * 4096 : nullptr;
@@ -1601,6 +1605,7 @@ static int run(int mode, const void* act, const void* sA, const int8_t* w, const
   if (out && !acc_out && !split_out && ((uintptr_t)out & 15) == 0 && N % 8 == 0 && p.debug_exit == 0 && long_wanted(pl)) {
     p.stages = pl.stages;
     p.stage_at = (int)(pl.smem - 1024);
+    p.keep_w = pl.tiles_m > 2 && (size_t)N * K / 2 + (size_t)M * K * (mode_is_int(mode) ? 1 : 2) <= L2_KEEPS;
     pl.smem += STAGE_BYTES;
     if (pl.pair) {
       switch (mode) {
