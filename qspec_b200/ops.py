@@ -1195,10 +1195,10 @@ def seq_hgrn2(p: torch.Tensor, f_b: torch.Tensor, lower: torch.Tensor, norm_w: t
     if out.shape != (ntok, H * DV) or state.shape[1:] != (H, D, DV) or scratch.numel() < ntok * H * (DV + 3 * D) or norm_w.numel() != DV \
             or f_b.numel() != H * D or lower.numel() != H * D:
         raise ValueError("seq_hgrn2: shapes do not match")
-    lib, nseg = _lib.load_seq(), 0 if seg_starts is None else seg_starts.numel()
-    ws = _chunk_workspace(lib.qspec_seq_hgrn2_chunk_bytes, nseg, ntok, H, D, DV, p.device, _sdt(p))
+    lib, nseg, dt = _lib.load_seq(), 0 if seg_starts is None else seg_starts.numel(), _sdt(p)
+    ws = _chunk_workspace(lib.qspec_seq_hgrn2_chunk_bytes, nseg, ntok, H, D, DV, p.device, dt)
     _seq(lib.qspec_seq_hgrn2_chunked(_ptr(p), p.shape[1], _ptr(f_b), _ptr(lower), _ptr(norm_w), _ptr(state), _ptr(scratch), _ptr(out),
-                                     _ptr(meta), _ptr(seg_starts), nseg, ntok, H, D, DV, float(eps), _sdt(p), _ptr(ws),
+                                     _ptr(meta), _ptr(seg_starts), nseg, ntok, H, D, DV, float(eps), dt, _ptr(ws),
                                      0 if ws is None else ws.numel(), _stream()), "seq_hgrn2")
 
 
